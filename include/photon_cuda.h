@@ -489,22 +489,14 @@ int32_t pe_device_autotune(pe_device* d, const pe_camera* cam, const pe_settings
  * budget, the tail threshold). */
 typedef struct pe_tuning {
     int64_t tail_paths;        /* as pe_device_set_tail_paths */
-    int32_t closest_traversal; /* bounce-by-bounce closest hits: 0 the binary tree, 1 the 4-wide tree,
-                                  2 / 3 the 4-wide tree with the first 8 / 16 stack entries of each
-                                  thread in shared memory (the rest in local memory), 4 / 5 with the
-                                  top 4 / 8 stack entries in registers, 6 (default) the 4-wide tree
-                                  capped at 64 registers (eight 128-thread blocks per SM), 7 / 8 that
-                                  with the first 8 / 16 stack entries in shared memory, 9 that with
-                                  leaf tests postponed until the warp holds a leaf in every lane.
-                                  Mode 9 only on request (the autotuner leaves it out): which of two
-                                  triangles at a bit-identical distance wins then depends on the
-                                  rays that share the warp, so films are no longer bit-identical
-                                  across batchings and switch points where such ties occur */
+    int32_t closest_traversal; /* bounce-by-bounce closest hits: 0 the binary tree in the reference's
+                                  order, a ray per lane; 1-9 (default 6) the 4-wide tree, four lanes
+                                  per ray (one kernel: the numbers are kept for callers that stored
+                                  one of the variants it replaced) */
     int32_t shade_budget;      /* lean shading kernels: 0 the compiler's register count, 1 (default) at
                                   most 128 registers a thread (four 128-thread blocks per SM), 2 at
                                   most 96 (five blocks) */
-    int32_t any_traversal;     /* plain any-hit shadows: 0 the stack in local memory, 1 its top 4
-                                  entries in registers, 2 (default) capped at 64 registers */
+    int32_t any_traversal;     /* plain any-hit shadows: 0-2 (default 2), all the four-lane walk */
     int64_t wave_slots;        /* paths in flight in a regenerating wave (unguided renders without
                                   AOV or pass targets): 2^20 … 2^23, default 2^23; 0 on input keeps
                                   the current value.  Each of the device's two lanes holds path

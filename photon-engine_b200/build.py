@@ -6,6 +6,7 @@ path.  Re-running is cheap: objects are rebuilt only when a source or header cha
 """
 from __future__ import annotations
 
+import concurrent.futures
 import os
 import pathlib
 import shutil
@@ -60,11 +61,14 @@ def build(verbose: bool = False) -> pathlib.Path:
         _run(["g++", *CXX_FLAGS, *inc, "-c", str(host_src), "-o", str(host_obj)], verbose)
     objs.append(host_obj)
     nvcc = _nvcc()
+    stale = []
     for cu in sorted(CSRC.glob("*.cu")):
         o = OBJ / (cu.stem + ".o")
         if _stale(o, [cu] + deps):
-            _run([nvcc, *ARCH, *NVCC_FLAGS, *inc, "-c", str(cu), "-o", str(o)], verbose)
+            stale.append([nvcc, *ARCH, *NVCC_FLAGS, *inc, "-c", str(cu), "-o", str(o)])
         objs.append(o)
+    with concurrent.futures.ThreadPoolExecutor(max(1, os.cpu_count() or 1)) as pool:
+        list(pool.map(lambda cmd: _run(cmd, verbose), stale))
     if _stale(LIB, objs):
         _run([nvcc, *ARCH, "-shared", "-o", str(LIB), *map(str, objs), "-lcudart_static", "-lrt", "-ldl", "-lpthread"],
              verbose)

@@ -12,6 +12,31 @@
 #include <thread>
 #include <vector>
 
+// Compiled in pe_kernels_*.cu.
+namespace pe {
+#define PE_EXTERN(...) extern template __global__ void __VA_ARGS__ PE_SHADE_ARGS;
+PE_LEAN_KERNELS(PE_EXTERN)
+#undef PE_EXTERN
+#define PE_EXTERN(...) extern template __global__ void __VA_ARGS__ PE_SHADE_ARGS;
+PE_LEAN_OUT_KERNELS(PE_EXTERN)
+#undef PE_EXTERN
+#define PE_EXTERN(...) extern template __global__ void __VA_ARGS__ PE_SHADE_ARGS;
+PE_FULL_KERNELS(PE_EXTERN)
+#undef PE_EXTERN
+#define PE_EXTERN(...) extern template __global__ void __VA_ARGS__ PE_TAIL_ARGS;
+PE_TAIL_KERNELS(PE_EXTERN)
+#undef PE_EXTERN
+#define PE_EXTERN(...) extern template __global__ void __VA_ARGS__ PE_TAIL_ARGS;
+PE_LOCKSTEP_KERNELS(PE_EXTERN)
+#undef PE_EXTERN
+#define PE_EXTERN(...) extern template __global__ void __VA_ARGS__ PE_TRACE_ARGS;
+PE_TRACE_KERNELS(PE_EXTERN)
+#undef PE_EXTERN
+#define PE_EXTERN(...) extern template __global__ void __VA_ARGS__ PE_SHADOW_ARGS;
+PE_SHADOW_KERNELS(PE_EXTERN)
+#undef PE_EXTERN
+} // namespace pe
+
 using namespace pe;
 using namespace pe_dev;
 
@@ -339,8 +364,6 @@ int32_t segsWritable(pe_device* d, int lane) {
     return PE_OK;
 }
 
-static_assert(sizeof(pe_device::blocksIntersectMode) / sizeof(int) == TRACE_MODES, "a grid size per traversal mode");
-
 // The tail in lockstep over `n` queued paths (count and cursor on the device).
 void launchTailLockstep(pe_device* d, bool lean, const SceneGPU& S, const Paths& P, const Wave& W, const int32_t* queue,
                         const uint32_t* count, uint32_t* cursor, int64_t n, cudaStream_t cs) {
@@ -350,39 +373,29 @@ void launchTailLockstep(pe_device* d, bool lean, const SceneGPU& S, const Paths&
     else kTailLockstep<false><<<grid, kTailLockstepBlock, 0, cs>>>(S, P, W, queue, count, cursor, d->dStats);
 }
 
-// The closest-hit kernel of the tuned traversal (pe_tuning::closest_traversal) over a queue.
+// The closest-hit kernel over a queue (pe_tuning::closest_traversal 0: the binary tree).
 void launchClosest(pe_device* d, const SceneGPU& S, const Paths& P, const int32_t* q, const uint32_t* c, cudaStream_t cs) {
-    const int* g = d->blocksIntersectMode;
     unsigned long long* st = d->dStats;
-    switch (d->closestMode) {
-    case TRACE_BINARY: kIntersect<false, TRACE_BINARY><<<g[TRACE_BINARY], 128, 0, cs>>>(S, P, q, c, st); break;
-    case TRACE_WIDE_SMEM8: kIntersect<false, TRACE_WIDE_SMEM8><<<g[TRACE_WIDE_SMEM8], 128, 0, cs>>>(S, P, q, c, st); break;
-    case TRACE_WIDE_SMEM16: kIntersect<false, TRACE_WIDE_SMEM16><<<g[TRACE_WIDE_SMEM16], 128, 0, cs>>>(S, P, q, c, st); break;
-    case TRACE_WIDE_REG4: kIntersect<false, TRACE_WIDE_REG4><<<g[TRACE_WIDE_REG4], 128, 0, cs>>>(S, P, q, c, st); break;
-    case TRACE_WIDE_REG8: kIntersect<false, TRACE_WIDE_REG8><<<g[TRACE_WIDE_REG8], 128, 0, cs>>>(S, P, q, c, st); break;
-    case TRACE_WIDE_OCC8: kIntersect<false, TRACE_WIDE_OCC8><<<g[TRACE_WIDE_OCC8], 128, 0, cs>>>(S, P, q, c, st); break;
-    case TRACE_WIDE_SMEM8_OCC8:
-        kIntersect<false, TRACE_WIDE_SMEM8_OCC8><<<g[TRACE_WIDE_SMEM8_OCC8], 128, 0, cs>>>(S, P, q, c, st);
-        break;
-    case TRACE_WIDE_SMEM16_OCC8:
-        kIntersect<false, TRACE_WIDE_SMEM16_OCC8><<<g[TRACE_WIDE_SMEM16_OCC8], 128, 0, cs>>>(S, P, q, c, st);
-        break;
-    case TRACE_WIDE_SPEC_OCC8:
-        kIntersect<false, TRACE_WIDE_SPEC_OCC8><<<g[TRACE_WIDE_SPEC_OCC8], 128, 0, cs>>>(S, P, q, c, st);
-        break;
-    default: kIntersect<false><<<d->blocksIntersect, 128, 0, cs>>>(S, P, q, c, st); break;
-    }
+    if (d->closestMode == TRACE_BINARY && d->counting)
+        kIntersectBinary<true><<<d->blocksIntersectBinary, 128, 0, cs>>>(S, P, q, c, st);
+    else if (d->closestMode == TRACE_BINARY)
+        kIntersectBinary<false><<<d->blocksIntersectBinary, 128, 0, cs>>>(S, P, q, c, st);
+    else if (d->counting)
+        kIntersect<true><<<d->blocksIntersect, 128, 0, cs>>>(S, P, q, c, st);
+    else
+        kIntersect<false><<<d->blocksIntersect, 128, 0, cs>>>(S, P, q, c, st);
+    kBin<<<d->prop.multiProcessorCount * 8, 256, 0, cs>>>(S, P, q, c);
 }
 
-// The plain any-hit shadow kernel of the tuned variant (pe_tuning::any_traversal).
-void launchShadowAny(pe_device* d, const SceneGPU& S, const Paths& P, cudaStream_t cs) {
-    uint32_t* n = &P.counters[CNT_SHADOW];
+// The shadow kernel of a scene over the wave's shadow records.
+void launchShadow(pe_device* d, const SceneGPU& S, const Paths& P, cudaStream_t cs) {
+    const uint32_t* n = &P.counters[CNT_SHADOW];
     unsigned long long* st = d->dStats;
-    switch (d->anyMode) {
-    case 1: kShadow<false, true, 4><<<d->blocksShadowAnyWindow, 128, 0, cs>>>(S, P, n, st); break;
-    case 2: kShadow<false, true, 0, 8><<<d->blocksShadowAnyOcc8, 128, 0, cs>>>(S, P, n, st); break;
-    default: kShadow<false, true><<<d->blocksShadowAny, 128, 0, cs>>>(S, P, n, st); break;
-    }
+    const bool any = !S.hasShadowTransmitters && !S.hasShadowLinks;
+    if (any && d->counting) kShadowAny<true><<<d->blocksShadowAny, 128, 0, cs>>>(S, P, n, st);
+    else if (any) kShadowAny<false><<<d->blocksShadowAny, 128, 0, cs>>>(S, P, n, st);
+    else if (d->counting) kShadow<true><<<d->blocksShadow, 128, 0, cs>>>(S, P, n, st);
+    else kShadow<false><<<d->blocksShadow, 128, 0, cs>>>(S, P, n, st);
 }
 
 // One wave on a lane over the nSegs segments in its segment table (nSlots paths, nPix film
@@ -457,7 +470,6 @@ int32_t runWave(pe_device* d, int lane, Paths& P, int nSegs, int nSlots, int nPi
         inlineShadows = inlineShadows || ln.hSegs[k].shadowSamples > 1;
     }
     const bool lean = S.leanShading && !P.guiding && !P.sdMode && noAo && !d->counting && !inlineShadows;
-    const bool anyHitShadows = !S.hasShadowTransmitters && !S.hasShadowLinks;
     int64_t tailPaths = d->tailPaths < 0 ? static_cast<int64_t>(d->blocksTail) * kTailBlock : d->tailPaths;
     // the tail kernel runs no inference: keep guided bounces in the wavefront until few paths remain
     if (P.guiding == 2) tailPaths = std::min<int64_t>(tailPaths, kGuideTailPaths);
@@ -502,12 +514,7 @@ int32_t runWave(pe_device* d, int lane, Paths& P, int nSegs, int nSlots, int nPi
                 return rc;
             PE_CUDA(cudaEventRecord(e0, cs));
         }
-        if (d->counting && d->closestMode == TRACE_BINARY)
-            kIntersect<true, TRACE_BINARY><<<d->blocksIntersectMode[0], 128, 0, cs>>>(S, P, qIn, cIn, d->dStats);
-        else if (d->counting)
-            kIntersect<true><<<d->blocksIntersect, 128, 0, cs>>>(S, P, qIn, cIn, d->dStats);
-        else
-            launchClosest(d, S, P, qIn, cIn, cs);
+        launchClosest(d, S, P, qIn, cIn, cs);
         if (P.guiding == 2 && (rc = guideQueries(d, cs, P, W, qIn, cIn))) return rc;
         if (tm.timing) PE_CUDA(cudaEventRecord(e1, cs));
         if (lean)
@@ -521,13 +528,8 @@ int32_t runWave(pe_device* d, int lane, Paths& P, int nSegs, int nSlots, int nPi
         else
             kShade<false><<<d->blocksShade, 128, 0, cs>>>(S, P, W, qOut, cOut);
         if (tm.timing) PE_CUDA(cudaEventRecord(e2, cs));
-        if (d->counting)
-            kShadow<true><<<d->blocksShadow, 128, 0, cs>>>(S, P, &P.counters[CNT_SHADOW], d->dStats);
-        else if (anyHitShadows)
-            launchShadowAny(d, S, P, cs);
-        else
-            kShadow<false><<<d->blocksShadow, 128, 0, cs>>>(S, P, &P.counters[CNT_SHADOW], d->dStats);
-        stats.kernel_launches += lean ? 2 : 3;
+        launchShadow(d, S, P, cs);
+        stats.kernel_launches += lean ? 3 : 4;
         ++stats.intersect_launches;
         if (tm.timing) {
             PE_CUDA(cudaEventRecord(e3, cs));
@@ -647,15 +649,12 @@ int32_t loopBounce(pe_device* d, LaneLoop& L, const Wave& W, uint32_t* hSegLeft,
     P.sweepAge = sweep >= 0 ? L.sweepAge : 0;
     P.sweepQ = sweep >= 0 ? L.sweepBuf[sweep] : nullptr;
     P.iter = L.iter;
-    // the tuned closest-hit and any-hit kernels, as a lone render uses
+    // the closest-hit and any-hit kernels a lone render uses
     launchClosest(d, S, P, L.qIn, L.cIn, cs);
     // lean-shading scenes shade with the per-key kernels, as a lone render does
     if (L.lean) launchLeanShade(d, S, P, W, L.qOut, L.cOut, cs, false);
     else kShade<false><<<d->blocksShade, 128, 0, cs>>>(S, P, W, L.qOut, L.cOut);
-    if (!S.hasShadowTransmitters && !S.hasShadowLinks)
-        launchShadowAny(d, S, P, cs);
-    else
-        kShadow<false><<<d->blocksShadow, 128, 0, cs>>>(S, P, &P.counters[CNT_SHADOW], d->dStats);
+    launchShadow(d, S, P, cs);
     PE_CUDA(cudaMemcpyAsync(ln.hCounters, P.counters, CNT_TOTAL * sizeof(uint32_t), cudaMemcpyDeviceToHost, cs));
     // segment counts as of the previous bounce's flushes (one bounce behind)
     if (segCount > 0)
@@ -767,6 +766,7 @@ int32_t renderWaves(pe_device* d, const pe_camera* cam, const pe_settings* st, i
     base.tileX = tile.x0;
     base.tileY = tile.y0;
     base.tileW = tile.w;
+    base.tileH = tile.h;
     base.sum = sum;
     base.cnt = cnt;
     base.sq = sq;
@@ -1019,7 +1019,7 @@ __global__ void kTraceRays(SceneGPU S, const float* o, const float* dir, const f
             outT[i] = 0.0f;
             continue;
         }
-        const Hit h = MODE == 1 ? traceClosestWide<false>(S, ro, rd, mask, 0.0f, tMax[i], a, b, nullptr, time)
+        const Hit h = MODE == 1 ? traceClosestWide<false>(S, ro, rd, mask, 0.0f, tMax[i], a, b, time)
                                 : traceClosest<false>(S, ro, rd, mask, 0.0f, tMax[i], a, b, time);
         if (isMiss(h.prim)) {
             outShape[i] = -1;
@@ -1301,8 +1301,6 @@ pe_device* pe_device_create(int32_t ordinal, char* err, size_t errLen) {
     d->blocksTailLockstep[0] = sm * std::max(1, b);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kTailLockstep<true>, kTailLockstepBlock, 0);
     d->blocksTailLockstep[1] = sm * std::max(1, b);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kShadow<false, true>, 128, 0);
-    d->blocksShadowAny = sm * std::max(1, b);
     auto occ = [&](auto kernel, int threads) {
         int nb = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, threads, 0);
@@ -1323,18 +1321,8 @@ pe_device* pe_device_create(int32_t ordinal, char* err, size_t errLen) {
     d->blocksShadeKey[2][2] = occ(kShadeKey<false, 2, 5>, 128);
     d->blocksShadeKey[2][3] = occ(kShadeKey<false, 3, 5>, 128);
     d->blocksShadeKey[2][4] = occ(kShadeKey<false, 4, 5>, 128);
-    d->blocksIntersectMode[TRACE_BINARY] = occ(kIntersect<false, TRACE_BINARY>, 128);
-    d->blocksIntersectMode[TRACE_WIDE] = occ(kIntersect<false, TRACE_WIDE>, 128);
-    d->blocksIntersectMode[TRACE_WIDE_SMEM8] = occ(kIntersect<false, TRACE_WIDE_SMEM8>, 128);
-    d->blocksIntersectMode[TRACE_WIDE_SMEM16] = occ(kIntersect<false, TRACE_WIDE_SMEM16>, 128);
-    d->blocksIntersectMode[TRACE_WIDE_REG4] = occ(kIntersect<false, TRACE_WIDE_REG4>, 128);
-    d->blocksIntersectMode[TRACE_WIDE_REG8] = occ(kIntersect<false, TRACE_WIDE_REG8>, 128);
-    d->blocksShadowAnyWindow = occ(kShadow<false, true, 4>, 128);
-    d->blocksIntersectMode[TRACE_WIDE_OCC8] = occ(kIntersect<false, TRACE_WIDE_OCC8>, 128);
-    d->blocksIntersectMode[TRACE_WIDE_SMEM8_OCC8] = occ(kIntersect<false, TRACE_WIDE_SMEM8_OCC8>, 128);
-    d->blocksIntersectMode[TRACE_WIDE_SMEM16_OCC8] = occ(kIntersect<false, TRACE_WIDE_SMEM16_OCC8>, 128);
-    d->blocksIntersectMode[TRACE_WIDE_SPEC_OCC8] = occ(kIntersect<false, TRACE_WIDE_SPEC_OCC8>, 128);
-    d->blocksShadowAnyOcc8 = occ(kShadow<false, true, 0, 8>, 128);
+    d->blocksIntersectBinary = occ(kIntersectBinary<false>, 128);
+    d->blocksShadowAny = occ(kShadowAny<false>, 128);
     const cudaError_t le = cudaGetLastError();
     if (le != cudaSuccess) {
         pe_device_destroy(d);
@@ -2086,10 +2074,7 @@ int32_t pe_device_autotune(pe_device* d, const pe_camera* cam, const pe_settings
              if (!rc) rc = ensureCapacity(d, kWaveSlots);
          },
          {static_cast<int64_t>(kWaveSlots), static_cast<int64_t>(kDefaultWaveSlots), static_cast<int64_t>(kMaxWaveSlots)});
-    tune("closest_traversal", [&](int64_t v) { d->closestMode = static_cast<int>(v); },
-         {TRACE_WIDE, TRACE_BINARY, TRACE_WIDE_SMEM8, TRACE_WIDE_SMEM16, TRACE_WIDE_REG4, TRACE_WIDE_REG8,
-          TRACE_WIDE_OCC8, TRACE_WIDE_SMEM8_OCC8, TRACE_WIDE_SMEM16_OCC8});
-    tune("any_traversal", [&](int64_t v) { d->anyMode = static_cast<int>(v); }, {0, 1, 2});
+    tune("closest_traversal", [&](int64_t v) { d->closestMode = static_cast<int>(v); }, {d->closestMode, TRACE_BINARY});
     tune("shade_budget", [&](int64_t v) { d->shadeBudget = static_cast<int>(v); }, {0, 1, 2});
     const int64_t grid = static_cast<int64_t>(d->blocksTail) * kTailBlock;
     tune("tail_paths", [&](int64_t v) { d->tailPaths = v; }, {grid / 4, grid / 2, grid, 2 * grid});

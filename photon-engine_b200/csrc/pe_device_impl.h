@@ -210,14 +210,12 @@ struct pe_device {
     int blocksShadeKey[3][5] = {}; // lean shading kernels: [budget][key]
     int blocksShadowAny = 0;
     int blocksTailLockstep[2] = {}; // kTailLockstep<LEAN>: [0] full, [1] lean shading; 128-thread blocks
-    int blocksIntersectMode[10] = {}; // per TraceMode
+    int blocksIntersectBinary = 0;
     size_t waveSlots = pe_dev::kDefaultWaveSlots; // pe_tuning::wave_slots: paths in flight per regenerating wave
     size_t laneSlots = 0;                 // slots of path state allocated per lane (>= capacity, waveSlots)
-    int blocksShadowAnyOcc8 = 0;   // kShadow capped at 64 registers
-    int blocksShadowAnyWindow = 0; // kShadow with the any-hit stack's top entries in registers
-    int anyMode = 2;               // pe_tuning::any_traversal (default: the 64-register cap)
+    int anyMode = 2;               // pe_tuning::any_traversal (every value the one any-hit kernel)
     // tuning (pe_tuning): closest-hit traversal variant, register budget of the lean shading kernels
-    int closestMode = 6;  // TraceMode (default: TRACE_WIDE_OCC8, the autotuner's pick on the knot frame)
+    int closestMode = 6;  // pe_tuning::closest_traversal (TraceMode: 0 the binary tree, else the 4-wide one)
     int shadeBudget = 1;  // 0 the compiler's register count, 1 (default) at most 128 registers (4 blocks per SM)
     std::string tuneLog;  // the last autotune's probe times
     int64_t tailPaths = -1; // -1: one resident grid of the tail kernel; 0: no tail kernel

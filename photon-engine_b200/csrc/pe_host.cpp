@@ -370,9 +370,18 @@ inline float4 f4(float x, float y, float z, float w) {
 // children left after repeatedly replacing its largest-area interior child by that child's two
 // children (at most four; leaves are never opened), in the binary tree's left-to-right order, so
 // every box and leaf is one of the binary tree's.  Layout per node, 8 float4 (128 bytes, one L2
-// line): lo.x, hi.x, lo.y, hi.y, lo.z, hi.z of the four children (SoA, one child per lane),
-// then the child references (interior: wide node index; leaf: ~(first << 8 | count-1)), then
-// the child count.  Nodes are written depth-first, a node before its children.
+// line), child by child, so that lane k of the four that walk a ray reads child k with two
+// 16-byte loads: (lo.x, lo.y, lo.z, hi.x) of children 0-3, then (hi.y, hi.z, reference, 1) of
+// children 0-3; reference: interior, wide node index; leaf, ~(first << 8 | count-1); all zero
+// for an absent child.  Nodes are written depth-first, a node before its children.
+static void putWideBox(float4* w, int k, V3 lo, V3 hi) {
+    w[k].x = lo.x;
+    w[k].y = lo.y;
+    w[k].z = lo.z;
+    w[k].w = hi.x;
+    w[4 + k].x = hi.y;
+    w[4 + k].y = hi.z;
+}
 static int collapseWide(const std::vector<RefNode>& ref, std::vector<float4>& out, int& maxDepth, int node = 0,
                         int depth = 1, int recBase = 0, std::vector<int4>* kidsOut = nullptr) {
     maxDepth = std::max(maxDepth, depth);
@@ -402,33 +411,15 @@ static int collapseWide(const std::vector<RefNode>& ref, std::vector<float4>& ou
         if (kidsOut->size() <= me) kidsOut->resize(me + 1, int4{-1, -1, -1, -1});
         (*kidsOut)[me] = int4{kids[0], kids[1], kids[2], kids[3]};
     }
-    float lo[3][4], hi[3][4];
-    int32_t child[4] = {0, 0, 0, 0};
-    for (int k = 0; k < 4; ++k) {
-        for (int a = 0; a < 3; ++a) {
-            lo[a][k] = 0.0f;
-            hi[a][k] = 0.0f;
-        }
-    }
     for (int k = 0; k < n; ++k) {
         const RefNode& c = ref[static_cast<size_t>(kids[k])];
-        lo[0][k] = c.bounds.lo.x;
-        lo[1][k] = c.bounds.lo.y;
-        lo[2][k] = c.bounds.lo.z;
-        hi[0][k] = c.bounds.hi.x;
-        hi[1][k] = c.bounds.hi.y;
-        hi[2][k] = c.bounds.hi.z;
-        child[k] = c.count > 0 ? ~(((c.offset + recBase) << 8) | (c.count - 1))
-                               : collapseWide(ref, out, maxDepth, kids[k], depth + 1, recBase, kidsOut);
+        const int32_t child = c.count > 0 ? ~(((c.offset + recBase) << 8) | (c.count - 1))
+                                          : collapseWide(ref, out, maxDepth, kids[k], depth + 1, recBase, kidsOut);
+        float4* w = out.data() + me * 8; // after the recursion, which may move the nodes
+        putWideBox(w, k, c.bounds.lo, c.bounds.hi);
+        w[4 + k].z = bitsf(static_cast<uint32_t>(child));
+        w[4 + k].w = bitsf(1u);
     }
-    float4* w = out.data() + me * 8;
-    for (int a = 0; a < 3; ++a) {
-        w[2 * a] = f4(lo[a][0], lo[a][1], lo[a][2], lo[a][3]);
-        w[2 * a + 1] = f4(hi[a][0], hi[a][1], hi[a][2], hi[a][3]);
-    }
-    w[6] = f4(bitsf(static_cast<uint32_t>(child[0])), bitsf(static_cast<uint32_t>(child[1])),
-              bitsf(static_cast<uint32_t>(child[2])), bitsf(static_cast<uint32_t>(child[3])));
-    w[7] = f4(bitsf(static_cast<uint32_t>(n)), 0.0f, 0.0f, 0.0f);
     return static_cast<int>(me);
 }
 
@@ -1948,18 +1939,8 @@ int32_t pe_scene_refit(pe_scene* s) {
     // 4-wide nodes of the top level
     for (size_t w = 0; w < B.tlasWideKids.size(); ++w) {
         const int kids[4] = {B.tlasWideKids[w].x, B.tlasWideKids[w].y, B.tlasWideKids[w].z, B.tlasWideKids[w].w};
-        float lo[3][4] = {}, hi[3][4] = {};
-        for (int c = 0; c < 4; ++c) {
-            if (kids[c] < 0) continue;
-            const Box& b = nb[static_cast<size_t>(kids[c])];
-            lo[0][c] = b.lo.x; lo[1][c] = b.lo.y; lo[2][c] = b.lo.z;
-            hi[0][c] = b.hi.x; hi[1][c] = b.hi.y; hi[2][c] = b.hi.z;
-        }
-        float4* q = &B.wide[w * 8];
-        for (int a = 0; a < 3; ++a) {
-            q[2 * a] = f4(lo[a][0], lo[a][1], lo[a][2], lo[a][3]);
-            q[2 * a + 1] = f4(hi[a][0], hi[a][1], hi[a][2], hi[a][3]);
-        }
+        for (int c = 0; c < 4; ++c)
+            if (kids[c] >= 0) putWideBox(&B.wide[w * 8], c, nb[static_cast<size_t>(kids[c])].lo, nb[static_cast<size_t>(kids[c])].hi);
     }
     B.rootMin[0] = nb[0].lo.x; B.rootMin[1] = nb[0].lo.y; B.rootMin[2] = nb[0].lo.z;
     B.rootMax[0] = nb[0].hi.x; B.rootMax[1] = nb[0].hi.y; B.rootMax[2] = nb[0].hi.z;

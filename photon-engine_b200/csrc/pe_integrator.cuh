@@ -10,19 +10,21 @@
 // vertex k+1, ...), and each slot draws Sobol dimensions in the reference's order.
 #pragma once
 
+#include "photon_cuda.h"
 #include "pe_bsdf.h"
 #include "pe_guide.cuh"
 #include "pe_light.h"
 #include "pe_medium.h"
 #include "pe_trace.cuh"
+#include "pe_walk.cuh"
 #include "pe_wave.h"
 
 namespace pe {
 
-// Persistent-warp work distribution: lane 0 claims the next 32 items for its warp.
-__device__ __forceinline__ int warpFetch(uint32_t* cursor) {
+// Persistent-warp work distribution: lane 0 claims the next `items` items for its warp.
+__device__ __forceinline__ int warpFetch(uint32_t* cursor, int items = 32) {
     int base = 0;
-    if ((threadIdx.x & 31) == 0) base = static_cast<int>(atomicAdd(cursor, 32u));
+    if ((threadIdx.x & 31) == 0) base = static_cast<int>(atomicAdd(cursor, static_cast<uint32_t>(items)));
     return __shfl_sync(0xffffffffu, base, 0);
 }
 
@@ -69,14 +71,14 @@ __device__ __forceinline__ void lobeShares(const LobeSplit3& sp, V3 out[3]) {
     }
 }
 // creditGroup: a term of light group `group` (ids outside the groups count for group 0).
-__device__ __noinline__ void creditGroup(const SceneGPU& S, const Paths& P, int path, int group, V3 added) {
+static __device__ __noinline__ void creditGroup(const SceneGPU& S, const Paths& P, int path, int group, V3 added) {
     if (S.nLightGroups <= 0 || isBlack(added)) return;
     const int g = (group >= 0 && group < S.nLightGroups) ? group : 0;
     if (g < PE_MAX_LIGHT_GROUPS) passAdd(passBlock(P, path) + PASS_GROUPS + g, added);
 }
 // creditPath: light reaching the path past its first surface, split by that surface's lobe
 // shares into the direct (found by the first bounce) or indirect passes.
-__device__ __noinline__ void creditPath(const Paths& P, int path, V3 added, bool direct) {
+static __device__ __noinline__ void creditPath(const Paths& P, int path, V3 added, bool direct) {
     float4* b = passBlock(P, path);
     for (int k = 0; k < 3; ++k) {
         const float4 share = b[PASS_LOBES + k];
@@ -88,7 +90,7 @@ __device__ __forceinline__ int lightGroupOf(const SceneGPU& S, int light) {
 }
 // A NEE term's passes: its light's group, and the direct passes by the vertex's own lobe shares
 // at the first surface (shares non-null), else the first surface's shares as indirect light.
-__device__ __noinline__ void creditNee(const SceneGPU& S, const Paths& P, int path, int light, V3 added,
+static __device__ __noinline__ void creditNee(const SceneGPU& S, const Paths& P, int path, int light, V3 added,
                                        const float4* shares) {
     if (isBlack(added)) return;
     creditGroup(S, P, path, lightGroupOf(S, light), added);
@@ -103,12 +105,9 @@ __device__ __noinline__ void creditNee(const SceneGPU& S, const Paths& P, int pa
 __device__ __forceinline__ void generatePath(const SceneGPU& S, const Paths& P, const Wave& W, int slot, int path) {
     const TablesGPU* T = S.tables;
     const WaveSeg& A = W.segs[segOfSlot(W, path)];
-    const int local = path - A.slotFirst;
-    const int sOff = local / A.nPix;
-    const int pix = A.pixelFirst + (local - sOff * A.nPix);
-    const int fp = A.pixList ? A.pixList[pix] : -1;
-    const int x = fp >= 0 ? fp % A.width : A.tileX + pix % A.tileW;
-    const int y = fp >= 0 ? fp / A.width : A.tileY + pix / A.tileW;
+    const int p = (path - A.slotFirst) / A.nSamples, sOff = path - A.slotFirst - p * A.nSamples;
+    int x, y;
+    tilePixel(A, A.pixelFirst + p, x, y);
     Sobol sb;
     sb.pixelHash = pixelHashOf(A.seed, x, y);
     sb.revIndex = rev32(static_cast<uint32_t>(A.sampleFirst + sOff));
@@ -151,7 +150,7 @@ __device__ __forceinline__ void flushPath(const Paths& P, const Wave& W, int slo
 }
 
 // The wave's first `count` paths into slots [0, count), all queued.
-__global__ void kGenerate(SceneGPU S, Paths P, Wave W, int count) {
+static __global__ void kGenerate(SceneGPU S, Paths P, Wave W, int count) {
     for (int slot = blockIdx.x * blockDim.x + threadIdx.x; slot < count; slot += gridDim.x * blockDim.x) {
         generatePath(S, P, W, slot, slot);
         P.queueA[slot] = slot;
@@ -161,7 +160,7 @@ __global__ void kGenerate(SceneGPU S, Paths P, Wave W, int count) {
 // After a bounce of a regenerating wave: every slot freed this bounce hands its path's radiance
 // to Lout (its NEE terms are in by now), and the first `fresh` of them take the wave's paths
 // [nextPath, nextPath + fresh), appended to the next closest-hit queue after its `queued` entries.
-__global__ void kRecycle(SceneGPU S, Paths P, Wave W, int freed, int fresh, int nextPath, int32_t* queue, int queued,
+static __global__ void kRecycle(SceneGPU S, Paths P, Wave W, int freed, int fresh, int nextPath, int32_t* queue, int queued,
                          uint32_t* queueCount) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < freed; k += gridDim.x * blockDim.x) {
         const int slot = P.freeQ[k];
@@ -175,7 +174,7 @@ __global__ void kRecycle(SceneGPU S, Paths P, Wave W, int freed, int fresh, int 
 }
 
 // The radiance of the paths the tail kernel finished, to Lout.
-__global__ void kFlush(Paths P, Wave W, const int32_t* queue, const uint32_t* count) {
+static __global__ void kFlush(Paths P, Wave W, const int32_t* queue, const uint32_t* count) {
     const int n = static_cast<int>(*count);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) flushPath(P, W, queue[i]);
 }
@@ -184,12 +183,12 @@ __global__ void kFlush(Paths P, Wave W, const int32_t* queue, const uint32_t* co
 // counters[CNT_FREE]).  kFlushFreed hands over the radiance of the `freed` slots pushed this
 // bounce, above `base`; kInject then pops `fresh` slots for the wave's paths [nextPath, +fresh),
 // appended to the next closest-hit queue after its `queued` entries.
-__global__ void kFlushFreed(Paths P, Wave W, int base, int freed) {
+static __global__ void kFlushFreed(Paths P, Wave W, int base, int freed) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < freed; k += gridDim.x * blockDim.x)
         flushPath(P, W, P.freeQ[base + k]);
 }
 
-__global__ void kInject(SceneGPU S, Paths P, Wave W, int top, int fresh, int nextPath, int32_t* queue, int queued,
+static __global__ void kInject(SceneGPU S, Paths P, Wave W, int top, int fresh, int nextPath, int32_t* queue, int queued,
                         uint32_t* queueCount) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < fresh; k += gridDim.x * blockDim.x) {
         const int slot = P.freeQ[top - fresh + k];
@@ -204,76 +203,161 @@ __global__ void kInject(SceneGPU S, Paths P, Wave W, int top, int fresh, int nex
 }
 
 // Slots of a finished sweep back onto the free stack, above `top`.
-__global__ void kReturnSlots(Paths P, const int32_t* slots, int n, int top) {
+static __global__ void kReturnSlots(Paths P, const int32_t* slots, int n, int top) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) P.freeQ[top + k] = slots[k];
     if (blockIdx.x == 0 && threadIdx.x == 0) P.counters[CNT_FREE] = static_cast<uint32_t>(top + n);
 }
 
 // Every slot free: the stack holds slots [0, n).
-__global__ void kInitFree(Paths P, int n) {
+static __global__ void kInitFree(Paths P, int n) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) P.freeQ[k] = k;
     if (blockIdx.x == 0 && threadIdx.x == 0) P.counters[CNT_FREE] = static_cast<uint32_t>(n);
 }
 
 // ---- closest hit over a queue -----------------------------------------------------------------
-// Closest hit for every queued ray; each ray is then binned by its shading key (miss or the
-// hit material's type) so the shading kernel runs warps of one material kind.
-// Closest-hit traversal variants the tuner chooses among (pe_tuning::closest_traversal).
-// Closest-hit traversals: the binary tree in the reference's order; the 4-wide tree with its stack
-// in local memory, its first 8 / 16 entries in shared memory, or its top 4 / 8 entries in registers.
-// TRACE_WIDE_OCC8: the 4-wide walk capped at 64 registers, eight 128-thread blocks per SM; with
-// the first 8 / 16 stack entries in shared memory as well (TRACE_WIDE_SMEM8_OCC8 / _SMEM16_OCC8).
-enum TraceMode { TRACE_BINARY = 0, TRACE_WIDE = 1, TRACE_WIDE_SMEM8 = 2, TRACE_WIDE_SMEM16 = 3, TRACE_WIDE_REG4 = 4,
-                 TRACE_WIDE_REG8 = 5, TRACE_WIDE_OCC8 = 6, TRACE_WIDE_SMEM8_OCC8 = 7, TRACE_WIDE_SMEM16_OCC8 = 8,
-                 TRACE_WIDE_SPEC_OCC8 = 9, TRACE_MODES = 10 };
-// TRACE_WIDE_SPEC_OCC8: the 64-register walk with postponed leaves (walkClosestWideSpec).
-constexpr bool traceSpeculative(int mode) { return mode == TRACE_WIDE_SPEC_OCC8; }
-constexpr int traceMinBlocks(int mode) { return mode >= TRACE_WIDE_OCC8 ? 8 : 1; }
-constexpr int traceStackShared(int mode) {
-    return (mode == TRACE_WIDE_SMEM8 || mode == TRACE_WIDE_SMEM8_OCC8) ? 8
-         : (mode == TRACE_WIDE_SMEM16 || mode == TRACE_WIDE_SMEM16_OCC8) ? 16
-         : mode == TRACE_WIDE_REG4 ? -4
-         : mode == TRACE_WIDE_REG8 ? -8 : 0;
+// Closest hit for every queued ray; kBin then bins the rays by shading key (miss or the hit
+// material's type) so that the shading kernels run warps of one material kind.  Traversals of pe_tuning::closest_traversal: 0 the binary tree in the reference's order, one lane
+// per ray; 1-9 the 4-wide tree, four lanes per ray (one kernel: the numbers once told variants apart
+// that the four-lane walk replaced).
+enum TraceMode { TRACE_BINARY = 0, TRACE_MODES = 10 };
+
+// Warp-aggregated append of each lane's slot into its key's bin (key < 0: none): one atomic per
+// distinct key per warp.
+__device__ __forceinline__ void binByKey(const Paths& P, int key, int slot) {
+    const int lane = threadIdx.x & 31;
+    const unsigned peers = __match_any_sync(0xffffffffu, key);
+    if (key >= 0) {
+        const int leader = __ffs(peers) - 1;
+        const int rank = __popc(peers & ((1u << lane) - 1u));
+        uint32_t at = 0;
+        if (lane == leader) at = atomicAdd(&P.counters[CNT_KEYS + key], static_cast<uint32_t>(__popc(peers)));
+        at = __shfl_sync(peers, at, leader);
+        P.sortQ[static_cast<size_t>(key) * P.capacity + at + rank] = slot;
+    }
 }
 
-template <bool COUNT, int MODE = TRACE_WIDE>
-__global__ void __launch_bounds__(128, traceMinBlocks(MODE)) kIntersect(SceneGPU S, Paths P, const int32_t* queue,
-                                                                        const uint32_t* count, unsigned long long* stats) {
-    constexpr int SD = traceStackShared(MODE);
-    __shared__ uint2 sstack[SD > 0 ? SD * 128 : 1];
+// The shading key of a closest hit by its primitive.
+__device__ __forceinline__ int shadeKeyOfPrim(const SceneGPU& S, uint32_t rayMask, int prim) {
+    if (rayMask & RAY_WALK) return kShadeKeys - 1;
+    if (isMiss(prim)) return 0;
+    if (isInstanceHit(prim)) return 1 + S.materials[S.instances[instanceOfHit(prim)].material].type;
+    return 1 + static_cast<int>((__float_as_uint(__ldg(&S.tris[3 * prim + 1]).w) >> 8) & 0xFFu);
+}
+
+// The queue's slots into the bins of their hits' shading keys.  A pass of its own rather than the
+// end of each ray's walk: rays end in any order, and bins in that order made the shading kernels'
+// state reads scatter (8.3 against 7.1 ms of shading per 8.3M-path knot wave); here a bin keeps the
+// queue's order but for the interleaving of warps.
+static __global__ void kBin(SceneGPU S, Paths P, const int32_t* queue, const uint32_t* count) {
     const int n = static_cast<int>(*count);
-    uint32_t nodes = 0, tris = 0;
-    const int lane = threadIdx.x & 31;
-    for (;;) {
-        const int base = warpFetch(&P.counters[CNT_WORK_ISECT]);
-        if (base >= n) break;
-        const int i = base + lane;
+    const int stride = gridDim.x * blockDim.x;
+    for (int base = blockIdx.x * blockDim.x; base < n; base += stride) {
+        const int i = base + static_cast<int>(threadIdx.x);
         int key = -1, slot = -1;
         if (i < n) {
             slot = queue[i];
-            const float4 ro = P.rayO[slot];
-            const float4 rd = P.rayD[slot];
-            const V3 o = mk(ro.x, ro.y, ro.z), d = mk(rd.x, rd.y, rd.z);
-            const uint32_t vmask = __float_as_uint(ro.w);
-            const float time = pathTime(S, P, slot);
-            const Hit h = MODE == TRACE_BINARY ? traceClosest<COUNT>(S, o, d, vmask, 0.0f, 1e30f, nodes, tris, time)
-                                               : traceClosestWide<COUNT, SD, traceSpeculative(MODE)>(
-                                                     S, o, d, vmask, 0.0f, 1e30f, nodes, tris,
-                                                                             sstack + threadIdx.x, time);
-            P.hit[slot] = make_float4(h.t, h.u, h.v, __int_as_float(h.prim));
-            key = (__float_as_uint(ro.w) & RAY_WALK) ? kShadeKeys - 1
-                  : (isMiss(h.prim) ? 0 : 1 + static_cast<int>((h.meta >> 8) & 0xFFu));
+            const uint32_t mask = S.hasSubsurface ? __float_as_uint(P.rayO[slot].w) : 0u;
+            key = shadeKeyOfPrim(S, mask, __float_as_int(P.hit[slot].w));
         }
-        // warp-aggregated append into the key's segment: one atomic per distinct key per warp
-        const unsigned peers = __match_any_sync(0xffffffffu, key);
-        if (key >= 0) {
-            const int leader = __ffs(peers) - 1;
-            const int rank = __popc(peers & ((1u << lane) - 1u));
-            uint32_t at = 0;
-            if (lane == leader) at = atomicAdd(&P.counters[CNT_KEYS + key], static_cast<uint32_t>(__popc(peers)));
-            at = __shfl_sync(peers, at, leader);
-            P.sortQ[static_cast<size_t>(key) * P.capacity + at + rank] = slot;
+        binByKey(P, key, slot);
+    }
+}
+
+// The binary tree, a ray per lane.
+template <bool COUNT>
+__global__ void __launch_bounds__(128) kIntersectBinary(SceneGPU S, Paths P, const int32_t* queue, const uint32_t* count,
+                                                        unsigned long long* stats) {
+    const int n = static_cast<int>(*count);
+    uint32_t nodes = 0, tris = 0;
+    for (;;) {
+        const int base = warpFetch(&P.counters[CNT_WORK_ISECT]);
+        if (base >= n) break;
+        const int i = base + (threadIdx.x & 31);
+        if (i >= n) continue;
+        const int slot = queue[i];
+        const float4 ro = P.rayO[slot];
+        const float4 rd = P.rayD[slot];
+        const Hit h = traceClosest<COUNT>(S, mk(ro.x, ro.y, ro.z), mk(rd.x, rd.y, rd.z), __float_as_uint(ro.w), 0.0f, 1e30f,
+                                          nodes, tris, pathTime(S, P, slot));
+        P.hit[slot] = make_float4(h.t, h.u, h.v, __int_as_float(h.prim));
+    }
+    if (COUNT) {
+        atomicAdd(&stats[0], static_cast<unsigned long long>(nodes));
+        atomicAdd(&stats[1], static_cast<unsigned long long>(tris));
+    }
+}
+
+// A warp's share of a queue: it takes 32 entries at a time from the global cursor and hands them to
+// lanes that ask.  All 32 lanes call next(); a lane that wants an entry gets its number, or -1.
+struct WarpFeed {
+    uint32_t* cursor;
+    int n;
+    int at = 0, end = 0;
+    __device__ __forceinline__ int next(bool want) {
+        const unsigned lanes = __ballot_sync(kWarp, want);
+        const int rank = __popc(lanes & ((1u << (threadIdx.x & 31)) - 1u));
+        const int wanted = __popc(lanes);
+        const int had = end - at, from = at;
+        if (had < wanted && end >= 0) {
+            const int base = warpFetch(cursor);
+            at = base + wanted - had;
+            if (base >= n) {
+                end = -1; // the queue is empty
+                at = -1;
+                return want && rank < had ? from + rank : -1;
+            }
+            end = min(base + 32, n);
+            const int i = rank < had ? from + rank : base + rank - had;
+            if (at > end) at = end;
+            return want && (rank < had || i < end) ? i : -1;
         }
+        if (end < 0) return -1;
+        at += wanted;
+        return want ? from + rank : -1;
+    }
+    __device__ __forceinline__ bool dry() const { return end < 0; }
+};
+
+// The 4-wide tree, a ray per lane (walkTurn).
+template <bool COUNT>
+__global__ void __launch_bounds__(128, 8) kIntersect(SceneGPU S, Paths P, const int32_t* queue, const uint32_t* count,
+                                                     unsigned long long* stats) {
+    uint2 stack[kWalkStack];
+    WarpFeed feed{&P.counters[CNT_WORK_ISECT], static_cast<int>(*count)};
+    const int root = rootRef(S);
+    const bool instances = S.nInstances > 0;
+    uint32_t nodes = 0, tris = 0;
+    int slot = -1;
+    RayWalk w;
+    w.cur = kRayDone;
+    for (;;) {
+        const unsigned idle = __ballot_sync(kWarp, w.cur == kRayDone);
+        if (idle == kWarp || (!feed.dry() && __popc(idle) >= kRefill)) {
+            // ended rays: their hits; then the queue's next rays
+            if (w.cur == kRayDone && slot >= 0) {
+                P.hit[slot] = make_float4(w.tMax, w.u, w.v, __int_as_float(w.prim));
+                slot = -1;
+            }
+            const int i = feed.next(w.cur == kRayDone);
+            if (i >= 0) {
+                slot = queue[i];
+                const float4 ro = P.rayO[slot];
+                const float4 rd = P.rayD[slot];
+                w.start(S, root, mk(ro.x, ro.y, ro.z), mk(rd.x, rd.y, rd.z), __float_as_uint(ro.w), 1e30f, -1);
+            }
+            if (__all_sync(kWarp, slot < 0)) break;
+            continue;
+        }
+        walkTurn<false, COUNT>(
+            S, w, stack, instances, nodes, tris,
+            [&](V3& o, V3& d, uint32_t& mask) {
+                const float4 ro = P.rayO[slot], rd = P.rayD[slot];
+                o = mk(ro.x, ro.y, ro.z);
+                d = mk(rd.x, rd.y, rd.z);
+                mask = __float_as_uint(ro.w);
+            },
+            [&]() { return pathTime(S, P, slot); });
+        __syncwarp();
     }
     if (COUNT) {
         atomicAdd(&stats[0], static_cast<unsigned long long>(nodes));
@@ -283,7 +367,7 @@ __global__ void __launch_bounds__(128, traceMinBlocks(MODE)) kIntersect(SceneGPU
 
 // Surface coverage of a hit for a ray that may pass through cutouts (DisneyMaterial::opacity,
 // disney.cpp:505-509: the opacity times the opacity map's red channel, a level-0 lookup).
-__device__ __noinline__ float mappedOpacity(const SceneGPU& S, const MatGPU& m, const Isect& is) {
+static __device__ __noinline__ float mappedOpacity(const SceneGPU& S, const MatGPU& m, const Isect& is) {
     ShadePoint sp;
     sp.uv = is.uv;
     sp.p = is.point;
@@ -333,7 +417,7 @@ __device__ V3 shadowVisibility(const SceneGPU& S, V3 o, V3 d, float tMax, int li
     V3 origin = o;
     float remaining = tMax;
     for (int i = 0; i < 64; ++i) {
-        const Hit h = traceClosestWide<COUNT>(S, origin, d, VIS_SHADOW, 0.0f, remaining, nodes, tris, nullptr, time);
+        const Hit h = traceClosestWide<COUNT>(S, origin, d, VIS_SHADOW, 0.0f, remaining, nodes, tris, time);
         if (isMiss(h.prim)) return T;
         Isect is;
         fillHit(S, h, origin, d, is, time);
@@ -367,13 +451,27 @@ __device__ __forceinline__ V3 neeTerm(V3 fLi, V3 vis, float scalar, V3 thr, bool
 }
 
 // ---- any hit over the shadow queue ------------------------------------------------------------
-// ANY: the scene has neither shadow-transmitting surfaces nor shadow links, so visibility is
-// the plain any-hit query (and the transmittance walk is compiled out).
-// AW: the any-hit walk's top AW stack entries in registers (0: all in local memory).
-// MINB: at least this many 128-thread blocks per SM (8: a 64-register cap).
-template <bool COUNT, bool ANY = false, int AW = 0, int MINB = 1>
-__global__ void __launch_bounds__(128, MINB) kShadow(SceneGPU S, Paths P, const uint32_t* count,
-                                                    unsigned long long* stats) {
+// Shadow record i's visibility, found, into its path's radiance.
+__device__ __forceinline__ void addShadowTerm(const SceneGPU& S, const Paths& P, int i, int slot, float scalar, V3 vis) {
+    const float4 sc = P.shC[i];
+    const float4 st = P.shT[i];
+    const V3 c = neeTerm(mk(sc.x, sc.y, sc.z), vis, scalar, mk(st.x, st.y, st.z), (__float_as_uint(sc.w) & 1u) != 0, st.w);
+    if (!isFinite3(c)) return;
+    float4 L = P.L[slot];
+    L.x += c.x;
+    L.y += c.y;
+    L.z += c.z;
+    P.L[slot] = L;
+    if (P.pass) {
+        const int light = static_cast<int>(__float_as_uint(sc.w) >> 1) - 1;
+        const float4* shares = P.shPass + 3 * static_cast<size_t>(i);
+        creditNee(S, P, pathOfSlot(P, slot), light, c, shares[0].w != 0.0f ? shares : nullptr);
+    }
+}
+
+// Scenes with shadow-transmitting surfaces or shadow links: a ray per lane, the transmittance walk.
+template <bool COUNT>
+__global__ void __launch_bounds__(128) kShadow(SceneGPU S, Paths P, const uint32_t* count, unsigned long long* stats) {
     const int n = static_cast<int>(*count);
     uint32_t nodes = 0, tris = 0;
     for (;;) {
@@ -385,25 +483,55 @@ __global__ void __launch_bounds__(128, MINB) kShadow(SceneGPU S, Paths P, const 
         const float4 so = P.shO[i];
         const float4 sd = P.shD[i];
         const int light = static_cast<int>(__float_as_uint(P.shC[i].w) >> 1) - 1;
-        const float time = pathTime(S, P, slot);
-        const V3 vis = ANY ? (traceAnyWide<COUNT, AW>(S, mk(so.x, so.y, so.z), mk(sd.x, sd.y, sd.z), VIS_SHADOW, 0.0f, so.w,
-                                                  nodes, tris, time) ? mk(0.0f) : mk(1.0f))
-                           : shadowVisibility<COUNT>(S, mk(so.x, so.y, so.z), mk(sd.x, sd.y, sd.z), so.w, light, nodes, tris,
-                                                     time);
-        if (isBlack(vis)) continue;
-        const float4 sc = P.shC[i];
-        const float4 st = P.shT[i];
-        const V3 c = neeTerm(mk(sc.x, sc.y, sc.z), vis, sd.w, mk(st.x, st.y, st.z), (__float_as_uint(sc.w) & 1u) != 0, st.w);
-        if (!isFinite3(c)) continue;
-        float4 L = P.L[slot];
-        L.x += c.x;
-        L.y += c.y;
-        L.z += c.z;
-        P.L[slot] = L;
-        if (P.pass) {
-            const float4* shares = P.shPass + 3 * static_cast<size_t>(i);
-            creditNee(S, P, pathOfSlot(P, slot), light, c, shares[0].w != 0.0f ? shares : nullptr);
+        const V3 vis = shadowVisibility<COUNT>(S, mk(so.x, so.y, so.z), mk(sd.x, sd.y, sd.z), so.w, light, nodes, tris,
+                                               pathTime(S, P, slot));
+        if (!isBlack(vis)) addShadowTerm(S, P, i, slot, sd.w, vis);
+    }
+    if (COUNT) {
+        atomicAdd(&stats[2], static_cast<unsigned long long>(nodes));
+        atomicAdd(&stats[3], static_cast<unsigned long long>(tris));
+    }
+}
+
+// Every other scene: the plain any-hit query, a ray per lane (walkTurn).
+template <bool COUNT>
+__global__ void __launch_bounds__(128, 8) kShadowAny(SceneGPU S, Paths P, const uint32_t* count, unsigned long long* stats) {
+    uint32_t stack[kWalkStack];
+    WarpFeed feed{&P.counters[CNT_WORK_SHADOW], static_cast<int>(*count)};
+    const int root = rootRef(S);
+    const bool instances = S.nInstances > 0;
+    uint32_t nodes = 0, tris = 0;
+    int rec = -1;
+    RayWalk w;
+    w.cur = kRayDone;
+    for (;;) {
+        const unsigned idle = __ballot_sync(kWarp, w.cur == kRayDone);
+        if (idle == kWarp || (!feed.dry() && __popc(idle) >= kRefill)) {
+            if (w.cur == kRayDone && rec >= 0) {
+                if (w.prim == 0) addShadowTerm(S, P, rec, P.shadowQ[rec], P.shD[rec].w, mk(1.0f));
+                rec = -1;
+            }
+            __syncwarp();
+            const int i = feed.next(w.cur == kRayDone);
+            if (i >= 0) {
+                rec = i;
+                const float4 so = P.shO[i];
+                const float4 sd = P.shD[i];
+                w.start(S, root, mk(so.x, so.y, so.z), mk(sd.x, sd.y, sd.z), VIS_SHADOW, so.w, 0);
+            }
+            if (__all_sync(kWarp, rec < 0)) break;
+            continue;
         }
+        walkTurn<true, COUNT>(
+            S, w, stack, instances, nodes, tris,
+            [&](V3& o, V3& d, uint32_t& mask) {
+                const float4 so = P.shO[rec], sd = P.shD[rec];
+                o = mk(so.x, so.y, so.z);
+                d = mk(sd.x, sd.y, sd.z);
+                mask = VIS_SHADOW;
+            },
+            [&]() { return pathTime(S, P, P.shadowQ[rec]); });
+        __syncwarp();
     }
     if (COUNT) {
         atomicAdd(&stats[2], static_cast<unsigned long long>(nodes));
@@ -435,7 +563,7 @@ enum SegmentOutcome { SEG_SURFACE = 0, SEG_SCATTERED = 1, SEG_END = 2 };
 // Absorption and scattering over the segment a path just travelled inside the medium of the
 // innermost volume boundary it entered (path_tracer.cpp:456-479).  SEG_SCATTERED sets up the
 // next ray (origin newO, direction newD).
-__device__ __noinline__ int mediumSegment(const TablesGPU* T, const MatGPU& mm, V3 segStart, V3 dir, bool hit, V3 hitPoint,
+static __device__ __noinline__ int mediumSegment(const TablesGPU* T, const MatGPU& mm, V3 segStart, V3 dir, bool hit, V3 hitPoint,
                                           Sobol& sb, V3& thr, uint32_t& volCtr, V3& newO, V3& newD) {
     const float dirLen = length(dir);
     const float segment = hit ? length(hitPoint - segStart) : kFltMax;
@@ -470,7 +598,7 @@ __device__ __forceinline__ bool guidable(const MatGPU& m) {
     return (m.flags & (MF_DELTA | MF_VOLUME_BOUNDARY | MF_TRANSMITS_SHADOWS)) == 0;
 }
 
-__device__ __noinline__ void slotLobes(const Paths& P, int slot, Lobes& L) {
+static __device__ __noinline__ void slotLobes(const Paths& P, int slot, Lobes& L) {
     float o[kNetUsedOut];
     for (int j = 0; j < kNetUsedOut / 4; ++j) {
         const float4 v = P.guideOut[static_cast<size_t>(slot) * 10 + j];
@@ -482,7 +610,7 @@ __device__ __noinline__ void slotLobes(const Paths& P, int slot, Lobes& L) {
     decodeLobes(o, L);
 }
 
-__device__ __noinline__ float guidePdf(const Paths& P, int slot, V3 w) {
+static __device__ __noinline__ float guidePdf(const Paths& P, int slot, V3 w) {
     Lobes L;
     slotLobes(P, slot, L);
     return lobesPdf(L, w);
@@ -490,7 +618,7 @@ __device__ __noinline__ float guidePdf(const Paths& P, int slot, V3 w) {
 
 // Training record of a path's first guidable vertex; its radiance along wi is what the path adds
 // from here on (kGuideCollect).  False when the path has one already.
-__device__ __noinline__ bool guideRecord(const Paths& P, int slot, V3 p, V3 n, V3 wo, V3 wi, V3 thrBefore) {
+static __device__ __noinline__ bool guideRecord(const Paths& P, int slot, V3 p, V3 n, V3 wo, V3 wi, V3 thrBefore) {
     float4* rec = P.guideRec + static_cast<size_t>(slot) * 6;
     if (rec[4].w != 0.0f) return false;
     rec[0] = make_float4(p.x, p.y, p.z, 0.0f);
@@ -505,7 +633,7 @@ __device__ __noinline__ bool guideRecord(const Paths& P, int slot, V3 p, V3 n, V
 // One-sample MIS of the proposal and the BSDF, 50/50 (path_tracer.cpp:703-735 with the
 // learned mixture in place of the SD-tree): the branch number picks the strategy, the
 // proposal draws a lobe from the rest of it and a direction from one get2D.
-__device__ __noinline__ bool guidedSample(const TablesGPU* T, const MatGPU& mat, V3 wo, const ShadePoint& sp, const Paths& P,
+static __device__ __noinline__ bool guidedSample(const TablesGPU* T, const MatGPU& mat, V3 wo, const ShadePoint& sp, const Paths& P,
                                           int slot, Sobol& sb, BsdfSample& bs) {
     Lobes L;
     slotLobes(P, slot, L);
@@ -539,7 +667,7 @@ __device__ __noinline__ bool guidedSample(const TablesGPU* T, const MatGPU& mat,
 // The same one-sample MIS with the SD-tree's sampling quadtree rooted at `root`
 // (path_tracer.cpp:703-735): a direction from one get2D on the guide branch, the BSDF's
 // get1D + get2D on the other.
-__device__ __noinline__ bool sdGuidedSample(const TablesGPU* T, const MatGPU& mat, V3 wo, const ShadePoint& sp,
+static __device__ __noinline__ bool sdGuidedSample(const TablesGPU* T, const MatGPU& mat, V3 wo, const ShadePoint& sp,
                                             const SdQuad* tree, int root, Sobol& sb, BsdfSample& bs) {
     const float uBranch = get1D(sb);
     if (uBranch < 0.5f) {
@@ -571,7 +699,7 @@ __device__ __noinline__ bool sdGuidedSample(const TablesGPU* T, const MatGPU& ma
 // ---- surface effects of Li that cast rays of their own ------------------------------------------
 // Contact ambient occlusion (approxAo, path_tracer.cpp:27-45): `samples` cosine rays of at most
 // 0.35 over the shading normal; the path's throughput is scaled by lerp(1, visibility, strength).
-__device__ __noinline__ float approxAo(const SceneGPU& S, const Isect& is, Sobol& sb, float strength, int samples,
+static __device__ __noinline__ float approxAo(const SceneGPU& S, const Isect& is, Sobol& sb, float strength, int samples,
                                        float time) {
     if (strength <= 0.0f || samples <= 0) return 1.0f;
     const TablesGPU* T = S.tables;
@@ -591,7 +719,7 @@ __device__ __noinline__ float approxAo(const SceneGPU& S, const Isect& is, Sobol
 // around the hit, each probed along one of the frame's axes (normal ½, tangents ¼ each) from both
 // sides with rays of 2·radius; the outward normals of hits on the same shape within 1.5·radius,
 // weighted by their projection on the probe axis, average with a quarter of the own normal.
-__device__ __noinline__ V3 roundedEdgeNormal(const SceneGPU& S, const Isect& is, float radius, Sobol& sb, float time) {
+static __device__ __noinline__ V3 roundedEdgeNormal(const SceneGPU& S, const Isect& is, float radius, Sobol& sb, float time) {
     const TablesGPU* T = S.tables;
     const V3 N = is.normal;
     const Frame f = frameFromNormal(N);
@@ -613,7 +741,7 @@ __device__ __noinline__ V3 roundedEdgeNormal(const SceneGPU& S, const Isect& is,
             const float sign = k == 0 ? 1.0f : -1.0f;
             const V3 origin = is.point + s * d.x + t * d.y + axis * (sign * radius);
             const V3 rdir = axis * -sign;
-            const Hit h = traceClosestWide<false>(S, origin, rdir, VIS_ALL, 0.0f, 2.0f * radius, n0, n1, nullptr, time);
+            const Hit h = traceClosestWide<false>(S, origin, rdir, VIS_ALL, 0.0f, 2.0f * radius, n0, n1, time);
             if (isMiss(h.prim)) continue;
             Isect hit;
             fillHit(S, h, origin, rdir, hit, time);
@@ -632,7 +760,7 @@ __device__ __noinline__ V3 roundedEdgeNormal(const SceneGPU& S, const Isect& is,
 // Shadow catcher (path_tracer.cpp:515-563): a camera ray that hits the catcher sees the
 // background `bg` times the share `ratio` of the direct light, over 4 × shadowSamples NEE
 // samples, that reaches the hit point.
-__device__ __noinline__ V3 shadowCatcher(const SceneGPU& S, const Isect& is, V3 dir, int shadowSamples, Sobol& sb,
+static __device__ __noinline__ V3 shadowCatcher(const SceneGPU& S, const Isect& is, V3 dir, int shadowSamples, Sobol& sb,
                                          float& ratioOut, float time) {
     const TablesGPU* T = S.tables;
     V3 bg = mk(0.0f);
@@ -727,10 +855,7 @@ __device__ __forceinline__ bool shadeSlot(const SceneGPU& S, const Paths& P, con
         skips = (ctr >> 24) & 0xFF;
     Sobol sb;
     sb.pixelHash = __float_as_uint(pp.w);
-    {
-        const int sOff = (path - A.slotFirst) / A.nPix;
-        sb.revIndex = rev32(static_cast<uint32_t>(A.sampleFirst + sOff));
-    }
+    sb.revIndex = rev32(static_cast<uint32_t>(A.sampleFirst + sampleOfPath(A, path)));
     sb.dim = __float_as_uint(lp.w);
     V3 thr = mk(th.x, th.y, th.z);
     const V3 dir = mk(rd.x, rd.y, rd.z);
@@ -1341,7 +1466,7 @@ __global__ void __launch_bounds__(kTailBlock) kTail(SceneGPU S, Paths P, Wave W,
             const float4 ro = P.rayO[slot];
             const float4 rd = P.rayD[slot];
             const Hit h = traceClosestWide<COUNT>(S, mk(ro.x, ro.y, ro.z), mk(rd.x, rd.y, rd.z), __float_as_uint(ro.w), 0.0f,
-                                              1e30f, nodes, tris, nullptr, pathTime(S, P, slot));
+                                              1e30f, nodes, tris, pathTime(S, P, slot));
             ++rays;
             P.hit[slot] = make_float4(h.t, h.u, h.v, __int_as_float(h.prim));
             if (!shadeSlot<true, COUNT, OUT>(S, P, A, slot, path, shNodes, shTris, shRays)) break;
@@ -1392,7 +1517,7 @@ __global__ void __launch_bounds__(kTailLockstepBlock) kTailLockstep(SceneGPU S, 
             const float4 ro = P.rayO[slot];
             const float4 rd = P.rayD[slot];
             const Hit h = traceClosestWide<false>(S, mk(ro.x, ro.y, ro.z), mk(rd.x, rd.y, rd.z), __float_as_uint(ro.w), 0.0f,
-                                              1e30f, nodes, tris, nullptr, pathTime(S, P, slot));
+                                              1e30f, nodes, tris, pathTime(S, P, slot));
             ++rays;
             P.hit[slot] = make_float4(h.t, h.u, h.v, __int_as_float(h.prim));
         }
@@ -1414,7 +1539,7 @@ __global__ void __launch_bounds__(kTailLockstepBlock) kTailLockstep(SceneGPU S, 
 // ---- film: Film::addSample in sample order per pixel (src/core/image/film.cpp:56-69) ----------
 // The AOV films of one pixel (addAovs, renderer.cpp:219-224): albedo and alpha by addSample,
 // the normal by addSampleSigned (film.cpp:73-85), in sample order.
-__device__ __noinline__ void filmAovs(const Paths& P, const WaveSeg& A, int p, int pix) {
+static __device__ __noinline__ void filmAovs(const Paths& P, const WaveSeg& A, int p, int pix) {
     const size_t n = static_cast<size_t>(A.width) * static_cast<size_t>(A.height);
     for (int f = 0; f < 3; ++f) {
         float* fsum = A.aov + static_cast<size_t>(f) * 5 * n;
@@ -1423,7 +1548,7 @@ __device__ __noinline__ void filmAovs(const Paths& P, const WaveSeg& A, int p, i
         float r = fsum[3 * pix + 0], g = fsum[3 * pix + 1], b = fsum[3 * pix + 2], q = fsq[pix];
         uint32_t c = fcnt[pix];
         for (int s = 0; s < A.nSamples; ++s) {
-            const int path = A.slotFirst + s * A.nPix + p;
+            const int path = pathOfSample(A, p, s);
             V3 v;
             if (f == 0) {
                 const float4 a = P.aovA[path];
@@ -1455,7 +1580,7 @@ __device__ __noinline__ void filmAovs(const Paths& P, const WaveSeg& A, int p, i
 
 // The render-pass films of one pixel (addPasses, renderer.cpp:206-217), in sample order: light
 // passes, depth, ids and light groups by addSample, the position by addSampleSigned.
-__device__ __noinline__ void filmPasses(const Paths& P, const WaveSeg& A, int p, int pix) {
+static __device__ __noinline__ void filmPasses(const Paths& P, const WaveSeg& A, int p, int pix) {
     const size_t n = static_cast<size_t>(A.width) * static_cast<size_t>(A.height);
     const int nFilms = PFILM_GROUPS + (P.passStride - PASS_GROUPS);
     for (int f = 0; f < nFilms; ++f) {
@@ -1471,7 +1596,7 @@ __device__ __noinline__ void filmPasses(const Paths& P, const WaveSeg& A, int p,
         float r = fsum[3 * pix + 0], g = fsum[3 * pix + 1], b = fsum[3 * pix + 2], q = fsq[pix];
         uint32_t c = fcnt[pix];
         for (int s = 0; s < A.nSamples; ++s) {
-            const float4* blk = passBlock(P, A.slotFirst + s * A.nPix + p);
+            const float4* blk = passBlock(P, pathOfSample(A, p, s));
             const float4 v4 = blk[slotOf];
             V3 v = mk(v4.x, v4.y, v4.z);
             if (f == PFILM_DEPTH || f == PFILM_POSITION) {
@@ -1498,7 +1623,7 @@ __device__ __noinline__ void filmPasses(const Paths& P, const WaveSeg& A, int p,
     if (A.cryptoObj) {
         // each sample's Cryptomatte ids; the host adds them to its CryptoFilms
         for (int s = 0; s < A.nSamples; ++s) {
-            const float4 id = passBlock(P, A.slotFirst + s * A.nPix + p)[PASS_CRYPTO];
+            const float4 id = passBlock(P, pathOfSample(A, p, s))[PASS_CRYPTO];
             const size_t o = static_cast<size_t>(A.sampleFirst + s - A.cryptoFirst) * n + static_cast<size_t>(pix);
             A.cryptoObj[o] = id.x;
             A.cryptoMat[o] = id.y;
@@ -1506,19 +1631,20 @@ __device__ __noinline__ void filmPasses(const Paths& P, const WaveSeg& A, int p,
     }
 }
 
-__global__ void kFilm(Paths P, Wave W, unsigned long long* rejected) {
+static __global__ void kFilm(Paths P, Wave W, unsigned long long* rejected) {
     unsigned long long rej = 0;
     for (int wp = blockIdx.x * blockDim.x + threadIdx.x; wp < W.nPix; wp += gridDim.x * blockDim.x) {
         const WaveSeg& A = W.segs[segOfPixel(W, wp)];
         const int p = wp - A.pixFirst;
-        const int tp = A.pixelFirst + p;
-        const int pix = A.pixList ? A.pixList[tp] : (A.tileY + tp / A.tileW) * A.width + A.tileX + tp % A.tileW;
+        int px, py;
+        tilePixel(A, A.pixelFirst + p, px, py);
+        const int pix = py * A.width + px;
         float* sum = A.sum;
         float sr = sum[3 * pix + 0], sg = sum[3 * pix + 1], sbb = sum[3 * pix + 2];
         float sq = A.sq[pix];
         uint32_t c = A.cnt[pix];
         for (int s = 0; s < A.nSamples; ++s) {
-            const int path = A.slotFirst + s * A.nPix + p;
+            const int path = pathOfSample(A, p, s);
             const float4 L = P.Lout ? P.Lout[path] : P.L[path];
             ++c;
             const bool ok = finitef(L.x) && finitef(L.y) && finitef(L.z) && L.x >= 0.0f && L.y >= 0.0f && L.z >= 0.0f;
@@ -1542,5 +1668,29 @@ __global__ void kFilm(Paths P, Wave W, unsigned long long* rejected) {
     }
     if (rej) atomicAdd(rejected, rej);
 }
+
+// ---- instantiations ---------------------------------------------------------------------------
+// The kernels below are compiled in translation units of their own (pe_kernels_*.cu), side by side;
+// PE_LEAN_KERNELS(K) and its siblings expand K(kernel) over a unit's instantiations.
+#define PE_SHADE_ARGS (SceneGPU, Paths, Wave, int32_t*, uint32_t*)
+#define PE_LEAN_KERNELS(K)                                                                         \
+    K(kShadeKey<false, 0, 1>) K(kShadeKey<false, 1, 1>) K(kShadeKey<false, 2, 1>)                  \
+    K(kShadeKey<false, 3, 1>) K(kShadeKey<false, 4, 1>) K(kShadeKey<false, 0, 4>)                  \
+    K(kShadeKey<false, 1, 4>) K(kShadeKey<false, 2, 4>) K(kShadeKey<false, 3, 4>)                  \
+    K(kShadeKey<false, 4, 4>) K(kShadeKey<false, 0, 5>) K(kShadeKey<false, 1, 5>)                  \
+    K(kShadeKey<false, 2, 5>) K(kShadeKey<false, 3, 5>) K(kShadeKey<false, 4, 5>)
+#define PE_LEAN_OUT_KERNELS(K)                                                                     \
+    K(kShadeKey<true, 0, 1>) K(kShadeKey<true, 1, 1>) K(kShadeKey<true, 2, 1>)                     \
+    K(kShadeKey<true, 3, 1>) K(kShadeKey<true, 4, 1>)
+#define PE_FULL_KERNELS(K)                                                                         \
+    K(kShade<false, false>) K(kShade<true, false>) K(kShade<false, true>) K(kShade<true, true>)
+#define PE_TAIL_ARGS (SceneGPU, Paths, Wave, const int32_t*, const uint32_t*, uint32_t*, unsigned long long*)
+#define PE_TAIL_KERNELS(K) K(kTail<false, true>) K(kTail<true, false>) K(kTail<true, true>)
+#define PE_LOCKSTEP_KERNELS(K) K(kTailLockstep<false>) K(kTailLockstep<true>)
+#define PE_TRACE_ARGS (SceneGPU, Paths, const int32_t*, const uint32_t*, unsigned long long*)
+#define PE_TRACE_KERNELS(K)                                                                        \
+    K(kIntersect<false>) K(kIntersect<true>) K(kIntersectBinary<false>) K(kIntersectBinary<true>)
+#define PE_SHADOW_ARGS (SceneGPU, Paths, const uint32_t*, unsigned long long*)
+#define PE_SHADOW_KERNELS(K) K(kShadow<false>) K(kShadow<true>) K(kShadowAny<false>) K(kShadowAny<true>)
 
 } // namespace pe

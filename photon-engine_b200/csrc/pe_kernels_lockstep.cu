@@ -1,0 +1,8 @@
+// pe_kernels_lockstep.cu — the lockstep tail kernels (pe_integrator.cuh), compiled on their own.
+#include "pe_integrator.cuh"
+
+namespace pe {
+#define PE_INSTANTIATE(...) template __global__ void __VA_ARGS__ PE_TAIL_ARGS;
+PE_LOCKSTEP_KERNELS(PE_INSTANTIATE)
+#undef PE_INSTANTIATE
+} // namespace pe

@@ -1,0 +1,11 @@
+// pe_kernels_trace.cu — the closest-hit and any-hit kernels (pe_integrator.cuh), compiled on their own.
+#include "pe_integrator.cuh"
+
+namespace pe {
+#define PE_INSTANTIATE(...) template __global__ void __VA_ARGS__ PE_TRACE_ARGS;
+PE_TRACE_KERNELS(PE_INSTANTIATE)
+#undef PE_INSTANTIATE
+#define PE_INSTANTIATE(...) template __global__ void __VA_ARGS__ PE_SHADOW_ARGS;
+PE_SHADOW_KERNELS(PE_INSTANTIATE)
+#undef PE_INSTANTIATE
+} // namespace pe

@@ -313,6 +313,7 @@ int planPaths(pe_server* S, int li, int budget) {
             seg.tileX = 0;
             seg.tileY = 0;
             seg.tileW = r.st.width;
+            seg.tileH = r.st.height;
             seg.sum = r.sum;
             seg.cnt = r.cnt;
             seg.sq = r.sq;

@@ -251,13 +251,13 @@ __device__ __forceinline__ int localOfHit(int32_t prim) { return static_cast<int
 template <bool COUNT, int LEVEL>
 __device__ void walkClosest(const SceneGPU& S, int cur, V3 o, V3 d, V3 inv, uint32_t mask, float tMin, float& tMax,
                             Hit& best, uint32_t& nodeVisits, uint32_t& triTests, float time);
-template <bool COUNT, int SD, int LEVEL>
+template <bool COUNT, int LEVEL>
 __device__ void walkClosestWide(const SceneGPU& S, int cur, V3 o, V3 d, V3 inv, uint32_t mask, float tMin, float& tMax,
-                                Hit& best, uint32_t& nodeVisits, uint32_t& triTests, uint2* sstack, float time);
+                                Hit& best, uint32_t& nodeVisits, uint32_t& triTests, float time);
 template <bool COUNT, int LEVEL>
 __device__ bool walkAny(const SceneGPU& S, int cur, V3 o, V3 d, V3 inv, uint32_t mask, float tMin, float tMax,
                         uint32_t& nodeVisits, uint32_t& triTests, float time);
-template <bool COUNT, int LEVEL, int AW = 0>
+template <bool COUNT, int LEVEL>
 __device__ bool walkAnyWide(const SceneGPU& S, int cur, V3 o, V3 d, V3 inv, uint32_t mask, float tMin, float tMax,
                             uint32_t& nodeVisits, uint32_t& triTests, float time);
 
@@ -314,7 +314,7 @@ __device__ __noinline__ void instanceClosest(const SceneGPU& S, int inst, uint32
     h.u = h.v = 0.0f;
     float tm = tMax;
     if (WIDE)
-        walkClosestWide<COUNT, 0, 1>(S, I.rootWide, lo, ld, linv, 0x1Fu, tMin, tm, h, nodeVisits, triTests, nullptr, 0.0f);
+        walkClosestWide<COUNT, 1>(S, I.rootWide, lo, ld, linv, 0x1Fu, tMin, tm, h, nodeVisits, triTests, 0.0f);
     else
         walkClosest<COUNT, 1>(S, I.rootBinary, lo, ld, linv, 0x1Fu, tMin, tm, h, nodeVisits, triTests, 0.0f);
     if (h.prim < 0) return;
@@ -547,31 +547,27 @@ __device__ bool traceAny(const SceneGPU& S, V3 o, V3 d, uint32_t mask, float tMi
 constexpr float kInf = std::numeric_limits<float>::infinity();
 
 struct WideNode {
-    float4 lx, hx, ly, hy, lz, hz;
-    int4 child;
-    int count;
+    float4 a[4], b[4]; // per child: (lo.x, lo.y, lo.z, hi.x), (hi.y, hi.z, reference, present)
 };
 __device__ __forceinline__ WideNode loadWide(const float4* w, int i) {
     WideNode n;
     const float4* p = w + 8 * static_cast<size_t>(i);
-    n.lx = __ldg(p + 0);
-    n.hx = __ldg(p + 1);
-    n.ly = __ldg(p + 2);
-    n.hy = __ldg(p + 3);
-    n.lz = __ldg(p + 4);
-    n.hz = __ldg(p + 5);
-    const float4 c = __ldg(p + 6);
-    n.child = make_int4(__float_as_int(c.x), __float_as_int(c.y), __float_as_int(c.z), __float_as_int(c.w));
-    n.count = __float_as_int(__ldg(reinterpret_cast<const float*>(p + 7)));
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        n.a[k] = __ldg(p + k);
+        n.b[k] = __ldg(p + 4 + k);
+    }
     return n;
 }
+__device__ __forceinline__ bool wideSlab(const float4 a, const float4 b, V3 o, V3 inv, float tMin, float tMax, float& tn) {
+    return __float_as_int(b.w) != 0 && slab(a.x, a.w, a.y, b.x, a.z, b.y, o, inv, tMin, tMax, tn);
+}
+__device__ __forceinline__ int wideRef(const float4 b) { return __float_as_int(b.z); }
 // Entry distances of the four children (+inf where a child is absent or missed).
 __device__ __forceinline__ void wideSlabs(const WideNode& n, V3 o, V3 inv, float tMin, float tMax, float t[4]) {
     float tn;
-    t[0] = slab(n.lx.x, n.hx.x, n.ly.x, n.hy.x, n.lz.x, n.hz.x, o, inv, tMin, tMax, tn) ? tn : kInf;
-    t[1] = slab(n.lx.y, n.hx.y, n.ly.y, n.hy.y, n.lz.y, n.hz.y, o, inv, tMin, tMax, tn) ? tn : kInf;
-    t[2] = n.count > 2 && slab(n.lx.z, n.hx.z, n.ly.z, n.hy.z, n.lz.z, n.hz.z, o, inv, tMin, tMax, tn) ? tn : kInf;
-    t[3] = n.count > 3 && slab(n.lx.w, n.hx.w, n.ly.w, n.hy.w, n.lz.w, n.hz.w, o, inv, tMin, tMax, tn) ? tn : kInf;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) t[k] = wideSlab(n.a[k], n.b[k], o, inv, tMin, tMax, tn) ? tn : kInf;
 }
 // Compare-exchange on (distance, child order): a total order, so equal distances keep child order.
 __device__ __forceinline__ void cmpx(float& ta, int& ra, int& ka, float& tb, int& rb, int& kb) {
@@ -582,65 +578,13 @@ __device__ __forceinline__ void cmpx(float& ta, int& ra, int& ka, float& tb, int
     }
 }
 
-// A traversal stack whose top K entries live in registers (shifted on every push and pop, so
-// every index is static) and the rest in the thread's local memory: a walk pushes and pops mostly
-// within a few entries of the top, so most of its stack traffic never reaches memory.
-template <typename T, int K, int N>
-struct WindowStack {
-    T top[K];
-    T rest[N - K];
-    int n = 0;
-    __device__ __forceinline__ void push(T e) {
-        if (n >= K) rest[n - K] = top[K - 1];
-#pragma unroll
-        for (int i = K - 1; i > 0; --i) top[i] = top[i - 1];
-        top[0] = e;
-        ++n;
-    }
-    __device__ __forceinline__ T pop() {
-        const T e = top[0];
-#pragma unroll
-        for (int i = 0; i < K - 1; ++i) top[i] = top[i + 1];
-        --n;
-        if (n >= K) top[K - 1] = rest[n - K];
-        return e;
-    }
-    __device__ __forceinline__ bool empty() const { return n == 0; }
-};
-
-// The closest-hit walk's stack of (reference, entry distance) pairs.  SD > 0: its first SD entries
-// in shared memory (`shared` points at the thread's column of a [SD][128] block array, stride 128),
-// the rest in local memory; SD == 0: all in local memory; SD < 0: the top −SD entries in registers.
-template <int SD, bool WINDOW = (SD < 0)>
-struct TraceStack;
-template <int SD>
-struct TraceStack<SD, false> {
-    uint2* shared;
-    uint2 local[kWideStack - SD];
-    int sp = 0;
-    __device__ __forceinline__ void push(uint2 e) {
-        if (SD > 0 && sp < SD) shared[sp * 128] = e;
-        else local[sp - SD] = e;
-        ++sp;
-    }
-    __device__ __forceinline__ uint2 pop() {
-        --sp;
-        return (SD > 0 && sp < SD) ? shared[sp * 128] : local[sp - SD];
-    }
-    __device__ __forceinline__ bool empty() const { return sp == 0; }
-};
-template <int SD>
-struct TraceStack<SD, true> : WindowStack<uint2, -SD, kWideStack> {
-    uint2* shared;
-};
-
-// The 4-wide walk from reference `cur`.  SD: stack entries kept in shared memory (`sstack`:
-// this thread's column); 0 keeps all in local memory.
-template <bool COUNT, int SD, int LEVEL>
+// The 4-wide walk by one lane from reference `cur`: rays cast inside the shading code (contact
+// occlusion, rounded edges, transmitted shadows).  The queues' rays take the four-lane walk below.
+template <bool COUNT, int LEVEL>
 __device__ void walkClosestWide(const SceneGPU& S, int cur, V3 o, V3 d, V3 inv, uint32_t mask, float tMin, float& tMax,
-                                Hit& best, uint32_t& nodeVisits, uint32_t& triTests, uint2* sstack, float time) {
-    TraceStack<SD> stack;
-    stack.shared = sstack;
+                                Hit& best, uint32_t& nodeVisits, uint32_t& triTests, float time) {
+    uint2 stack[kWideStack];
+    int sp = 0;
     for (;;) {
         while (cur >= 0) {
             if (COUNT) ++nodeVisits;
@@ -648,7 +592,7 @@ __device__ void walkClosestWide(const SceneGPU& S, int cur, V3 o, V3 d, V3 inv, 
             float t[4];
             wideSlabs(n, o, inv, tMin, tMax, t);
             float t0 = t[0], t1 = t[1], t2 = t[2], t3 = t[3];
-            int r0 = n.child.x, r1 = n.child.y, r2 = n.child.z, r3 = n.child.w;
+            int r0 = wideRef(n.b[0]), r1 = wideRef(n.b[1]), r2 = wideRef(n.b[2]), r3 = wideRef(n.b[3]);
             int k0 = 0, k1 = 1, k2 = 2, k3 = 3;
             cmpx(t0, r0, k0, t1, r1, k1);
             cmpx(t2, r2, k2, t3, r3, k3);
@@ -657,8 +601,8 @@ __device__ void walkClosestWide(const SceneGPU& S, int cur, V3 o, V3 d, V3 inv, 
             cmpx(t1, r1, k1, t2, r2, k2);
             if (t0 == kInf) {
                 bool found = false;
-                while (!stack.empty()) {
-                    const uint2 e = stack.pop();
+                while (sp > 0) {
+                    const uint2 e = stack[--sp];
                     if (__uint_as_float(e.y) <= tMax) {
                         cur = static_cast<int>(e.x);
                         found = true;
@@ -669,17 +613,17 @@ __device__ void walkClosestWide(const SceneGPU& S, int cur, V3 o, V3 d, V3 inv, 
                 continue;
             }
             // farther children first onto the stack, so they pop nearest first
-            if (t3 != kInf) stack.push(make_uint2(static_cast<uint32_t>(r3), __float_as_uint(t3)));
-            if (t2 != kInf) stack.push(make_uint2(static_cast<uint32_t>(r2), __float_as_uint(t2)));
-            if (t1 != kInf) stack.push(make_uint2(static_cast<uint32_t>(r1), __float_as_uint(t1)));
+            if (t3 != kInf) stack[sp++] = make_uint2(static_cast<uint32_t>(r3), __float_as_uint(t3));
+            if (t2 != kInf) stack[sp++] = make_uint2(static_cast<uint32_t>(r2), __float_as_uint(t2));
+            if (t1 != kInf) stack[sp++] = make_uint2(static_cast<uint32_t>(r1), __float_as_uint(t1));
             cur = r0;
         }
         int first, count;
         leafRange(cur, first, count);
         testLeafClosest<COUNT, LEVEL, true>(S, first, count, o, d, mask, tMin, tMax, best, nodeVisits, triTests, time);
         bool found = false;
-        while (!stack.empty()) {
-            const uint2 e = stack.pop();
+        while (sp > 0) {
+            const uint2 e = stack[--sp];
             if (__uint_as_float(e.y) <= tMax) {
                 cur = static_cast<int>(e.x);
                 found = true;
@@ -690,77 +634,9 @@ __device__ void walkClosestWide(const SceneGPU& S, int cur, V3 o, V3 d, V3 inv, 
     }
 }
 
-// The 4-wide walk with postponed leaves (speculative traversal after Aila and Laine, "Understanding
-// the Efficiency of Ray Traversal on GPUs", 2009): a lane that reaches a leaf keeps it aside and
-// goes on descending until every active lane of its warp holds one, then the warp tests its
-// leaves together, so leaf tests and node steps stop interleaving across the lanes.  Leaves are
-// tested in another order than the depth-first walk's and tMax shrinks later, so a few more nodes
-// are visited; every leaf that can hold a closer hit is still tested, so the distance is the same.
-template <bool COUNT, int SD, int LEVEL>
-__device__ void walkClosestWideSpec(const SceneGPU& S, int cur, V3 o, V3 d, V3 inv, uint32_t mask, float tMin,
-                                    float& tMax, Hit& best, uint32_t& nodeVisits, uint32_t& triTests, uint2* sstack,
-                                    float time) {
-    TraceStack<SD> stack;
-    stack.shared = sstack;
-    auto popNext = [&]() {
-        while (!stack.empty()) {
-            const uint2 e = stack.pop();
-            if (__uint_as_float(e.y) <= tMax) {
-                cur = static_cast<int>(e.x);
-                return true;
-            }
-        }
-        return false;
-    };
-    bool alive = true;       // `cur` holds a reference still to visit
-    bool hasLeaf = false;    // a leaf is kept aside for the next test
-    int leafRef = 0;
-    while (alive || hasLeaf) {
-        while (alive && (cur >= 0 || !hasLeaf)) {
-            if (cur < 0) {
-                // a leaf and none kept aside: keep it, take the next reference
-                leafRef = cur;
-                hasLeaf = true;
-                alive = popNext();
-            } else {
-                if (COUNT) ++nodeVisits;
-                const WideNode n = loadWide(S.wide, cur);
-                float t[4];
-                wideSlabs(n, o, inv, tMin, tMax, t);
-                float t0 = t[0], t1 = t[1], t2 = t[2], t3 = t[3];
-                int r0 = n.child.x, r1 = n.child.y, r2 = n.child.z, r3 = n.child.w;
-                int k0 = 0, k1 = 1, k2 = 2, k3 = 3;
-                cmpx(t0, r0, k0, t1, r1, k1);
-                cmpx(t2, r2, k2, t3, r3, k3);
-                cmpx(t0, r0, k0, t2, r2, k2);
-                cmpx(t1, r1, k1, t3, r3, k3);
-                cmpx(t1, r1, k1, t2, r2, k2);
-                if (t0 == kInf) {
-                    alive = popNext();
-                } else {
-                    if (t3 != kInf) stack.push(make_uint2(static_cast<uint32_t>(r3), __float_as_uint(t3)));
-                    if (t2 != kInf) stack.push(make_uint2(static_cast<uint32_t>(r2), __float_as_uint(t2)));
-                    if (t1 != kInf) stack.push(make_uint2(static_cast<uint32_t>(r1), __float_as_uint(t1)));
-                    cur = r0;
-                }
-            }
-            // every lane still walking holds a leaf: test them together
-            if (!__any_sync(__activemask(), !hasLeaf)) break;
-        }
-        if (hasLeaf) {
-            int first, count;
-            leafRange(leafRef, first, count);
-            testLeafClosest<COUNT, LEVEL, true>(S, first, count, o, d, mask, tMin, tMax, best, nodeVisits, triTests, time);
-            hasLeaf = false;
-            // the reference in hand may have become too far while the leaf was aside; it is an
-            // interior node or a leaf, tested against tMax when it is visited or kept
-        }
-    }
-}
-
-template <bool COUNT, int SD = 0, bool SPEC = false>
+template <bool COUNT>
 __device__ Hit traceClosestWide(const SceneGPU& S, V3 o, V3 d, uint32_t mask, float tMin, float tMax,
-                                uint32_t& nodeVisits, uint32_t& triTests, uint2* sstack = nullptr, float time = 0.0f) {
+                                uint32_t& nodeVisits, uint32_t& triTests, float time = 0.0f) {
     Hit best;
     best.prim = -1;
     best.meta = 0;
@@ -771,48 +647,14 @@ __device__ Hit traceClosestWide(const SceneGPU& S, V3 o, V3 d, uint32_t mask, fl
     if (S.nTris == 0) return best;
     if (!slab(S.rootMin[0], S.rootMax[0], S.rootMin[1], S.rootMax[1], S.rootMin[2], S.rootMax[2], o, inv, tMin, tMax, tn))
         return best;
-    if (SPEC)
-        walkClosestWideSpec<COUNT, SD, 0>(S, rootRef(S), o, d, inv, mask, tMin, tMax, best, nodeVisits, triTests, sstack,
-                                          time);
-    else
-        walkClosestWide<COUNT, SD, 0>(S, rootRef(S), o, d, inv, mask, tMin, tMax, best, nodeVisits, triTests, sstack, time);
+    walkClosestWide<COUNT, 0>(S, rootRef(S), o, d, inv, mask, tMin, tMax, best, nodeVisits, triTests, time);
     return best;
 }
 
-// Any hit over the 4-wide tree from reference `cur`: the answer does not depend on the order.
-// AW > 0: the top AW stack entries in registers (WindowStack), else all in local memory.
-template <bool COUNT, int LEVEL, int AW>
+// Any hit over the 4-wide tree by one lane from reference `cur`: the answer does not depend on the order.
+template <bool COUNT, int LEVEL>
 __device__ bool walkAnyWide(const SceneGPU& S, int cur, V3 o, V3 d, V3 inv, uint32_t mask, float tMin, float tMax,
                             uint32_t& nodeVisits, uint32_t& triTests, float time) {
-    if constexpr (AW > 0) {
-        WindowStack<int, AW, kWideStack> stack;
-        for (;;) {
-            while (cur >= 0) {
-                if (COUNT) ++nodeVisits;
-                const WideNode n = loadWide(S.wide, cur);
-                float t[4];
-                wideSlabs(n, o, inv, tMin, tMax, t);
-                int next = 0;
-                bool have = false;
-                if (t[0] != kInf) { next = n.child.x; have = true; }
-                if (t[1] != kInf) { if (!have) { next = n.child.y; have = true; } else stack.push(n.child.y); }
-                if (t[2] != kInf) { if (!have) { next = n.child.z; have = true; } else stack.push(n.child.z); }
-                if (t[3] != kInf) { if (!have) { next = n.child.w; have = true; } else stack.push(n.child.w); }
-                if (!have) {
-                    if (stack.empty()) return false;
-                    cur = stack.pop();
-                } else {
-                    cur = next;
-                }
-            }
-            int first, count;
-            leafRange(cur, first, count);
-            if (testLeafAny<COUNT, LEVEL, true>(S, first, count, o, d, mask, tMin, tMax, nodeVisits, triTests, time))
-                return true;
-            if (stack.empty()) return false;
-            cur = stack.pop();
-        }
-    }
     int stackRef[kWideStack];
     int sp = 0;
     for (;;) {
@@ -825,10 +667,16 @@ __device__ bool walkAnyWide(const SceneGPU& S, int cur, V3 o, V3 d, V3 inv, uint
             // sentinel reference: the leaf of primitive 0 alone is encoded as ~0 = -1)
             int next = 0;
             bool have = false;
-            if (t[0] != kInf) { next = n.child.x; have = true; }
-            if (t[1] != kInf) { if (!have) { next = n.child.y; have = true; } else stackRef[sp++] = n.child.y; }
-            if (t[2] != kInf) { if (!have) { next = n.child.z; have = true; } else stackRef[sp++] = n.child.z; }
-            if (t[3] != kInf) { if (!have) { next = n.child.w; have = true; } else stackRef[sp++] = n.child.w; }
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (t[k] != kInf) {
+                    if (!have) {
+                        next = wideRef(n.b[k]);
+                        have = true;
+                    } else {
+                        stackRef[sp++] = wideRef(n.b[k]);
+                    }
+                }
             if (!have) {
                 if (sp == 0) return false;
                 cur = stackRef[--sp];
@@ -844,7 +692,7 @@ __device__ bool walkAnyWide(const SceneGPU& S, int cur, V3 o, V3 d, V3 inv, uint
     }
 }
 
-template <bool COUNT, int AW = 0>
+template <bool COUNT>
 __device__ bool traceAnyWide(const SceneGPU& S, V3 o, V3 d, uint32_t mask, float tMin, float tMax, uint32_t& nodeVisits,
                              uint32_t& triTests, float time = 0.0f) {
     const V3 inv = mk(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
@@ -852,7 +700,7 @@ __device__ bool traceAnyWide(const SceneGPU& S, V3 o, V3 d, uint32_t mask, float
     if (S.nTris == 0) return false;
     if (!slab(S.rootMin[0], S.rootMax[0], S.rootMin[1], S.rootMax[1], S.rootMin[2], S.rootMax[2], o, inv, tMin, tMax, tn))
         return false;
-    return walkAnyWide<COUNT, 0, AW>(S, rootRef(S), o, d, inv, mask, tMin, tMax, nodeVisits, triTests, time);
+    return walkAnyWide<COUNT, 0>(S, rootRef(S), o, d, inv, mask, tMin, tMax, nodeVisits, triTests, time);
 }
 
 // Shutter time of the path in `slot` (Ray::time): read only where the scene has moving instances.

@@ -141,12 +141,13 @@ enum SdModeBits { SD_RECORD = 1, SD_SAMPLE = 2 };
 constexpr int kGuideTrainRows = 1 << 16;
 
 // One request's share of a wave: a rectangle of its film, a range of its sample indices and its
-// render settings.  Wave slots [slotFirst, slotFirst + nPix·nSamples) are its paths, sample-major
-// (slot = slotFirst + s·nPix + p), and its pixels are wave pixels [pixFirst, pixFirst + nPix).
+// render settings.  Wave slots [slotFirst, slotFirst + nPix·nSamples) are its paths, pixel by pixel
+// (slot = slotFirst + p·nSamples + s; neighbouring paths are samples of one pixel, then of the
+// pixels around it: tilePixel), and its pixels are wave pixels [pixFirst, pixFirst + nPix).
 struct WaveSeg {
     CamDev cam;
     int width, height;      // film
-    int tileX, tileY, tileW; // rendered rectangle of the film (whole frame: 0, 0, width)
+    int tileX, tileY, tileW, tileH; // rendered rectangle of the film (whole frame: 0, 0, width, height)
     const int32_t* pixList;  // film pixel (y·width + x) of each tile-linear pixel, or null: the rectangle
     int pixelFirst, nPix;   // range of tile-linear pixel indices in this wave
     int sampleFirst, nSamples;
@@ -182,6 +183,29 @@ struct Wave {
 };
 
 #ifdef __CUDACC__
+// Sample (of the segment's nSamples) of a wave path.
+__device__ __forceinline__ int sampleOfPath(const WaveSeg& A, int path) {
+    const int local = path - A.slotFirst;
+    return local - (local / A.nSamples) * A.nSamples;
+}
+__device__ __forceinline__ int pathOfSample(const WaveSeg& A, int p, int s) { return A.slotFirst + p * A.nSamples + s; }
+// Film position of the segment's tile-linear pixel tp.  The rectangle is numbered in bands of four
+// rows, down each band's columns, so that the 32 paths of a warp look at a compact patch of the film
+// (their camera rays meet the same nodes and their first hits the same surfaces).
+__device__ __forceinline__ void tilePixel(const WaveSeg& A, int tp, int& x, int& y) {
+    if (A.pixList) {
+        const int fp = A.pixList[tp];
+        x = fp % A.width;
+        y = fp / A.width;
+        return;
+    }
+    const int band = tp / (4 * A.tileW);
+    const int rows = A.tileH - 4 * band < 4 ? A.tileH - 4 * band : 4;
+    const int in = tp - band * 4 * A.tileW;
+    const int col = in / rows;
+    x = A.tileX + col;
+    y = A.tileY + 4 * band + (in - col * rows);
+}
 // Wave path index held by a slot.
 __device__ __forceinline__ int pathOfSlot(const Paths& P, int slot) { return P.pathOf ? P.pathOf[slot] : slot; }
 // Segment owning a wave path / a wave pixel (binary search; one segment for a lone request).
