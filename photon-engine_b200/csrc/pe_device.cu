@@ -972,7 +972,7 @@ int32_t renderAdaptive(pe_device* d, const pe_camera* cam, const pe_settings* st
 // WIDE: the traversal the render kernels use (4-wide tree); else the binary tree in the
 // reference's visiting order.
 template <bool WIDE>
-__global__ void kTracePrimary(SceneGPU S, WaveSeg A, int nPix, int32_t* outShape, int32_t* outPrim, float* outT) {
+__global__ void kTracePrimary(const __grid_constant__ SceneGPU S, const __grid_constant__ WaveSeg A, int nPix, int32_t* outShape, int32_t* outPrim, float* outT) {
     for (int pix = blockIdx.x * blockDim.x + threadIdx.x; pix < nPix; pix += gridDim.x * blockDim.x) {
         const int x = pix % A.width, y = pix / A.width;
         Sobol sb;
@@ -1008,7 +1008,7 @@ __global__ void kTracePrimary(SceneGPU S, WaveSeg A, int nPix, int32_t* outShape
 // Ray queries of pe_device_trace_rays: closest hit (binary tree in the reference's visiting
 // order, or the 4-wide tree) or any hit (4-wide), at a shutter time.
 template <int MODE>
-__global__ void kTraceRays(SceneGPU S, const float* o, const float* dir, const float* tMax, int n, uint32_t mask,
+__global__ void kTraceRays(const __grid_constant__ SceneGPU S, const float* o, const float* dir, const float* tMax, int n, uint32_t mask,
                            float time, int32_t* outShape, int32_t* outPrim, float* outT) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const V3 ro = mk(o[3 * i], o[3 * i + 1], o[3 * i + 2]), rd = mk(dir[3 * i], dir[3 * i + 1], dir[3 * i + 2]);
@@ -1056,7 +1056,7 @@ __global__ void kSobol(const TablesGPU* T, uint64_t seed, const int32_t* px, con
     }
 }
 
-__global__ void kBsdfProbe(SceneGPU S, int material, const pe_bsdf_query* q, int n, pe_bsdf_result* out) {
+__global__ void kBsdfProbe(const __grid_constant__ SceneGPU S, int material, const pe_bsdf_query* q, int n, pe_bsdf_result* out) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const MatGPU& m = S.materials[material];
         ShadePoint sp;

@@ -44,7 +44,7 @@ __device__ __forceinline__ void storeRow8(unsigned char* tile, int row, int k0, 
 // Queries: 3 float4 per row (position | shading normal | direction to the viewer).  Row r's 40
 // mixture outputs go to out[slot(r) · 10 ...] as 10 float4; mark[slot] = 1 tells the shading
 // kernel that this bounce's proposal is there.
-__global__ void __launch_bounds__(kTcRows) kGuideInferTC(GuideNet g, const float4* q, const int32_t* slots,
+__global__ void __launch_bounds__(kTcRows) kGuideInferTC(const __grid_constant__ GuideNet g, const float4* q, const int32_t* slots,
                                                          const uint32_t* count, int nFixed, float4* out, uint32_t* mark,
                                                          uint32_t* err) {
     extern __shared__ __align__(1024) unsigned char sm[];
@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(kTcRows) kGuideInferTC(GuideNet g, const float
     if (warp == 0) tmemDealloc(tmem, kTmemCols);
 }
 
-__global__ void kGuideInferSimt(GuideNet g, const float4* q, int n, float4* out) {
+__global__ void kGuideInferSimt(const __grid_constant__ GuideNet g, const float4* q, int n, float4* out) {
     for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < n; row += gridDim.x * blockDim.x) {
         const float4 a = q[3 * row], b = q[3 * row + 1], c = q[3 * row + 2];
         float x[kNetIn], h1[kNetHidden], h2[kNetHidden], h3[kNetHidden], o[kNetOut];
@@ -192,7 +192,7 @@ __device__ __forceinline__ void layerBackward(const float* W, float* gW, float* 
     __syncwarp();
 }
 
-__global__ void __launch_bounds__(kTrainWarps * 32) kGuideTrain(GuideNet g, const float4* samples, const uint32_t* count,
+__global__ void __launch_bounds__(kTrainWarps * 32) kGuideTrain(const __grid_constant__ GuideNet g, const float4* samples, const uint32_t* count,
                                                                 int nFixed, float* gradMlp, float* gradGrid, float* loss) {
     extern __shared__ float smf[];
     float* P = smf;                                  // kNetParams
@@ -273,7 +273,7 @@ __global__ void kGuideHalf(const float* p, __half* h, int n) {
 // ---- rendering: per-bounce queries and per-wave training samples -------------------------------
 // Query rows for the queued rays whose hit the next shading step may sample with the proposal:
 // surface hits (not random-walk steps) below the depth limit on guidable materials.
-__global__ void kGuideQuery(SceneGPU S, Paths P, Wave W, const int32_t* queue, const uint32_t* count) {
+__global__ void kGuideQuery(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P, const __grid_constant__ Wave W, const int32_t* queue, const uint32_t* count) {
     const int n = static_cast<int>(*count);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int slot = queue[i];
@@ -315,7 +315,7 @@ __global__ void kGuideQuery(SceneGPU S, Paths P, Wave W, const int32_t* queue, c
 // (point, normal, view direction, sampled direction ω, throughput before the bounce) and the
 // radiance the path had gathered before anything arrived along ω; what the path added since,
 // over that throughput, is f·cos·L(ω)/pdf for this one sample — the weight c of −c·log q(ω).
-__global__ void kGuideCollect(Paths P, int nSlots) {
+__global__ void kGuideCollect(const __grid_constant__ Paths P, int nSlots) {
     for (int s = (blockIdx.x * blockDim.x + threadIdx.x) * P.guideStride; s < nSlots;
          s += gridDim.x * blockDim.x * P.guideStride) {
         float4* rec = P.guideRec + static_cast<size_t>(s) * 6;

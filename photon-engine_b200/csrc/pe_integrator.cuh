@@ -150,7 +150,7 @@ __device__ __forceinline__ void flushPath(const Paths& P, const Wave& W, int slo
 }
 
 // The wave's first `count` paths into slots [0, count), all queued.
-static __global__ void kGenerate(SceneGPU S, Paths P, Wave W, int count) {
+static __global__ void kGenerate(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P, const __grid_constant__ Wave W, int count) {
     for (int slot = blockIdx.x * blockDim.x + threadIdx.x; slot < count; slot += gridDim.x * blockDim.x) {
         generatePath(S, P, W, slot, slot);
         P.queueA[slot] = slot;
@@ -160,7 +160,7 @@ static __global__ void kGenerate(SceneGPU S, Paths P, Wave W, int count) {
 // After a bounce of a regenerating wave: every slot freed this bounce hands its path's radiance
 // to Lout (its NEE terms are in by now), and the first `fresh` of them take the wave's paths
 // [nextPath, nextPath + fresh), appended to the next closest-hit queue after its `queued` entries.
-static __global__ void kRecycle(SceneGPU S, Paths P, Wave W, int freed, int fresh, int nextPath, int32_t* queue, int queued,
+static __global__ void kRecycle(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P, const __grid_constant__ Wave W, int freed, int fresh, int nextPath, int32_t* queue, int queued,
                          uint32_t* queueCount) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < freed; k += gridDim.x * blockDim.x) {
         const int slot = P.freeQ[k];
@@ -174,7 +174,7 @@ static __global__ void kRecycle(SceneGPU S, Paths P, Wave W, int freed, int fres
 }
 
 // The radiance of the paths the tail kernel finished, to Lout.
-static __global__ void kFlush(Paths P, Wave W, const int32_t* queue, const uint32_t* count) {
+static __global__ void kFlush(const __grid_constant__ Paths P, const __grid_constant__ Wave W, const int32_t* queue, const uint32_t* count) {
     const int n = static_cast<int>(*count);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) flushPath(P, W, queue[i]);
 }
@@ -183,12 +183,12 @@ static __global__ void kFlush(Paths P, Wave W, const int32_t* queue, const uint3
 // counters[CNT_FREE]).  kFlushFreed hands over the radiance of the `freed` slots pushed this
 // bounce, above `base`; kInject then pops `fresh` slots for the wave's paths [nextPath, +fresh),
 // appended to the next closest-hit queue after its `queued` entries.
-static __global__ void kFlushFreed(Paths P, Wave W, int base, int freed) {
+static __global__ void kFlushFreed(const __grid_constant__ Paths P, const __grid_constant__ Wave W, int base, int freed) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < freed; k += gridDim.x * blockDim.x)
         flushPath(P, W, P.freeQ[base + k]);
 }
 
-static __global__ void kInject(SceneGPU S, Paths P, Wave W, int top, int fresh, int nextPath, int32_t* queue, int queued,
+static __global__ void kInject(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P, const __grid_constant__ Wave W, int top, int fresh, int nextPath, int32_t* queue, int queued,
                         uint32_t* queueCount) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < fresh; k += gridDim.x * blockDim.x) {
         const int slot = P.freeQ[top - fresh + k];
@@ -203,13 +203,13 @@ static __global__ void kInject(SceneGPU S, Paths P, Wave W, int top, int fresh, 
 }
 
 // Slots of a finished sweep back onto the free stack, above `top`.
-static __global__ void kReturnSlots(Paths P, const int32_t* slots, int n, int top) {
+static __global__ void kReturnSlots(const __grid_constant__ Paths P, const int32_t* slots, int n, int top) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) P.freeQ[top + k] = slots[k];
     if (blockIdx.x == 0 && threadIdx.x == 0) P.counters[CNT_FREE] = static_cast<uint32_t>(top + n);
 }
 
 // Every slot free: the stack holds slots [0, n).
-static __global__ void kInitFree(Paths P, int n) {
+static __global__ void kInitFree(const __grid_constant__ Paths P, int n) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) P.freeQ[k] = k;
     if (blockIdx.x == 0 && threadIdx.x == 0) P.counters[CNT_FREE] = static_cast<uint32_t>(n);
 }
@@ -248,7 +248,7 @@ __device__ __forceinline__ int shadeKeyOfPrim(const SceneGPU& S, uint32_t rayMas
 // end of each ray's walk: rays end in any order, and bins in that order made the shading kernels'
 // state reads scatter (8.3 against 7.1 ms of shading per 8.3M-path knot wave); here a bin keeps the
 // queue's order but for the interleaving of warps.
-static __global__ void kBin(SceneGPU S, Paths P, const int32_t* queue, const uint32_t* count) {
+static __global__ void kBin(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P, const int32_t* queue, const uint32_t* count) {
     const int n = static_cast<int>(*count);
     const int stride = gridDim.x * blockDim.x;
     for (int base = blockIdx.x * blockDim.x; base < n; base += stride) {
@@ -265,7 +265,7 @@ static __global__ void kBin(SceneGPU S, Paths P, const int32_t* queue, const uin
 
 // The binary tree, a ray per lane.
 template <bool COUNT>
-__global__ void __launch_bounds__(128) kIntersectBinary(SceneGPU S, Paths P, const int32_t* queue, const uint32_t* count,
+__global__ void __launch_bounds__(128) kIntersectBinary(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P, const int32_t* queue, const uint32_t* count,
                                                         unsigned long long* stats) {
     const int n = static_cast<int>(*count);
     uint32_t nodes = 0, tris = 0;
@@ -320,7 +320,7 @@ struct WarpFeed {
 
 // The 4-wide tree, a ray per lane (walkTurn).
 template <bool COUNT>
-__global__ void __launch_bounds__(128, 8) kIntersect(SceneGPU S, Paths P, const int32_t* queue, const uint32_t* count,
+__global__ void __launch_bounds__(128, 8) kIntersect(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P, const int32_t* queue, const uint32_t* count,
                                                      unsigned long long* stats) {
     uint2 stack[kWalkStack];
     WarpFeed feed{&P.counters[CNT_WORK_ISECT], static_cast<int>(*count)};
@@ -471,7 +471,7 @@ __device__ __forceinline__ void addShadowTerm(const SceneGPU& S, const Paths& P,
 
 // Scenes with shadow-transmitting surfaces or shadow links: a ray per lane, the transmittance walk.
 template <bool COUNT>
-__global__ void __launch_bounds__(128) kShadow(SceneGPU S, Paths P, const uint32_t* count, unsigned long long* stats) {
+__global__ void __launch_bounds__(128) kShadow(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P, const uint32_t* count, unsigned long long* stats) {
     const int n = static_cast<int>(*count);
     uint32_t nodes = 0, tris = 0;
     for (;;) {
@@ -495,7 +495,7 @@ __global__ void __launch_bounds__(128) kShadow(SceneGPU S, Paths P, const uint32
 
 // Every other scene: the plain any-hit query, a ray per lane (walkTurn).
 template <bool COUNT>
-__global__ void __launch_bounds__(128, 8) kShadowAny(SceneGPU S, Paths P, const uint32_t* count, unsigned long long* stats) {
+__global__ void __launch_bounds__(128, 8) kShadowAny(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P, const uint32_t* count, unsigned long long* stats) {
     uint32_t stack[kWalkStack];
     WarpFeed feed{&P.counters[CNT_WORK_SHADOW], static_cast<int>(*count)};
     const int root = rootRef(S);
@@ -1368,7 +1368,7 @@ __device__ __forceinline__ bool shadeSlot(const SceneGPU& S, const Paths& P, con
 // INLINE: NEE shadow rays are traced here, each sample's term added in the sample loop's order
 // (waves with shadowQuality > 1, whose several records per vertex the shadow queue does not hold).
 template <bool OUT, bool INLINE = false>
-__global__ void __launch_bounds__(128, 6) kShade(SceneGPU S, Paths P, Wave W, int32_t* nextQueue, uint32_t* nextCount) {
+__global__ void __launch_bounds__(128, 6) kShade(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P, const __grid_constant__ Wave W, int32_t* nextQueue, uint32_t* nextCount) {
     uint32_t seg[kShadeKeys];
     int n = 0;
     for (int k = 0; k < kShadeKeys; ++k) {
@@ -1412,7 +1412,7 @@ __global__ void __launch_bounds__(128, 6) kShade(SceneGPU S, Paths P, Wave W, in
 // MINB: at least this many 128-thread blocks per SM (__launch_bounds__), i.e. a register budget
 // of 65536 / (128·MINB) per thread; 1 leaves the count to the compiler (pe_tuning::shade_budget).
 template <bool OUT, int KEY, int MINB = 1>
-__global__ void __launch_bounds__(128, MINB) kShadeKey(SceneGPU S, Paths P, Wave W, int32_t* nextQueue, uint32_t* nextCount) {
+__global__ void __launch_bounds__(128, MINB) kShadeKey(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P, const __grid_constant__ Wave W, int32_t* nextQueue, uint32_t* nextCount) {
     const int n = static_cast<int>(P.counters[CNT_KEYS + KEY]);
     const int32_t* bin = P.sortQ + static_cast<size_t>(KEY) * P.capacity;
     const int lane = threadIdx.x & 31;
@@ -1448,7 +1448,7 @@ __global__ void __launch_bounds__(128, MINB) kShadeKey(SceneGPU S, Paths P, Wave
 constexpr int kTailBlock = 32;
 
 template <bool COUNT, bool OUT>
-__global__ void __launch_bounds__(kTailBlock) kTail(SceneGPU S, Paths P, Wave W, const int32_t* queue, const uint32_t* count,
+__global__ void __launch_bounds__(kTailBlock) kTail(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P, const __grid_constant__ Wave W, const int32_t* queue, const uint32_t* count,
                                              uint32_t* cursor, unsigned long long* stats) {
     const int n = static_cast<int>(*count);
     uint32_t nodes = 0, tris = 0, shNodes = 0, shTris = 0, rays = 0, shRays = 0;
@@ -1492,7 +1492,7 @@ __global__ void __launch_bounds__(kTailBlock) kTail(SceneGPU S, Paths P, Wave W,
 // one.  Each path's queries and terms are kTail's, so the film is the same bit for bit.
 constexpr int kTailLockstepBlock = 128;
 template <bool LEAN>
-__global__ void __launch_bounds__(kTailLockstepBlock) kTailLockstep(SceneGPU S, Paths P, Wave W, const int32_t* queue,
+__global__ void __launch_bounds__(kTailLockstepBlock) kTailLockstep(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P, const __grid_constant__ Wave W, const int32_t* queue,
                                                                   const uint32_t* count, uint32_t* cursor,
                                                                   unsigned long long* stats) {
     const int n = static_cast<int>(*count);
@@ -1631,7 +1631,7 @@ static __device__ __noinline__ void filmPasses(const Paths& P, const WaveSeg& A,
     }
 }
 
-static __global__ void kFilm(Paths P, Wave W, unsigned long long* rejected) {
+static __global__ void kFilm(const __grid_constant__ Paths P, const __grid_constant__ Wave W, unsigned long long* rejected) {
     unsigned long long rej = 0;
     for (int wp = blockIdx.x * blockDim.x + threadIdx.x; wp < W.nPix; wp += gridDim.x * blockDim.x) {
         const WaveSeg& A = W.segs[segOfPixel(W, wp)];
@@ -1672,7 +1672,7 @@ static __global__ void kFilm(Paths P, Wave W, unsigned long long* rejected) {
 // ---- instantiations ---------------------------------------------------------------------------
 // The kernels below are compiled in translation units of their own (pe_kernels_*.cu), side by side;
 // PE_LEAN_KERNELS(K) and its siblings expand K(kernel) over a unit's instantiations.
-#define PE_SHADE_ARGS (SceneGPU, Paths, Wave, int32_t*, uint32_t*)
+#define PE_SHADE_ARGS (const __grid_constant__ SceneGPU, const __grid_constant__ Paths, const __grid_constant__ Wave, int32_t*, uint32_t*)
 #define PE_LEAN_KERNELS(K)                                                                         \
     K(kShadeKey<false, 0, 1>) K(kShadeKey<false, 1, 1>) K(kShadeKey<false, 2, 1>)                  \
     K(kShadeKey<false, 3, 1>) K(kShadeKey<false, 4, 1>) K(kShadeKey<false, 0, 4>)                  \
@@ -1684,13 +1684,13 @@ static __global__ void kFilm(Paths P, Wave W, unsigned long long* rejected) {
     K(kShadeKey<true, 3, 1>) K(kShadeKey<true, 4, 1>)
 #define PE_FULL_KERNELS(K)                                                                         \
     K(kShade<false, false>) K(kShade<true, false>) K(kShade<false, true>) K(kShade<true, true>)
-#define PE_TAIL_ARGS (SceneGPU, Paths, Wave, const int32_t*, const uint32_t*, uint32_t*, unsigned long long*)
+#define PE_TAIL_ARGS (const __grid_constant__ SceneGPU, const __grid_constant__ Paths, const __grid_constant__ Wave, const int32_t*, const uint32_t*, uint32_t*, unsigned long long*)
 #define PE_TAIL_KERNELS(K) K(kTail<false, true>) K(kTail<true, false>) K(kTail<true, true>)
 #define PE_LOCKSTEP_KERNELS(K) K(kTailLockstep<false>) K(kTailLockstep<true>)
-#define PE_TRACE_ARGS (SceneGPU, Paths, const int32_t*, const uint32_t*, unsigned long long*)
+#define PE_TRACE_ARGS (const __grid_constant__ SceneGPU, const __grid_constant__ Paths, const int32_t*, const uint32_t*, unsigned long long*)
 #define PE_TRACE_KERNELS(K)                                                                        \
     K(kIntersect<false>) K(kIntersect<true>) K(kIntersectBinary<false>) K(kIntersectBinary<true>)
-#define PE_SHADOW_ARGS (SceneGPU, Paths, const uint32_t*, unsigned long long*)
+#define PE_SHADOW_ARGS (const __grid_constant__ SceneGPU, const __grid_constant__ Paths, const uint32_t*, unsigned long long*)
 #define PE_SHADOW_KERNELS(K) K(kShadow<false>) K(kShadow<true>) K(kShadowAny<false>) K(kShadowAny<true>)
 
 } // namespace pe

@@ -20,7 +20,7 @@ namespace {
 // Incident radiance of each recorded vertex: what the path gathered after it, over its
 // throughput after the bounce, as luminance over the sampling pdf (the reference's
 // lum(suffix) / max(pdf, 1e-4)); splatted into the building quadtree of the vertex's leaf.
-__global__ void kSdRecord(Paths P, int nSlots) {
+__global__ void kSdRecord(const __grid_constant__ Paths P, int nSlots) {
     const SdField& F = P.sd;
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < nSlots; s += gridDim.x * blockDim.x) {
         const uint32_t n = P.sdCount[s];
