@@ -318,8 +318,10 @@ typedef struct pe_render_stats {
     uint64_t rejected;         /* non-finite / negative samples counted black */
     uint64_t waves;
     float ms_total;            /* device time of the last render call */
-    float ms_intersect;        /* device time in closest-hit traversal */
-    float ms_shadow;           /* device time in any-hit traversal */
+    float ms_intersect;        /* device time in ray traversal: closest hits, and the plain any-hit shadow
+                                  rays traced in the same launches */
+    float ms_shadow;           /* device time in shadow launches of their own (scenes with shadow
+                                  transmitters or shadow links, regenerating waves over moving instances) */
     float ms_shade;
     uint64_t intersect_launches;
     uint64_t node_visits;      /* closest-hit BVH node visits (counting enabled only) */
@@ -484,18 +486,16 @@ int64_t pe_device_tail_paths(pe_device* d);
 int32_t pe_device_autotune(pe_device* d, const pe_camera* cam, const pe_settings* st, int32_t probe_spp, int64_t* chosen);
 
 /* B200 tuning knobs with no counterpart in the reference engine; none changes a film.  The
- * autotuner above sets all five by coordinate descent on probe renders of the caller's frame
- * (paths in flight per wave, closest-hit traversal, any-hit traversal, the shading register
- * budget, the tail threshold). */
+ * autotuner above sets paths in flight per wave, the closest-hit traversal and the tail threshold
+ * by coordinate descent on probe renders of the caller's frame. */
 typedef struct pe_tuning {
     int64_t tail_paths;        /* as pe_device_set_tail_paths */
     int32_t closest_traversal; /* bounce-by-bounce closest hits: 0 the binary tree in the reference's
                                   order, a ray per lane; 1-9 (default 6) the 4-wide tree, four lanes
                                   per ray (one kernel: the numbers are kept for callers that stored
                                   one of the variants it replaced) */
-    int32_t shade_budget;      /* lean shading kernels: 0 the compiler's register count, 1 (default) at
-                                  most 128 registers a thread (four 128-thread blocks per SM), 2 at
-                                  most 96 (five blocks) */
+    int32_t shade_budget;      /* lean shading kernels: 0-2 (default 1), all at most 128 registers a
+                                  thread for surfaces (four 128-thread blocks per SM) */
     int32_t any_traversal;     /* plain any-hit shadows: 0-2 (default 2), all the four-lane walk */
     int64_t wave_slots;        /* paths in flight in a regenerating wave (unguided renders without
                                   AOV or pass targets): 2^20 … 2^23, default 2^23; 0 on input keeps

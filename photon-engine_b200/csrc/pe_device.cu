@@ -23,6 +23,9 @@ PE_LEAN_OUT_KERNELS(PE_EXTERN)
 #define PE_EXTERN(...) extern template __global__ void __VA_ARGS__ PE_SHADE_ARGS;
 PE_FULL_KERNELS(PE_EXTERN)
 #undef PE_EXTERN
+#define PE_EXTERN(...) extern template __global__ void __VA_ARGS__ PE_SHADE_ARGS;
+PE_FULL_OUT_KERNELS(PE_EXTERN)
+#undef PE_EXTERN
 #define PE_EXTERN(...) extern template __global__ void __VA_ARGS__ PE_TAIL_ARGS;
 PE_TAIL_KERNELS(PE_EXTERN)
 #undef PE_EXTERN
@@ -31,6 +34,9 @@ PE_LOCKSTEP_KERNELS(PE_EXTERN)
 #undef PE_EXTERN
 #define PE_EXTERN(...) extern template __global__ void __VA_ARGS__ PE_TRACE_ARGS;
 PE_TRACE_KERNELS(PE_EXTERN)
+#undef PE_EXTERN
+#define PE_EXTERN(...) extern template __global__ void __VA_ARGS__ PE_BINARY_ARGS;
+PE_BINARY_KERNELS(PE_EXTERN)
 #undef PE_EXTERN
 #define PE_EXTERN(...) extern template __global__ void __VA_ARGS__ PE_SHADOW_ARGS;
 PE_SHADOW_KERNELS(PE_EXTERN)
@@ -57,7 +63,9 @@ int32_t allocLane(WaveLane& ln, size_t slots) {
     float4** scols[] = {&P.shO, &P.shD, &P.shC, &P.shT};
     for (float4** c : scols)
         if ((st = devAlloc(ln.bufs, *c, slots))) return st;
-    if ((st = devAlloc(ln.bufs, P.counters, CNT_TOTAL))) return st;
+    uint32_t* counters = nullptr;
+    if ((st = devAlloc(ln.bufs, counters, kCounters))) return st;
+    setCounters(P, counters);
     if ((st = devAlloc(ln.bufs, P.cone, slots))) return st;
     if ((st = devAlloc(ln.bufs, P.time, slots))) return st;
     // path regeneration: slot → path, freed slots, radiance of kStreamFactor × slots paths
@@ -231,7 +239,9 @@ int32_t leanShadingOf(const SceneGPU& G, const std::vector<MatGPU>& mats) {
 constexpr size_t kNoAllocSlots = size_t(1) << 15;
 constexpr size_t kNoAllocColumn = kNoAllocSlots * sizeof(float4);   // 512 KiB, 256-aligned
 constexpr size_t kNoAllocIndex = kNoAllocSlots * sizeof(int32_t);    // 128 KiB, 256-aligned
-constexpr size_t kNoAllocBytes = 14 * kNoAllocColumn + (3 + kShadeKeys) * kNoAllocIndex + 256;
+constexpr size_t kNoAllocCounters = 512;                             // bytes
+static_assert(kCounters * sizeof(uint32_t) <= kNoAllocCounters, "the scratch holds every counter");
+constexpr size_t kNoAllocBytes = 14 * kNoAllocColumn + (3 + kShadeKeys) * kNoAllocIndex + kNoAllocCounters;
 static __device__ __align__(256) unsigned char g_noAllocScratch[kNoAllocBytes];
 
 // Path-state view of the scratch whose device address is `base`.
@@ -244,48 +254,21 @@ Paths noAllocPaths(unsigned char* base) {
     col(P.med);
     col(P.shO); col(P.shD); col(P.shC); col(P.shT);
     idx(P.queueA, 1); idx(P.queueB, 1); idx(P.shadowQ, 1); idx(P.sortQ, kShadeKeys);
-    P.counters = reinterpret_cast<uint32_t*>(base + off);
+    setCounters(P, reinterpret_cast<uint32_t*>(base + off));
     P.capacity = static_cast<uint32_t>(kNoAllocSlots);
     return P;
 }
 
-// The lean shading kernels of one bounce, one per shading key whose material type the scene
-// uses (the miss key always); returns the number of launches.
-int launchLeanShade(pe_device* d, const SceneGPU& S, const Paths& P, const Wave& W, int32_t* qOut, uint32_t* cOut,
-                    cudaStream_t cs, bool out) {
-    int n = 0;
-    const int budget = d->shadeBudget;
-    auto one = [&](auto kernel, int key) {
-        if (key > 0 && !(S.materialTypes & (1 << (key - 1)))) return;
-        kernel<<<d->blocksShadeKey[budget][key], 128, 0, cs>>>(S, P, W, qOut, cOut);
-        ++n;
-    };
-    if (!out && budget == 2) {
-        one(kShadeKey<false, 0, 5>, 0);
-        one(kShadeKey<false, 1, 5>, 1);
-        one(kShadeKey<false, 2, 5>, 2);
-        one(kShadeKey<false, 3, 5>, 3);
-        one(kShadeKey<false, 4, 5>, 4);
-    } else if (!out && budget == 1) {
-        one(kShadeKey<false, 0, 4>, 0);
-        one(kShadeKey<false, 1, 4>, 1);
-        one(kShadeKey<false, 2, 4>, 2);
-        one(kShadeKey<false, 3, 4>, 3);
-        one(kShadeKey<false, 4, 4>, 4);
-    } else if (out) {
-        one(kShadeKey<true, 0>, 0);
-        one(kShadeKey<true, 1>, 1);
-        one(kShadeKey<true, 2>, 2);
-        one(kShadeKey<true, 3>, 3);
-        one(kShadeKey<true, 4>, 4);
+// The lean shading kernels of one bounce; returns the number of launches.
+int launchLeanShade(pe_device* d, const SceneGPU& S, const Paths& P, const Wave& W, int32_t* qOut, cudaStream_t cs, bool out) {
+    if (out) {
+        kShadeMiss<true><<<d->blocksShadeMiss[1], 128, 0, cs>>>(S, P, W, qOut);
+        kShadeSurface<true><<<d->blocksShadeSurface[1], 128, 0, cs>>>(S, P, W, qOut);
     } else {
-        one(kShadeKey<false, 0>, 0);
-        one(kShadeKey<false, 1>, 1);
-        one(kShadeKey<false, 2>, 2);
-        one(kShadeKey<false, 3>, 3);
-        one(kShadeKey<false, 4>, 4);
+        kShadeMiss<false><<<d->blocksShadeMiss[0], 128, 0, cs>>>(S, P, W, qOut);
+        kShadeSurface<false><<<d->blocksShadeSurface[0], 128, 0, cs>>>(S, P, W, qOut);
     }
-    return n;
+    return 2;
 }
 
 int32_t timerEvent(pe_device* d, RenderTimer& tm, cudaEvent_t& e) {
@@ -366,43 +349,55 @@ int32_t segsWritable(pe_device* d, int lane) {
 
 // The tail in lockstep over `n` queued paths (count and cursor on the device).
 void launchTailLockstep(pe_device* d, bool lean, const SceneGPU& S, const Paths& P, const Wave& W, const int32_t* queue,
-                        const uint32_t* count, uint32_t* cursor, int64_t n, cudaStream_t cs) {
+                        const uint32_t* count, uint32_t* cursor, int64_t n, bool traced, cudaStream_t cs) {
     const int grid = static_cast<int>(std::max<int64_t>(
         1, std::min<int64_t>(d->blocksTailLockstep[lean ? 1 : 0], (n + kTailLockstepBlock - 1) / kTailLockstepBlock)));
-    if (lean) kTailLockstep<true><<<grid, kTailLockstepBlock, 0, cs>>>(S, P, W, queue, count, cursor, d->dStats);
-    else kTailLockstep<false><<<grid, kTailLockstepBlock, 0, cs>>>(S, P, W, queue, count, cursor, d->dStats);
+    if (lean) kTailLockstep<true><<<grid, kTailLockstepBlock, 0, cs>>>(S, P, W, queue, count, cursor, traced ? 1 : 0, d->dStats);
+    else kTailLockstep<false><<<grid, kTailLockstepBlock, 0, cs>>>(S, P, W, queue, count, cursor, traced ? 1 : 0, d->dStats);
 }
 
-// The closest-hit kernel over a queue (pe_tuning::closest_traversal 0: the binary tree).
-void launchClosest(pe_device* d, const SceneGPU& S, const Paths& P, const int32_t* q, const uint32_t* c, cudaStream_t cs) {
+// A bounce's ray queries: the closest hits of its queue, with `shadows` the any-hit queries of the
+// shadow records the bounce before left, then the hits binned by shading key.  Returns the launches.
+int launchTrace(pe_device* d, const SceneGPU& S, const Paths& P, const int32_t* q, bool shadows, cudaStream_t cs) {
     unsigned long long* st = d->dStats;
-    if (d->closestMode == TRACE_BINARY && d->counting)
-        kIntersectBinary<true><<<d->blocksIntersectBinary, 128, 0, cs>>>(S, P, q, c, st);
-    else if (d->closestMode == TRACE_BINARY)
-        kIntersectBinary<false><<<d->blocksIntersectBinary, 128, 0, cs>>>(S, P, q, c, st);
-    else if (d->counting)
-        kIntersect<true><<<d->blocksIntersect, 128, 0, cs>>>(S, P, q, c, st);
-    else
-        kIntersect<false><<<d->blocksIntersect, 128, 0, cs>>>(S, P, q, c, st);
-    kBin<<<d->prop.multiProcessorCount * 8, 256, 0, cs>>>(S, P, q, c);
+    int n = 2;
+    if (d->closestMode == TRACE_BINARY) {
+        if (d->counting) kIntersectBinary<true><<<d->blocksIntersectBinary, 128, 0, cs>>>(S, P, q, st);
+        else kIntersectBinary<false><<<d->blocksIntersectBinary, 128, 0, cs>>>(S, P, q, st);
+        if (shadows) {
+            ++n;
+            if (d->counting) kShadowAny<true><<<d->blocksShadowAny, 128, 0, cs>>>(S, P, st);
+            else kShadowAny<false><<<d->blocksShadowAny, 128, 0, cs>>>(S, P, st);
+        }
+    } else if (d->counting) {
+        kTrace<true><<<d->blocksIntersect, 128, 0, cs>>>(S, P, q, shadows ? 1 : 0, st);
+    } else {
+        kTrace<false><<<d->blocksIntersect, 128, 0, cs>>>(S, P, q, shadows ? 1 : 0, st);
+    }
+    kBin<<<d->prop.multiProcessorCount * 8, 256, 0, cs>>>(S, P, q);
+    return n;
 }
 
-// The shadow kernel of a scene over the wave's shadow records.
+// Shadow rays that a scene's closest hits need not wait with (launchTrace).
+bool plainShadows(const SceneGPU& S) { return !S.hasShadowTransmitters && !S.hasShadowLinks; }
+
+// The shadow rays of the records counted in P.now, in a launch of their own.
 void launchShadow(pe_device* d, const SceneGPU& S, const Paths& P, cudaStream_t cs) {
-    const uint32_t* n = &P.counters[CNT_SHADOW];
     unsigned long long* st = d->dStats;
-    const bool any = !S.hasShadowTransmitters && !S.hasShadowLinks;
-    if (any && d->counting) kShadowAny<true><<<d->blocksShadowAny, 128, 0, cs>>>(S, P, n, st);
-    else if (any) kShadowAny<false><<<d->blocksShadowAny, 128, 0, cs>>>(S, P, n, st);
-    else if (d->counting) kShadow<true><<<d->blocksShadow, 128, 0, cs>>>(S, P, n, st);
-    else kShadow<false><<<d->blocksShadow, 128, 0, cs>>>(S, P, n, st);
+    const bool any = plainShadows(S);
+    if (any && d->counting) kShadowAny<true><<<d->blocksShadowAny, 128, 0, cs>>>(S, P, st);
+    else if (any) kShadowAny<false><<<d->blocksShadowAny, 128, 0, cs>>>(S, P, st);
+    else if (d->counting) kShadow<true><<<d->blocksShadow, 128, 0, cs>>>(S, P, st);
+    else kShadow<false><<<d->blocksShadow, 128, 0, cs>>>(S, P, st);
 }
 
 // One wave on a lane over the nSegs segments in its segment table (nSlots paths, nPix film
-// pixels): uploads the table, generates the camera rays, traces them bounce by bounce (closest
-// hit → shade → any hit) until the live paths fit the tail kernel, which finishes them, and adds
-// every sample to its segment's film in sample order, after the previous wave's film kernel.
-// The host waits for each bounce's queue count, not for the tail or the film kernel.
+// pixels): uploads the table, generates the camera rays, traces them bounce by bounce (closest hits
+// and the shadow rays of the bounce before → shade) until the live paths fit the tail kernel, which
+// finishes them, and adds every sample to its segment's film in sample order, after the previous
+// wave's film kernel.  The host reads a bounce's counts while the next bounce's rays are traced, so
+// the device does not wait for it; only a wave that still has paths to start in freed slots waits
+// for the counts first.
 int32_t runWave(pe_device* d, int lane, Paths& P, int nSegs, int nSlots, int nPix, RenderTimer& tm) {
     WaveLane& ln = d->lanes[lane];
     const cudaStream_t cs = ln.stream;
@@ -451,120 +446,137 @@ int32_t runWave(pe_device* d, int lane, Paths& P, int nSegs, int nSlots, int nPi
     }
     const int firstPaths = static_cast<int>(std::min<int64_t>(nSlots, slotCap));
     int nextPath = firstPaths;
+    // shadow rays go with the next bounce's closest hits, unless a moving instance's shutter time
+    // would be gone with the slot by then
+    const bool movingRegen = regen && S.motions;
+    const bool lateShadows = plainShadows(S) && !movingRegen;
+    P.direct = regen && !movingRegen ? 1 : 0;
+    int block = 0;
+    setBlock(P, block);
+    PE_CUDA(cudaMemsetAsync(P.blocks, 0, kCounters * sizeof(uint32_t), cs));
     kGenerate<<<sm * 8, 256, 0, cs>>>(S, P, W, firstPaths);
     ++stats.kernel_launches;
     ++stats.waves;
     uint32_t live = static_cast<uint32_t>(firstPaths);
-    PE_CUDA(cudaMemsetAsync(&P.counters[1], 0, (CNT_TOTAL - 1) * sizeof(uint32_t), cs));
-    PE_CUDA(cudaMemcpyAsync(&P.counters[0], &live, sizeof(uint32_t), cudaMemcpyHostToDevice, cs));
     int32_t* qIn = P.queueA;
     int32_t* qOut = P.queueB;
-    uint32_t* cIn = &P.counters[0];
-    uint32_t* cOut = &P.counters[1];
     stats.paths += static_cast<uint64_t>(nSlots);
     // lean shading (one specialised kernel per shading key) for plain surface scenes that
-    // neither guide nor record; shadows without transmitters or shadow links are plain any-hits
+    // neither guide nor record
     bool noAo = true, inlineShadows = false;
     for (int k = 0; k < nSegs; ++k) {
         noAo = noAo && !(ln.hSegs[k].aoStrength > 0.0f);
         inlineShadows = inlineShadows || ln.hSegs[k].shadowSamples > 1;
     }
     const bool lean = S.leanShading && !P.guiding && !P.sdMode && noAo && !d->counting && !inlineShadows;
+    const bool out = P.aovA || P.pass;
     int64_t tailPaths = d->tailPaths < 0 ? static_cast<int64_t>(d->blocksTail) * kTailBlock : d->tailPaths;
     // the tail kernel runs no inference: keep guided bounces in the wavefront until few paths remain
     if (P.guiding == 2) tailPaths = std::min<int64_t>(tailPaths, kGuideTailPaths);
-    for (int iter = 0; live > 0; ++iter) {
-        if (static_cast<int64_t>(live) <= tailPaths && nextPath == nSlots) {
-            // the rest of the wave: one thread per path until it ends
-            const int grid = static_cast<int>(
-                std::min<int64_t>(d->blocksTail, (static_cast<int64_t>(live) + kTailBlock - 1) / kTailBlock));
-            cudaEvent_t t0 = nullptr, t1 = nullptr;
-            if (tm.timing) {
-                if ((rc = timerEvent(d, tm, t0)) || (rc = timerEvent(d, tm, t1))) return rc;
-                PE_CUDA(cudaEventRecord(t0, cs));
-            }
-            const bool out = P.aovA || P.pass;
-            if (lean && !d->counting && !out)
-                launchTailLockstep(d, true, S, P, W, qIn, cIn, &P.counters[CNT_WORK_TAIL], live, cs);
-            else if (d->counting && out)
-                kTail<true, true><<<grid, kTailBlock, 0, cs>>>(S, P, W, qIn, cIn, &P.counters[CNT_WORK_TAIL], d->dStats);
-            else if (d->counting)
-                kTail<true, false><<<grid, kTailBlock, 0, cs>>>(S, P, W, qIn, cIn, &P.counters[CNT_WORK_TAIL], d->dStats);
-            else if (out)
-                kTail<false, true><<<grid, kTailBlock, 0, cs>>>(S, P, W, qIn, cIn, &P.counters[CNT_WORK_TAIL], d->dStats);
-            else
-                launchTailLockstep(d, false, S, P, W, qIn, cIn, &P.counters[CNT_WORK_TAIL], live, cs);
-            if (tm.timing) {
-                PE_CUDA(cudaEventRecord(t1, cs));
-                tm.tail.push_back({tm.evUsed - 2, tm.evUsed - 1});
-            }
-            ++stats.kernel_launches;
-            stats.tail_paths += live;
-            if (regen) {
-                kFlush<<<sm * 4, 256, 0, cs>>>(P, W, qIn, cIn);
-                ++stats.kernel_launches;
-            }
-            break;
-        }
-        stats.closest_rays += live;
-        cudaEvent_t e0 = nullptr, e1 = nullptr, e2 = nullptr, e3 = nullptr;
-        if (tm.timing) {
-            if ((rc = timerEvent(d, tm, e0)) || (rc = timerEvent(d, tm, e1)) || (rc = timerEvent(d, tm, e2)) ||
-                (rc = timerEvent(d, tm, e3)))
-                return rc;
-            PE_CUDA(cudaEventRecord(e0, cs));
-        }
-        launchClosest(d, S, P, qIn, cIn, cs);
-        if (P.guiding == 2 && (rc = guideQueries(d, cs, P, W, qIn, cIn))) return rc;
-        if (tm.timing) PE_CUDA(cudaEventRecord(e1, cs));
-        if (lean)
-            stats.kernel_launches += launchLeanShade(d, S, P, W, qOut, cOut, cs, P.aovA || P.pass);
-        else if (inlineShadows && (P.aovA || P.pass))
-            kShade<true, true><<<d->blocksShade, 128, 0, cs>>>(S, P, W, qOut, cOut);
-        else if (inlineShadows)
-            kShade<false, true><<<d->blocksShade, 128, 0, cs>>>(S, P, W, qOut, cOut);
-        else if (P.aovA || P.pass)
-            kShade<true><<<d->blocksShade, 128, 0, cs>>>(S, P, W, qOut, cOut);
+    auto mark = [&](cudaEvent_t& e) -> int32_t {
+        if (!tm.timing) return PE_OK;
+        const int32_t r = timerEvent(d, tm, e);
+        if (r) return r;
+        PE_CUDA(cudaEventRecord(e, cs));
+        return PE_OK;
+    };
+    auto spent = [&](std::vector<std::pair<size_t, size_t>>& v) {
+        if (tm.timing) v.push_back({tm.evUsed - 2, tm.evUsed - 1});
+    };
+    // the rest of the wave: one thread per path until it ends
+    auto tail = [&](bool traced) -> int32_t {
+        const int grid = static_cast<int>(
+            std::min<int64_t>(d->blocksTail, (static_cast<int64_t>(live) + kTailBlock - 1) / kTailBlock));
+        uint32_t* count = &P.now[BC_QUEUE];
+        uint32_t* cursor = &P.counters[CNT_WORK_TAIL];
+        cudaEvent_t e = nullptr;
+        int32_t r = mark(e);
+        if (r) return r;
+        if (d->counting && out)
+            kTail<true, true><<<grid, kTailBlock, 0, cs>>>(S, P, W, qIn, count, cursor, traced ? 1 : 0, d->dStats);
+        else if (d->counting)
+            kTail<true, false><<<grid, kTailBlock, 0, cs>>>(S, P, W, qIn, count, cursor, traced ? 1 : 0, d->dStats);
+        else if (out)
+            kTail<false, true><<<grid, kTailBlock, 0, cs>>>(S, P, W, qIn, count, cursor, traced ? 1 : 0, d->dStats);
         else
-            kShade<false><<<d->blocksShade, 128, 0, cs>>>(S, P, W, qOut, cOut);
-        if (tm.timing) PE_CUDA(cudaEventRecord(e2, cs));
-        launchShadow(d, S, P, cs);
-        stats.kernel_launches += lean ? 3 : 4;
-        ++stats.intersect_launches;
-        if (tm.timing) {
-            PE_CUDA(cudaEventRecord(e3, cs));
-            tm.isect.push_back({tm.evUsed - 4, tm.evUsed - 3});
-            tm.shade.push_back({tm.evUsed - 3, tm.evUsed - 2});
-            tm.shadow.push_back({tm.evUsed - 2, tm.evUsed - 1});
+            launchTailLockstep(d, lean, S, P, W, qIn, count, cursor, live, traced, cs);
+        if ((r = mark(e))) return r;
+        spent(tm.tail);
+        ++stats.kernel_launches;
+        stats.tail_paths += live;
+        if (regen && !P.direct) {
+            kFlush<<<sm * 4, 256, 0, cs>>>(P, W, qIn, count);
+            ++stats.kernel_launches;
         }
-        PE_CUDA(cudaMemcpyAsync(ln.hCounters, P.counters, CNT_TOTAL * sizeof(uint32_t), cudaMemcpyDeviceToHost, cs));
-        PE_CUDA(cudaStreamSynchronize(cs));
-        stats.shadow_rays += ln.hCounters[CNT_SHADOW];
-        live = cOut == &P.counters[1] ? ln.hCounters[1] : ln.hCounters[0];
-        if (regen) {
-            // ended paths hand over their radiance; their slots take the wave's next paths
-            const int freed = static_cast<int>(ln.hCounters[CNT_FREE]);
+        return PE_OK;
+    };
+    if (static_cast<int64_t>(live) <= tailPaths && nextPath == nSlots) {
+        if ((rc = tail(false))) return rc;
+        live = 0;
+    }
+    bool counted = true;    // `live` is the count of the queue in hand
+    bool shadows = false;   // shadow rays of the bounce before wait for the next trace
+    for (int iter = 0; live > 0 || !counted; ++iter) {
+        cudaEvent_t e = nullptr;
+        auto readCounts = [&]() -> int32_t {
+            PE_CUDA(cudaEventSynchronize(ln.evCounts));
+            stats.shadow_rays += ln.hCounters[block * kBounceBlock + BC_SHADOW];
+            live = ln.hCounters[block * kBounceBlock + BC_QUEUE];
+            counted = true;
+            return PE_OK;
+        };
+        if (!counted && regen && nextPath < nSlots) {
+            // the slots of ended paths take the wave's next paths
+            if ((rc = readCounts())) return rc;
+            const int freed = static_cast<int>(ln.hCounters[2 * kBounceBlock + CNT_FREE]);
             const int fresh = std::min(freed, nSlots - nextPath);
             if (freed > 0) {
-                kRecycle<<<sm * 4, 256, 0, cs>>>(S, P, W, freed, fresh, nextPath, qOut, static_cast<int>(live), cOut);
+                kRecycle<<<sm * 4, 256, 0, cs>>>(S, P, W, freed, fresh, nextPath, qIn, static_cast<int>(live),
+                                                 &P.now[BC_QUEUE]);
                 ++stats.kernel_launches;
                 PE_CUDA(cudaMemsetAsync(&P.counters[CNT_FREE], 0, sizeof(uint32_t), cs));
             }
             nextPath += fresh;
             live += static_cast<uint32_t>(fresh);
         }
+        if ((rc = mark(e))) return rc;
+        stats.kernel_launches += launchTrace(d, S, P, qIn, shadows, cs);
+        if (P.guiding == 2 && (rc = guideQueries(d, cs, P, W, qIn, &P.now[BC_QUEUE]))) return rc;
+        if ((rc = mark(e))) return rc;
+        spent(tm.isect);
+        if (!counted && (rc = readCounts())) return rc;
+        if (live == 0) break;
+        stats.closest_rays += live;
+        ++stats.intersect_launches;
+        if (iter > 0 && static_cast<int64_t>(live) <= tailPaths && nextPath == nSlots) {
+            if ((rc = tail(true))) return rc;
+            break;
+        }
+        if (lean) stats.kernel_launches += launchLeanShade(d, S, P, W, qOut, cs, out);
+        else if (inlineShadows && out) kShade<true, true><<<d->blocksShade, 128, 0, cs>>>(S, P, W, qOut);
+        else if (inlineShadows) kShade<false, true><<<d->blocksShade, 128, 0, cs>>>(S, P, W, qOut);
+        else if (out) kShade<true, false><<<d->blocksShade, 128, 0, cs>>>(S, P, W, qOut);
+        else kShade<false, false><<<d->blocksShade, 128, 0, cs>>>(S, P, W, qOut);
+        if (!lean) ++stats.kernel_launches;
+        if ((rc = mark(e))) return rc;
+        spent(tm.shade);
+        block = 1 - block;
+        setBlock(P, block);
+        std::swap(qIn, qOut);
+        if (!lateShadows) {
+            launchShadow(d, S, P, cs);
+            ++stats.kernel_launches;
+            if ((rc = mark(e))) return rc;
+            spent(tm.shadow);
+        }
+        shadows = lateShadows;
+        PE_CUDA(cudaMemcpyAsync(ln.hCounters, P.blocks, kCounters * sizeof(uint32_t), cudaMemcpyDeviceToHost, cs));
+        PE_CUDA(cudaEventRecord(ln.evCounts, cs));
+        counted = false;
         if (iter > kMaxWavefrontIterations * (regen ? kStreamFactor + 1 : 1)) {
             setError("wavefront did not drain after " + std::to_string(kMaxWavefrontIterations) + " iterations");
             return PE_ERR_DEVICE;
         }
-        // swap queues; reset the consumed queue's counter, the shadow counter, the work
-        // cursors and the shading-key bins
-        PE_CUDA(cudaMemsetAsync(cIn, 0, sizeof(uint32_t), cs));
-        PE_CUDA(cudaMemsetAsync(&P.counters[CNT_SHADOW], 0, (CNT_KEYS + kShadeKeys - CNT_SHADOW) * sizeof(uint32_t),
-                                cs));
-        if (lean) PE_CUDA(cudaMemsetAsync(&P.counters[CNT_WORK_KEYS], 0, kShadeKeys * sizeof(uint32_t), cs));
-        std::swap(qIn, qOut);
-        std::swap(cIn, cOut);
     }
     // films accumulate in wave order: after the other lane's last film kernel
     if (d->filmLane >= 0 && d->filmLane != lane) PE_CUDA(cudaStreamWaitEvent(cs, d->evFilm, 0));
@@ -608,14 +620,15 @@ int32_t loopBegin(pe_device* d, LaneLoop& L, uint32_t* segLeft) {
     L.sweeping = 0;
     L.qIn = P.queueA;
     L.qOut = P.queueB;
-    L.cIn = &P.counters[0];
-    L.cOut = &P.counters[1];
+    L.block = 0;
+    setBlock(P, 0);
+    P.direct = 0;
     L.live = 0;
     L.freeTop = static_cast<int>(P.capacity);
     L.nextPath = 0;
     L.pathCap = static_cast<int>(static_cast<int64_t>(P.capacity) * kStreamFactor);
     L.iter = 0;
-    PE_CUDA(cudaMemsetAsync(P.counters, 0, CNT_TOTAL * sizeof(uint32_t), cs));
+    PE_CUDA(cudaMemsetAsync(P.blocks, 0, kCounters * sizeof(uint32_t), cs));
     kInitFree<<<d->prop.multiProcessorCount * 4, 256, 0, cs>>>(P, static_cast<int>(P.capacity));
     PE_CUDA(cudaGetLastError());
     return PE_OK;
@@ -627,7 +640,7 @@ int32_t loopInject(pe_device* d, LaneLoop& L, const Wave& W, int fresh) {
     Paths& P = ln.paths;
     P.iter = L.iter;
     kInject<<<d->prop.multiProcessorCount * 4, 256, 0, ln.stream>>>(L.scene, P, W, L.freeTop, fresh, L.nextPath, L.qIn,
-                                                                    static_cast<int>(L.live), L.cIn);
+                                                                    static_cast<int>(L.live), &P.now[BC_QUEUE]);
     PE_CUDA(cudaGetLastError());
     L.freeTop -= fresh;
     L.nextPath += fresh;
@@ -649,26 +662,30 @@ int32_t loopBounce(pe_device* d, LaneLoop& L, const Wave& W, uint32_t* hSegLeft,
     P.sweepAge = sweep >= 0 ? L.sweepAge : 0;
     P.sweepQ = sweep >= 0 ? L.sweepBuf[sweep] : nullptr;
     P.iter = L.iter;
-    // the closest-hit and any-hit kernels a lone render uses
-    launchClosest(d, S, P, L.qIn, L.cIn, cs);
-    // lean-shading scenes shade with the per-key kernels, as a lone render does
-    if (L.lean) launchLeanShade(d, S, P, W, L.qOut, L.cOut, cs, false);
-    else kShade<false><<<d->blocksShade, 128, 0, cs>>>(S, P, W, L.qOut, L.cOut);
+    // the kernels a lone render uses; shadow rays before the bounce's end, as the slots of ended
+    // paths are handed on then
+    launchTrace(d, S, P, L.qIn, false, cs);
+    if (L.lean) launchLeanShade(d, S, P, W, L.qOut, cs, false);
+    else kShade<false, false><<<d->blocksShade, 128, 0, cs>>>(S, P, W, L.qOut);
+    L.block = 1 - L.block;
+    setBlock(P, L.block);
+    std::swap(L.qIn, L.qOut);
     launchShadow(d, S, P, cs);
-    PE_CUDA(cudaMemcpyAsync(ln.hCounters, P.counters, CNT_TOTAL * sizeof(uint32_t), cudaMemcpyDeviceToHost, cs));
+    PE_CUDA(cudaMemcpyAsync(ln.hCounters, P.blocks, kCounters * sizeof(uint32_t), cudaMemcpyDeviceToHost, cs));
     // segment counts as of the previous bounce's flushes (one bounce behind)
     if (segCount > 0)
         PE_CUDA(cudaMemcpyAsync(hSegLeft + segFirst, dSegLeft + segFirst, static_cast<size_t>(segCount) * sizeof(uint32_t),
                                 cudaMemcpyDeviceToHost, cs));
     PE_CUDA(cudaStreamSynchronize(cs));
-    L.live = L.cOut == &P.counters[1] ? ln.hCounters[1] : ln.hCounters[0];
-    const int top = static_cast<int>(ln.hCounters[CNT_FREE]);
+    const uint32_t* waveCounters = ln.hCounters + 2 * kBounceBlock;
+    L.live = ln.hCounters[L.block * kBounceBlock + BC_QUEUE];
+    const int top = static_cast<int>(waveCounters[CNT_FREE]);
     const int freed = top - L.freeTop;
     if (freed > 0) {
         kFlushFreed<<<d->prop.multiProcessorCount * 4, 256, 0, cs>>>(P, W, L.freeTop, freed);
     }
     L.freeTop = top;
-    const int swept = static_cast<int>(ln.hCounters[CNT_SWEEP]);
+    const int swept = static_cast<int>(waveCounters[CNT_SWEEP]);
     if (sweep >= 0 && swept > 0) {
         // the swept paths run to their end on the side stream, then hand over their radiance
         PE_CUDA(cudaMemcpyAsync(&L.sweepCnt[sweep], &P.counters[CNT_SWEEP], sizeof(uint32_t), cudaMemcpyDeviceToDevice, cs));
@@ -677,17 +694,12 @@ int32_t loopBounce(pe_device* d, LaneLoop& L, const Wave& W, uint32_t* hSegLeft,
         PE_CUDA(cudaStreamWaitEvent(L.side, L.evReady[sweep], 0));
         PE_CUDA(cudaMemsetAsync(&L.sweepCursor[sweep], 0, sizeof(uint32_t), L.side));
         launchTailLockstep(d, L.lean, S, P, W, L.sweepBuf[sweep], &L.sweepCnt[sweep], &L.sweepCursor[sweep],
-                           static_cast<int64_t>(swept), L.side);
+                           static_cast<int64_t>(swept), false, L.side);
         kFlush<<<d->prop.multiProcessorCount * 4, 256, 0, L.side>>>(P, W, L.sweepBuf[sweep], &L.sweepCnt[sweep]);
         PE_CUDA(cudaEventRecord(L.evDone[sweep], L.side));
         L.sweepN[sweep] = swept;
         L.sweeping += swept;
     }
-    PE_CUDA(cudaMemsetAsync(L.cIn, 0, sizeof(uint32_t), cs));
-    PE_CUDA(cudaMemsetAsync(&P.counters[CNT_SHADOW], 0, (CNT_KEYS + kShadeKeys - CNT_SHADOW) * sizeof(uint32_t), cs));
-    if (L.lean) PE_CUDA(cudaMemsetAsync(&P.counters[CNT_WORK_KEYS], 0, kShadeKeys * sizeof(uint32_t), cs));
-    std::swap(L.qIn, L.qOut);
-    std::swap(L.cIn, L.cOut);
     if (++L.iter > kMaxWavefrontIterations * 64) {
         setError("continuous wave exceeded its bounce bound");
         return PE_ERR_DEVICE;
@@ -701,8 +713,9 @@ int32_t loopTail(pe_device* d, LaneLoop& L, const Wave& W) {
     WaveLane& ln = *L.ln;
     Paths& P = ln.paths;
     const cudaStream_t cs = ln.stream;
-    launchTailLockstep(d, L.lean, L.scene, P, W, L.qIn, L.cIn, &P.counters[CNT_WORK_TAIL], static_cast<int64_t>(L.live), cs);
-    kFlush<<<d->prop.multiProcessorCount * 4, 256, 0, cs>>>(P, W, L.qIn, L.cIn);
+    launchTailLockstep(d, L.lean, L.scene, P, W, L.qIn, &P.now[BC_QUEUE], &P.counters[CNT_WORK_TAIL],
+                       static_cast<int64_t>(L.live), false, cs);
+    kFlush<<<d->prop.multiProcessorCount * 4, 256, 0, cs>>>(P, W, L.qIn, &P.now[BC_QUEUE]);
     L.live = 0;
     PE_CUDA(cudaGetLastError());
     return PE_OK;
@@ -1278,7 +1291,8 @@ pe_device* pe_device_create(int32_t ordinal, char* err, size_t errLen) {
                 cudaSuccess ||
             cudaMalloc(&ln.dSegs, kMaxSegs * sizeof(WaveSeg)) != cudaSuccess ||
             cudaMallocHost(&ln.hSegs, kMaxSegs * sizeof(WaveSeg)) != cudaSuccess ||
-            cudaMallocHost(&ln.hCounters, 32 * sizeof(uint32_t)) != cudaSuccess ||
+            cudaMallocHost(&ln.hCounters, kCounters * sizeof(uint32_t)) != cudaSuccess ||
+            cudaEventCreateWithFlags(&ln.evCounts, cudaEventDisableTiming) != cudaSuccess ||
             cudaEventCreateWithFlags(&ln.evSegs, cudaEventDisableTiming) != cudaSuccess ||
             cudaEventCreate(&ln.evDone) != cudaSuccess) {
             pe_device_destroy(d);
@@ -1289,9 +1303,9 @@ pe_device* pe_device_create(int32_t ordinal, char* err, size_t errLen) {
     cudaMemcpy(d->dTables, &d->hTables, sizeof(TablesGPU), cudaMemcpyHostToDevice);
     int b = 0;
     const int sm = d->prop.multiProcessorCount;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kIntersect<false>, 128, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kTrace<false>, 128, 0);
     d->blocksIntersect = sm * std::max(1, b);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kShade<false>, 128, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kShade<false, false>, 128, 0);
     d->blocksShade = sm * std::max(1, b);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kShadow<false>, 128, 0);
     d->blocksShadow = sm * std::max(1, b);
@@ -1306,21 +1320,10 @@ pe_device* pe_device_create(int32_t ordinal, char* err, size_t errLen) {
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, threads, 0);
         return sm * std::max(1, nb);
     };
-    d->blocksShadeKey[0][0] = occ(kShadeKey<false, 0>, 128);
-    d->blocksShadeKey[0][1] = occ(kShadeKey<false, 1>, 128);
-    d->blocksShadeKey[0][2] = occ(kShadeKey<false, 2>, 128);
-    d->blocksShadeKey[0][3] = occ(kShadeKey<false, 3>, 128);
-    d->blocksShadeKey[0][4] = occ(kShadeKey<false, 4>, 128);
-    d->blocksShadeKey[1][0] = occ(kShadeKey<false, 0, 4>, 128);
-    d->blocksShadeKey[1][1] = occ(kShadeKey<false, 1, 4>, 128);
-    d->blocksShadeKey[1][2] = occ(kShadeKey<false, 2, 4>, 128);
-    d->blocksShadeKey[1][3] = occ(kShadeKey<false, 3, 4>, 128);
-    d->blocksShadeKey[1][4] = occ(kShadeKey<false, 4, 4>, 128);
-    d->blocksShadeKey[2][0] = occ(kShadeKey<false, 0, 5>, 128);
-    d->blocksShadeKey[2][1] = occ(kShadeKey<false, 1, 5>, 128);
-    d->blocksShadeKey[2][2] = occ(kShadeKey<false, 2, 5>, 128);
-    d->blocksShadeKey[2][3] = occ(kShadeKey<false, 3, 5>, 128);
-    d->blocksShadeKey[2][4] = occ(kShadeKey<false, 4, 5>, 128);
+    d->blocksShadeMiss[0] = occ(kShadeMiss<false>, 128);
+    d->blocksShadeMiss[1] = occ(kShadeMiss<true>, 128);
+    d->blocksShadeSurface[0] = occ(kShadeSurface<false>, 128);
+    d->blocksShadeSurface[1] = occ(kShadeSurface<true>, 128);
     d->blocksIntersectBinary = occ(kIntersectBinary<false>, 128);
     d->blocksShadowAny = occ(kShadowAny<false>, 128);
     const cudaError_t le = cudaGetLastError();
@@ -1354,6 +1357,7 @@ void pe_device_destroy(pe_device* d) {
         if (ln.hSegs) cudaFreeHost(ln.hSegs);
         if (ln.hCounters) cudaFreeHost(ln.hCounters);
         if (ln.evSegs) cudaEventDestroy(ln.evSegs);
+        if (ln.evCounts) cudaEventDestroy(ln.evCounts);
         if (ln.evDone) cudaEventDestroy(ln.evDone);
         if (l == 1 && ln.stream) cudaStreamDestroy(ln.stream);
     }
@@ -1980,7 +1984,7 @@ int32_t pe_device_render_tile_noalloc(pe_device* d, const pe_camera* cam, const 
     if (count <= 0) return PE_OK;
     Paths P = noAllocPaths(d->noAllocBase);
     // The array keeps the previous call's contents; the queue and shadow counters must start at 0.
-    PE_CUDA(cudaMemsetAsync(P.counters, 0, 256, d->stream));
+    PE_CUDA(cudaMemsetAsync(P.blocks, 0, kNoAllocCounters, d->stream));
     return renderWaves(d, cam, st, first, count, nullptr, sumRgb, sampleCount, sumLumSq, &P, kNoAllocSlots, false,
                        Tile{x0, y0, w, h});
 }
@@ -2075,7 +2079,6 @@ int32_t pe_device_autotune(pe_device* d, const pe_camera* cam, const pe_settings
          },
          {static_cast<int64_t>(kWaveSlots), static_cast<int64_t>(kDefaultWaveSlots), static_cast<int64_t>(kMaxWaveSlots)});
     tune("closest_traversal", [&](int64_t v) { d->closestMode = static_cast<int>(v); }, {d->closestMode, TRACE_BINARY});
-    tune("shade_budget", [&](int64_t v) { d->shadeBudget = static_cast<int>(v); }, {0, 1, 2});
     const int64_t grid = static_cast<int64_t>(d->blocksTail) * kTailBlock;
     tune("tail_paths", [&](int64_t v) { d->tailPaths = v; }, {grid / 4, grid / 2, grid, 2 * grid});
     d->guideKind = savedKind;

@@ -67,7 +67,8 @@ struct WaveLane {
     WaveSeg* dSegs = nullptr;
     cudaEvent_t evSegs = nullptr;     // the segment upload of the lane's last wave
     bool segsInFlight = false;
-    uint32_t* hCounters = nullptr;    // pinned
+    uint32_t* hCounters = nullptr;    // pinned: the lane's counters (kCounters) after its last shading
+    cudaEvent_t evCounts = nullptr;   // ... once that copy has landed
     float4* aovA = nullptr;           // AOVs per slot (allocated on first use, in aovBufs)
     float4* aovN = nullptr;
     std::vector<DevBuf> aovBufs;
@@ -207,7 +208,7 @@ struct pe_device {
     bool counting = false;
     pe_render_stats stats{};
     int blocksIntersect = 0, blocksShade = 0, blocksShadow = 0, blocksGen = 0, blocksTail = 0;
-    int blocksShadeKey[3][5] = {}; // lean shading kernels: [budget][key]
+    int blocksShadeMiss[2] = {}, blocksShadeSurface[2] = {}; // lean shading: [recording AOVs or passes]
     int blocksShadowAny = 0;
     int blocksTailLockstep[2] = {}; // kTailLockstep<LEAN>: [0] full, [1] lean shading; 128-thread blocks
     int blocksIntersectBinary = 0;
@@ -216,7 +217,7 @@ struct pe_device {
     int anyMode = 2;               // pe_tuning::any_traversal (every value the one any-hit kernel)
     // tuning (pe_tuning): closest-hit traversal variant, register budget of the lean shading kernels
     int closestMode = 6;  // pe_tuning::closest_traversal (TraceMode: 0 the binary tree, else the 4-wide one)
-    int shadeBudget = 1;  // 0 the compiler's register count, 1 (default) at most 128 registers (4 blocks per SM)
+    int shadeBudget = 1;  // pe_tuning::shade_budget (every value the 128-register kernels)
     std::string tuneLog;  // the last autotune's probe times
     int64_t tailPaths = -1; // -1: one resident grid of the tail kernel; 0: no tail kernel
     unsigned char* noAllocBase = nullptr; // device address of g_noAllocScratch on this device
@@ -294,8 +295,7 @@ struct LaneLoop {
     SceneGPU scene{};   // the wave's scene (each lane may trace its own)
     int32_t* qIn = nullptr;
     int32_t* qOut = nullptr;
-    uint32_t* cIn = nullptr;
-    uint32_t* cOut = nullptr;
+    int block = 0;      // bounce block of the next closest-hit queue
     uint32_t live = 0;  // paths in the next closest-hit queue
     bool lean = false;  // the lean per-key shading kernels (a lean-shading scene, no segment with AO)
     int freeTop = 0;    // free slots on the stack

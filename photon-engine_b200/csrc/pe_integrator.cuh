@@ -155,16 +155,18 @@ static __global__ void kGenerate(const __grid_constant__ SceneGPU S, const __gri
         generatePath(S, P, W, slot, slot);
         P.queueA[slot] = slot;
     }
+    if (blockIdx.x == 0 && threadIdx.x == 0) P.now[BC_QUEUE] = static_cast<uint32_t>(count);
 }
 
 // After a bounce of a regenerating wave: every slot freed this bounce hands its path's radiance
-// to Lout (its NEE terms are in by now), and the first `fresh` of them take the wave's paths
-// [nextPath, nextPath + fresh), appended to the next closest-hit queue after its `queued` entries.
+// to Lout (its NEE terms are in by now; in direct waves it did so when it ended), and the first
+// `fresh` of them take the wave's paths [nextPath, nextPath + fresh), appended to the next
+// closest-hit queue after its `queued` entries.
 static __global__ void kRecycle(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P, const __grid_constant__ Wave W, int freed, int fresh, int nextPath, int32_t* queue, int queued,
                          uint32_t* queueCount) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < freed; k += gridDim.x * blockDim.x) {
         const int slot = P.freeQ[k];
-        flushPath(P, W, slot);
+        if (!P.direct) flushPath(P, W, slot);
         if (k < fresh) {
             generatePath(S, P, W, slot, nextPath + k);
             queue[queued + k] = slot;
@@ -230,7 +232,7 @@ __device__ __forceinline__ void binByKey(const Paths& P, int key, int slot) {
         const int leader = __ffs(peers) - 1;
         const int rank = __popc(peers & ((1u << lane) - 1u));
         uint32_t at = 0;
-        if (lane == leader) at = atomicAdd(&P.counters[CNT_KEYS + key], static_cast<uint32_t>(__popc(peers)));
+        if (lane == leader) at = atomicAdd(&P.now[BC_KEYS + key], static_cast<uint32_t>(__popc(peers)));
         at = __shfl_sync(peers, at, leader);
         P.sortQ[static_cast<size_t>(key) * P.capacity + at + rank] = slot;
     }
@@ -248,9 +250,10 @@ __device__ __forceinline__ int shadeKeyOfPrim(const SceneGPU& S, uint32_t rayMas
 // end of each ray's walk: rays end in any order, and bins in that order made the shading kernels'
 // state reads scatter (8.3 against 7.1 ms of shading per 8.3M-path knot wave); here a bin keeps the
 // queue's order but for the interleaving of warps.
-static __global__ void kBin(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P, const int32_t* queue, const uint32_t* count) {
-    const int n = static_cast<int>(*count);
+static __global__ void kBin(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P, const int32_t* queue) {
+    const int n = static_cast<int>(P.now[BC_QUEUE]);
     const int stride = gridDim.x * blockDim.x;
+    if (blockIdx.x == 0 && threadIdx.x < kBounceBlock) P.next[threadIdx.x] = 0u; // the next bounce's counters
     for (int base = blockIdx.x * blockDim.x; base < n; base += stride) {
         const int i = base + static_cast<int>(threadIdx.x);
         int key = -1, slot = -1;
@@ -265,12 +268,12 @@ static __global__ void kBin(const __grid_constant__ SceneGPU S, const __grid_con
 
 // The binary tree, a ray per lane.
 template <bool COUNT>
-__global__ void __launch_bounds__(128) kIntersectBinary(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P, const int32_t* queue, const uint32_t* count,
+__global__ void __launch_bounds__(128) kIntersectBinary(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P, const int32_t* queue,
                                                         unsigned long long* stats) {
-    const int n = static_cast<int>(*count);
+    const int n = static_cast<int>(P.now[BC_QUEUE]);
     uint32_t nodes = 0, tris = 0;
     for (;;) {
-        const int base = warpFetch(&P.counters[CNT_WORK_ISECT]);
+        const int base = warpFetch(&P.now[BC_WORK_ISECT]);
         if (base >= n) break;
         const int i = base + (threadIdx.x & 31);
         if (i >= n) continue;
@@ -317,53 +320,6 @@ struct WarpFeed {
     }
     __device__ __forceinline__ bool dry() const { return end < 0; }
 };
-
-// The 4-wide tree, a ray per lane (walkTurn).
-template <bool COUNT>
-__global__ void __launch_bounds__(128, 8) kIntersect(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P, const int32_t* queue, const uint32_t* count,
-                                                     unsigned long long* stats) {
-    uint2 stack[kWalkStack];
-    WarpFeed feed{&P.counters[CNT_WORK_ISECT], static_cast<int>(*count)};
-    const int root = rootRef(S);
-    const bool instances = S.nInstances > 0;
-    uint32_t nodes = 0, tris = 0;
-    int slot = -1;
-    RayWalk w;
-    w.cur = kRayDone;
-    for (;;) {
-        const unsigned idle = __ballot_sync(kWarp, w.cur == kRayDone);
-        if (idle == kWarp || (!feed.dry() && __popc(idle) >= kRefill)) {
-            // ended rays: their hits; then the queue's next rays
-            if (w.cur == kRayDone && slot >= 0) {
-                P.hit[slot] = make_float4(w.tMax, w.u, w.v, __int_as_float(w.prim));
-                slot = -1;
-            }
-            const int i = feed.next(w.cur == kRayDone);
-            if (i >= 0) {
-                slot = queue[i];
-                const float4 ro = P.rayO[slot];
-                const float4 rd = P.rayD[slot];
-                w.start(S, root, mk(ro.x, ro.y, ro.z), mk(rd.x, rd.y, rd.z), __float_as_uint(ro.w), 1e30f, -1);
-            }
-            if (__all_sync(kWarp, slot < 0)) break;
-            continue;
-        }
-        walkTurn<false, COUNT>(
-            S, w, stack, instances, nodes, tris,
-            [&](V3& o, V3& d, uint32_t& mask) {
-                const float4 ro = P.rayO[slot], rd = P.rayD[slot];
-                o = mk(ro.x, ro.y, ro.z);
-                d = mk(rd.x, rd.y, rd.z);
-                mask = __float_as_uint(ro.w);
-            },
-            [&]() { return pathTime(S, P, slot); });
-        __syncwarp();
-    }
-    if (COUNT) {
-        atomicAdd(&stats[0], static_cast<unsigned long long>(nodes));
-        atomicAdd(&stats[1], static_cast<unsigned long long>(tris));
-    }
-}
 
 // Surface coverage of a hit for a ray that may pass through cutouts (DisneyMaterial::opacity,
 // disney.cpp:505-509: the opacity times the opacity map's red channel, a level-0 lookup).
@@ -453,15 +409,16 @@ __device__ __forceinline__ V3 neeTerm(V3 fLi, V3 vis, float scalar, V3 thr, bool
 // ---- any hit over the shadow queue ------------------------------------------------------------
 // Shadow record i's visibility, found, into its path's radiance.
 __device__ __forceinline__ void addShadowTerm(const SceneGPU& S, const Paths& P, int i, int slot, float scalar, V3 vis) {
+    float4* const at = slot >= 0 ? P.L + slot : P.Lout + ~slot; // ~path: the path has ended (Paths::direct)
     const float4 sc = P.shC[i];
     const float4 st = P.shT[i];
     const V3 c = neeTerm(mk(sc.x, sc.y, sc.z), vis, scalar, mk(st.x, st.y, st.z), (__float_as_uint(sc.w) & 1u) != 0, st.w);
     if (!isFinite3(c)) return;
-    float4 L = P.L[slot];
+    float4 L = *at;
     L.x += c.x;
     L.y += c.y;
     L.z += c.z;
-    P.L[slot] = L;
+    *at = L;
     if (P.pass) {
         const int light = static_cast<int>(__float_as_uint(sc.w) >> 1) - 1;
         const float4* shares = P.shPass + 3 * static_cast<size_t>(i);
@@ -471,11 +428,11 @@ __device__ __forceinline__ void addShadowTerm(const SceneGPU& S, const Paths& P,
 
 // Scenes with shadow-transmitting surfaces or shadow links: a ray per lane, the transmittance walk.
 template <bool COUNT>
-__global__ void __launch_bounds__(128) kShadow(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P, const uint32_t* count, unsigned long long* stats) {
-    const int n = static_cast<int>(*count);
+__global__ void __launch_bounds__(128) kShadow(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P, unsigned long long* stats) {
+    const int n = static_cast<int>(P.now[BC_SHADOW]);
     uint32_t nodes = 0, tris = 0;
     for (;;) {
-        const int base = warpFetch(&P.counters[CNT_WORK_SHADOW]);
+        const int base = warpFetch(&P.now[BC_WORK_SHADOW]);
         if (base >= n) break;
         const int i = base + (threadIdx.x & 31);
         if (i >= n) continue;
@@ -493,14 +450,50 @@ __global__ void __launch_bounds__(128) kShadow(const __grid_constant__ SceneGPU 
     }
 }
 
-// Every other scene: the plain any-hit query, a ray per lane (walkTurn).
+// The closest hits of a queue over the 4-wide tree, a ray per lane (walkTurn); all 32 lanes call it.
 template <bool COUNT>
-__global__ void __launch_bounds__(128, 8) kShadowAny(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P, const uint32_t* count, unsigned long long* stats) {
-    uint32_t stack[kWalkStack];
-    WarpFeed feed{&P.counters[CNT_WORK_SHADOW], static_cast<int>(*count)};
-    const int root = rootRef(S);
-    const bool instances = S.nInstances > 0;
-    uint32_t nodes = 0, tris = 0;
+__device__ __forceinline__ void traceQueue(const SceneGPU& S, const Paths& P, const int32_t* queue, uint2* stack, int root,
+                                           bool instances, uint32_t& nodes, uint32_t& tris) {
+    WarpFeed feed{&P.now[BC_WORK_ISECT], static_cast<int>(P.now[BC_QUEUE])};
+    int slot = -1;
+    RayWalk w;
+    w.cur = kRayDone;
+    for (;;) {
+        const unsigned idle = __ballot_sync(kWarp, w.cur == kRayDone);
+        if (idle == kWarp || (!feed.dry() && __popc(idle) >= kRefill)) {
+            // ended rays: their hits; then the queue's next rays
+            if (w.cur == kRayDone && slot >= 0) {
+                P.hit[slot] = make_float4(w.tMax, w.u, w.v, __int_as_float(w.prim));
+                slot = -1;
+            }
+            const int i = feed.next(w.cur == kRayDone);
+            if (i >= 0) {
+                slot = queue[i];
+                const float4 ro = P.rayO[slot];
+                const float4 rd = P.rayD[slot];
+                w.start(S, root, mk(ro.x, ro.y, ro.z), mk(rd.x, rd.y, rd.z), __float_as_uint(ro.w), 1e30f, -1);
+            }
+            if (__all_sync(kWarp, slot < 0)) break;
+            continue;
+        }
+        walkTurn<false, COUNT>(
+            S, w, stack, instances, nodes, tris,
+            [&](V3& o, V3& d, uint32_t& mask) {
+                const float4 ro = P.rayO[slot], rd = P.rayD[slot];
+                o = mk(ro.x, ro.y, ro.z);
+                d = mk(rd.x, rd.y, rd.z);
+                mask = __float_as_uint(ro.w);
+            },
+            [&]() { return pathTime(S, P, slot); });
+        __syncwarp();
+    }
+}
+
+// The plain any-hit queries of the shadow records, a ray per lane.
+template <bool COUNT>
+__device__ __forceinline__ void traceShadows(const SceneGPU& S, const Paths& P, uint32_t* stack, int root, bool instances,
+                                             uint32_t& nodes, uint32_t& tris) {
+    WarpFeed feed{&P.now[BC_WORK_SHADOW], static_cast<int>(P.now[BC_SHADOW])};
     int rec = -1;
     RayWalk w;
     w.cur = kRayDone;
@@ -533,6 +526,36 @@ __global__ void __launch_bounds__(128, 8) kShadowAny(const __grid_constant__ Sce
             [&]() { return pathTime(S, P, P.shadowQ[rec]); });
         __syncwarp();
     }
+}
+
+// A bounce's ray queries in one launch: the closest hits of its queue, then (`shadows`) the shadow
+// rays the bounce before left.  The two do not depend on each other (shadow rays only add to the
+// radiance that the next shading reads), and a launch's time for a short queue is that of its longest
+// ray; warps that run out of closest hits go on with shadow rays while the long ones finish.
+template <bool COUNT>
+__global__ void __launch_bounds__(128, 8) kTrace(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P,
+                                                 const int32_t* queue, int shadows, unsigned long long* stats) {
+    uint2 stack[kWalkStack];
+    const int root = rootRef(S);
+    const bool instances = S.nInstances > 0;
+    uint32_t nodes = 0, tris = 0, shNodes = 0, shTris = 0;
+    traceQueue<COUNT>(S, P, queue, stack, root, instances, nodes, tris);
+    if (shadows) traceShadows<COUNT>(S, P, reinterpret_cast<uint32_t*>(stack), root, instances, shNodes, shTris);
+    if (COUNT) {
+        atomicAdd(&stats[0], static_cast<unsigned long long>(nodes));
+        atomicAdd(&stats[1], static_cast<unsigned long long>(tris));
+        atomicAdd(&stats[2], static_cast<unsigned long long>(shNodes));
+        atomicAdd(&stats[3], static_cast<unsigned long long>(shTris));
+    }
+}
+
+// The shadow rays alone (waves whose radiance is needed before the next closest hits).
+template <bool COUNT>
+__global__ void __launch_bounds__(128, 8) kShadowAny(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P,
+                                                     unsigned long long* stats) {
+    uint32_t stack[kWalkStack];
+    uint32_t nodes = 0, tris = 0;
+    traceShadows<COUNT>(S, P, stack, rootRef(S), S.nInstances > 0, nodes, tris);
     if (COUNT) {
         atomicAdd(&stats[2], static_cast<unsigned long long>(nodes));
         atomicAdd(&stats[3], static_cast<unsigned long long>(tris));
@@ -875,6 +898,7 @@ __device__ __forceinline__ bool shadeSlot(const SceneGPU& S, const Paths& P, con
     bool done = false;
     bool vertex = false; // a surface vertex to shade (NEE + BSDF sampling) below
     bool exitVertex = false; // ... the exit vertex of a subsurface walk
+    int shadowRec = -1;      // this vertex's record in the shadow queue
     V3 wo = -dir;
     if (!LEAN && (flags & PF_WALK)) {
         // one step of the random walk (path_tracer.cpp:263-303)
@@ -1195,9 +1219,14 @@ __device__ __forceinline__ bool shadeSlot(const SceneGPU& S, const Paths& P, con
                         }
                     }
                 } else {
-                    // shadow queue append (one record per sample)
-                    const uint32_t pos = atomicAdd(&P.counters[CNT_SHADOW], 1u);
-                    P.shadowQ[pos] = slot;
+                    // shadow queue append (waves with one shadow sample per vertex), one atomic per
+                    // group of lanes that are here together
+                    const unsigned here = __activemask();
+                    const int lane = threadIdx.x & 31, leader = __ffs(here) - 1;
+                    uint32_t pos = 0;
+                    if (lane == leader) pos = atomicAdd(&P.next[BC_SHADOW], static_cast<uint32_t>(__popc(here)));
+                    pos = __shfl_sync(here, pos, leader) + __popc(here & ((1u << lane) - 1u));
+                    shadowRec = static_cast<int>(pos);
                     P.shO[pos] = make_float4(so.x, so.y, so.z, stMax);
                     P.shD[pos] = make_float4(sd.x, sd.y, sd.z, scalar);
                     // flags: bit 0 indirect, bits 1.. the light index + 1 (0: the environment)
@@ -1345,7 +1374,9 @@ __device__ __forceinline__ bool shadeSlot(const SceneGPU& S, const Paths& P, con
         }
     }
     // write back
-    P.L[slot] = L;
+    if (P.direct && !cont) P.Lout[path] = L;
+    else P.L[slot] = L;
+    if (!INLINE_SHADOW && shadowRec >= 0) P.shadowQ[shadowRec] = P.direct && !cont ? ~path : slot;
     if (cont) {
         if (cones) P.cone[slot] = cone;
         P.rayO[slot] = ro;
@@ -1368,17 +1399,17 @@ __device__ __forceinline__ bool shadeSlot(const SceneGPU& S, const Paths& P, con
 // INLINE: NEE shadow rays are traced here, each sample's term added in the sample loop's order
 // (waves with shadowQuality > 1, whose several records per vertex the shadow queue does not hold).
 template <bool OUT, bool INLINE = false>
-__global__ void __launch_bounds__(128, 6) kShade(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P, const __grid_constant__ Wave W, int32_t* nextQueue, uint32_t* nextCount) {
+__global__ void __launch_bounds__(128, 6) kShade(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P, const __grid_constant__ Wave W, int32_t* nextQueue) {
     uint32_t seg[kShadeKeys];
     int n = 0;
     for (int k = 0; k < kShadeKeys; ++k) {
-        seg[k] = P.counters[CNT_KEYS + k];
+        seg[k] = P.now[BC_KEYS + k];
         n += static_cast<int>(seg[k]);
     }
     const int lane = threadIdx.x & 31;
     uint32_t unused0 = 0, unused1 = 0, unused2 = 0;
     for (;;) {
-        const int base = warpFetch(&P.counters[CNT_WORK_SHADE]);
+        const int base = warpFetch(&P.now[BC_WORK_SHADE]);
         if (base >= n) break;
         const int i = base + lane;
         bool cont = false, sweepable = false;
@@ -1399,26 +1430,23 @@ __global__ void __launch_bounds__(128, 6) kShade(const __grid_constant__ SceneGP
         // a continuous wave sweeps its interactive paths that have lived sweepAge bounces into a
         // tail launch, so that their requests do not wait on one bounce per wavefront step
         const bool old = P.sweepAge > 0 && cont && sweepable && P.iter - P.born[slot] >= P.sweepAge;
-        queuePush(nextQueue, nextCount, cont && !old, slot);
+        queuePush(nextQueue, &P.next[BC_QUEUE], cont && !old, slot);
         if (P.sweepAge > 0) queuePush(P.sweepQ, &P.counters[CNT_SWEEP], old, slot);
         // a regenerating wave refills the slots of ended paths
         if (P.pathOf) queuePush(P.freeQ, &P.counters[CNT_FREE], !cont && slot >= 0, slot);
     }
 }
 
-// The lean shading kernel of one shading key: the rays of that key's bin only, shaded by the
-// shadeSlot instantiation that carries the code of that key alone (waves of lean-shading scenes
-// without guiding; one launch per key, each with the registers its key needs).
-// MINB: at least this many 128-thread blocks per SM (__launch_bounds__), i.e. a register budget
-// of 65536 / (128·MINB) per thread; 1 leaves the count to the compiler (pe_tuning::shade_budget).
-template <bool OUT, int KEY, int MINB = 1>
-__global__ void __launch_bounds__(128, MINB) kShadeKey(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P, const __grid_constant__ Wave W, int32_t* nextQueue, uint32_t* nextCount) {
-    const int n = static_cast<int>(P.counters[CNT_KEYS + KEY]);
+// Lean shading of one shading key's bin by the shadeSlot instantiation that carries the code of that
+// key alone; all 32 lanes call it.
+template <bool OUT, int KEY>
+__device__ __forceinline__ void shadeBin(const SceneGPU& S, const Paths& P, const Wave& W, int32_t* nextQueue) {
+    const int n = static_cast<int>(P.now[BC_KEYS + KEY]);
     const int32_t* bin = P.sortQ + static_cast<size_t>(KEY) * P.capacity;
     const int lane = threadIdx.x & 31;
     uint32_t unused0 = 0, unused1 = 0, unused2 = 0;
-    for (;;) {
-        const int base = warpFetch(&P.counters[CNT_WORK_KEYS + KEY]);
+    while (n > 0) {
+        const int base = warpFetch(&P.now[BC_WORK_KEYS + KEY]);
         if (base >= n) break;
         const int i = base + lane;
         bool cont = false, sweepable = false;
@@ -1430,18 +1458,39 @@ __global__ void __launch_bounds__(128, MINB) kShadeKey(const __grid_constant__ S
             cont = shadeSlot<false, false, OUT, KEY>(S, P, A, slot, path, unused0, unused1, unused2);
             sweepable = (A.flags & SEG_SWEEP) != 0;
         }
-        // continuous waves sweep interactive paths that have lived sweepAge bounces, as kShade does
-        const bool old = P.sweepAge > 0 && cont && sweepable && P.iter - P.born[slot] >= P.sweepAge;
-        queuePush(nextQueue, nextCount, cont && !old, slot);
-        if (P.sweepAge > 0) queuePush(P.sweepQ, &P.counters[CNT_SWEEP], old, slot);
+        if (KEY != 0) {
+            // continuous waves sweep interactive paths that have lived sweepAge bounces, as kShade does
+            const bool old = P.sweepAge > 0 && cont && sweepable && P.iter - P.born[slot] >= P.sweepAge;
+            queuePush(nextQueue, &P.next[BC_QUEUE], cont && !old, slot);
+            if (P.sweepAge > 0) queuePush(P.sweepQ, &P.counters[CNT_SWEEP], old, slot);
+        }
         if (P.pathOf) queuePush(P.freeQ, &P.counters[CNT_FREE], !cont && slot >= 0, slot);
     }
+}
+
+// The lean shading kernels of a bounce (waves of lean-shading scenes without guiding): the misses,
+// whose code is small (75 registers), and the surfaces, whose four kinds follow each other in one
+// launch at 128 registers (four 128-thread blocks per SM), so that one kind's last warps overlap the
+// next kind's first.
+template <bool OUT>
+__global__ void __launch_bounds__(128) kShadeMiss(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P,
+                                                  const __grid_constant__ Wave W, int32_t* nextQueue) {
+    shadeBin<OUT, 0>(S, P, W, nextQueue);
+}
+template <bool OUT>
+__global__ void __launch_bounds__(128, 4) kShadeSurface(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P,
+                                                        const __grid_constant__ Wave W, int32_t* nextQueue) {
+    shadeBin<OUT, 2>(S, P, W, nextQueue);
+    shadeBin<OUT, 1>(S, P, W, nextQueue);
+    shadeBin<OUT, 3>(S, P, W, nextQueue);
+    shadeBin<OUT, 4>(S, P, W, nextQueue);
 }
 
 // ---- tail: the last paths of a wave, each run to its end by one thread -------------------------
 // Once a wave's live queue fits in one resident grid, per-bounce launches cost more than they
 // save: each thread takes a path from the queue, alternates closest-hit queries with shadeSlot
-// (shadow rays inline) until the path ends, then takes the next.  The arithmetic and the order of
+// (shadow rays inline) until the path ends, then takes the next (`traced`: the queue's paths have
+// their first hits).  The arithmetic and the order of
 // L's terms are the wavefront's, so the film is the same bit for bit.  This one-warp-per-block
 // form serves the counting pass and waves with AOV or pass outputs; plain waves and the request
 // server's sweeps and drains use kTailLockstep below.
@@ -1449,7 +1498,7 @@ constexpr int kTailBlock = 32;
 
 template <bool COUNT, bool OUT>
 __global__ void __launch_bounds__(kTailBlock) kTail(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P, const __grid_constant__ Wave W, const int32_t* queue, const uint32_t* count,
-                                             uint32_t* cursor, unsigned long long* stats) {
+                                             uint32_t* cursor, int traced, unsigned long long* stats) {
     const int n = static_cast<int>(*count);
     uint32_t nodes = 0, tris = 0, shNodes = 0, shTris = 0, rays = 0, shRays = 0;
     for (;;) {
@@ -1463,12 +1512,14 @@ __global__ void __launch_bounds__(kTailBlock) kTail(const __grid_constant__ Scen
                 atomicAdd(&stats[7], 1ull);
                 break;
             }
-            const float4 ro = P.rayO[slot];
-            const float4 rd = P.rayD[slot];
-            const Hit h = traceClosestWide<COUNT>(S, mk(ro.x, ro.y, ro.z), mk(rd.x, rd.y, rd.z), __float_as_uint(ro.w), 0.0f,
-                                              1e30f, nodes, tris, pathTime(S, P, slot));
-            ++rays;
-            P.hit[slot] = make_float4(h.t, h.u, h.v, __int_as_float(h.prim));
+            if (q > 0 || !traced) {
+                const float4 ro = P.rayO[slot];
+                const float4 rd = P.rayD[slot];
+                const Hit h = traceClosestWide<COUNT>(S, mk(ro.x, ro.y, ro.z), mk(rd.x, rd.y, rd.z), __float_as_uint(ro.w),
+                                                      0.0f, 1e30f, nodes, tris, pathTime(S, P, slot));
+                ++rays;
+                P.hit[slot] = make_float4(h.t, h.u, h.v, __int_as_float(h.prim));
+            }
             if (!shadeSlot<true, COUNT, OUT>(S, P, A, slot, path, shNodes, shTris, shRays)) break;
         }
     }
@@ -1493,7 +1544,7 @@ __global__ void __launch_bounds__(kTailBlock) kTail(const __grid_constant__ Scen
 constexpr int kTailLockstepBlock = 128;
 template <bool LEAN>
 __global__ void __launch_bounds__(kTailLockstepBlock) kTailLockstep(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P, const __grid_constant__ Wave W, const int32_t* queue,
-                                                                  const uint32_t* count, uint32_t* cursor,
+                                                                  const uint32_t* count, uint32_t* cursor, int traced,
                                                                   unsigned long long* stats) {
     const int n = static_cast<int>(*count);
     uint32_t nodes = 0, tris = 0, shNodes = 0, shTris = 0, rays = 0, shRays = 0;
@@ -1513,7 +1564,7 @@ __global__ void __launch_bounds__(kTailLockstepBlock) kTailLockstep(const __grid
             }
         }
         if (!__syncthreads_or(slot >= 0)) break;
-        if (slot >= 0) {
+        if (slot >= 0 && (q > 0 || !traced)) {
             const float4 ro = P.rayO[slot];
             const float4 rd = P.rayD[slot];
             const Hit h = traceClosestWide<false>(S, mk(ro.x, ro.y, ro.z), mk(rd.x, rd.y, rd.z), __float_as_uint(ro.w), 0.0f,
@@ -1672,25 +1723,24 @@ static __global__ void kFilm(const __grid_constant__ Paths P, const __grid_const
 // ---- instantiations ---------------------------------------------------------------------------
 // The kernels below are compiled in translation units of their own (pe_kernels_*.cu), side by side;
 // PE_LEAN_KERNELS(K) and its siblings expand K(kernel) over a unit's instantiations.
-#define PE_SHADE_ARGS (const __grid_constant__ SceneGPU, const __grid_constant__ Paths, const __grid_constant__ Wave, int32_t*, uint32_t*)
-#define PE_LEAN_KERNELS(K)                                                                         \
-    K(kShadeKey<false, 0, 1>) K(kShadeKey<false, 1, 1>) K(kShadeKey<false, 2, 1>)                  \
-    K(kShadeKey<false, 3, 1>) K(kShadeKey<false, 4, 1>) K(kShadeKey<false, 0, 4>)                  \
-    K(kShadeKey<false, 1, 4>) K(kShadeKey<false, 2, 4>) K(kShadeKey<false, 3, 4>)                  \
-    K(kShadeKey<false, 4, 4>) K(kShadeKey<false, 0, 5>) K(kShadeKey<false, 1, 5>)                  \
-    K(kShadeKey<false, 2, 5>) K(kShadeKey<false, 3, 5>) K(kShadeKey<false, 4, 5>)
-#define PE_LEAN_OUT_KERNELS(K)                                                                     \
-    K(kShadeKey<true, 0, 1>) K(kShadeKey<true, 1, 1>) K(kShadeKey<true, 2, 1>)                     \
-    K(kShadeKey<true, 3, 1>) K(kShadeKey<true, 4, 1>)
-#define PE_FULL_KERNELS(K)                                                                         \
-    K(kShade<false, false>) K(kShade<true, false>) K(kShade<false, true>) K(kShade<true, true>)
-#define PE_TAIL_ARGS (const __grid_constant__ SceneGPU, const __grid_constant__ Paths, const __grid_constant__ Wave, const int32_t*, const uint32_t*, uint32_t*, unsigned long long*)
+#define PE_SHADE_ARGS                                                                              \
+    (const __grid_constant__ SceneGPU, const __grid_constant__ Paths, const __grid_constant__ Wave, int32_t*)
+#define PE_LEAN_KERNELS(K) K(kShadeMiss<false>) K(kShadeSurface<false>)
+#define PE_LEAN_OUT_KERNELS(K) K(kShadeMiss<true>) K(kShadeSurface<true>)
+#define PE_FULL_KERNELS(K) K(kShade<false, false>) K(kShade<false, true>)
+#define PE_FULL_OUT_KERNELS(K) K(kShade<true, false>) K(kShade<true, true>)
+#define PE_TAIL_ARGS                                                                               \
+    (const __grid_constant__ SceneGPU, const __grid_constant__ Paths, const __grid_constant__ Wave, const int32_t*, \
+     const uint32_t*, uint32_t*, int, unsigned long long*)
 #define PE_TAIL_KERNELS(K) K(kTail<false, true>) K(kTail<true, false>) K(kTail<true, true>)
 #define PE_LOCKSTEP_KERNELS(K) K(kTailLockstep<false>) K(kTailLockstep<true>)
-#define PE_TRACE_ARGS (const __grid_constant__ SceneGPU, const __grid_constant__ Paths, const int32_t*, const uint32_t*, unsigned long long*)
-#define PE_TRACE_KERNELS(K)                                                                        \
-    K(kIntersect<false>) K(kIntersect<true>) K(kIntersectBinary<false>) K(kIntersectBinary<true>)
-#define PE_SHADOW_ARGS (const __grid_constant__ SceneGPU, const __grid_constant__ Paths, const uint32_t*, unsigned long long*)
+#define PE_TRACE_ARGS                                                                              \
+    (const __grid_constant__ SceneGPU, const __grid_constant__ Paths, const int32_t*, int, unsigned long long*)
+#define PE_TRACE_KERNELS(K) K(kTrace<false>) K(kTrace<true>)
+#define PE_BINARY_ARGS                                                                             \
+    (const __grid_constant__ SceneGPU, const __grid_constant__ Paths, const int32_t*, unsigned long long*)
+#define PE_BINARY_KERNELS(K) K(kIntersectBinary<false>) K(kIntersectBinary<true>)
+#define PE_SHADOW_ARGS (const __grid_constant__ SceneGPU, const __grid_constant__ Paths, unsigned long long*)
 #define PE_SHADOW_KERNELS(K) K(kShadow<false>) K(kShadow<true>) K(kShadowAny<false>) K(kShadowAny<true>)
 
 } // namespace pe

@@ -701,7 +701,7 @@ pe_server* pe_server_create(pe_device* d, uint64_t budget, char* err, size_t err
         if (express(li)) {
             // the express lane: its own path state, on the highest-priority streams
             ok = cudaStreamCreateWithPriority(&R.own.stream, cudaStreamNonBlocking, hiPrio) == cudaSuccess &&
-                 cudaMallocHost(&R.own.hCounters, 32 * sizeof(uint32_t)) == cudaSuccess &&
+                 cudaMallocHost(&R.own.hCounters, kCounters * sizeof(uint32_t)) == cudaSuccess &&
                  allocLane(R.own, kExpressSlots) == PE_OK;
             R.loop.ln = &R.own;
         } else {

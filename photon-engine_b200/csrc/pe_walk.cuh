@@ -111,9 +111,26 @@ __device__ __forceinline__ void walkTurn(const SceneGPU& S, RayWalk& w, T* stack
         else return static_cast<uint32_t>(ref);
     };
     bool pop = false;
-    if (w.cur >= 0) {
+    // the turn's loads, issued together whichever unit the lane is at: a node's eight float4, or
+    // the three of a leaf's next primitive
+    const bool isNode = w.cur >= 0, isLeaf = !isNode && w.cur != kRayDone;
+    int pi, more;
+    leafRange(w.cur, pi, more);
+    --more;
+    const float4* at = isNode ? S.wide + 8 * static_cast<size_t>(w.cur) : S.tris + 3 * static_cast<size_t>(pi);
+    WideNode n;
+    if (isNode || isLeaf) {
+        n.a[0] = __ldg(at);
+        n.a[1] = __ldg(at + 1);
+        n.a[2] = __ldg(at + 2);
+    }
+    if (isNode) {
+        n.a[3] = __ldg(at + 3);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) n.b[k] = __ldg(at + 4 + k);
+    }
+    if (isNode) {
         if (COUNT) ++nodeVisits;
-        const WideNode n = loadWide(S.wide, w.cur);
         float t[4];
         bool hit[4];
 #pragma unroll
@@ -159,12 +176,8 @@ __device__ __forceinline__ void walkTurn(const SceneGPU& S, RayWalk& w, T* stack
             }
         }
     }
-    if (w.cur < 0 && w.cur != kRayDone && !pop) {
-        int pi, more;
-        leafRange(w.cur, pi, more);
-        --more;
-        const float4 a = __ldg(&S.tris[3 * pi + 0]);
-        const float4 b = __ldg(&S.tris[3 * pi + 1]);
+    if (isLeaf) {
+        const float4 a = n.a[0], b = n.a[1];
         const uint32_t meta = __float_as_uint(b.w);
         bool enter = false;
         if ((meta & w.mask) != 0u) {
@@ -174,7 +187,7 @@ __device__ __forceinline__ void walkTurn(const SceneGPU& S, RayWalk& w, T* stack
                 float t, u = 0.0f, v = 0.0f;
                 const bool in = (meta & PRIM_SPHERE)
                                     ? sphereLean(a, w.o, w.d, 0.0f, w.tMax, t)
-                                    : triLean(a, b, __ldg(&S.tris[3 * pi + 2]), w.o, w.d, 0.0f, w.tMax, t, u, v);
+                                    : triLean(a, b, n.a[2], w.o, w.d, 0.0f, w.tMax, t, u, v);
                 if (in) {
                     if (ANY) {
                         w.prim = 1;

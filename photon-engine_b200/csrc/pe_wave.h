@@ -109,9 +109,15 @@ struct Paths {
     int32_t sweepAge;
     int32_t iter;        // current bounce of the continuous wave
     uint32_t capacity;
-    // [0] queue A count, [1] queue B count, [2] shadow count, [3] closest-hit work cursor,
-    // [4] any-hit work cursor, [5] shade work cursor, [6..11] rays per shading key, [12] errors,
-    // [13] tail work cursor, [14] guide query rows, [15] training samples
+    // bounce counters (BounceCounters): two blocks that the bounces of a wave use in turn.  A bounce
+    // traces and shades what `now` counts and appends to what `next` counts; kBin clears `next`.
+    uint32_t* blocks;
+    uint32_t* now;
+    uint32_t* next;
+    // 1: a path that ends hands its radiance to Lout at once, and a shadow ray still to be traced
+    // for its last vertex adds to Lout (shadowQ holds ~path); its slot is free for another path
+    int32_t direct;
+    // wave counters (CounterSlots)
     uint32_t* counters;
 };
 
@@ -127,10 +133,15 @@ enum PassFilms { PFILM_DEPTH = 8, PFILM_POSITION = 9, PFILM_OBJECT = 10, PFILM_M
 
 // Shading keys: 0 = miss, 1 + material type (Lambert, Disney, Dielectric, Mirror), 5 = random-walk step.
 constexpr int kShadeKeys = 6;
-enum CounterSlots { CNT_QA = 0, CNT_QB = 1, CNT_SHADOW = 2, CNT_WORK_ISECT = 3, CNT_WORK_SHADOW = 4,
-                    CNT_WORK_SHADE = 5, CNT_KEYS = 6, CNT_ERRORS = 12, CNT_WORK_TAIL = 13, CNT_GUIDE_Q = 14,
-                    CNT_TRAIN = 15, CNT_FREE = 16, CNT_SWEEP = 17, CNT_WORK_KEYS = 18,
-                    CNT_TOTAL = CNT_WORK_KEYS + kShadeKeys };
+// Counters of one bounce: the closest-hit queue's entries, the shadow records, the work cursors of
+// the trace and shading kernels, the rays per shading key and their bins' cursors.
+enum BounceCounters { BC_QUEUE = 0, BC_SHADOW = 1, BC_WORK_ISECT = 2, BC_WORK_SHADOW = 3, BC_WORK_SHADE = 4, BC_KEYS = 5,
+                      BC_WORK_KEYS = BC_KEYS + kShadeKeys, BC_TOTAL = BC_WORK_KEYS + kShadeKeys };
+constexpr int kBounceBlock = 32; // counters from one block to the next
+static_assert(BC_TOTAL <= kBounceBlock, "a bounce's counters fit its block");
+// Counters of a wave, after the two bounce blocks.
+enum CounterSlots { CNT_WORK_TAIL = 0, CNT_GUIDE_Q = 1, CNT_TRAIN = 2, CNT_FREE = 3, CNT_SWEEP = 4, CNT_WAVE = 5 };
+constexpr int kCounters = 2 * kBounceBlock + CNT_WAVE; // all of them, from Paths::blocks on
 // Paths per wave with regeneration, as a multiple of the slots.
 constexpr int kStreamFactor = 16;
 // Vertices an SD-tree training path records (the reference records up to 32; its paths in these
@@ -181,6 +192,19 @@ struct Wave {
     int nSlots;
     int nPix;
 };
+
+// Path state whose counters start at `p` (kCounters words).
+inline void setCounters(Paths& P, uint32_t* p) {
+    P.blocks = p;
+    P.now = p;
+    P.next = p + kBounceBlock;
+    P.counters = p + 2 * kBounceBlock;
+}
+// ... at bounce block b.
+inline void setBlock(Paths& P, int b) {
+    P.now = P.blocks + b * kBounceBlock;
+    P.next = P.blocks + (1 - b) * kBounceBlock;
+}
 
 #ifdef __CUDACC__
 // Sample (of the segment's nSamples) of a wave path.
