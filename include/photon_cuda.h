@@ -476,12 +476,12 @@ int32_t pe_device_last_stats(pe_device* d, pe_render_stats* out);
 int32_t pe_device_set_counting(pe_device* d, int32_t enabled);
 /* B200 tuning knob with no counterpart in the reference engine.  A wave's paths are traced
  * bounce by bounce (one closest-hit, shade and any-hit launch per bounce) until at most `paths`
- * remain live; those finish in one launch that runs each path to its end on one thread.  The
- * film is the same either way.  -1 (default) = the paths one resident grid holds, 0 = never. */
+ * remain live; those finish in one launch that runs each path to its end.  The film is the same
+ * either way.  -1 (default) = 448 paths per SM in scenes of plain surfaces, 224 in others, 0 = never. */
 int32_t pe_device_set_tail_paths(pe_device* d, int64_t paths);
 int64_t pe_device_tail_paths(pe_device* d);
 /* Autotuner (no reference counterpart): renders probe_spp samples of the view with each of a few
- * tail thresholds (1/4, 1/2, 1 and 2 resident grids) into a scratch film, twice, and keeps the
+ * tail thresholds (1/4, 1/2, 1 and 2 times the default) into a scratch film, twice, and keeps the
  * fastest of the second round; chosen (may be NULL) receives it.  The caller's films are untouched. */
 int32_t pe_device_autotune(pe_device* d, const pe_camera* cam, const pe_settings* st, int32_t probe_spp, int64_t* chosen);
 

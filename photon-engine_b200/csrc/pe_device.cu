@@ -32,6 +32,12 @@ PE_TAIL_KERNELS(PE_EXTERN)
 #define PE_EXTERN(...) extern template __global__ void __VA_ARGS__ PE_TAIL_ARGS;
 PE_LOCKSTEP_KERNELS(PE_EXTERN)
 #undef PE_EXTERN
+#define PE_EXTERN(...) extern template __global__ void __VA_ARGS__ PE_TAIL_WARPS_ARGS;
+PE_TAIL_WARPS_LEAN_KERNELS(PE_EXTERN)
+#undef PE_EXTERN
+#define PE_EXTERN(...) extern template __global__ void __VA_ARGS__ PE_TAIL_WARPS_ARGS;
+PE_TAIL_WARPS_FULL_KERNELS(PE_EXTERN)
+#undef PE_EXTERN
 #define PE_EXTERN(...) extern template __global__ void __VA_ARGS__ PE_TRACE_ARGS;
 PE_TRACE_KERNELS(PE_EXTERN)
 #undef PE_EXTERN
@@ -284,7 +290,7 @@ int32_t timerEvent(pe_device* d, RenderTimer& tm, cudaEvent_t& e) {
 // Starts a render call's statistics and its device clock.
 int32_t beginRender(pe_device* d) {
     std::memset(&d->stats, 0, sizeof(d->stats));
-    PE_CUDA(cudaMemsetAsync(d->dStats, 0, 8 * sizeof(unsigned long long), d->stream));
+    PE_CUDA(cudaMemsetAsync(d->dStats, 0, kDeviceStats * sizeof(unsigned long long), d->stream));
     PE_CUDA(cudaEventRecord(d->evStart, d->stream));
     PE_CUDA(cudaStreamWaitEvent(d->lanes[1].stream, d->evStart, 0));
     d->filmLane = -1;
@@ -301,7 +307,7 @@ int32_t endRender(pe_device* d, const RenderTimer& tm) {
     }
     d->lanes[0].pending = false;
     PE_CUDA(cudaEventRecord(d->evStop, d->stream));
-    unsigned long long hs[8] = {};
+    unsigned long long hs[kDeviceStats] = {};
     PE_CUDA(cudaMemcpyAsync(hs, d->dStats, sizeof(hs), cudaMemcpyDeviceToHost, d->stream));
     PE_CUDA(cudaStreamSynchronize(d->stream));
     PE_CUDA(cudaGetLastError());
@@ -326,7 +332,7 @@ int32_t endRender(pe_device* d, const RenderTimer& tm) {
     stats.shadow_node_visits = hs[2];
     stats.shadow_tri_tests = hs[3];
     stats.rejected = hs[4];
-    stats.closest_rays += hs[5];
+    stats.closest_rays += hs[5] + hs[8];
     stats.shadow_rays += hs[6];
     stats.tail_closest_rays = hs[5];
     stats.tail_shadow_rays = hs[6];
@@ -347,18 +353,36 @@ int32_t segsWritable(pe_device* d, int lane) {
     return PE_OK;
 }
 
-// The tail in lockstep over `n` queued paths (count and cursor on the device).
-void launchTailLockstep(pe_device* d, bool lean, const SceneGPU& S, const Paths& P, const Wave& W, const int32_t* queue,
-                        const uint32_t* count, uint32_t* cursor, int64_t n, bool traced, cudaStream_t cs) {
-    const int grid = static_cast<int>(std::max<int64_t>(
-        1, std::min<int64_t>(d->blocksTailLockstep[lean ? 1 : 0], (n + kTailLockstepBlock - 1) / kTailLockstepBlock)));
-    if (lean) kTailLockstep<true><<<grid, kTailLockstepBlock, 0, cs>>>(S, P, W, queue, count, cursor, traced ? 1 : 0, d->dStats);
-    else kTailLockstep<false><<<grid, kTailLockstepBlock, 0, cs>>>(S, P, W, queue, count, cursor, traced ? 1 : 0, d->dStats);
+// Shadow rays that a scene's closest hits need not wait with (launchTrace).
+bool plainShadows(const SceneGPU& S) { return !S.hasShadowTransmitters && !S.hasShadowLinks; }
+
+// The tail kernel over `n` queued paths (count and cursor on the device) of a wave without pass
+// outputs; `inlineShadows`: its segments take several shadow samples per vertex, `out`: it records AOVs.
+void launchTail(pe_device* d, bool lean, bool inlineShadows, bool out, const SceneGPU& S, const Paths& P, const Wave& W,
+                const int32_t* queue, const uint32_t* count, uint32_t* cursor, int64_t n, bool traced, cudaStream_t cs) {
+    const int hits = traced ? 1 : 0;
+    if (inlineShadows || !plainShadows(S)) {
+        const int grid = static_cast<int>(std::max<int64_t>(
+            1, std::min<int64_t>(d->blocksTailLockstep, (n + kTailLockstepBlock - 1) / kTailLockstepBlock)));
+        kTailLockstep<0><<<grid, kTailLockstepBlock, 0, cs>>>(S, P, W, queue, count, cursor, hits, d->dStats);
+        return;
+    }
+    const int64_t warps = static_cast<int64_t>(d->blocksTailWarps[lean ? 1 : 0][out ? 1 : 0]) * (kTailWarpsBlock / 32);
+
+    const int perWarp = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(32, (n + warps - 1) / warps)));
+    const int64_t perBlock = static_cast<int64_t>(perWarp) * (kTailWarpsBlock / 32);
+    const int grid = static_cast<int>(
+        std::max<int64_t>(1, std::min<int64_t>(warps / (kTailWarpsBlock / 32), (n + perBlock - 1) / perBlock)));
+    if (lean && out) kTailWarps<true, true><<<grid, kTailWarpsBlock, 0, cs>>>(S, P, W, queue, count, cursor, hits, perWarp, d->dStats);
+    else if (lean) kTailWarps<true, false><<<grid, kTailWarpsBlock, 0, cs>>>(S, P, W, queue, count, cursor, hits, perWarp, d->dStats);
+    else if (out) kTailWarps<false, true><<<grid, kTailWarpsBlock, 0, cs>>>(S, P, W, queue, count, cursor, hits, perWarp, d->dStats);
+    else kTailWarps<false, false><<<grid, kTailWarpsBlock, 0, cs>>>(S, P, W, queue, count, cursor, hits, perWarp, d->dStats);
 }
 
 // A bounce's ray queries: the closest hits of its queue, with `shadows` the any-hit queries of the
 // shadow records the bounce before left, then the hits binned by shading key.  Returns the launches.
-int launchTrace(pe_device* d, const SceneGPU& S, const Paths& P, const int32_t* q, bool shadows, cudaStream_t cs) {
+int launchTrace(pe_device* d, const SceneGPU& S, const Paths& P, const Wave& W, const int32_t* q, bool shadows,
+                cudaStream_t cs) {
     unsigned long long* st = d->dStats;
     int n = 2;
     if (d->closestMode == TRACE_BINARY) {
@@ -369,17 +393,17 @@ int launchTrace(pe_device* d, const SceneGPU& S, const Paths& P, const int32_t* 
             if (d->counting) kShadowAny<true><<<d->blocksShadowAny, 128, 0, cs>>>(S, P, st);
             else kShadowAny<false><<<d->blocksShadowAny, 128, 0, cs>>>(S, P, st);
         }
-    } else if (d->counting) {
-        kTrace<true><<<d->blocksIntersect, 128, 0, cs>>>(S, P, q, shadows ? 1 : 0, st);
     } else {
-        kTrace<false><<<d->blocksIntersect, 128, 0, cs>>>(S, P, q, shadows ? 1 : 0, st);
+        const int sh = shadows ? 1 : 0, grid = d->blocksIntersect;
+        const bool scatter = S.hasVolumes || S.hasSubsurface;
+        if (d->counting && scatter) kTrace<true, true><<<grid, 128, 0, cs>>>(S, P, W, q, sh, st);
+        else if (d->counting) kTrace<true, false><<<grid, 128, 0, cs>>>(S, P, W, q, sh, st);
+        else if (scatter) kTrace<false, true><<<grid, 128, 0, cs>>>(S, P, W, q, sh, st);
+        else kTrace<false, false><<<grid, 128, 0, cs>>>(S, P, W, q, sh, st);
     }
     kBin<<<d->prop.multiProcessorCount * 8, 256, 0, cs>>>(S, P, q);
     return n;
 }
-
-// Shadow rays that a scene's closest hits need not wait with (launchTrace).
-bool plainShadows(const SceneGPU& S) { return !S.hasShadowTransmitters && !S.hasShadowLinks; }
 
 // The shadow rays of the records counted in P.now, in a launch of their own.
 void launchShadow(pe_device* d, const SceneGPU& S, const Paths& P, cudaStream_t cs) {
@@ -389,6 +413,16 @@ void launchShadow(pe_device* d, const SceneGPU& S, const Paths& P, cudaStream_t 
     else if (any) kShadowAny<false><<<d->blocksShadowAny, 128, 0, cs>>>(S, P, st);
     else if (d->counting) kShadow<true><<<d->blocksShadow, 128, 0, cs>>>(S, P, st);
     else kShadow<false><<<d->blocksShadow, 128, 0, cs>>>(S, P, st);
+}
+
+// Live paths at or below which a wave's rest goes to the tail kernel unless the caller says otherwise.
+// Below the line a bounce of the whole wave costs more than its rays: it lasts as long as its longest
+// ray and path (about 0.35 ms on the torus knot, however few rays).  448 paths per SM measured best
+// or within 2 % from 64x64 to 1920x1080 films of lean-shading scenes (256x256 x 1 spp, ms, at half
+// this line / at it: Cornell 0.51 / 0.33, knot 2.19 / 2.09, room 2.33 / 1.99, grid 2.81 / 2.48); half of it
+// for the others, whose tail kernel carries all shading code (media 1280x720 x 4 spp: 19.7 / 21.2).
+int64_t defaultTailPaths(const pe_device* d, bool lean) {
+    return static_cast<int64_t>(d->prop.multiProcessorCount) * (lean ? 448 : 224);
 }
 
 // One wave on a lane over the nSegs segments in its segment table (nSlots paths, nPix film
@@ -470,7 +504,7 @@ int32_t runWave(pe_device* d, int lane, Paths& P, int nSegs, int nSlots, int nPi
     }
     const bool lean = S.leanShading && !P.guiding && !P.sdMode && noAo && !d->counting && !inlineShadows;
     const bool out = P.aovA || P.pass;
-    int64_t tailPaths = d->tailPaths < 0 ? static_cast<int64_t>(d->blocksTail) * kTailBlock : d->tailPaths;
+    int64_t tailPaths = d->tailPaths < 0 ? defaultTailPaths(d, lean) : d->tailPaths;
     // the tail kernel runs no inference: keep guided bounces in the wavefront until few paths remain
     if (P.guiding == 2) tailPaths = std::min<int64_t>(tailPaths, kGuideTailPaths);
     auto mark = [&](cudaEvent_t& e) -> int32_t {
@@ -496,10 +530,10 @@ int32_t runWave(pe_device* d, int lane, Paths& P, int nSegs, int nSlots, int nPi
             kTail<true, true><<<grid, kTailBlock, 0, cs>>>(S, P, W, qIn, count, cursor, traced ? 1 : 0, d->dStats);
         else if (d->counting)
             kTail<true, false><<<grid, kTailBlock, 0, cs>>>(S, P, W, qIn, count, cursor, traced ? 1 : 0, d->dStats);
-        else if (out)
+        else if (P.pass || (out && (inlineShadows || !plainShadows(S))))
             kTail<false, true><<<grid, kTailBlock, 0, cs>>>(S, P, W, qIn, count, cursor, traced ? 1 : 0, d->dStats);
         else
-            launchTailLockstep(d, lean, S, P, W, qIn, count, cursor, live, traced, cs);
+            launchTail(d, lean, inlineShadows, out, S, P, W, qIn, count, cursor, live, traced, cs);
         if ((r = mark(e))) return r;
         spent(tm.tail);
         ++stats.kernel_launches;
@@ -540,7 +574,7 @@ int32_t runWave(pe_device* d, int lane, Paths& P, int nSegs, int nSlots, int nPi
             live += static_cast<uint32_t>(fresh);
         }
         if ((rc = mark(e))) return rc;
-        stats.kernel_launches += launchTrace(d, S, P, qIn, shadows, cs);
+        stats.kernel_launches += launchTrace(d, S, P, W, qIn, shadows, cs);
         if (P.guiding == 2 && (rc = guideQueries(d, cs, P, W, qIn, &P.now[BC_QUEUE]))) return rc;
         if ((rc = mark(e))) return rc;
         spent(tm.isect);
@@ -664,7 +698,7 @@ int32_t loopBounce(pe_device* d, LaneLoop& L, const Wave& W, uint32_t* hSegLeft,
     P.iter = L.iter;
     // the kernels a lone render uses; shadow rays before the bounce's end, as the slots of ended
     // paths are handed on then
-    launchTrace(d, S, P, L.qIn, false, cs);
+    launchTrace(d, S, P, W, L.qIn, false, cs);
     if (L.lean) launchLeanShade(d, S, P, W, L.qOut, cs, false);
     else kShade<false, false><<<d->blocksShade, 128, 0, cs>>>(S, P, W, L.qOut);
     L.block = 1 - L.block;
@@ -693,7 +727,7 @@ int32_t loopBounce(pe_device* d, LaneLoop& L, const Wave& W, uint32_t* hSegLeft,
         PE_CUDA(cudaEventRecord(L.evReady[sweep], cs));
         PE_CUDA(cudaStreamWaitEvent(L.side, L.evReady[sweep], 0));
         PE_CUDA(cudaMemsetAsync(&L.sweepCursor[sweep], 0, sizeof(uint32_t), L.side));
-        launchTailLockstep(d, L.lean, S, P, W, L.sweepBuf[sweep], &L.sweepCnt[sweep], &L.sweepCursor[sweep],
+        launchTail(d, L.lean, false, false, S, P, W, L.sweepBuf[sweep], &L.sweepCnt[sweep], &L.sweepCursor[sweep],
                            static_cast<int64_t>(swept), false, L.side);
         kFlush<<<d->prop.multiProcessorCount * 4, 256, 0, L.side>>>(P, W, L.sweepBuf[sweep], &L.sweepCnt[sweep]);
         PE_CUDA(cudaEventRecord(L.evDone[sweep], L.side));
@@ -713,7 +747,7 @@ int32_t loopTail(pe_device* d, LaneLoop& L, const Wave& W) {
     WaveLane& ln = *L.ln;
     Paths& P = ln.paths;
     const cudaStream_t cs = ln.stream;
-    launchTailLockstep(d, L.lean, L.scene, P, W, L.qIn, &P.now[BC_QUEUE], &P.counters[CNT_WORK_TAIL],
+    launchTail(d, L.lean, false, false, L.scene, P, W, L.qIn, &P.now[BC_QUEUE], &P.counters[CNT_WORK_TAIL],
                        static_cast<int64_t>(L.live), false, cs);
     kFlush<<<d->prop.multiProcessorCount * 4, 256, 0, cs>>>(P, W, L.qIn, &P.now[BC_QUEUE]);
     L.live = 0;
@@ -1279,7 +1313,7 @@ pe_device* pe_device_create(int32_t ordinal, char* err, size_t errLen) {
         cudaEventCreate(&d->evStart) != cudaSuccess || cudaEventCreate(&d->evStop) != cudaSuccess ||
         cudaEventCreate(&d->evT0) != cudaSuccess || cudaEventCreate(&d->evT1) != cudaSuccess ||
         cudaMalloc(&d->dTables, sizeof(TablesGPU)) != cudaSuccess ||
-        cudaMalloc(&d->dStats, 8 * sizeof(unsigned long long)) != cudaSuccess ||
+        cudaMalloc(&d->dStats, kDeviceStats * sizeof(unsigned long long)) != cudaSuccess ||
         cudaMalloc(&d->dFilters, static_cast<size_t>(kFilterSlots) * (kFilterBins + 1) * sizeof(float)) != cudaSuccess ||
         cudaEventCreateWithFlags(&d->evFilm, cudaEventDisableTiming) != cudaSuccess) {
         pe_device_destroy(d);
@@ -1303,7 +1337,7 @@ pe_device* pe_device_create(int32_t ordinal, char* err, size_t errLen) {
     cudaMemcpy(d->dTables, &d->hTables, sizeof(TablesGPU), cudaMemcpyHostToDevice);
     int b = 0;
     const int sm = d->prop.multiProcessorCount;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kTrace<false>, 128, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kTrace<false, true>, 128, 0);
     d->blocksIntersect = sm * std::max(1, b);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kShade<false, false>, 128, 0);
     d->blocksShade = sm * std::max(1, b);
@@ -1311,15 +1345,16 @@ pe_device* pe_device_create(int32_t ordinal, char* err, size_t errLen) {
     d->blocksShadow = sm * std::max(1, b);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kTail<true, false>, kTailBlock, 0);
     d->blocksTail = sm * std::max(1, b);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kTailLockstep<false>, kTailLockstepBlock, 0);
-    d->blocksTailLockstep[0] = sm * std::max(1, b);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kTailLockstep<true>, kTailLockstepBlock, 0);
-    d->blocksTailLockstep[1] = sm * std::max(1, b);
     auto occ = [&](auto kernel, int threads) {
         int nb = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, threads, 0);
         return sm * std::max(1, nb);
     };
+    d->blocksTailLockstep = occ(kTailLockstep<0>, kTailLockstepBlock);
+    d->blocksTailWarps[0][0] = occ(kTailWarps<false, false>, kTailWarpsBlock);
+    d->blocksTailWarps[0][1] = occ(kTailWarps<false, true>, kTailWarpsBlock);
+    d->blocksTailWarps[1][0] = occ(kTailWarps<true, false>, kTailWarpsBlock);
+    d->blocksTailWarps[1][1] = occ(kTailWarps<true, true>, kTailWarpsBlock);
     d->blocksShadeMiss[0] = occ(kShadeMiss<false>, 128);
     d->blocksShadeMiss[1] = occ(kShadeMiss<true>, 128);
     d->blocksShadeSurface[0] = occ(kShadeSurface<false>, 128);
@@ -2079,7 +2114,7 @@ int32_t pe_device_autotune(pe_device* d, const pe_camera* cam, const pe_settings
          },
          {static_cast<int64_t>(kWaveSlots), static_cast<int64_t>(kDefaultWaveSlots), static_cast<int64_t>(kMaxWaveSlots)});
     tune("closest_traversal", [&](int64_t v) { d->closestMode = static_cast<int>(v); }, {d->closestMode, TRACE_BINARY});
-    const int64_t grid = static_cast<int64_t>(d->blocksTail) * kTailBlock;
+    const int64_t grid = defaultTailPaths(d, true);
     tune("tail_paths", [&](int64_t v) { d->tailPaths = v; }, {grid / 4, grid / 2, grid, 2 * grid});
     d->guideKind = savedKind;
     d->guide.mode = savedMode;
@@ -2157,7 +2192,7 @@ int32_t pe_device_set_tail_paths(pe_device* d, int64_t paths) {
 
 int64_t pe_device_tail_paths(pe_device* d) {
     if (!d) return -1;
-    return d->tailPaths < 0 ? static_cast<int64_t>(d->blocksTail) * kTailBlock : d->tailPaths;
+    return d->tailPaths < 0 ? defaultTailPaths(d, true) : d->tailPaths;
 }
 
 int32_t pe_device_set_counting(pe_device* d, int32_t enabled) {

@@ -34,6 +34,7 @@ struct DevBuf {
     size_t bytes = 0;
 };
 
+constexpr int kDeviceStats = 9;                  // pe_device::dStats
 constexpr int kFilterSlots = 16;
 constexpr int kMaxSegs = 64;                    // requests sharing one wave
 constexpr size_t kWaveSlots = size_t(1) << 21;  // paths in flight per wave (guided, AOV and pass waves; servers)
@@ -210,7 +211,8 @@ struct pe_device {
     int blocksIntersect = 0, blocksShade = 0, blocksShadow = 0, blocksGen = 0, blocksTail = 0;
     int blocksShadeMiss[2] = {}, blocksShadeSurface[2] = {}; // lean shading: [recording AOVs or passes]
     int blocksShadowAny = 0;
-    int blocksTailLockstep[2] = {}; // kTailLockstep<LEAN>: [0] full, [1] lean shading; 128-thread blocks
+    int blocksTailLockstep = 0;     // 128-thread blocks
+    int blocksTailWarps[2][2] = {}; // kTailWarps: [lean shading][AOVs]
     int blocksIntersectBinary = 0;
     size_t waveSlots = pe_dev::kDefaultWaveSlots; // pe_tuning::wave_slots: paths in flight per regenerating wave
     size_t laneSlots = 0;                 // slots of path state allocated per lane (>= capacity, waveSlots)
@@ -219,7 +221,7 @@ struct pe_device {
     int closestMode = 6;  // pe_tuning::closest_traversal (TraceMode: 0 the binary tree, else the 4-wide one)
     int shadeBudget = 1;  // pe_tuning::shade_budget (every value the 128-register kernels)
     std::string tuneLog;  // the last autotune's probe times
-    int64_t tailPaths = -1; // -1: one resident grid of the tail kernel; 0: no tail kernel
+    int64_t tailPaths = -1; // -1: defaultTailPaths; 0: no tail kernel
     unsigned char* noAllocBase = nullptr; // device address of g_noAllocScratch on this device
     void* stage = nullptr;                 // pinned staging of the batch film (host-film render)
     size_t stageBytes = 0;

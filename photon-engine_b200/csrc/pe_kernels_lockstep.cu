@@ -1,4 +1,4 @@
-// pe_kernels_lockstep.cu — the lockstep tail kernels (pe_integrator.cuh), compiled on their own.
+// pe_kernels_lockstep.cu — the tail kernel with inline shadow rays (pe_integrator.cuh), compiled on their own.
 #include "pe_integrator.cuh"
 
 namespace pe {

@@ -77,6 +77,7 @@ struct RayWalk {
     int sp;
     int inst;        // the instance the ray is in, -1 at the top level
     bool finite;     // inv is finite
+    bool any;        // WALK_MIXED: this ray asks for any hit
 
     __device__ __forceinline__ void setRay(V3 o_, V3 d_) {
         o = o_;
@@ -100,10 +101,12 @@ struct RayWalk {
     }
 };
 
-// One turn of the walk for every lane of the warp that has a reference.  ANY: to the first hit,
-// else to the closest.  T: uint2 (reference, entry distance), or for any hit uint32_t (reference).
+// What a warp's rays ask for: the closest hit, any hit, or (RayWalk::any) some the one and some the other.
+enum WalkKind { WALK_CLOSEST, WALK_ANY, WALK_MIXED };
+
+// One turn of the walk for every lane of the warp that has a reference.  T: uint2 (reference, entry distance), or for any hit uint32_t (reference).
 // world(o, d, mask) gives the lane's ray back when it leaves an instance, time() its shutter time.
-template <bool ANY, bool COUNT, typename T, typename World, typename Time>
+template <WalkKind KIND, bool COUNT, typename T, typename World, typename Time>
 __device__ __forceinline__ void walkTurn(const SceneGPU& S, RayWalk& w, T* stack, bool instances, uint32_t& nodeVisits,
                                          uint32_t& triTests, World world, Time time) {
     auto entry = [](int ref, float t) {
@@ -140,7 +143,7 @@ __device__ __forceinline__ void walkTurn(const SceneGPU& S, RayWalk& w, T* stack
             if (k >= 2) hit[k] = hit[k] && __float_as_int(n.b[k].w) != 0; // two children at least
         }
         const int count = (hit[0] ? 1 : 0) + (hit[1] ? 1 : 0) + (hit[2] ? 1 : 0) + (hit[3] ? 1 : 0);
-        if constexpr (ANY) {
+        if constexpr (KIND == WALK_ANY) {
             // the first child hit is next, the others wait on the stack
             bool have = false;
             int next = 0;
@@ -189,7 +192,7 @@ __device__ __forceinline__ void walkTurn(const SceneGPU& S, RayWalk& w, T* stack
                                     ? sphereLean(a, w.o, w.d, 0.0f, w.tMax, t)
                                     : triLean(a, b, n.a[2], w.o, w.d, 0.0f, w.tMax, t, u, v);
                 if (in) {
-                    if (ANY) {
+                    if (KIND == WALK_ANY || (KIND == WALK_MIXED && w.any)) {
                         w.prim = 1;
                         w.sp = 0;
                         more = 0;
