@@ -131,18 +131,15 @@ const float* filterTable(pe_device* d, int type, float width, uint64_t wave, cud
 int32_t ensureFilm(pe_device* d, int w, int h) {
     if (w == d->filmW && h == d->filmH && d->fSum) return PE_OK;
     cudaFree(d->fSum);
-    cudaFree(d->fCnt);
-    cudaFree(d->fSq);
     d->fSum = nullptr;
     d->fCnt = nullptr;
     d->fSq = nullptr;
+    // one block: sum 3n, count n, sum of squares n
     const size_t n = static_cast<size_t>(w) * static_cast<size_t>(h);
-    PE_CUDA(cudaMalloc(&d->fSum, n * 3 * sizeof(float)));
-    PE_CUDA(cudaMalloc(&d->fCnt, n * sizeof(uint32_t)));
-    PE_CUDA(cudaMalloc(&d->fSq, n * sizeof(float)));
-    PE_CUDA(cudaMemsetAsync(d->fSum, 0, n * 3 * sizeof(float), d->stream));
-    PE_CUDA(cudaMemsetAsync(d->fCnt, 0, n * sizeof(uint32_t), d->stream));
-    PE_CUDA(cudaMemsetAsync(d->fSq, 0, n * sizeof(float), d->stream));
+    PE_CUDA(cudaMalloc(&d->fSum, n * kFilmFloats * sizeof(float)));
+    d->fCnt = reinterpret_cast<uint32_t*>(d->fSum + 3 * n);
+    d->fSq = d->fSum + 4 * n;
+    PE_CUDA(cudaMemsetAsync(d->fSum, 0, n * kFilmFloats * sizeof(float), d->stream));
     d->filmW = w;
     d->filmH = h;
     return PE_OK;
@@ -307,8 +304,8 @@ int32_t endRender(pe_device* d, const RenderTimer& tm) {
     }
     d->lanes[0].pending = false;
     PE_CUDA(cudaEventRecord(d->evStop, d->stream));
-    unsigned long long hs[kDeviceStats] = {};
-    PE_CUDA(cudaMemcpyAsync(hs, d->dStats, sizeof(hs), cudaMemcpyDeviceToHost, d->stream));
+    unsigned long long* hs = d->hStats;
+    PE_CUDA(cudaMemcpyAsync(hs, d->dStats, kDeviceStats * sizeof(*hs), cudaMemcpyDeviceToHost, d->stream));
     PE_CUDA(cudaStreamSynchronize(d->stream));
     PE_CUDA(cudaGetLastError());
     float ms = 0.0f;
@@ -1314,6 +1311,7 @@ pe_device* pe_device_create(int32_t ordinal, char* err, size_t errLen) {
         cudaEventCreate(&d->evT0) != cudaSuccess || cudaEventCreate(&d->evT1) != cudaSuccess ||
         cudaMalloc(&d->dTables, sizeof(TablesGPU)) != cudaSuccess ||
         cudaMalloc(&d->dStats, kDeviceStats * sizeof(unsigned long long)) != cudaSuccess ||
+        cudaMallocHost(&d->hStats, kDeviceStats * sizeof(unsigned long long)) != cudaSuccess ||
         cudaMalloc(&d->dFilters, static_cast<size_t>(kFilterSlots) * (kFilterBins + 1) * sizeof(float)) != cudaSuccess ||
         cudaEventCreateWithFlags(&d->evFilm, cudaEventDisableTiming) != cudaSuccess) {
         pe_device_destroy(d);
@@ -1404,12 +1402,12 @@ void pe_device_destroy(pe_device* d) {
     cudaFree(d->adaptClean);
     cudaFree(d->adaptCount);
     cudaFree(d->fSum);
-    cudaFree(d->fCnt);
-    cudaFree(d->fSq);
     cudaFree(d->dTables);
     cudaFree(d->dStats);
     cudaFree(d->dFilters);
     if (d->stage) cudaFreeHost(d->stage);
+    if (d->hStats) cudaFreeHost(d->hStats);
+    for (cudaEvent_t e : d->evLanded) cudaEventDestroy(e);
     for (cudaEvent_t e : d->evPool) cudaEventDestroy(e);
     if (d->evStart) cudaEventDestroy(d->evStart);
     if (d->evT0) cudaEventDestroy(d->evT0);
@@ -1589,9 +1587,7 @@ int32_t pe_device_film_clear(pe_device* d) {
     }
     if (!d->fSum) return PE_OK;
     const size_t n = static_cast<size_t>(d->filmW) * static_cast<size_t>(d->filmH);
-    PE_CUDA(cudaMemsetAsync(d->fSum, 0, n * 3 * sizeof(float), d->stream));
-    PE_CUDA(cudaMemsetAsync(d->fCnt, 0, n * sizeof(uint32_t), d->stream));
-    PE_CUDA(cudaMemsetAsync(d->fSq, 0, n * sizeof(float), d->stream));
+    PE_CUDA(cudaMemsetAsync(d->fSum, 0, n * kFilmFloats * sizeof(float), d->stream));
     return PE_OK;
 }
 
@@ -1612,17 +1608,103 @@ int32_t pe_device_film_read(pe_device* d, float* sum, uint32_t* cnt, float* sq) 
     return PE_OK;
 }
 
-// Adds a device film block (5 floats per pixel: sum 3n, count n, sum of squares n) to a Film's
-// host arrays as Film::addBatch does (film.cpp:119-137); a null array is skipped.
-static void mergeFilm(const float* fs, size_t n, float* sum, uint32_t* cnt, float* sq) {
-    const uint32_t* fc = reinterpret_cast<const uint32_t*>(fs + 3 * n);
-    const float* fq = fs + 4 * n;
-    if (sum)
-        for (size_t i = 0; i < 3 * n; ++i) sum[i] += fs[i];
-    if (cnt)
-        for (size_t i = 0; i < n; ++i) cnt[i] += fc[i];
-    if (sq)
-        for (size_t i = 0; i < n; ++i) sq[i] += fq[i];
+// A device film block (kFilmFloats per pixel: sum 3n, count n, sum of squares n) and the host arrays
+// it is added to as Film::addBatch does (film.cpp:119-137); a null array is skipped.
+struct FilmDest {
+    const float* dev;
+    float* sum;
+    uint32_t* cnt;
+    float* sq;
+};
+
+// Adds the tile's pixels of each device film to its host arrays; `traced` (may be null) gets the
+// samples the first film counts.  The tile's rows go through pinned staging in pieces of about 1 MB,
+// at most 16, each merged by a thread of its own as soon as its copy has landed, while later pieces
+// copy; a piece's staging serves one film after another.  A film of one piece is copied and merged by
+// the caller: starting 15 threads and 48 copies cost a 256x256 film 0.25 ms.
+static int32_t mergeFilms(pe_device* d, const std::vector<FilmDest>& films, size_t n, size_t W, Tile tile, uint64_t* traced) {
+    const size_t bytes = n * kFilmFloats * sizeof(float);
+    if (d->stageBytes < bytes) {
+        if (d->stage) cudaFreeHost(d->stage);
+        d->stage = nullptr;
+        d->stageBytes = 0;
+        PE_CUDA(cudaMallocHost(&d->stage, bytes));
+        d->stageBytes = bytes;
+    }
+    float* s = reinterpret_cast<float*>(d->stage);
+    uint32_t* c = reinterpret_cast<uint32_t*>(s + 3 * n);
+    float* q = s + 4 * n;
+    const size_t rows = static_cast<size_t>(tile.h);
+    const size_t cores = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
+    const size_t pieces = std::max<size_t>(1, std::min(cores, rows * W * kFilmFloats * sizeof(float) >> 20));
+    const size_t chunk = (rows + pieces - 1) / pieces;
+    while (d->evLanded.size() < pieces) {
+        cudaEvent_t e;
+        PE_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        d->evLanded.push_back(e);
+    }
+    // piece t of film f on its way to the staging
+    auto fetch = [&](size_t t, size_t f) -> cudaError_t {
+        const FilmDest& F = films[f];
+        const size_t r0 = std::min(rows, t * chunk), r1 = std::min(rows, (t + 1) * chunk);
+        const size_t b = (static_cast<size_t>(tile.y0) + r0) * W, e = (static_cast<size_t>(tile.y0) + r1) * W;
+        cudaError_t err = cudaSuccess;
+        if (e - b == n) {
+            err = cudaMemcpyAsync(s, F.dev, bytes, cudaMemcpyDeviceToHost, d->stream);
+        } else if (e > b) {
+            err = cudaMemcpyAsync(s + 3 * b, F.dev + 3 * b, 3 * (e - b) * sizeof(float), cudaMemcpyDeviceToHost, d->stream);
+            if (err == cudaSuccess)
+                err = cudaMemcpyAsync(c + b, F.dev + 3 * n + b, (e - b) * sizeof(uint32_t), cudaMemcpyDeviceToHost, d->stream);
+            if (err == cudaSuccess && F.sq)
+                err = cudaMemcpyAsync(q + b, F.dev + 4 * n + b, (e - b) * sizeof(float), cudaMemcpyDeviceToHost, d->stream);
+        }
+        return err == cudaSuccess ? cudaEventRecord(d->evLanded[t], d->stream) : err;
+    };
+    std::vector<uint64_t> partial(pieces, 0);
+    std::vector<cudaError_t> failed(pieces, cudaSuccess);
+    auto merge = [&](size_t t) {
+        for (size_t f = 0; f < films.size(); ++f) {
+            if (f > 0) failed[t] = fetch(t, f);
+            if (failed[t] == cudaSuccess) failed[t] = cudaEventSynchronize(d->evLanded[t]);
+            if (failed[t] != cudaSuccess) return;
+            const FilmDest& F = films[f];
+            for (size_t r = t * chunk; r < std::min(rows, (t + 1) * chunk); ++r) {
+                const size_t b = (static_cast<size_t>(tile.y0) + r) * W + static_cast<size_t>(tile.x0);
+                const size_t e = b + static_cast<size_t>(tile.w);
+                if (f == 0 && traced)
+                    for (size_t i = b; i < e; ++i) partial[t] += c[i];
+                if (F.cnt)
+                    for (size_t i = b; i < e; ++i) F.cnt[i] += c[i];
+                if (F.sum)
+                    for (size_t i = 3 * b; i < 3 * e; ++i) F.sum[i] += s[i];
+                if (F.sq)
+                    for (size_t i = b; i < e; ++i) F.sq[i] += q[i];
+            }
+        }
+    };
+    for (size_t t = 0; t < pieces; ++t) PE_CUDA(fetch(t, 0));
+    std::vector<std::thread> pool;
+    size_t own = 1; // pieces from here on that have no thread are the caller's
+    try {
+        for (; own < pieces; ++own)
+            pool.emplace_back([&, t = own] {
+                failed[t] = cudaSetDevice(d->ordinal);
+                if (failed[t] == cudaSuccess) merge(t);
+            });
+    } catch (const std::exception&) {
+    }
+    merge(0);
+    for (size_t t = own; t < pieces; ++t) merge(t);
+    for (std::thread& th : pool) th.join();
+    if (traced) *traced = 0;
+    for (size_t t = 0; t < pieces; ++t) {
+        if (failed[t] != cudaSuccess) {
+            setError(std::string("film read-back failed: ") + cudaMsg(failed[t]));
+            return PE_ERR_CUDA;
+        }
+        if (traced) *traced += partial[t];
+    }
+    return PE_OK;
 }
 
 // RenderDevice::render with AOV and / or pass targets: per-slot outputs on both lanes, zeroed
@@ -1664,7 +1746,7 @@ static int32_t renderTargets(pe_device* d, const pe_camera* cam, const pe_settin
         PE_CUDA(cudaMemsetAsync(d->aovFilm, 0, n * 15 * sizeof(float), d->stream));
     }
     const int32_t stride = PASS_GROUPS + d->lightGroups;
-    const size_t passFloats = static_cast<size_t>(PFILM_GROUPS + d->lightGroups) * 5 * n;
+    const size_t passFloats = static_cast<size_t>(PFILM_GROUPS + d->lightGroups) * kFilmFloats * n;
     if (passes) {
         for (WaveLane& ln : d->lanes)
             if (!ln.pass || ln.passStride != stride) {
@@ -1714,18 +1796,14 @@ static int32_t renderTargets(pe_device* d, const pe_camera* cam, const pe_settin
     } reset{d, cryptoBuf};
     rc = pe_device_render(d, cam, st, first, count, cancel, sumRgb, sampleCount, sumLumSq, traced);
     if (rc != PE_OK && rc != PE_ERR_CANCELLED) return rc;
+    std::vector<FilmDest> dests;
     if (aovs) {
-        std::vector<float> h(n * 15);
-        PE_CUDA(cudaMemcpyAsync(h.data(), d->aovFilm, n * 15 * sizeof(float), cudaMemcpyDeviceToHost, d->stream));
-        PE_CUDA(cudaStreamSynchronize(d->stream));
-        mergeFilm(h.data(), n, aovs->albedo_sum, aovs->albedo_count, aovs->albedo_sum_sq);
-        mergeFilm(h.data() + 5 * n, n, aovs->normal_sum, aovs->normal_count, nullptr);
-        mergeFilm(h.data() + 10 * n, n, aovs->alpha_sum, aovs->alpha_count, aovs->alpha_sum_sq);
+        const float* f = d->aovFilm;
+        dests.push_back({f, aovs->albedo_sum, aovs->albedo_count, aovs->albedo_sum_sq});
+        dests.push_back({f + kFilmFloats * n, aovs->normal_sum, aovs->normal_count, nullptr});
+        dests.push_back({f + 2 * kFilmFloats * n, aovs->alpha_sum, aovs->alpha_count, aovs->alpha_sum_sq});
     }
     if (passes) {
-        std::vector<float> h(passFloats);
-        PE_CUDA(cudaMemcpyAsync(h.data(), d->passFilm, passFloats * sizeof(float), cudaMemcpyDeviceToHost, d->stream));
-        PE_CUDA(cudaStreamSynchronize(d->stream));
         const pe_film_arrays* films[PFILM_GROUPS + PE_MAX_LIGHT_GROUPS];
         for (int k = 0; k < PE_LIGHT_PASSES; ++k) films[k] = &passes->light[k];
         films[PFILM_DEPTH] = &passes->depth;
@@ -1734,8 +1812,14 @@ static int32_t renderTargets(pe_device* d, const pe_camera* cam, const pe_settin
         films[PFILM_MATERIAL] = &passes->material_id;
         for (int g = 0; g < d->lightGroups; ++g) films[PFILM_GROUPS + g] = &passes->groups[g];
         for (int f = 0; f < PFILM_GROUPS + d->lightGroups; ++f)
-            mergeFilm(h.data() + static_cast<size_t>(f) * 5 * n, n, films[f]->sum, films[f]->count,
-                      f == PFILM_POSITION ? nullptr : films[f]->sum_sq);
+            dests.push_back({d->passFilm + static_cast<size_t>(f) * kFilmFloats * n, films[f]->sum, films[f]->count,
+                             f == PFILM_POSITION ? nullptr : films[f]->sum_sq});
+    }
+    if (!dests.empty()) {
+        const int32_t mr = mergeFilms(d, dests, n, static_cast<size_t>(st->width), Tile{0, 0, st->width, st->height}, nullptr);
+        if (mr) return mr;
+    }
+    if (passes) {
         if (cryptoBuf) {
             PE_CUDA(cudaMemcpyAsync(passes->crypto_object, cryptoBuf, cryptoFloats * sizeof(float),
                                     cudaMemcpyDeviceToHost, d->stream));
@@ -1780,76 +1864,8 @@ static int32_t renderHostFilm(pe_device* d, const pe_camera* cam, const pe_setti
                                    true, tile);
     if (rr != PE_OK && rr != PE_ERR_CANCELLED) return rr;
     const size_t n = static_cast<size_t>(st->width) * static_cast<size_t>(st->height);
-    const size_t bytes = n * 5 * sizeof(float);
-    if (d->stageBytes < bytes) {
-        if (d->stage) cudaFreeHost(d->stage);
-        d->stage = nullptr;
-        d->stageBytes = 0;
-        PE_CUDA(cudaMallocHost(&d->stage, bytes));
-        d->stageBytes = bytes;
-    }
-    float* s = reinterpret_cast<float*>(d->stage);
-    uint32_t* c = reinterpret_cast<uint32_t*>(s + 3 * n);
-    float* q = s + 4 * n;
-    const unsigned hw = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
-    const size_t rows = static_cast<size_t>(tile.h), W = static_cast<size_t>(st->width);
-    const size_t chunk = (rows + hw - 1) / hw;
-    // the tile's rows come back in hw pieces, one copy each on the device stream; each piece is
-    // merged by its own thread as soon as its copy has landed, while the later pieces copy
-    std::vector<cudaEvent_t> landed(hw, nullptr);
-    struct EventsGuard {
-        std::vector<cudaEvent_t>& ev;
-        ~EventsGuard() {
-            for (cudaEvent_t e : ev)
-                if (e) cudaEventDestroy(e);
-        }
-    } eventsGuard{landed};
-    for (unsigned t = 0; t < hw; ++t) {
-        const size_t r0 = std::min(rows, t * chunk), r1 = std::min(rows, (t + 1) * chunk);
-        const size_t b = (static_cast<size_t>(tile.y0) + r0) * W, e = (static_cast<size_t>(tile.y0) + r1) * W;
-        if (e > b) {
-            PE_CUDA(cudaMemcpyAsync(s + 3 * b, d->fSum + 3 * b, 3 * (e - b) * sizeof(float), cudaMemcpyDeviceToHost,
-                                    d->stream));
-            PE_CUDA(cudaMemcpyAsync(c + b, d->fCnt + b, (e - b) * sizeof(uint32_t), cudaMemcpyDeviceToHost, d->stream));
-            PE_CUDA(cudaMemcpyAsync(q + b, d->fSq + b, (e - b) * sizeof(float), cudaMemcpyDeviceToHost, d->stream));
-        }
-        PE_CUDA(cudaEventCreateWithFlags(&landed[t], cudaEventDisableTiming));
-        PE_CUDA(cudaEventRecord(landed[t], d->stream));
-    }
-    std::vector<uint64_t> partial(hw, 0);
-    std::vector<int> copyFailed(hw, 0);
-    auto merge = [&](unsigned t) {
-        uint64_t tr = 0;
-        if (cudaEventSynchronize(landed[t]) != cudaSuccess) {
-            copyFailed[t] = 1;
-            return;
-        }
-        for (size_t r = t * chunk; r < std::min(rows, (t + 1) * chunk); ++r) {
-            const size_t b = (static_cast<size_t>(tile.y0) + r) * W + static_cast<size_t>(tile.x0);
-            const size_t e = b + static_cast<size_t>(tile.w);
-            for (size_t i = b; i < e; ++i) tr += c[i];
-            if (sampleCount)
-                for (size_t i = b; i < e; ++i) sampleCount[i] += c[i];
-            if (sumRgb)
-                for (size_t i = 3 * b; i < 3 * e; ++i) sumRgb[i] += s[i];
-            if (sumLumSq)
-                for (size_t i = b; i < e; ++i) sumLumSq[i] += q[i];
-        }
-        partial[t] = tr;
-    };
-    std::vector<std::thread> pool;
-    for (unsigned t = 1; t < hw; ++t) pool.emplace_back(merge, t);
-    merge(0);
-    for (auto& th : pool) th.join();
-    for (int f : copyFailed)
-        if (f) {
-            setError(std::string("film read-back failed: ") + cudaMsg(cudaGetLastError()));
-            return PE_ERR_CUDA;
-        }
-    uint64_t tr = 0;
-    for (uint64_t p : partial) tr += p;
-    if (traced) *traced = tr;
-    return rr;
+    const int32_t mr = mergeFilms(d, {{d->fSum, sumRgb, sampleCount, sumLumSq}}, n, static_cast<size_t>(st->width), tile, traced);
+    return mr ? mr : rr;
 }
 
 int32_t pe_device_render(pe_device* d, const pe_camera* cam, const pe_settings* st, int32_t first, int32_t count,

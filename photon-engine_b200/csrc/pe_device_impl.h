@@ -34,6 +34,7 @@ struct DevBuf {
     size_t bytes = 0;
 };
 
+constexpr size_t kFilmFloats = 5;                // words per pixel of a device film: sum 3, count, sum of squares
 constexpr int kDeviceStats = 9;                  // pe_device::dStats
 constexpr int kFilterSlots = 16;
 constexpr int kMaxSegs = 64;                    // requests sharing one wave
@@ -195,8 +196,10 @@ struct pe_device {
     cudaEvent_t evFilm = nullptr;     // after the last film kernel of the render call
     int filmLane = -1;                // lane that recorded evFilm (-1: none yet)
     // [0] nodes, [1] tris (closest), [2] nodes, [3] tris (any), [4] rejected, [5] closest rays,
-    // [6] shadow rays (both of the tail kernel), [7] paths ended at the per-path query bound
+    // [6] shadow rays (both of the tail kernel), [7] paths ended at the per-path query bound,
+    // [8] closest rays of scattered segments traced with their bounce's
     unsigned long long* dStats = nullptr;
+    unsigned long long* hStats = nullptr;  // pinned copy at a render call's end
     // resident film
     int filmW = 0, filmH = 0;
     float* fSum = nullptr;
@@ -225,6 +228,7 @@ struct pe_device {
     unsigned char* noAllocBase = nullptr; // device address of g_noAllocScratch on this device
     void* stage = nullptr;                 // pinned staging of the batch film (host-film render)
     size_t stageBytes = 0;
+    std::vector<cudaEvent_t> evLanded;     // per piece of a read-back film: its copy has landed
     std::string noAllocError;
     pe_dev::GuideState guide;
     float* aovTarget = nullptr;     // AOV films of the render in progress (pe_device_render_aovs)
