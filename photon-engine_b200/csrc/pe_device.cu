@@ -1148,6 +1148,17 @@ __global__ void kBsdfProbe(const __grid_constant__ SceneGPU S, int material, con
 
 namespace pe_dev {
 
+// Bucket tables of an environment's CDFs: block y the conditional CDF of row y, the last the marginal.
+constexpr int kMaxCdfBuckets = 2048;
+__global__ void kCdfGuide(const __grid_constant__ EnvGPU e, uint16_t* cond, uint16_t* marginal) {
+    const bool last = blockIdx.x == static_cast<unsigned>(e.height);
+    const float* cdf = last ? e.marginalCdf : e.condCdf + static_cast<size_t>(blockIdx.x) * static_cast<size_t>(e.width + 1);
+    const int n = last ? e.height : e.width, buckets = last ? e.marginalBuckets : e.condBuckets;
+    uint16_t* out = last ? marginal : cond + static_cast<size_t>(blockIdx.x) * static_cast<size_t>(buckets + 1);
+    for (int k = threadIdx.x; k <= buckets; k += blockDim.x)
+        out[k] = static_cast<uint16_t>(cdfUpper(cdf, 0, n + 1, static_cast<float>(k) / static_cast<float>(buckets)));
+}
+
 int32_t uploadScene(pe_device* d, const pe_scene* s, SceneGPU& G, std::vector<DevBuf>& bufs) {
     G = SceneGPU{};
     const HostBuild& B = s->build;
@@ -1201,10 +1212,28 @@ int32_t uploadScene(pe_device* d, const pe_scene* s, SceneGPU& G, std::vector<De
     if ((rc = upload(d, bufs, E.image, e.image)) || (rc = upload(d, bufs, E.func, e.misFunc)) ||
         (rc = upload(d, bufs, E.marginalCdf, e.misMarg)) || (rc = upload(d, bufs, E.condCdf, e.misCond)))
         return rc;
+    if (E.valid && E.width < 65535 && E.height < 65535) {
+        // where each bucket of u ends up in the sampling CDFs (sampleCdf)
+        auto buckets = [](int n) {
+            int g = 1;
+            while (2 * g <= n && g < kMaxCdfBuckets) g *= 2;
+            return g;
+        };
+        uint16_t* guide = nullptr;
+        E.marginalBuckets = buckets(E.height);
+        E.condBuckets = buckets(E.width);
+        const size_t condWords = static_cast<size_t>(E.height) * static_cast<size_t>(E.condBuckets + 1);
+        if ((rc = devAlloc(bufs, guide, condWords + static_cast<size_t>(E.marginalBuckets) + 1))) return rc;
+        E.condGuide = guide;
+        E.marginalGuide = guide + condWords;
+        kCdfGuide<<<E.height + 1, 256, 0, d->stream>>>(E, guide, guide + condWords);
+        PE_CUDA(cudaGetLastError());
+    }
     // the shadow catcher samples the environment without MIS compensation (sampleLiFull)
     G.envFull = E;
     if (B.catcherShape >= 0) {
         EnvGPU& F = G.envFull;
+        F.condGuide = F.marginalGuide = nullptr;
         F.funcInt = e.fullInt;
         F.valid = e.fullValid ? 1 : 0;
         if ((rc = upload(d, bufs, F.func, e.fullFunc)) || (rc = upload(d, bufs, F.marginalCdf, e.fullMarg)) ||

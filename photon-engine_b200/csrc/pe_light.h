@@ -77,7 +77,9 @@ PE_HD SphRect setupSphRect(V3 ref, V3 corner, V3 ex, V3 ey) {
 }
 PE_HD V3 sampleSphRect(const SphRect& r, V2 u) {
     const float au = u.x * r.solidAngle - r.g2g3;
-    const float fu = (cosf(au) * r.b0 - r.b1) / sinf(au);
+    float sinAu, cosAu;
+    sinCos(au, sinAu, cosAu);
+    const float fu = (cosAu * r.b0 - r.b1) / sinAu;
     float cu = copysignf(1.0f, fu) / sqrtf(fu * fu + r.b0 * r.b0);
     cu = sclamp(cu, -0.9999999f, 0.9999999f);
     float xu = -(cu * r.z0) / sqrtf(smax(0.0f, 1.0f - cu * cu));
@@ -199,15 +201,18 @@ PE_HD V2 dirToEquirect(V3 direction, float rotation) {
     const V3 d = normalize(direction);
     const float theta = acosf(sclamp(d.y, -1.0f, 1.0f));
     float phi = atan2f(-d.z, d.x) + kPi + rotation;
-    phi = fmodf(phi, kTwoPi);
+    // fmod of a value already in [0, 2π) is the value itself; the library call loops
+    if (!(phi >= 0.0f && phi < kTwoPi)) phi = fmodf(phi, kTwoPi);
     if (phi < 0.0f) phi += kTwoPi;
     return mk2(phi / kTwoPi, theta / kPi);
 }
 PE_HD V3 equirectToDir(float u, float v, float rotation) {
     const float theta = v * kPi;
     const float a = u * kTwoPi - kPi - rotation;
-    const float st = sinf(theta);
-    return mk(st * cosf(a), cosf(theta), -st * sinf(a));
+    float st, ct, sa, ca;
+    sinCos(theta, st, ct);
+    sinCos(a, sa, ca);
+    return mk(st * ca, ct, -st * sa);
 }
 PE_HD V3 envPixel(const EnvGPU& e, int x, int y) {
     const float* p = e.image + 3 * (static_cast<size_t>(y) * static_cast<size_t>(e.width) + static_cast<size_t>(x));
@@ -223,8 +228,14 @@ PE_HD V3 sampleEquirect(const EnvGPU& e, float u, float v) {
     const int y0 = static_cast<int>(floorf(y));
     const float fx = x - static_cast<float>(x0);
     const float fy = y - static_cast<float>(y0);
-    int xa = x0 % w; if (xa < 0) xa += w;
-    int xb = (x0 + 1) % w; if (xb < 0) xb += w;
+    // x0 is in [-1, w - 1] but for a NaN direction
+    int xa = x0 < 0 ? x0 + w : x0, xb = x0 + 1 >= w ? x0 + 1 - w : x0 + 1;
+    if (x0 < -1 || x0 >= w) {
+        xa = x0 % w;
+        if (xa < 0) xa += w;
+        xb = (x0 + 1) % w;
+        if (xb < 0) xb += w;
+    }
     const int ya = iclamp(y0, 0, h - 1), yb = iclamp(y0 + 1, 0, h - 1);
     const V3 c0 = envPixel(e, xa, ya) * (1.0f - fx) + envPixel(e, xb, ya) * fx;
     const V3 c1 = envPixel(e, xa, yb) * (1.0f - fx) + envPixel(e, xb, yb) * fx;
@@ -260,26 +271,34 @@ PE_HDN float envPdf(const EnvGPU& e, V3 wi) {
     if (e.sunPdfWeight < 1.0f) pdf += (1.0f - e.sunPdfWeight) * envImagePdf(e, wi);
     return pdf;
 }
-// First i with cdf[i] > u over n+1 entries (std::upper_bound), minus one, clamped to [0, n-1].
-PE_HD int cdfFind(const float* cdf, int n, float u) {
-    int lo = 0, count = n + 1;
-    while (count > 0) {
-        const int step = count / 2;
-        const int it = lo + step;
-        if (!(u < cdf[it])) {
-            lo = it + 1;
-            count -= step + 1;
-        } else {
-            count = step;
-        }
+// First i in [lo, hi) with cdf[i] > u, else hi (std::upper_bound).
+PE_HD int cdfUpper(const float* cdf, int lo, int hi, float u) {
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (u < cdf[mid]) hi = mid;
+        else lo = mid + 1;
     }
-    int i = lo - 1;
+    return lo;
+}
+// std::upper_bound over n+1 entries, minus one, clamped to [0, n-1].  `guide` (may be null): the upper
+// bounds of k / buckets for k = 0..buckets, buckets a power of two, so that u's own lies between those
+// of its bucket's ends.  A search of 2049 entries is eleven dependent loads; with as many buckets as
+// entries one pair of table words and a probe or two are left.
+PE_HD int cdfFind(const float* cdf, int n, float u, const uint16_t* guide, int buckets) {
+    int lo = 0, hi = n + 1;
+    if (guide && u >= 0.0f && u < 1.0f) {
+        const int k = static_cast<int>(u * static_cast<float>(buckets));
+        lo = guide[k];
+        hi = guide[k + 1];
+    }
+    int i = cdfUpper(cdf, lo, hi, u) - 1;
     if (i < 0) i = 0;
     if (i >= n) i = n - 1;
     return i;
 }
-PE_HD void sampleCdf(const float* cdf, int n, float u, int& index, float& pdf, float& coord) {
-    const int i = cdfFind(cdf, n, u);
+PE_HD void sampleCdf(const float* cdf, int n, float u, const uint16_t* guide, int buckets, int& index, float& pdf,
+                     float& coord) {
+    const int i = cdfFind(cdf, n, u, guide, buckets);
     pdf = cdf[i + 1] - cdf[i];
     float du = pdf > 0.0f ? (u - cdf[i]) / pdf : 0.0f;
     du = sclamp(du, 0.0f, 1.0f);
@@ -297,9 +316,10 @@ PE_HD LightSample envSampleImage(const EnvGPU& e, V2 s) {
     }
     int ri, ci;
     float rpdf, rc, cpdf, cc;
-    sampleCdf(e.marginalCdf, e.height, s.y, ri, rpdf, rc);
+    sampleCdf(e.marginalCdf, e.height, s.y, e.marginalGuide, e.marginalBuckets, ri, rpdf, rc);
     const float* cond = e.condCdf + static_cast<size_t>(ri) * static_cast<size_t>(e.width + 1);
-    sampleCdf(cond, e.width, s.x, ci, cpdf, cc);
+    const uint16_t* guide = e.condGuide ? e.condGuide + static_cast<size_t>(ri) * static_cast<size_t>(e.condBuckets + 1) : nullptr;
+    sampleCdf(cond, e.width, s.x, guide, e.condBuckets, ci, cpdf, cc);
     const float theta = rc * kPi;
     const float sinTheta = smax(sinf(theta), 1e-6f);
     ls.wi = normalize(equirectToDir(cc, rc, e.rotation));

@@ -126,6 +126,17 @@ PE_HD float lerpf(float a, float b, float t) { return a + t * (b - a); }
 // Color3f::clamp = max(lo, min(v, hi)) per channel (spectrum.h:57-62).
 PE_HD V3 clamp3(V3 c, float lo, float hi) { return mk(smax(lo, smin(c.x, hi)), smax(lo, smin(c.y, hi)), smax(lo, smin(c.z, hi))); }
 
+// Sine and cosine of one angle.  On the device sincosf gives the bits of sinf and cosf (checked for
+// every finite float) with one range reduction.
+PE_HD void sinCos(float x, float& s, float& c) {
+#if defined(__CUDA_ARCH__)
+    sincosf(x, &s, &c);
+#else
+    s = sinf(x);
+    c = cosf(x);
+#endif
+}
+
 // Orthonormal basis of Duff et al. 2017 (src/core/math/frame.h:32-44).
 struct Frame {
     V3 s, t, n;
@@ -190,7 +201,9 @@ PE_HD V2 sampleDiskConcentric(V2 u) {
         r = sy;
         theta = kPiOver2 - kPiOver4 * (sx / sy);
     }
-    return mk2(r * cosf(theta), r * sinf(theta));
+    float st, ct;
+    sinCos(theta, st, ct);
+    return mk2(r * ct, r * st);
 }
 PE_HD V3 sampleCosineHemisphere(V2 u) {
     const V2 d = sampleDiskConcentric(u);
@@ -202,7 +215,9 @@ PE_HD V3 sampleUniformSphere(V2 u) {
     const float z = 1.0f - 2.0f * u.x;
     const float r = sqrtf(smax(0.0f, 1.0f - z * z));
     const float phi = kTwoPi * u.y;
-    return mk(r * cosf(phi), r * sinf(phi), z);
+    float sp, cp;
+    sinCos(phi, sp, cp);
+    return mk(r * cp, r * sp, z);
 }
 PE_HD float uniformSpherePdf() { return 0.25f * kInvPi; }
 PE_HD V2 sampleUniformTriangle(V2 u) {

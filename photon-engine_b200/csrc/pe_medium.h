@@ -104,7 +104,9 @@ PE_HD V3 sampleHG(V3 d, float g, V2 u) {
     const float sinTheta = sqrtf(smax(0.0f, 1.0f - cosTheta * cosTheta));
     const float phi = kTwoPi * u.y;
     const Frame f = frameFromNormal(d);
-    return normalize(toWorld(f, mk(sinTheta * cosf(phi), sinTheta * sinf(phi), cosTheta)));
+    float sp, cp;
+    sinCos(phi, sp, cp);
+    return normalize(toWorld(f, mk(sinTheta * cp, sinTheta * sp, cosTheta)));
 }
 
 // Per-path stack of the volume-boundary materials a refracted path is inside (at most four;

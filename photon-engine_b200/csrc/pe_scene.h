@@ -206,11 +206,14 @@ struct EnvGPU {
     float sunRadiance[3];
     float funcInt;      // m_mis.funcInt
     int32_t valid;      // m_mis.valid()
-    int32_t pad[3];
+    int32_t marginalBuckets, condBuckets; // powers of two (sampleCdf)
+    int32_t pad;
     const float* image; // w*h*3
     const float* func;  // w*h
     const float* marginalCdf; // h+1
     const float* condCdf;     // h*(w+1)
+    const uint16_t* marginalGuide; // marginalBuckets+1, or null: where the bucket ends of u fall in the CDF
+    const uint16_t* condGuide;     // h*(condBuckets+1), or null
 };
 
 struct SceneGPU {
