@@ -60,8 +60,10 @@ PE_HD V3 ggxSampleVisibleNormal(V3 wo, float ax, float ay, float u1, float u2) {
     const V3 t2 = cross(vh, t1);
     const float r = sqrtf(u1);
     const float phi = kTwoPi * u2;
-    const float p1 = r * cosf(phi);
-    float p2 = r * sinf(phi);
+    float sp, cp;
+    sinCos(phi, sp, cp);
+    const float p1 = r * cp;
+    float p2 = r * sp;
     const float s = 0.5f * (1.0f + vh.z);
     p2 = (1.0f - s) * sqrtf(smax(0.0f, 1.0f - p1 * p1)) + s * p2;
     const V3 nh = t1 * p1 + t2 * p2 + vh * sqrtf(smax(0.0f, 1.0f - p1 * p1 - p2 * p2));
@@ -603,86 +605,6 @@ struct LobeSplit3 {
     V3 diffuse, glossy, transmission;
 };
 
-// Sum of all lobes f(wo, wi) (disney.cpp:223-311).  split (may be null) receives the sum in
-// lobe groups as DisneyMaterial::evalSplit forms it (disney.cpp:654-658).
-PE_HDN V3 disneyEval(const TablesGPU* T, V3 wo, V3 wi, const DisneyParams& p, LobeSplit3* split) {
-    const Frame frame = shadingFrame(p.normal, p.tangent);
-    const V3 woL = toLocal(frame, wo);
-    const V3 wiL = toLocal(frame, wi);
-    if (split) split->diffuse = split->glossy = split->transmission = mk(0.0f);
-    if (woL.z <= 0.0f) return mk(0.0f);
-    const float cosThetaO = woL.z;
-    const float coatO = coatTransmit(T, p, cosThetaO);
-    const V3 cTint = coatTintFactor(p);
-    const float stW = p.inFlake ? 0.0f : sclamp(p.specTrans, 0.0f, 1.0f) * (1.0f - p.metallic);
-    const float opaqueDielectric = (1.0f - p.metallic) * (1.0f - sclamp(p.specTrans, 0.0f, 1.0f));
-    const float trans = p.inFlake ? 0.0f : sclamp(p.diffuseTransmission, 0.0f, 1.0f) * opaqueDielectric;
-    if (wiL.z <= 0.0f) {
-        V3 ft = mk(0.0f);
-        if (trans > 0.0f) {
-            const float muI = -wiL.z;
-            const DielectricLayer dl = makeLayer(T, p);
-            const V3 sc = resolvedSheenColor(p);
-            const float sh = sheenScale(T, p, smax3(sc.x, sc.y, sc.z), cosThetaO, muI);
-            ft += p.base * (trans * kInvPi * coatO * layerFactor(T, dl, cosThetaO, muI) * sh) * cTint;
-        }
-        if (stW > 0.0f) ft += evalSpecTransmission(woL, wiL, p) * coatO * cTint;
-        if (split) split->transmission = ft;
-        return ft;
-    }
-    const V3 hL = normalize(woL + wiL);
-    const float cosThetaI = wiL.z;
-    const float cosThetaD = dot(woL, hL);
-    V3 base, baseDiffuse = mk(0.0f);
-    if (p.inFlake) {
-        base = evalFlake(wo, wi, p);
-    } else {
-        const DielectricLayer dl = makeLayer(T, p);
-        const float diffW = opaqueDielectric * (1.0f - sclamp(p.diffuseTransmission, 0.0f, 1.0f)) * (1.0f - p.subsurface);
-        const V3 fDiffuse = diffW > 0.0f ? eonEval(p.base, p.diffuseRoughness, wiL, woL) *
-                                               (diffW * layerFactor(T, dl, cosThetaO, cosThetaI))
-                                         : mk(0.0f);
-        float ax, ay;
-        anisoAlpha(p.roughness, p.anisotropy, ax, ay);
-        const float D = ggxD(hL, ax, ay);
-        const float G = ggxG(woL, wiL, ax, ay);
-        V3 F = specularFresnel(p, cosThetaD);
-        if (stW > 0.0f && !p.frontFace) {
-            const float fInt = fresnelDielectric(-cosThetaD, 1.0f, p.ior);
-            F = lerp3(F, mk(fInt), stW);
-        }
-        const V3 fSpecular = (F * D * G) / (4.0f * cosThetaO * cosThetaI) * multiScatterFactor(T, p, cosThetaO, ax, ay);
-        base = fDiffuse + fSpecular;
-        baseDiffuse = fDiffuse;
-        const V3 sc = resolvedSheenColor(p);
-        if (!isBlack(sc)) {
-            const float s = sheenScale(T, p, smax3(sc.x, sc.y, sc.z), cosThetaO, cosThetaI);
-            base = base * s + evalSheen(T, sc, p, cosThetaO, cosThetaI, hL.z);
-            baseDiffuse = baseDiffuse * s;
-        }
-    }
-    if (p.clearCoat <= 0.0f) {
-        if (split) {
-            split->diffuse = baseDiffuse;
-            split->glossy = base - baseDiffuse;
-        }
-        return base;
-    }
-    const float alphaC = p.clearCoatRoughness * p.clearCoatRoughness;
-    const float Dc = ggxD(hL, alphaC, alphaC);
-    const float Gc = ggxG(woL, wiL, alphaC, alphaC);
-    const float f0c = coatF0(p);
-    const float Fc = schlickClamped(f0c, cosThetaD);
-    const float msC = 1.0f + f0c * (1.0f / ggxDirectionalAlbedo(T, cosThetaO, alphaC) - 1.0f);
-    const V3 fCoat = mk(p.clearCoat * Fc * Dc * Gc / (4.0f * cosThetaO * cosThetaI) * msC);
-    const V3 coatAtt = cTint * (coatO * coatTransmit(T, p, cosThetaI));
-    if (split) {
-        split->diffuse = baseDiffuse * coatAtt;
-        split->glossy = (base - baseDiffuse) * coatAtt + fCoat;
-    }
-    return base * coatAtt + fCoat;
-}
-
 struct LobeWeights {
     float coat, spec, diffRefl, trans, sss, specTrans;
 };
@@ -708,36 +630,143 @@ PE_HD LobeWeights disneyLobeWeights(const DisneyParams& p) {
     return w;
 }
 
-PE_HDN float disneyPdf(V3 wo, V3 wi, const DisneyParams& p) {
-    const Frame frame = shadingFrame(p.normal, p.tangent);
-    const V3 woL = toLocal(frame, wo);
-    const V3 wiL = toLocal(frame, wi);
-    if (woL.z <= 0.0f) return 0.0f;
-    const LobeWeights lw = disneyLobeWeights(p);
+// A Disney vertex: the resolved parameters and everything of f, its pdf and the sampled lobes that
+// depends on the outgoing direction alone.  A vertex evaluates f and pdf twice (the light sample, the
+// sampled direction) and used to build the shading frame five times, the parameters twice and the
+// outgoing side's table lookups, masking terms and D with each of them.
+struct DisneyVertex {
+    DisneyParams p;
+    Frame frame;
+    V3 wo, woL;
+    LobeWeights lw;
+    float stW, trans, diffW;       // weights of specular transmission, diffuse transmission and diffuse reflection
+    DielectricLayer layer;         // where trans or diffW need it
+    float layerO;                  // its transmittance towards wo
+    float ax, ay, lambdaO;         // base specular (not in a flake)
+    V3 multi;
+    V3 sheen;
+    float coatO;                   // 1 without a coat
+    V3 coatTint;
+    float coatAlpha, coatLambdaO, coatF0, coatMulti;
+};
+PE_HDN void disneyVertex(const TablesGPU* T, const MatGPU& m, V3 wo, const ShadePoint& sp, DisneyVertex& v) {
+    v.p = disneyResolve(m, sp);
+    const DisneyParams& p = v.p;
+    v.frame = shadingFrame(p.normal, p.tangent);
+    v.wo = wo;
+    v.woL = toLocal(v.frame, wo);
+    v.lw = disneyLobeWeights(p);
+    const float cosThetaO = v.woL.z;
+    if (cosThetaO <= 0.0f) return;
+    v.coatO = coatTransmit(T, p, cosThetaO);
+    v.coatTint = coatTintFactor(p);
+    v.stW = p.inFlake ? 0.0f : sclamp(p.specTrans, 0.0f, 1.0f) * (1.0f - p.metallic);
+    const float opaqueDielectric = (1.0f - p.metallic) * (1.0f - sclamp(p.specTrans, 0.0f, 1.0f));
+    v.trans = p.inFlake ? 0.0f : sclamp(p.diffuseTransmission, 0.0f, 1.0f) * opaqueDielectric;
+    v.diffW = opaqueDielectric * (1.0f - sclamp(p.diffuseTransmission, 0.0f, 1.0f)) * (1.0f - p.subsurface);
+    if (v.trans > 0.0f || (!p.inFlake && v.diffW > 0.0f)) {
+        v.layer = makeLayer(T, p);
+        v.layerO = layerTransmit(T, v.layer, cosThetaO);
+    }
+    if (!p.inFlake) {
+        anisoAlpha(p.roughness, p.anisotropy, v.ax, v.ay);
+        v.lambdaO = ggxLambda(v.woL, v.ax, v.ay);
+        v.multi = multiScatterFactor(T, p, cosThetaO, v.ax, v.ay);
+        v.sheen = resolvedSheenColor(p);
+    }
+    if (p.clearCoat > 0.0f) {
+        v.coatAlpha = p.clearCoatRoughness * p.clearCoatRoughness;
+        v.coatLambdaO = ggxLambda(v.woL, v.coatAlpha, v.coatAlpha);
+        v.coatF0 = coatF0(p);
+        v.coatMulti = 1.0f + v.coatF0 * (1.0f / ggxDirectionalAlbedo(T, cosThetaO, v.coatAlpha) - 1.0f);
+    }
+}
+
+// ggxVisiblePdf with the outgoing direction's Λ and the half vector's D in hand.
+PE_HD float ggxVisiblePdfOf(float lambdaO, float cosThetaD, float D, float cosThetaO) {
+    const float cosO = fabsf(cosThetaO);
+    if (cosO <= 0.0f) return 0.0f;
+    return 1.0f / (1.0f + lambdaO) * fabsf(cosThetaD) * D / cosO;
+}
+
+// Sum of all lobes f(wo, wi) (disney.cpp:223-311) and the sampling density of wi.  split (may be null)
+// receives the sum in lobe groups as DisneyMaterial::evalSplit forms it (disney.cpp:654-658).
+PE_HDN V3 disneyEvalPdf(const TablesGPU* T, const DisneyVertex& v, V3 wi, float& pdf, LobeSplit3* split) {
+    const DisneyParams& p = v.p;
+    const V3 woL = v.woL;
+    const V3 wiL = toLocal(v.frame, wi);
+    if (split) split->diffuse = split->glossy = split->transmission = mk(0.0f);
+    pdf = 0.0f;
+    if (woL.z <= 0.0f) return mk(0.0f);
+    const float cosThetaO = woL.z;
     if (wiL.z <= 0.0f) {
-        float pdf = 0.0f;
-        if (lw.trans > 0.0f) pdf += lw.trans * cosineHemispherePdf(-wiL.z);
-        if (lw.specTrans > 0.0f) pdf += lw.specTrans * pdfSpecTransmission(woL, wiL, p);
-        return pdf;
+        V3 ft = mk(0.0f);
+        if (v.trans > 0.0f) {
+            const float muI = -wiL.z;
+            const V3 sc = resolvedSheenColor(p);
+            const float sh = sheenScale(T, p, smax3(sc.x, sc.y, sc.z), cosThetaO, muI);
+            ft += p.base * (v.trans * kInvPi * v.coatO * (v.layerO * layerTransmit(T, v.layer, muI) * v.layer.invOneMinusAvg) * sh) *
+                  v.coatTint;
+        }
+        if (v.stW > 0.0f) ft += evalSpecTransmission(woL, wiL, p) * v.coatO * v.coatTint;
+        if (split) split->transmission = ft;
+        if (v.lw.trans > 0.0f) pdf += v.lw.trans * cosineHemispherePdf(-wiL.z);
+        if (v.lw.specTrans > 0.0f) pdf += v.lw.specTrans * pdfSpecTransmission(woL, wiL, p);
+        return ft;
     }
     const V3 hL = normalize(woL + wiL);
+    const float cosThetaI = wiL.z;
     const float cosThetaD = dot(woL, hL);
-    if (cosThetaD <= 0.0f) return 0.0f;
-    const float pdfDiffuse = cosineHemispherePdf(wiL.z);
-    float pdfSpecular;
+    const bool sampled = cosThetaD > 0.0f; // wi has a density
+    V3 base, baseDiffuse = mk(0.0f);
+    float pdfSpecular = 0.0f;
     if (p.inFlake) {
-        pdfSpecular = pdfFlake(wo, wi, p);
+        base = evalFlake(v.wo, wi, p);
+        if (sampled) pdfSpecular = pdfFlake(v.wo, wi, p);
     } else {
-        float ax, ay;
-        anisoAlpha(p.roughness, p.anisotropy, ax, ay);
-        pdfSpecular = ggxVisiblePdf(woL, hL, ax, ay) / (4.0f * cosThetaD);
+        const V3 fDiffuse = v.diffW > 0.0f
+                                ? eonEval(p.base, p.diffuseRoughness, wiL, woL) *
+                                      (v.diffW * (v.layerO * layerTransmit(T, v.layer, cosThetaI) * v.layer.invOneMinusAvg))
+                                : mk(0.0f);
+        const float D = ggxD(hL, v.ax, v.ay);
+        const float G = 1.0f / (1.0f + v.lambdaO + ggxLambda(wiL, v.ax, v.ay));
+        V3 F = specularFresnel(p, cosThetaD);
+        if (v.stW > 0.0f && !p.frontFace) {
+            const float fInt = fresnelDielectric(-cosThetaD, 1.0f, p.ior);
+            F = lerp3(F, mk(fInt), v.stW);
+        }
+        const V3 fSpecular = (F * D * G) / (4.0f * cosThetaO * cosThetaI) * v.multi;
+        base = fDiffuse + fSpecular;
+        baseDiffuse = fDiffuse;
+        const V3 sc = v.sheen;
+        if (!isBlack(sc)) {
+            const float s = sheenScale(T, p, smax3(sc.x, sc.y, sc.z), cosThetaO, cosThetaI);
+            base = base * s + evalSheen(T, sc, p, cosThetaO, cosThetaI, hL.z);
+            baseDiffuse = baseDiffuse * s;
+        }
+        if (sampled) pdfSpecular = ggxVisiblePdfOf(v.lambdaO, cosThetaD, D, woL.z) / (4.0f * cosThetaD);
     }
     float pdfCoat = 0.0f;
-    if (lw.coat > 0.0f) {
-        const float alphaC = p.clearCoatRoughness * p.clearCoatRoughness;
-        pdfCoat = ggxVisiblePdf(woL, hL, alphaC, alphaC) / (4.0f * cosThetaD);
+    if (p.clearCoat <= 0.0f) {
+        if (split) {
+            split->diffuse = baseDiffuse;
+            split->glossy = base - baseDiffuse;
+        }
+    } else {
+        const float Dc = ggxD(hL, v.coatAlpha, v.coatAlpha);
+        const float Gc = 1.0f / (1.0f + v.coatLambdaO + ggxLambda(wiL, v.coatAlpha, v.coatAlpha));
+        const float Fc = schlickClamped(v.coatF0, cosThetaD);
+        const V3 fCoat = mk(p.clearCoat * Fc * Dc * Gc / (4.0f * cosThetaO * cosThetaI) * v.coatMulti);
+        const V3 coatAtt = v.coatTint * (v.coatO * coatTransmit(T, p, cosThetaI));
+        if (split) {
+            split->diffuse = baseDiffuse * coatAtt;
+            split->glossy = (base - baseDiffuse) * coatAtt + fCoat;
+        }
+        base = base * coatAtt + fCoat;
+        if (sampled && v.lw.coat > 0.0f) pdfCoat = ggxVisiblePdfOf(v.coatLambdaO, cosThetaD, Dc, woL.z) / (4.0f * cosThetaD);
     }
-    return lw.diffRefl * pdfDiffuse + lw.spec * pdfSpecular + lw.coat * pdfCoat;
+    if (sampled) pdf = v.lw.diffRefl * cosineHemispherePdf(wiL.z) + v.lw.spec * pdfSpecular + v.lw.coat * pdfCoat;
+    return base;
 }
 
 PE_HD bool disneySampleSpecularLobe(const DisneyParams& p, const Frame& frame, V3 wo, V3 woL, float u1, float u2,
@@ -765,22 +794,22 @@ PE_HD bool disneySampleSpecTransLobe(const DisneyParams& p, V3 woL, float u1, fl
 }
 
 // DisneyMaterial::sampleFull (disney.cpp:680-729).
-PE_HDN bool disneySample(const TablesGPU* T, V3 wo, const DisneyParams& p, float uc, V2 u, BsdfSample& out) {
+PE_HD bool disneySample(const TablesGPU* T, const DisneyVertex& v, float uc, V2 u, BsdfSample& out) {
+    const DisneyParams& p = v.p;
+    const LobeWeights& lw = v.lw;
     out.delta = false;
     out.subsurface = false;
     out.passThrough = false;
     out.weight = mk(0.0f);
-    const Frame frame = shadingFrame(p.normal, p.tangent);
-    const V3 woL = toLocal(frame, wo);
+    const V3 woL = v.woL;
     if (woL.z <= 0.0f) return false;
-    const LobeWeights lw = disneyLobeWeights(p);
     V3 wiL;
     if (uc < lw.coat) {
         const float alphaC = p.clearCoatRoughness * p.clearCoatRoughness;
         wiL = reflectV(woL, ggxSampleVisibleNormal(woL, alphaC, alphaC, u.x, u.y));
         if (wiL.z <= 0.0f) return false;
     } else if (uc < lw.coat + lw.spec) {
-        if (!disneySampleSpecularLobe(p, frame, wo, woL, u.x, u.y, wiL)) return false;
+        if (!disneySampleSpecularLobe(p, v.frame, v.wo, woL, u.x, u.y, wiL)) return false;
     } else if (uc < lw.coat + lw.spec + lw.specTrans) {
         if (!disneySampleSpecTransLobe(p, woL, u.x, u.y, wiL)) return false;
     } else if (uc < lw.coat + lw.spec + lw.specTrans + lw.diffRefl) {
@@ -795,7 +824,7 @@ PE_HDN bool disneySample(const TablesGPU* T, V3 wo, const DisneyParams& p, float
         const float sheenO = sheenScale(T, p, smax3(sc.x, sc.y, sc.z), woL.z, 1.0f);
         const float layerO = layerTransmit(T, makeLayer(T, p), woL.z);
         const float w = p.subsurface * opaqueDielectric * (1.0f - trans) * coatO * sheenO * layerO / smax(lw.sss, 1e-6f);
-        out.wi = normalize(toWorld(frame, wiL));
+        out.wi = normalize(toWorld(v.frame, wiL));
         out.subsurface = true;
         out.weight = coatTintFactor(p) * w;
         out.pdf = lw.sss * cosineHemispherePdf(-wiL.z);
@@ -805,9 +834,8 @@ PE_HDN bool disneySample(const TablesGPU* T, V3 wo, const DisneyParams& p, float
         wiL = sampleCosineHemisphere(u);
         wiL.z = -wiL.z;
     }
-    out.wi = normalize(toWorld(frame, wiL));
-    out.f = disneyEval(T, wo, out.wi, p, nullptr);
-    out.pdf = disneyPdf(wo, out.wi, p);
+    out.wi = normalize(toWorld(v.frame, wiL));
+    out.f = disneyEvalPdf(T, v, out.wi, out.pdf, nullptr);
     return out.pdf > 0.0f;
 }
 
@@ -1049,9 +1077,11 @@ PE_HDN bool glassSample(const MatGPU& m, V3 woW, const ShadePoint& sp, float uc,
 // ---------------------------------------------------------------------------------------------
 // Dispatch (Material::evalPdf / sampleFull).  MT >= 0 fixes the material type at compile time
 // (a kernel that shades one material kind carries only that kind's code); MT < 0 reads m.type.
+// `dv`: the vertex of a Disney material (disneyVertex), unused for the others.
+constexpr int kDisneyType = 1;
 template <int MT>
-PE_HD V3 bsdfEvalPdfT(const TablesGPU* T, const MatGPU& m, V3 wo, V3 wi, const ShadePoint& sp, float& pdf,
-                      LobeSplit3* split) {
+PE_HD V3 bsdfEvalPdfT(const TablesGPU* T, const MatGPU& m, V3 wo, V3 wi, const ShadePoint& sp, const DisneyVertex* dv,
+                      float& pdf, LobeSplit3* split) {
     const int type = MT >= 0 ? MT : m.type;
     if (split) split->diffuse = split->glossy = split->transmission = mk(0.0f);
     V3 f;
@@ -1059,11 +1089,8 @@ PE_HD V3 bsdfEvalPdfT(const TablesGPU* T, const MatGPU& m, V3 wo, V3 wi, const S
         case 0:
             f = lambertEval(m, wo, wi, sp.n, pdf);
             break;
-        case 1: {
-            const DisneyParams p = disneyResolve(m, sp);
-            pdf = disneyPdf(wo, wi, p);
-            return disneyEval(T, wo, wi, p, split);
-        }
+        case kDisneyType:
+            return disneyEvalPdf(T, *dv, wi, pdf, split);
         case 2:
             f = glassEval(m, wo, wi, sp, pdf);
             break;
@@ -1081,19 +1108,14 @@ PE_HD V3 bsdfEvalPdfT(const TablesGPU* T, const MatGPU& m, V3 wo, V3 wi, const S
     return f;
 }
 
-PE_HD V3 bsdfEvalPdf(const TablesGPU* T, const MatGPU& m, V3 wo, V3 wi, const ShadePoint& sp, float& pdf,
-                     LobeSplit3* split) {
-    return bsdfEvalPdfT<-1>(T, m, wo, wi, sp, pdf, split);
-}
-
 template <int MT>
-PE_HD bool bsdfSampleT(const TablesGPU* T, const MatGPU& m, V3 wo, const ShadePoint& sp, float uc, V2 u,
-                       BsdfSample& out) {
+PE_HD bool bsdfSampleT(const TablesGPU* T, const MatGPU& m, V3 wo, const ShadePoint& sp, const DisneyVertex* dv, float uc,
+                       V2 u, BsdfSample& out) {
     switch (MT >= 0 ? MT : m.type) {
         case 0:
             return lambertSample(m, wo, sp.n, u, out);
-        case 1:
-            return disneySample(T, wo, disneyResolve(m, sp), uc, u, out);
+        case kDisneyType:
+            return disneySample(T, *dv, uc, u, out);
         case 2:
             return glassSample(m, wo, sp, uc, u, out);
         case 3:
@@ -1101,11 +1123,6 @@ PE_HD bool bsdfSampleT(const TablesGPU* T, const MatGPU& m, V3 wo, const ShadePo
         default:
             return false;
     }
-}
-
-PE_HD bool bsdfSample(const TablesGPU* T, const MatGPU& m, V3 wo, const ShadePoint& sp, float uc, V2 u,
-                      BsdfSample& out) {
-    return bsdfSampleT<-1>(T, m, wo, sp, uc, u, out);
 }
 
 } // namespace pe

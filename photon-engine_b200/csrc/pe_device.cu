@@ -262,16 +262,29 @@ Paths noAllocPaths(unsigned char* base) {
     return P;
 }
 
-// The lean shading kernels of one bounce; returns the number of launches.
+// The lean shading kernels of one bounce, one per shading key whose material type the scene
+// uses (the miss key always); returns the number of launches.
 int launchLeanShade(pe_device* d, const SceneGPU& S, const Paths& P, const Wave& W, int32_t* qOut, cudaStream_t cs, bool out) {
+    int n = 0;
+    auto one = [&](auto kernel, int key) {
+        if (key > 0 && !(S.materialTypes & (1 << (key - 1)))) return;
+        kernel<<<d->blocksShadeKey[out ? 1 : 0][key], 128, 0, cs>>>(S, P, W, qOut);
+        ++n;
+    };
     if (out) {
-        kShadeMiss<true><<<d->blocksShadeMiss[1], 128, 0, cs>>>(S, P, W, qOut);
-        kShadeSurface<true><<<d->blocksShadeSurface[1], 128, 0, cs>>>(S, P, W, qOut);
+        one(kShadeKey<true, 0, 1>, 0);
+        one(kShadeKey<true, 1, 5>, 1);
+        one(kShadeKey<true, 2, 6>, 2);
+        one(kShadeKey<true, 3, 5>, 3);
+        one(kShadeKey<true, 4, 5>, 4);
     } else {
-        kShadeMiss<false><<<d->blocksShadeMiss[0], 128, 0, cs>>>(S, P, W, qOut);
-        kShadeSurface<false><<<d->blocksShadeSurface[0], 128, 0, cs>>>(S, P, W, qOut);
+        one(kShadeKey<false, 0, 1>, 0);
+        one(kShadeKey<false, 1, 5>, 1);
+        one(kShadeKey<false, 2, 6>, 2);
+        one(kShadeKey<false, 3, 5>, 3);
+        one(kShadeKey<false, 4, 5>, 4);
     }
-    return 2;
+    return n;
 }
 
 int32_t timerEvent(pe_device* d, RenderTimer& tm, cudaEvent_t& e) {
@@ -1115,7 +1128,9 @@ __global__ void kBsdfProbe(const __grid_constant__ SceneGPU S, int material, con
         pe_bsdf_result r;
         memset(&r, 0, sizeof(r));
         float pdf = 0.0f;
-        const V3 f = bsdfEvalPdf(S.tables, m, m3f(q[i].wo), m3f(q[i].wi), sp, pdf, nullptr);
+        DisneyVertex dv;
+        if (m.type == kDisneyType) disneyVertex(S.tables, m, m3f(q[i].wo), sp, dv);
+        const V3 f = bsdfEvalPdfT<-1>(S.tables, m, m3f(q[i].wo), m3f(q[i].wi), sp, &dv, pdf, nullptr);
         r.f[0] = f.x;
         r.f[1] = f.y;
         r.f[2] = f.z;
@@ -1126,7 +1141,7 @@ __global__ void kBsdfProbe(const __grid_constant__ SceneGPU S, int material, con
         bs.pdf = 0.0f;
         bs.delta = bs.passThrough = bs.subsurface = false;
         bs.weight = mk(0.0f);
-        r.sampled = bsdfSample(S.tables, m, m3f(q[i].wo), sp, q[i].uc, mk2(q[i].u[0], q[i].u[1]), bs) ? 1 : 0;
+        r.sampled = bsdfSampleT<-1>(S.tables, m, m3f(q[i].wo), sp, &dv, q[i].uc, mk2(q[i].u[0], q[i].u[1]), bs) ? 1 : 0;
         r.wi[0] = bs.wi.x;
         r.wi[1] = bs.wi.y;
         r.wi[2] = bs.wi.z;
@@ -1382,10 +1397,16 @@ pe_device* pe_device_create(int32_t ordinal, char* err, size_t errLen) {
     d->blocksTailWarps[0][1] = occ(kTailWarps<false, true>, kTailWarpsBlock);
     d->blocksTailWarps[1][0] = occ(kTailWarps<true, false>, kTailWarpsBlock);
     d->blocksTailWarps[1][1] = occ(kTailWarps<true, true>, kTailWarpsBlock);
-    d->blocksShadeMiss[0] = occ(kShadeMiss<false>, 128);
-    d->blocksShadeMiss[1] = occ(kShadeMiss<true>, 128);
-    d->blocksShadeSurface[0] = occ(kShadeSurface<false>, 128);
-    d->blocksShadeSurface[1] = occ(kShadeSurface<true>, 128);
+    d->blocksShadeKey[0][0] = occ(kShadeKey<false, 0, 1>, 128);
+    d->blocksShadeKey[0][1] = occ(kShadeKey<false, 1, 5>, 128);
+    d->blocksShadeKey[0][2] = occ(kShadeKey<false, 2, 6>, 128);
+    d->blocksShadeKey[0][3] = occ(kShadeKey<false, 3, 5>, 128);
+    d->blocksShadeKey[0][4] = occ(kShadeKey<false, 4, 5>, 128);
+    d->blocksShadeKey[1][0] = occ(kShadeKey<true, 0, 1>, 128);
+    d->blocksShadeKey[1][1] = occ(kShadeKey<true, 1, 5>, 128);
+    d->blocksShadeKey[1][2] = occ(kShadeKey<true, 2, 6>, 128);
+    d->blocksShadeKey[1][3] = occ(kShadeKey<true, 3, 5>, 128);
+    d->blocksShadeKey[1][4] = occ(kShadeKey<true, 4, 5>, 128);
     d->blocksIntersectBinary = occ(kIntersectBinary<false>, 128);
     d->blocksShadowAny = occ(kShadowAny<false>, 128);
     const cudaError_t le = cudaGetLastError();

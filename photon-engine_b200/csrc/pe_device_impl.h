@@ -212,7 +212,7 @@ struct pe_device {
     bool counting = false;
     pe_render_stats stats{};
     int blocksIntersect = 0, blocksShade = 0, blocksShadow = 0, blocksGen = 0, blocksTail = 0;
-    int blocksShadeMiss[2] = {}, blocksShadeSurface[2] = {}; // lean shading: [recording AOVs or passes]
+    int blocksShadeKey[2][5] = {}; // lean shading kernels: [recording AOVs or passes][key]
     int blocksShadowAny = 0;
     int blocksTailLockstep = 0;     // 128-thread blocks
     int blocksTailWarps[2][2] = {}; // kTailWarps: [lean shading][AOVs]

@@ -760,7 +760,7 @@ static __device__ __noinline__ bool guideRecord(const Paths& P, int slot, V3 p, 
 // learned mixture in place of the SD-tree): the branch number picks the strategy, the
 // proposal draws a lobe from the rest of it and a direction from one get2D.
 static __device__ __noinline__ bool guidedSample(const TablesGPU* T, const MatGPU& mat, V3 wo, const ShadePoint& sp, const Paths& P,
-                                          int slot, Sobol& sb, BsdfSample& bs) {
+                                          int slot, const DisneyVertex* dv, Sobol& sb, BsdfSample& bs) {
     Lobes L;
     slotLobes(P, slot, L);
     const float uBranch = get1D(sb);
@@ -769,7 +769,7 @@ static __device__ __noinline__ bool guidedSample(const TablesGPU* T, const MatGP
         const float gPdf = lobesPdf(L, gwi);
         if (!(gPdf > 0.0f)) return false;
         float bPdf = 0.0f;
-        const V3 f = bsdfEvalPdf(T, mat, wo, gwi, sp, bPdf, nullptr);
+        const V3 f = bsdfEvalPdfT<-1>(T, mat, wo, gwi, sp, dv, bPdf, nullptr);
         const float mixPdf = 0.5f * gPdf + 0.5f * bPdf;
         if (isBlack(f) || !(mixPdf > 0.0f)) return false;
         bs.wi = gwi;
@@ -783,7 +783,7 @@ static __device__ __noinline__ bool guidedSample(const TablesGPU* T, const MatGP
     }
     const float uc = get1D(sb);
     const V2 u2 = get2D(T, sb);
-    if (!bsdfSample(T, mat, wo, sp, uc, u2, bs)) return false;
+    if (!bsdfSampleT<-1>(T, mat, wo, sp, dv, uc, u2, bs)) return false;
     if (bs.subsurface) bs.weight = bs.weight * 2.0f;
     else if (bs.delta || bs.passThrough) bs.pdf *= 0.5f;
     else if (bs.pdf > 0.0f) bs.pdf = 0.5f * bs.pdf + 0.5f * lobesPdf(L, bs.wi);
@@ -794,14 +794,15 @@ static __device__ __noinline__ bool guidedSample(const TablesGPU* T, const MatGP
 // (path_tracer.cpp:703-735): a direction from one get2D on the guide branch, the BSDF's
 // get1D + get2D on the other.
 static __device__ __noinline__ bool sdGuidedSample(const TablesGPU* T, const MatGPU& mat, V3 wo, const ShadePoint& sp,
-                                            const SdQuad* tree, int root, Sobol& sb, BsdfSample& bs) {
+                                            const SdQuad* tree, int root, const DisneyVertex* dv, Sobol& sb,
+                                            BsdfSample& bs) {
     const float uBranch = get1D(sb);
     if (uBranch < 0.5f) {
         float gPdf = 0.0f;
         const V3 gwi = sdTreeSample(tree, root, get2D(T, sb), gPdf);
         if (!(gPdf > 0.0f)) return false;
         float bPdf = 0.0f;
-        const V3 f = bsdfEvalPdf(T, mat, wo, gwi, sp, bPdf, nullptr);
+        const V3 f = bsdfEvalPdfT<-1>(T, mat, wo, gwi, sp, dv, bPdf, nullptr);
         const float mixPdf = 0.5f * gPdf + 0.5f * bPdf;
         if (isBlack(f) || !(mixPdf > 0.0f)) return false;
         bs.wi = gwi;
@@ -815,7 +816,7 @@ static __device__ __noinline__ bool sdGuidedSample(const TablesGPU* T, const Mat
     }
     const float uc = get1D(sb);
     const V2 u2 = get2D(T, sb);
-    if (!bsdfSample(T, mat, wo, sp, uc, u2, bs)) return false;
+    if (!bsdfSampleT<-1>(T, mat, wo, sp, dv, uc, u2, bs)) return false;
     if (bs.subsurface) bs.weight = bs.weight * 2.0f;
     else if (bs.delta || bs.passThrough) bs.pdf *= 0.5f;
     else if (bs.pdf > 0.0f) bs.pdf = 0.5f * bs.pdf + 0.5f * sdTreePdf(tree, root, bs.wi);
@@ -1260,6 +1261,9 @@ __device__ __forceinline__ bool shadeSlot(const SceneGPU& S, const Paths& P, con
         sp.frontFace = is.frontFace;
         sp.wavelength = lambda;
         const bool isSpecular = (mat.flags & MF_DELTA) != 0;
+        DisneyVertex disney;
+        const DisneyVertex* dv = &disney;
+        if (MT == kDisneyType || (MT < 0 && mat.type == kDisneyType)) disneyVertex(T, mat, wo, sp, disney);
         // this bounce's proposal, when the inference kernel left one for the slot
         const bool useGuide = !LEAN && P.guiding == 2 && guidable(mat) && P.guideMark[slot] != 0u;
         if (useGuide) P.guideMark[slot] = 0u;
@@ -1300,7 +1304,7 @@ __device__ __forceinline__ bool shadeSlot(const SceneGPU& S, const Paths& P, con
                 float bsdfPdf = 0.0f;
                 LobeSplit3 split;
                 const bool firstShares = (OUT && P.pass) && depth == 0;
-                const V3 f = bsdfEvalPdfT<MT>(T, mat, wo, ls.wi, sp, bsdfPdf, firstShares ? &split : nullptr);
+                const V3 f = bsdfEvalPdfT<MT>(T, mat, wo, ls.wi, sp, dv, bsdfPdf, firstShares ? &split : nullptr);
                 const float cosTheta = fabsf(dot(ls.wi, is.normal));
                 if (isBlack(f) || !(cosTheta > 0.0f)) continue;
                 const float lightPdf = lightPmf * ls.pdf;
@@ -1370,13 +1374,13 @@ __device__ __forceinline__ bool shadeSlot(const SceneGPU& S, const Paths& P, con
         BsdfSample bs;
         bool sampled;
         if (useGuide) {
-            sampled = guidedSample(T, mat, wo, sp, P, slot, sb, bs);
+            sampled = guidedSample(T, mat, wo, sp, P, slot, dv, sb, bs);
         } else if (sdRoot >= 0) {
-            sampled = sdGuidedSample(T, mat, wo, sp, P.sd.samp, sdRoot, sb, bs);
+            sampled = sdGuidedSample(T, mat, wo, sp, P.sd.samp, sdRoot, dv, sb, bs);
         } else {
             const float uc = get1D(sb);
             const V2 u2 = get2D(T, sb);
-            sampled = bsdfSampleT<MT>(T, mat, wo, sp, uc, u2, bs);
+            sampled = bsdfSampleT<MT>(T, mat, wo, sp, dv, uc, u2, bs);
         }
         if (!sampled) {
             done = true;
@@ -1385,8 +1389,7 @@ __device__ __forceinline__ bool shadeSlot(const SceneGPU& S, const Paths& P, con
             // in the columns it does not need (lastP, lastN, pickP.x)
             V3 sigT, alb;
             float g = 0.0f;
-            const DisneyParams dp = disneyResolve(mat, sp);
-            if (!disneySubsurfaceCoeffs(mat, dp, sigT, alb, g)) {
+            if (!disneySubsurfaceCoeffs(mat, dv->p, sigT, alb, g)) {
                 done = true;
             } else {
                 thr *= bs.weight;
@@ -1428,7 +1431,7 @@ __device__ __forceinline__ bool shadeSlot(const SceneGPU& S, const Paths& P, con
                 } else {
                     LobeSplit3 split;
                     float unusedPdf = 0.0f;
-                    (void)bsdfEvalPdfT<MT>(T, mat, wo, wi, sp, unusedPdf, &split);
+                    (void)bsdfEvalPdfT<MT>(T, mat, wo, wi, sp, dv, unusedPdf, &split);
                     lobeShares(split, sh);
                 }
                 float4* b = passBlock(P, path);
@@ -1588,22 +1591,17 @@ __device__ __forceinline__ void shadeBin(const SceneGPU& S, const Paths& P, cons
     }
 }
 
-// The lean shading kernels of a bounce (waves of lean-shading scenes without guiding): the misses,
-// whose code is small (75 registers), and the surfaces, whose four kinds follow each other in one
-// launch at 128 registers (four 128-thread blocks per SM), so that one kind's last warps overlap the
-// next kind's first.
-template <bool OUT>
-__global__ void __launch_bounds__(128) kShadeMiss(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P,
-                                                  const __grid_constant__ Wave W, int32_t* nextQueue) {
-    shadeBin<OUT, 0>(S, P, W, nextQueue);
-}
-template <bool OUT>
-__global__ void __launch_bounds__(128, 4) kShadeSurface(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P,
-                                                        const __grid_constant__ Wave W, int32_t* nextQueue) {
-    shadeBin<OUT, 2>(S, P, W, nextQueue);
-    shadeBin<OUT, 1>(S, P, W, nextQueue);
-    shadeBin<OUT, 3>(S, P, W, nextQueue);
-    shadeBin<OUT, 4>(S, P, W, nextQueue);
+// The lean shading kernels (waves of lean-shading scenes without guiding), one per shading key.  They
+// wait for memory and instructions more than they issue, so blocks on the SM count for more than
+// registers: at least MINB 128-thread blocks per SM (96 registers for Lambert, 80 for Disney) — shading
+// of the 1920x1080 x 4-spp knot wave 9.5 / 7.1 / 6.7 / 6.4 / 6.3 ms at 2 / 4 / 5 / 6 / 8 blocks, of the
+// Cornell wave 4.20 / 2.85 / 2.70 / 2.82 / 3.24 ms.  All surface kinds in one launch
+// measured slower: the compiler keeps what the kinds share in registers across them and spills 1.2 KB
+// a thread (Cornell, Lambert alone: 3.11 against 2.84 ms of shading per 4.2M-path wave).
+template <bool OUT, int KEY, int MINB>
+__global__ void __launch_bounds__(128, MINB) kShadeKey(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P,
+                                                       const __grid_constant__ Wave W, int32_t* nextQueue) {
+    shadeBin<OUT, KEY>(S, P, W, nextQueue);
 }
 
 // ---- tail: the last paths of a wave, each run to its end by one thread -------------------------
@@ -1986,8 +1984,12 @@ static __global__ void kFilm(const __grid_constant__ Paths P, const __grid_const
 // PE_LEAN_KERNELS(K) and its siblings expand K(kernel) over a unit's instantiations.
 #define PE_SHADE_ARGS                                                                              \
     (const __grid_constant__ SceneGPU, const __grid_constant__ Paths, const __grid_constant__ Wave, int32_t*)
-#define PE_LEAN_KERNELS(K) K(kShadeMiss<false>) K(kShadeSurface<false>)
-#define PE_LEAN_OUT_KERNELS(K) K(kShadeMiss<true>) K(kShadeSurface<true>)
+#define PE_LEAN_KERNELS(K)                                                                         \
+    K(kShadeKey<false, 0, 1>) K(kShadeKey<false, 1, 5>) K(kShadeKey<false, 2, 6>)                  \
+    K(kShadeKey<false, 3, 5>) K(kShadeKey<false, 4, 5>)
+#define PE_LEAN_OUT_KERNELS(K)                                                                     \
+    K(kShadeKey<true, 0, 1>) K(kShadeKey<true, 1, 5>) K(kShadeKey<true, 2, 6>)                     \
+    K(kShadeKey<true, 3, 5>) K(kShadeKey<true, 4, 5>)
 #define PE_FULL_KERNELS(K) K(kShade<false, false>) K(kShade<false, true>)
 #define PE_FULL_OUT_KERNELS(K) K(kShade<true, false>) K(kShade<true, true>)
 #define PE_TAIL_ARGS                                                                               \
