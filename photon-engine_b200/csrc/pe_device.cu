@@ -404,12 +404,12 @@ int launchTrace(pe_device* d, const SceneGPU& S, const Paths& P, const Wave& W, 
             else kShadowAny<false><<<d->blocksShadowAny, 128, 0, cs>>>(S, P, st);
         }
     } else {
-        const int sh = shadows ? 1 : 0, grid = d->blocksIntersect;
-        const bool scatter = S.hasVolumes || S.hasSubsurface;
-        if (d->counting && scatter) kTrace<true, true><<<grid, 128, 0, cs>>>(S, P, W, q, sh, st);
-        else if (d->counting) kTrace<true, false><<<grid, 128, 0, cs>>>(S, P, W, q, sh, st);
-        else if (scatter) kTrace<false, true><<<grid, 128, 0, cs>>>(S, P, W, q, sh, st);
-        else kTrace<false, false><<<grid, 128, 0, cs>>>(S, P, W, q, sh, st);
+        const auto trace = [&](auto kernel) { kernel<<<d->blocksIntersect, 128, 0, cs>>>(S, P, W, q, shadows ? 1 : 0, st); };
+        const bool scatter = S.hasVolumes || S.hasSubsurface, inst = S.nInstances > 0;
+        if (d->counting) scatter ? (inst ? trace(kTrace<true, true, true>) : trace(kTrace<true, true, false>))
+                                 : (inst ? trace(kTrace<true, false, true>) : trace(kTrace<true, false, false>));
+        else scatter ? (inst ? trace(kTrace<false, true, true>) : trace(kTrace<false, true, false>))
+                     : (inst ? trace(kTrace<false, false, true>) : trace(kTrace<false, false, false>));
     }
     kBin<<<d->prop.multiProcessorCount * 8, 256, 0, cs>>>(S, P, q);
     return n;
@@ -1379,7 +1379,7 @@ pe_device* pe_device_create(int32_t ordinal, char* err, size_t errLen) {
     cudaMemcpy(d->dTables, &d->hTables, sizeof(TablesGPU), cudaMemcpyHostToDevice);
     int b = 0;
     const int sm = d->prop.multiProcessorCount;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kTrace<false, true>, 128, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kTrace<false, true, true>, 128, 0);
     d->blocksIntersect = sm * std::max(1, b);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kShade<false, false>, 128, 0);
     d->blocksShade = sm * std::max(1, b);

@@ -356,7 +356,7 @@ static __device__ __noinline__ int mediumSegment(const TablesGPU* T, const MatGP
     return SEG_SURFACE;
 }
 
-// The next segment of a path that scatters before the hit (t, u, v, prim) of its current ray: a step
+// The next segment of a path that scatters before the hit its current ray has in P.hit: a step
 // of a random subsurface walk (shadeSlot's PF_WALK state, path_tracer.cpp:263-303) or an event in the
 // medium the ray is in (mediumSegment).  True: the path's state has moved on to the segment `next`.
 // False, and nothing is changed: the ray's end is shadeSlot's to handle, which draws the same numbers.
@@ -364,8 +364,10 @@ struct ScatterRay {
     V3 o, d;
     uint32_t mask;
 };
-static __device__ __noinline__ bool scatterOn(const SceneGPU& S, const Paths& P, const Wave& W, int slot, float t, float u,
-                                              float v, int prim, ScatterRay& next) {
+static __device__ __noinline__ bool scatterOn(const SceneGPU& S, const Paths& P, const Wave& W, int slot, ScatterRay& next) {
+    const float4 hr = P.hit[slot];
+    const float t = hr.x, u = hr.y, v = hr.z;
+    const int prim = __float_as_int(hr.w);
     const float4 ro = P.rayO[slot];
     const uint32_t mask = __float_as_uint(ro.w);
     const bool walk = (mask & RAY_WALK) != 0;
@@ -583,10 +585,9 @@ __global__ void __launch_bounds__(128) kShadow(const __grid_constant__ SceneGPU 
 // segments a bounce: the bounce lasts as long as its longest chain (1280x720 x 4-spp media wave, rays
 // and shading and tail together: 19.8 ms at 2 and at 4, 20.7 at 8, 21.5 at 16, 30 unbounded, 21.7 at 0).
 constexpr int kScatterChain = 4;
-template <bool COUNT, bool SCATTER>
+template <bool COUNT, bool SCATTER, bool INSTANCES>
 __device__ __forceinline__ void traceQueue(const SceneGPU& S, const Paths& P, const Wave& W, const int32_t* queue,
-                                           uint2* stack, int root, bool instances, uint32_t& nodes, uint32_t& tris,
-                                           uint32_t& segments) {
+                                           uint2* stack, int root, uint32_t& nodes, uint32_t& tris, uint32_t& segments) {
     WarpFeed feed{&P.now[BC_WORK_ISECT], static_cast<int>(P.now[BC_QUEUE])};
     int slot = -1, chain = 0;
     RayWalk w;
@@ -594,16 +595,15 @@ __device__ __forceinline__ void traceQueue(const SceneGPU& S, const Paths& P, co
     for (;;) {
         const unsigned idle = __ballot_sync(kWarp, w.cur == kRayDone);
         if (idle == kWarp || (!feed.dry() && __popc(idle) >= kRefill)) {
-            // ended rays: their hits; then the queue's next rays
+            // ended rays (a hit is in P.hit already); then the queue's next rays
             if (w.cur == kRayDone && slot >= 0) {
                 ScatterRay next;
-                if (SCATTER && chain < kScatterChain &&
-                    scatterOn(S, P, W, slot, w.tMax, w.u, w.v, w.prim, next)) {
+                if (w.prim == -1) P.hit[slot] = make_float4(w.tMax, 0.0f, 0.0f, __int_as_float(-1));
+                if (SCATTER && chain < kScatterChain && scatterOn(S, P, W, slot, next)) {
                     w.start(S, root, next.o, next.d, next.mask, 1e30f, -1);
                     ++segments;
                     ++chain;
                 } else {
-                    P.hit[slot] = make_float4(w.tMax, w.u, w.v, __int_as_float(w.prim));
                     slot = -1;
                 }
             }
@@ -618,23 +618,24 @@ __device__ __forceinline__ void traceQueue(const SceneGPU& S, const Paths& P, co
             if (__all_sync(kWarp, slot < 0)) break;
             continue;
         }
-        walkTurn<WALK_CLOSEST, COUNT>(
-            S, w, stack, instances, nodes, tris,
+        walkTurn<WALK_CLOSEST, COUNT, INSTANCES>(
+            S, w, stack, nodes, tris,
             [&](V3& o, V3& d, uint32_t& mask) {
                 const float4 ro = P.rayO[slot], rd = P.rayD[slot];
                 o = mk(ro.x, ro.y, ro.z);
                 d = mk(rd.x, rd.y, rd.z);
                 mask = __float_as_uint(ro.w);
             },
-            [&]() { return pathTime(S, P, slot); });
+            [&]() { return pathTime(S, P, slot); },
+            [&](float t, float u, float v, int prim) { P.hit[slot] = make_float4(t, u, v, __int_as_float(prim)); });
         __syncwarp();
     }
 }
 
 // The plain any-hit queries of the shadow records, a ray per lane.
-template <bool COUNT>
-__device__ __forceinline__ void traceShadows(const SceneGPU& S, const Paths& P, uint32_t* stack, int root, bool instances,
-                                             uint32_t& nodes, uint32_t& tris) {
+template <bool COUNT, bool INSTANCES>
+__device__ __forceinline__ void traceShadows(const SceneGPU& S, const Paths& P, uint32_t* stack, int root, uint32_t& nodes,
+                                             uint32_t& tris) {
     WarpFeed feed{&P.now[BC_WORK_SHADOW], static_cast<int>(P.now[BC_SHADOW])};
     int rec = -1;
     RayWalk w;
@@ -657,15 +658,15 @@ __device__ __forceinline__ void traceShadows(const SceneGPU& S, const Paths& P, 
             if (__all_sync(kWarp, rec < 0)) break;
             continue;
         }
-        walkTurn<WALK_ANY, COUNT>(
-            S, w, stack, instances, nodes, tris,
+        walkTurn<WALK_ANY, COUNT, INSTANCES>(
+            S, w, stack, nodes, tris,
             [&](V3& o, V3& d, uint32_t& mask) {
                 const float4 so = P.shO[rec], sd = P.shD[rec];
                 o = mk(so.x, so.y, so.z);
                 d = mk(sd.x, sd.y, sd.z);
                 mask = VIS_SHADOW;
             },
-            [&]() { return pathTime(S, P, P.shadowQ[rec]); });
+            [&]() { return pathTime(S, P, P.shadowQ[rec]); }, [](float, float, float, int) {});
         __syncwarp();
     }
 }
@@ -675,17 +676,16 @@ __device__ __forceinline__ void traceShadows(const SceneGPU& S, const Paths& P, 
 // radiance that the next shading reads), and a launch's time for a short queue is that of its longest
 // ray; warps that run out of closest hits go on with shadow rays while the long ones finish.
 // SCATTER: the scene has media or subsurface walks (scatterOn's call costs the others 6 %).
-template <bool COUNT, bool SCATTER>
+template <bool COUNT, bool SCATTER, bool INSTANCES>
 __global__ void __launch_bounds__(128, 8) kTrace(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P,
                                                  const __grid_constant__ Wave W, const int32_t* queue, int shadows,
                                                  unsigned long long* stats) {
-    uint2 stack[kWalkStack];
+    uint2 stack[walkStack(INSTANCES)];
     const int root = rootRef(S);
-    const bool instances = S.nInstances > 0;
     uint32_t nodes = 0, tris = 0, shNodes = 0, shTris = 0, segments = 0;
-    traceQueue<COUNT, SCATTER>(S, P, W, queue, stack, root, instances, nodes, tris, segments);
+    traceQueue<COUNT, SCATTER, INSTANCES>(S, P, W, queue, stack, root, nodes, tris, segments);
     if (segments) atomicAdd(&stats[8], static_cast<unsigned long long>(segments));
-    if (shadows) traceShadows<COUNT>(S, P, reinterpret_cast<uint32_t*>(stack), root, instances, shNodes, shTris);
+    if (shadows) traceShadows<COUNT, INSTANCES>(S, P, reinterpret_cast<uint32_t*>(stack), root, shNodes, shTris);
     if (COUNT) {
         atomicAdd(&stats[0], static_cast<unsigned long long>(nodes));
         atomicAdd(&stats[1], static_cast<unsigned long long>(tris));
@@ -698,9 +698,9 @@ __global__ void __launch_bounds__(128, 8) kTrace(const __grid_constant__ SceneGP
 template <bool COUNT>
 __global__ void __launch_bounds__(128, 8) kShadowAny(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P,
                                                      unsigned long long* stats) {
-    uint32_t stack[kWalkStack];
+    uint32_t stack[walkStack(true)];
     uint32_t nodes = 0, tris = 0;
-    traceShadows<COUNT>(S, P, stack, rootRef(S), S.nInstances > 0, nodes, tris);
+    traceShadows<COUNT, true>(S, P, stack, rootRef(S), nodes, tris);
     if (COUNT) {
         atomicAdd(&stats[2], static_cast<unsigned long long>(nodes));
         atomicAdd(&stats[3], static_cast<unsigned long long>(tris));
@@ -1723,13 +1723,12 @@ __global__ void __launch_bounds__(kTailWarpsBlock) kTailWarps(const __grid_const
     __shared__ int slots[kTailWarpsBlock];
     __shared__ int blocked[kTailWarpsBlock];
     __shared__ uint8_t owners[kTailWarpsBlock / 32][64]; // each warp's rays: the lane they belong to, closest hits first
-    uint2 stack[kWalkStack];
+    uint2 stack[walkStack(true)];
     const int n = static_cast<int>(*count);
     const int tid = threadIdx.x, lane = tid & 31, warpBase = tid & ~31;
     const unsigned below = (1u << lane) - 1u;
     uint8_t* own = owners[tid >> 5];
     const int root = rootRef(S);
-    const bool instances = S.nInstances > 0;
     const bool scattering = (S.hasVolumes | S.hasSubsurface) != 0;
     uint32_t unused = 0, rays = 0, shRays = 0;
     int slot = -1, path = 0, q = 0;
@@ -1772,12 +1771,14 @@ __global__ void __launch_bounds__(kTailWarpsBlock) kTailWarps(const __grid_const
                     if (w.any) {
                         blocked[ray] = w.prim;
                         ray = -1;
-                    } else if (!LEAN && scattering && scatterOn(S, P, W, slots[ray], w.tMax, w.u, w.v, w.prim, next)) {
-                        w.start(S, root, next.o, next.d, next.mask, 1e30f, -1);
-                        ++rays;
                     } else {
-                        P.hit[slots[ray]] = make_float4(w.tMax, w.u, w.v, __int_as_float(w.prim));
-                        ray = -1;
+                        if (w.prim == -1) P.hit[slots[ray]] = make_float4(w.tMax, 0.0f, 0.0f, __int_as_float(-1));
+                        if (!LEAN && scattering && scatterOn(S, P, W, slots[ray], next)) {
+                            w.start(S, root, next.o, next.d, next.mask, 1e30f, -1);
+                            ++rays;
+                        } else {
+                            ray = -1;
+                        }
                     }
                 }
                 const unsigned without = __ballot_sync(kWarp, ray < 0);
@@ -1799,15 +1800,16 @@ __global__ void __launch_bounds__(kTailWarpsBlock) kTailWarps(const __grid_const
                 if (__all_sync(kWarp, ray < 0)) break;
                 continue;
             }
-            walkTurn<WALK_MIXED, false>(
-                S, w, stack, instances, unused, unused,
+            walkTurn<WALK_MIXED, false, true>(
+                S, w, stack, unused, unused,
                 [&](V3& o, V3& d, uint32_t& mask) {
                     const float4 ro = w.any ? recs[ray].o : P.rayO[slots[ray]], rd = w.any ? recs[ray].d : P.rayD[slots[ray]];
                     o = mk(ro.x, ro.y, ro.z);
                     d = mk(rd.x, rd.y, rd.z);
                     mask = w.any ? static_cast<uint32_t>(VIS_SHADOW) : __float_as_uint(ro.w);
                 },
-                [&]() { return pathTime(S, P, slots[ray]); });
+                [&]() { return pathTime(S, P, slots[ray]); },
+                [&](float t, float u, float v, int prim) { P.hit[slots[ray]] = make_float4(t, u, v, __int_as_float(prim)); });
             __syncwarp();
         }
         __syncthreads(); // the block shades together; hits and answers are visible
@@ -2005,7 +2007,10 @@ static __global__ void kFilm(const __grid_constant__ Paths P, const __grid_const
 #define PE_TRACE_ARGS                                                                              \
     (const __grid_constant__ SceneGPU, const __grid_constant__ Paths, const __grid_constant__ Wave, const int32_t*, int, \
      unsigned long long*)
-#define PE_TRACE_KERNELS(K) K(kTrace<false, false>) K(kTrace<false, true>) K(kTrace<true, false>) K(kTrace<true, true>)
+#define PE_TRACE_KERNELS(K)                                                                        \
+    K(kTrace<false, false, false>) K(kTrace<false, true, false>) K(kTrace<true, false, false>)     \
+    K(kTrace<true, true, false>) K(kTrace<false, false, true>) K(kTrace<false, true, true>)        \
+    K(kTrace<true, false, true>) K(kTrace<true, true, true>)
 #define PE_BINARY_ARGS                                                                             \
     (const __grid_constant__ SceneGPU, const __grid_constant__ Paths, const int32_t*, unsigned long long*)
 #define PE_BINARY_KERNELS(K) K(kIntersectBinary<false>) K(kIntersectBinary<true>)
