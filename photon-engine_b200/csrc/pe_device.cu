@@ -63,6 +63,7 @@ int32_t allocLane(WaveLane& ln, size_t slots) {
         if ((st = devAlloc(ln.bufs, *c, slots))) return st;
     if ((st = devAlloc(ln.bufs, P.queueA, slots))) return st;
     if ((st = devAlloc(ln.bufs, P.queueB, slots))) return st;
+    if ((st = devAlloc(ln.bufs, P.key, slots))) return st;
     if ((st = devAlloc(ln.bufs, P.sortQ, slots * kShadeKeys))) return st;
     // shadow records: one per slot (shadow quality 1)
     if ((st = devAlloc(ln.bufs, P.shadowQ, slots))) return st;
@@ -411,7 +412,7 @@ int launchTrace(pe_device* d, const SceneGPU& S, const Paths& P, const Wave& W, 
         else scatter ? (inst ? trace(kTrace<false, true, true>) : trace(kTrace<false, true, false>))
                      : (inst ? trace(kTrace<false, false, true>) : trace(kTrace<false, false, false>));
     }
-    kBin<<<d->prop.multiProcessorCount * 8, 256, 0, cs>>>(S, P, q);
+    kBin<<<d->prop.multiProcessorCount * 8, kBinBlock, 0, cs>>>(S, P, q);
     return n;
 }
 

@@ -223,21 +223,6 @@ static __global__ void kInitFree(const __grid_constant__ Paths P, int n) {
 // that the four-lane walk replaced).
 enum TraceMode { TRACE_BINARY = 0, TRACE_MODES = 10 };
 
-// Warp-aggregated append of each lane's slot into its key's bin (key < 0: none): one atomic per
-// distinct key per warp.
-__device__ __forceinline__ void binByKey(const Paths& P, int key, int slot) {
-    const int lane = threadIdx.x & 31;
-    const unsigned peers = __match_any_sync(0xffffffffu, key);
-    if (key >= 0) {
-        const int leader = __ffs(peers) - 1;
-        const int rank = __popc(peers & ((1u << lane) - 1u));
-        uint32_t at = 0;
-        if (lane == leader) at = atomicAdd(&P.now[BC_KEYS + key], static_cast<uint32_t>(__popc(peers)));
-        at = __shfl_sync(peers, at, leader);
-        P.sortQ[static_cast<size_t>(key) * P.capacity + at + rank] = slot;
-    }
-}
-
 // The shading key of a closest hit by its primitive.
 __device__ __forceinline__ int shadeKeyOfPrim(const SceneGPU& S, uint32_t rayMask, int prim) {
     if (rayMask & RAY_WALK) return kShadeKeys - 1;
@@ -246,23 +231,67 @@ __device__ __forceinline__ int shadeKeyOfPrim(const SceneGPU& S, uint32_t rayMas
     return 1 + static_cast<int>((__float_as_uint(__ldg(&S.tris[3 * prim + 1]).w) >> 8) & 0xFFu);
 }
 
+// The shading key of a hit by the record of its triangle or sphere.
+__device__ __forceinline__ uint8_t shadeKeyOfMeta(uint32_t rayMask, uint32_t meta) {
+    return static_cast<uint8_t>((rayMask & RAY_WALK) ? kShadeKeys - 1 : 1 + ((meta >> 8) & 0xFFu));
+}
+
 // The queue's slots into the bins of their hits' shading keys.  A pass of its own rather than the
 // end of each ray's walk: rays end in any order, and bins in that order made the shading kernels'
 // state reads scatter (8.3 against 7.1 ms of shading per 8.3M-path knot wave); here a bin keeps the
-// queue's order but for the interleaving of warps.
-static __global__ void kBin(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P, const int32_t* queue) {
+// queue's order but for the interleaving of blocks.  Bound by the latency of its loads and of the bins'
+// counters: the walk leaves a ray's key in a byte (instances' hits excepted), and a block takes each
+// bin's share for 1024 entries at once: 30 -> 11 us per million rays (traversal and binning of the
+// 256x256 x 64-spp Cornell wave 2.48 -> 2.21 ms, of the 1920x1080 x 4-spp knot wave 6.86 -> 6.53 ms).
+constexpr int kBinBlock = 256, kBinEach = 4;
+static __global__ void __launch_bounds__(kBinBlock) kBin(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P, const int32_t* queue) {
+    constexpr int kWarps = kBinBlock / 32;
+    __shared__ uint32_t count[kWarps][kShadeKeys], first[kWarps][kShadeKeys];
     const int n = static_cast<int>(P.now[BC_QUEUE]);
-    const int stride = gridDim.x * blockDim.x;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (blockIdx.x == 0 && threadIdx.x < kBounceBlock) P.next[threadIdx.x] = 0u; // the next bounce's counters
-    for (int base = blockIdx.x * blockDim.x; base < n; base += stride) {
-        const int i = base + static_cast<int>(threadIdx.x);
-        int key = -1, slot = -1;
-        if (i < n) {
-            slot = queue[i];
-            const uint32_t mask = S.hasSubsurface ? __float_as_uint(P.rayO[slot].w) : 0u;
-            key = shadeKeyOfPrim(S, mask, __float_as_int(P.hit[slot].w));
+    for (int base = blockIdx.x * kBinBlock * kBinEach; base < n; base += gridDim.x * kBinBlock * kBinEach) {
+        int slot[kBinEach], key[kBinEach];
+        uint32_t rank[kBinEach]; // among the warp's entries of the same key
+        uint32_t mine = 0;       // lane k: the warp's entries of key k
+#pragma unroll
+        for (int j = 0; j < kBinEach; ++j) {
+            const int i = base + (warp * kBinEach + j) * 32 + lane;
+            slot[j] = i < n ? queue[i] : -1;
         }
-        binByKey(P, key, slot);
+#pragma unroll
+        for (int j = 0; j < kBinEach; ++j) key[j] = slot[j] >= 0 ? P.key[slot[j]] : -1;
+#pragma unroll
+        for (int j = 0; j < kBinEach; ++j) {
+            if (key[j] == kKeyOfPrim) {
+                const uint32_t mask = S.hasSubsurface ? __float_as_uint(P.rayO[slot[j]].w) : 0u;
+                key[j] = shadeKeyOfPrim(S, mask, __float_as_int(P.hit[slot[j]].w));
+            }
+            const unsigned peers = __match_any_sync(kWarp, key[j]);
+            rank[j] = __popc(peers & ((1u << lane) - 1u)) + __shfl_sync(kWarp, mine, key[j] < 0 ? 0 : key[j]);
+#pragma unroll
+            for (int k = 0; k < kShadeKeys; ++k) {
+                const uint32_t c = __popc(__ballot_sync(kWarp, key[j] == k));
+                if (lane == k) mine += c;
+            }
+        }
+        if (lane < kShadeKeys) count[warp][lane] = mine;
+        __syncthreads();
+        if (threadIdx.x < kShadeKeys) {
+            uint32_t total = 0;
+#pragma unroll
+            for (int w = 0; w < kWarps; ++w) total += count[w][threadIdx.x];
+            uint32_t at = total ? atomicAdd(&P.now[BC_KEYS + threadIdx.x], total) : 0u;
+#pragma unroll
+            for (int w = 0; w < kWarps; ++w) {
+                first[w][threadIdx.x] = at;
+                at += count[w][threadIdx.x];
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < kBinEach; ++j)
+            if (key[j] >= 0) P.sortQ[static_cast<size_t>(key[j]) * P.capacity + first[warp][key[j]] + rank[j]] = slot[j];
     }
 }
 
@@ -283,6 +312,7 @@ __global__ void __launch_bounds__(128) kIntersectBinary(const __grid_constant__ 
         const Hit h = traceClosest<COUNT>(S, mk(ro.x, ro.y, ro.z), mk(rd.x, rd.y, rd.z), __float_as_uint(ro.w), 0.0f, 1e30f,
                                           nodes, tris, pathTime(S, P, slot));
         P.hit[slot] = make_float4(h.t, h.u, h.v, __int_as_float(h.prim));
+        P.key[slot] = kKeyOfPrim;
     }
     if (COUNT) {
         atomicAdd(&stats[0], static_cast<unsigned long long>(nodes));
@@ -598,7 +628,10 @@ __device__ __forceinline__ void traceQueue(const SceneGPU& S, const Paths& P, co
             // ended rays (a hit is in P.hit already); then the queue's next rays
             if (w.cur == kRayDone && slot >= 0) {
                 ScatterRay next;
-                if (w.prim == -1) P.hit[slot] = make_float4(w.tMax, 0.0f, 0.0f, __int_as_float(-1));
+                if (w.prim == -1) {
+                    P.hit[slot] = make_float4(w.tMax, 0.0f, 0.0f, __int_as_float(-1));
+                    P.key[slot] = static_cast<uint8_t>((w.mask & RAY_WALK) ? kShadeKeys - 1 : 0);
+                }
                 if (SCATTER && chain < kScatterChain && scatterOn(S, P, W, slot, next)) {
                     w.start(S, root, next.o, next.d, next.mask, 1e30f, -1);
                     ++segments;
@@ -627,7 +660,10 @@ __device__ __forceinline__ void traceQueue(const SceneGPU& S, const Paths& P, co
                 mask = __float_as_uint(ro.w);
             },
             [&]() { return pathTime(S, P, slot); },
-            [&](float t, float u, float v, int prim) { P.hit[slot] = make_float4(t, u, v, __int_as_float(prim)); });
+            [&](float t, float u, float v, int prim, uint32_t meta) {
+                P.hit[slot] = make_float4(t, u, v, __int_as_float(prim));
+                P.key[slot] = INSTANCES && w.inst >= 0 ? kKeyOfPrim : shadeKeyOfMeta(w.mask, meta);
+            });
         __syncwarp();
     }
 }
@@ -666,7 +702,7 @@ __device__ __forceinline__ void traceShadows(const SceneGPU& S, const Paths& P, 
                 d = mk(sd.x, sd.y, sd.z);
                 mask = VIS_SHADOW;
             },
-            [&]() { return pathTime(S, P, P.shadowQ[rec]); }, [](float, float, float, int) {});
+            [&]() { return pathTime(S, P, P.shadowQ[rec]); }, [](float, float, float, int, uint32_t) {});
         __syncwarp();
     }
 }
@@ -1809,7 +1845,7 @@ __global__ void __launch_bounds__(kTailWarpsBlock) kTailWarps(const __grid_const
                     mask = w.any ? static_cast<uint32_t>(VIS_SHADOW) : __float_as_uint(ro.w);
                 },
                 [&]() { return pathTime(S, P, slots[ray]); },
-                [&](float t, float u, float v, int prim) { P.hit[slots[ray]] = make_float4(t, u, v, __int_as_float(prim)); });
+                [&](float t, float u, float v, int prim, uint32_t) { P.hit[slots[ray]] = make_float4(t, u, v, __int_as_float(prim)); });
             __syncwarp();
         }
         __syncthreads(); // the block shades together; hits and answers are visible

@@ -107,7 +107,7 @@ enum WalkKind { WALK_CLOSEST, WALK_ANY, WALK_MIXED };
 
 // One turn of the walk for every lane of the warp that has a reference.  T: uint2 (reference, entry distance), or for any hit uint32_t (reference).
 // world(o, d, mask) gives the lane's ray back when it leaves an instance, time() its shutter time;
-// found(t, u, v, prim) takes a closest hit nearer than (or as near as) those before it.
+// found(t, u, v, prim, meta) takes a closest hit nearer than (or as near as) those before it.
 // INSTANCES: the scene has mesh instances.
 template <WalkKind KIND, bool COUNT, bool INSTANCES, typename T, typename World, typename Time, typename Found>
 __device__ __forceinline__ void walkTurn(const SceneGPU& S, RayWalk& w, T* stack, uint32_t& nodeVisits, uint32_t& triTests,
@@ -202,7 +202,7 @@ __device__ __forceinline__ void walkTurn(const SceneGPU& S, RayWalk& w, T* stack
                     } else {
                         w.tMax = t;
                         w.prim = !INSTANCES || w.inst < 0 ? pi : instanceHitCode(w.inst, pi - S.instances[w.inst].recBase);
-                        found(t, u, v, w.prim);
+                        found(t, u, v, w.prim, meta);
                     }
                 }
             }

@@ -70,6 +70,7 @@ struct Paths {
     float4* shD;     // shadow direction xyz, scalar (cos*w/(pdf*n))
     float4* shC;     // f*Li xyz, flags (bit0: indirect)
     float4* shT;     // throughput at NEE xyz
+    uint8_t* key;    // shading key of the slot's closest hit, or kKeyOfPrim (kBin)
     int32_t* sortQ;  // kShadeKeys segments of `capacity` slots: rays binned by shading key
     // learned proposal (null / 0 when off)
     float4* guideQ;      // 3 per query row, compacted per bounce: hit point | shading normal | view direction
@@ -133,6 +134,7 @@ enum PassFilms { PFILM_DEPTH = 8, PFILM_POSITION = 9, PFILM_OBJECT = 10, PFILM_M
 
 // Shading keys: 0 = miss, 1 + material type (Lambert, Disney, Dielectric, Mirror), 5 = random-walk step.
 constexpr int kShadeKeys = 6;
+constexpr uint8_t kKeyOfPrim = 255; // Paths::key: kBin derives the key from the hit's primitive
 // Counters of one bounce: the closest-hit queue's entries, the shadow records, the work cursors of
 // the trace and shading kernels, the rays per shading key and their bins' cursors.
 enum BounceCounters { BC_QUEUE = 0, BC_SHADOW = 1, BC_WORK_ISECT = 2, BC_WORK_SHADOW = 3, BC_WORK_SHADE = 4, BC_KEYS = 5,
