@@ -14,39 +14,31 @@
 
 // Compiled in pe_kernels_*.cu.
 namespace pe {
-#define PE_EXTERN(...) extern template __global__ void __VA_ARGS__ PE_SHADE_ARGS;
-PE_LEAN_KERNELS(PE_EXTERN)
-#undef PE_EXTERN
-#define PE_EXTERN(...) extern template __global__ void __VA_ARGS__ PE_SHADE_ARGS;
-PE_LEAN_OUT_KERNELS(PE_EXTERN)
-#undef PE_EXTERN
-#define PE_EXTERN(...) extern template __global__ void __VA_ARGS__ PE_SHADE_ARGS;
-PE_FULL_KERNELS(PE_EXTERN)
-#undef PE_EXTERN
-#define PE_EXTERN(...) extern template __global__ void __VA_ARGS__ PE_SHADE_ARGS;
-PE_FULL_OUT_KERNELS(PE_EXTERN)
-#undef PE_EXTERN
-#define PE_EXTERN(...) extern template __global__ void __VA_ARGS__ PE_TAIL_ARGS;
-PE_TAIL_KERNELS(PE_EXTERN)
-#undef PE_EXTERN
-#define PE_EXTERN(...) extern template __global__ void __VA_ARGS__ PE_TAIL_ARGS;
-PE_LOCKSTEP_KERNELS(PE_EXTERN)
-#undef PE_EXTERN
-#define PE_EXTERN(...) extern template __global__ void __VA_ARGS__ PE_TAIL_WARPS_ARGS;
-PE_TAIL_WARPS_LEAN_KERNELS(PE_EXTERN)
-#undef PE_EXTERN
-#define PE_EXTERN(...) extern template __global__ void __VA_ARGS__ PE_TAIL_WARPS_ARGS;
-PE_TAIL_WARPS_FULL_KERNELS(PE_EXTERN)
-#undef PE_EXTERN
-#define PE_EXTERN(...) extern template __global__ void __VA_ARGS__ PE_TRACE_ARGS;
-PE_TRACE_KERNELS(PE_EXTERN)
-#undef PE_EXTERN
-#define PE_EXTERN(...) extern template __global__ void __VA_ARGS__ PE_BINARY_ARGS;
-PE_BINARY_KERNELS(PE_EXTERN)
-#undef PE_EXTERN
-#define PE_EXTERN(...) extern template __global__ void __VA_ARGS__ PE_SHADOW_ARGS;
-PE_SHADOW_KERNELS(PE_EXTERN)
-#undef PE_EXTERN
+#define PE_K(...) extern template __global__ void __VA_ARGS__ PE_SHADE_ARGS;
+PE_LEAN_KEYS(PE_SHADE_KEY, false)
+PE_LEAN_KEYS(PE_SHADE_KEY, true)
+PE_MEDIA_KERNELS(PE_K)
+PE_GUIDE_KERNELS(PE_K)
+PE_FULL_KERNELS(PE_K)
+PE_FULL_OUT_KERNELS(PE_K)
+#undef PE_K
+#define PE_K(...) extern template __global__ void __VA_ARGS__ PE_TAIL_ARGS;
+PE_TAIL_KERNELS(PE_K)
+PE_LOCKSTEP_KERNELS(PE_K)
+#undef PE_K
+#define PE_K(...) extern template __global__ void __VA_ARGS__ PE_TAIL_WARPS_ARGS;
+PE_TAIL_WARPS_LEAN_KERNELS(PE_K)
+PE_TAIL_WARPS_FULL_KERNELS(PE_K)
+#undef PE_K
+#define PE_K(...) extern template __global__ void __VA_ARGS__ PE_TRACE_ARGS;
+PE_TRACE_KERNELS(PE_K)
+#undef PE_K
+#define PE_K(...) extern template __global__ void __VA_ARGS__ PE_BINARY_ARGS;
+PE_BINARY_KERNELS(PE_K)
+#undef PE_K
+#define PE_K(...) extern template __global__ void __VA_ARGS__ PE_SHADOW_ARGS;
+PE_SHADOW_KERNELS(PE_K)
+#undef PE_K
 } // namespace pe
 
 using namespace pe;
@@ -225,16 +217,17 @@ WaveSeg makeSeg(const pe_camera* cam, const pe_settings* st) {
 }
 
 
-// SceneGPU::leanShading of a scene: true when none of its materials and scene settings use a
-// shading feature that the lean shading kernels compile out.
-int32_t leanShadingOf(const SceneGPU& G, const std::vector<MatGPU>& mats) {
-    if (G.hasVolumes || G.hasSubsurface || G.hasMips || G.hasLightLinks || G.hasShadowLinks || G.catcherShape >= 0)
-        return 0;
+// SceneGPU::features of a scene.
+int32_t featuresOf(const SceneGPU& G, const std::vector<MatGPU>& mats) {
+    int32_t f = 0;
+    if (G.hasVolumes || G.hasSubsurface) f |= FEAT_MEDIA;
+    if (G.hasMips || G.hasLightLinks || G.hasShadowLinks || G.catcherShape >= 0) f |= FEAT_REST;
     for (const MatGPU& m : mats) {
-        if (m.roundEdge > 0.0f || (m.flags & (MF_DISPERSIVE | MF_VOLUME_BOUNDARY | MF_HAS_MEDIUM))) return 0;
-        if (m.type == PE_MAT_DISNEY && (m.opacity < 1.0f || m.texOpacity >= 0)) return 0;
+        if (m.flags & (MF_DISPERSIVE | MF_VOLUME_BOUNDARY | MF_HAS_MEDIUM)) f |= FEAT_MEDIA;
+        if (m.roundEdge > 0.0f) f |= FEAT_REST;
+        if (m.type == PE_MAT_DISNEY && (m.opacity < 1.0f || m.texOpacity >= 0)) f |= FEAT_REST;
     }
-    return 1;
+    return f;
 }
 
 // Scratch of pe_device_render_tile_noalloc: path-state columns, queues, shadow records and
@@ -263,29 +256,39 @@ Paths noAllocPaths(unsigned char* base) {
     return P;
 }
 
-// The lean shading kernels of one bounce, one per shading key whose material type the scene
-// uses (the miss key always); returns the number of launches.
-int launchLeanShade(pe_device* d, const SceneGPU& S, const Paths& P, const Wave& W, int32_t* qOut, cudaStream_t cs, bool out) {
-    int n = 0;
-    auto one = [&](auto kernel, int key) {
-        if (key > 0 && !(S.materialTypes & (1 << (key - 1)))) return;
-        kernel<<<d->blocksShadeKey[out ? 1 : 0][key], 128, 0, cs>>>(S, P, W, qOut);
-        ++n;
-    };
-    if (out) {
-        one(kShadeKey<true, 0, 1>, 0);
-        one(kShadeKey<true, 1, 5>, 1);
-        one(kShadeKey<true, 2, 6>, 2);
-        one(kShadeKey<true, 3, 5>, 3);
-        one(kShadeKey<true, 4, 5>, 4);
-    } else {
-        one(kShadeKey<false, 0, 1>, 0);
-        one(kShadeKey<false, 1, 5>, 1);
-        one(kShadeKey<false, 2, 6>, 2);
-        one(kShadeKey<false, 3, 5>, 3);
-        one(kShadeKey<false, 4, 5>, 4);
+// f(kernel, key) over the per-key shading kernels.
+template <typename F>
+void eachKeyKernel(bool out, F f) {
+#define PE_ONE(OUT, KEY, MINB) f(kShadeKey<OUT, KEY, MINB>, KEY);
+    if (out) { PE_LEAN_KEYS(PE_ONE, true) }
+    else { PE_LEAN_KEYS(PE_ONE, false) }
+#undef PE_ONE
+}
+
+// A bounce's shading; returns the number of launches.  Waves of plain surface scenes (no features): a kernel per
+// shading key whose material type the scene uses (the miss key always).  Others: one kernel over all
+// keys — a kernel per key measured slower for them (media 1280x720 x 4 spp 6.1 -> 6.5 ms of shading,
+// guided room 320x180 x 16 spp 3.45 -> 4.17: their bounces have fewer paths, and each launch its own last warps) —
+// with only the features of scenes with media or walks (6.1 -> 5.7 ms), of guided plain scenes (3.45 -> 3.25 ms),
+// or with all.
+int launchShade(pe_device* d, int features, bool inlineShadows, bool out, const SceneGPU& S, const Paths& P,
+                const Wave& W, int32_t* qOut, cudaStream_t cs) {
+    if (features == 0) {
+        int n = 0;
+        eachKeyKernel(out, [&](auto kernel, int key) {
+            if (key > 0 && !(S.materialTypes & (1 << (key - 1)))) return;
+            kernel<<<d->blocksShadeKey[out ? 1 : 0][key], 128, 0, cs>>>(S, P, W, qOut);
+            ++n;
+        });
+        return n;
     }
-    return n;
+    const auto shade = [&](auto kernel) { kernel<<<d->blocksShade, 128, 0, cs>>>(S, P, W, qOut); };
+    if (inlineShadows) out ? shade(kShade<FEAT_ALL, true, true>) : shade(kShade<FEAT_ALL, false, true>);
+    else if (out) shade(kShade<FEAT_ALL, true, false>);
+    else if (features == FEAT_MEDIA) shade(kShade<FEAT_MEDIA, false, false>);
+    else if (features == FEAT_GUIDE) shade(kShade<FEAT_GUIDE, false, false>);
+    else shade(kShade<FEAT_ALL, false, false>);
+    return 1;
 }
 
 int32_t timerEvent(pe_device* d, RenderTimer& tm, cudaEvent_t& e) {
@@ -369,7 +372,7 @@ bool plainShadows(const SceneGPU& S) { return !S.hasShadowTransmitters && !S.has
 
 // The tail kernel over `n` queued paths (count and cursor on the device) of a wave without pass
 // outputs; `inlineShadows`: its segments take several shadow samples per vertex, `out`: it records AOVs.
-void launchTail(pe_device* d, bool lean, bool inlineShadows, bool out, const SceneGPU& S, const Paths& P, const Wave& W,
+void launchTail(pe_device* d, int features, bool inlineShadows, bool out, const SceneGPU& S, const Paths& P, const Wave& W,
                 const int32_t* queue, const uint32_t* count, uint32_t* cursor, int64_t n, bool traced, cudaStream_t cs) {
     const int hits = traced ? 1 : 0;
     if (inlineShadows || !plainShadows(S)) {
@@ -378,16 +381,17 @@ void launchTail(pe_device* d, bool lean, bool inlineShadows, bool out, const Sce
         kTailLockstep<0><<<grid, kTailLockstepBlock, 0, cs>>>(S, P, W, queue, count, cursor, hits, d->dStats);
         return;
     }
+    const bool lean = features == 0;
     const int64_t warps = static_cast<int64_t>(d->blocksTailWarps[lean ? 1 : 0][out ? 1 : 0]) * (kTailWarpsBlock / 32);
-
     const int perWarp = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(32, (n + warps - 1) / warps)));
     const int64_t perBlock = static_cast<int64_t>(perWarp) * (kTailWarpsBlock / 32);
     const int grid = static_cast<int>(
         std::max<int64_t>(1, std::min<int64_t>(warps / (kTailWarpsBlock / 32), (n + perBlock - 1) / perBlock)));
-    if (lean && out) kTailWarps<true, true><<<grid, kTailWarpsBlock, 0, cs>>>(S, P, W, queue, count, cursor, hits, perWarp, d->dStats);
-    else if (lean) kTailWarps<true, false><<<grid, kTailWarpsBlock, 0, cs>>>(S, P, W, queue, count, cursor, hits, perWarp, d->dStats);
-    else if (out) kTailWarps<false, true><<<grid, kTailWarpsBlock, 0, cs>>>(S, P, W, queue, count, cursor, hits, perWarp, d->dStats);
-    else kTailWarps<false, false><<<grid, kTailWarpsBlock, 0, cs>>>(S, P, W, queue, count, cursor, hits, perWarp, d->dStats);
+    const auto tail = [&](auto kernel) {
+        kernel<<<grid, kTailWarpsBlock, 0, cs>>>(S, P, W, queue, count, cursor, hits, perWarp, d->dStats);
+    };
+    if (lean) out ? tail(kTailWarps<0, true>) : tail(kTailWarps<0, false>);
+    else out ? tail(kTailWarps<FEAT_ALL, true>) : tail(kTailWarps<FEAT_ALL, false>);
 }
 
 // A bounce's ray queries: the closest hits of its queue, with `shadows` the any-hit queries of the
@@ -506,16 +510,16 @@ int32_t runWave(pe_device* d, int lane, Paths& P, int nSegs, int nSlots, int nPi
     int32_t* qIn = P.queueA;
     int32_t* qOut = P.queueB;
     stats.paths += static_cast<uint64_t>(nSlots);
-    // lean shading (one specialised kernel per shading key) for plain surface scenes that
-    // neither guide nor record
     bool noAo = true, inlineShadows = false;
     for (int k = 0; k < nSegs; ++k) {
         noAo = noAo && !(ln.hSegs[k].aoStrength > 0.0f);
         inlineShadows = inlineShadows || ln.hSegs[k].shadowSamples > 1;
     }
-    const bool lean = S.leanShading && !P.guiding && !P.sdMode && noAo && !d->counting && !inlineShadows;
+    // the shading features this wave needs (kernels that count rays or trace shadow rays inline carry all)
+    const int features = d->counting || inlineShadows ? FEAT_ALL
+                                                      : S.features | (P.guiding || P.sdMode ? FEAT_GUIDE : 0) | (noAo ? 0 : FEAT_REST);
     const bool out = P.aovA || P.pass;
-    int64_t tailPaths = d->tailPaths < 0 ? defaultTailPaths(d, lean) : d->tailPaths;
+    int64_t tailPaths = d->tailPaths < 0 ? defaultTailPaths(d, features == 0) : d->tailPaths;
     // the tail kernel runs no inference: keep guided bounces in the wavefront until few paths remain
     if (P.guiding == 2) tailPaths = std::min<int64_t>(tailPaths, kGuideTailPaths);
     auto mark = [&](cudaEvent_t& e) -> int32_t {
@@ -544,7 +548,7 @@ int32_t runWave(pe_device* d, int lane, Paths& P, int nSegs, int nSlots, int nPi
         else if (P.pass || (out && (inlineShadows || !plainShadows(S))))
             kTail<false, true><<<grid, kTailBlock, 0, cs>>>(S, P, W, qIn, count, cursor, traced ? 1 : 0, d->dStats);
         else
-            launchTail(d, lean, inlineShadows, out, S, P, W, qIn, count, cursor, live, traced, cs);
+            launchTail(d, features, inlineShadows, out, S, P, W, qIn, count, cursor, live, traced, cs);
         if ((r = mark(e))) return r;
         spent(tm.tail);
         ++stats.kernel_launches;
@@ -597,12 +601,7 @@ int32_t runWave(pe_device* d, int lane, Paths& P, int nSegs, int nSlots, int nPi
             if ((rc = tail(true))) return rc;
             break;
         }
-        if (lean) stats.kernel_launches += launchLeanShade(d, S, P, W, qOut, cs, out);
-        else if (inlineShadows && out) kShade<true, true><<<d->blocksShade, 128, 0, cs>>>(S, P, W, qOut);
-        else if (inlineShadows) kShade<false, true><<<d->blocksShade, 128, 0, cs>>>(S, P, W, qOut);
-        else if (out) kShade<true, false><<<d->blocksShade, 128, 0, cs>>>(S, P, W, qOut);
-        else kShade<false, false><<<d->blocksShade, 128, 0, cs>>>(S, P, W, qOut);
-        if (!lean) ++stats.kernel_launches;
+        stats.kernel_launches += launchShade(d, features, inlineShadows, out, S, P, W, qOut, cs);
         if ((rc = mark(e))) return rc;
         spent(tm.shade);
         block = 1 - block;
@@ -710,8 +709,7 @@ int32_t loopBounce(pe_device* d, LaneLoop& L, const Wave& W, uint32_t* hSegLeft,
     // the kernels a lone render uses; shadow rays before the bounce's end, as the slots of ended
     // paths are handed on then
     launchTrace(d, S, P, W, L.qIn, false, cs);
-    if (L.lean) launchLeanShade(d, S, P, W, L.qOut, cs, false);
-    else kShade<false, false><<<d->blocksShade, 128, 0, cs>>>(S, P, W, L.qOut);
+    launchShade(d, L.features, false, false, S, P, W, L.qOut, cs);
     L.block = 1 - L.block;
     setBlock(P, L.block);
     std::swap(L.qIn, L.qOut);
@@ -738,7 +736,7 @@ int32_t loopBounce(pe_device* d, LaneLoop& L, const Wave& W, uint32_t* hSegLeft,
         PE_CUDA(cudaEventRecord(L.evReady[sweep], cs));
         PE_CUDA(cudaStreamWaitEvent(L.side, L.evReady[sweep], 0));
         PE_CUDA(cudaMemsetAsync(&L.sweepCursor[sweep], 0, sizeof(uint32_t), L.side));
-        launchTail(d, L.lean, false, false, S, P, W, L.sweepBuf[sweep], &L.sweepCnt[sweep], &L.sweepCursor[sweep],
+        launchTail(d, L.features, false, false, S, P, W, L.sweepBuf[sweep], &L.sweepCnt[sweep], &L.sweepCursor[sweep],
                            static_cast<int64_t>(swept), false, L.side);
         kFlush<<<d->prop.multiProcessorCount * 4, 256, 0, L.side>>>(P, W, L.sweepBuf[sweep], &L.sweepCnt[sweep]);
         PE_CUDA(cudaEventRecord(L.evDone[sweep], L.side));
@@ -758,7 +756,7 @@ int32_t loopTail(pe_device* d, LaneLoop& L, const Wave& W) {
     WaveLane& ln = *L.ln;
     Paths& P = ln.paths;
     const cudaStream_t cs = ln.stream;
-    launchTail(d, L.lean, false, false, L.scene, P, W, L.qIn, &P.now[BC_QUEUE], &P.counters[CNT_WORK_TAIL],
+    launchTail(d, L.features, false, false, L.scene, P, W, L.qIn, &P.now[BC_QUEUE], &P.counters[CNT_WORK_TAIL],
                        static_cast<int64_t>(L.live), false, cs);
     kFlush<<<d->prop.multiProcessorCount * 4, 256, 0, cs>>>(P, W, L.qIn, &P.now[BC_QUEUE]);
     L.live = 0;
@@ -1301,7 +1299,7 @@ int32_t uploadScene(pe_device* d, const pe_scene* s, SceneGPU& G, std::vector<De
     G.nInstances = static_cast<int32_t>(B.instances.size());
     // moving instances: null without, which also keeps the kernels from reading path times
     if (!B.motions.empty() && (rc = upload(d, bufs, G.motions, B.motions))) return rc;
-    G.leanShading = leanShadingOf(G, B.materials);
+    G.features = featuresOf(G, B.materials);
     G.materialTypes = 0;
     for (const MatGPU& m : B.materials) G.materialTypes |= 1 << m.type;
     G.nLightGroups = static_cast<int32_t>(B.groupNames.size());
@@ -1382,7 +1380,7 @@ pe_device* pe_device_create(int32_t ordinal, char* err, size_t errLen) {
     const int sm = d->prop.multiProcessorCount;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kTrace<false, true, true>, 128, 0);
     d->blocksIntersect = sm * std::max(1, b);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kShade<false, false>, 128, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kShade<FEAT_ALL, false, false>, 128, 0);
     d->blocksShade = sm * std::max(1, b);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kShadow<false>, 128, 0);
     d->blocksShadow = sm * std::max(1, b);
@@ -1394,20 +1392,12 @@ pe_device* pe_device_create(int32_t ordinal, char* err, size_t errLen) {
         return sm * std::max(1, nb);
     };
     d->blocksTailLockstep = occ(kTailLockstep<0>, kTailLockstepBlock);
-    d->blocksTailWarps[0][0] = occ(kTailWarps<false, false>, kTailWarpsBlock);
-    d->blocksTailWarps[0][1] = occ(kTailWarps<false, true>, kTailWarpsBlock);
-    d->blocksTailWarps[1][0] = occ(kTailWarps<true, false>, kTailWarpsBlock);
-    d->blocksTailWarps[1][1] = occ(kTailWarps<true, true>, kTailWarpsBlock);
-    d->blocksShadeKey[0][0] = occ(kShadeKey<false, 0, 1>, 128);
-    d->blocksShadeKey[0][1] = occ(kShadeKey<false, 1, 5>, 128);
-    d->blocksShadeKey[0][2] = occ(kShadeKey<false, 2, 6>, 128);
-    d->blocksShadeKey[0][3] = occ(kShadeKey<false, 3, 5>, 128);
-    d->blocksShadeKey[0][4] = occ(kShadeKey<false, 4, 5>, 128);
-    d->blocksShadeKey[1][0] = occ(kShadeKey<true, 0, 1>, 128);
-    d->blocksShadeKey[1][1] = occ(kShadeKey<true, 1, 5>, 128);
-    d->blocksShadeKey[1][2] = occ(kShadeKey<true, 2, 6>, 128);
-    d->blocksShadeKey[1][3] = occ(kShadeKey<true, 3, 5>, 128);
-    d->blocksShadeKey[1][4] = occ(kShadeKey<true, 4, 5>, 128);
+    d->blocksTailWarps[0][0] = occ(kTailWarps<FEAT_ALL, false>, kTailWarpsBlock);
+    d->blocksTailWarps[0][1] = occ(kTailWarps<FEAT_ALL, true>, kTailWarpsBlock);
+    d->blocksTailWarps[1][0] = occ(kTailWarps<0, false>, kTailWarpsBlock);
+    d->blocksTailWarps[1][1] = occ(kTailWarps<0, true>, kTailWarpsBlock);
+    for (int out = 0; out < 2; ++out)
+        eachKeyKernel(out, [&](auto kernel, int key) { d->blocksShadeKey[out][key] = occ(kernel, 128); });
     d->blocksIntersectBinary = occ(kIntersectBinary<false>, 128);
     d->blocksShadowAny = occ(kShadowAny<false>, 128);
     const cudaError_t le = cudaGetLastError();
@@ -1568,7 +1558,7 @@ int32_t pe_device_update_materials(pe_device* d, const pe_scene* s) {
     PE_CUDA(cudaMemcpyAsync(const_cast<MatGPU*>(d->scene.materials), s->build.materials.data(),
                             s->build.materials.size() * sizeof(MatGPU), cudaMemcpyHostToDevice, d->stream));
     PE_CUDA(cudaStreamSynchronize(d->stream));
-    d->scene.leanShading = leanShadingOf(d->scene, s->build.materials);
+    d->scene.features = featuresOf(d->scene, s->build.materials);
     ++d->sceneSerial;
     return PE_OK;
 }

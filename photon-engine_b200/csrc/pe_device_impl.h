@@ -212,7 +212,7 @@ struct pe_device {
     bool counting = false;
     pe_render_stats stats{};
     int blocksIntersect = 0, blocksShade = 0, blocksShadow = 0, blocksGen = 0, blocksTail = 0;
-    int blocksShadeKey[2][5] = {}; // lean shading kernels: [recording AOVs or passes][key]
+    int blocksShadeKey[2][pe::kShadeKeys] = {}; // per-key shading kernels: [recording AOVs or passes][key]
     int blocksShadowAny = 0;
     int blocksTailLockstep = 0;     // 128-thread blocks
     int blocksTailWarps[2][2] = {}; // kTailWarps: [lean shading][AOVs]
@@ -303,7 +303,7 @@ struct LaneLoop {
     int32_t* qOut = nullptr;
     int block = 0;      // bounce block of the next closest-hit queue
     uint32_t live = 0;  // paths in the next closest-hit queue
-    bool lean = false;  // the lean per-key shading kernels (a lean-shading scene, no segment with AO)
+    int features = 0;   // ShadeFeatures of the scene and the open segments
     int freeTop = 0;    // free slots on the stack
     int nextPath = 0;   // wave path index of the next injected path
     int pathCap = 0;    // paths the wave can hold (Lout)

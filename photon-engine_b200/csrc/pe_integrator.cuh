@@ -973,10 +973,9 @@ static __device__ __noinline__ V3 shadowCatcher(const SceneGPU& S, const Isect& 
 // shadow rays go to the any-hit queue or to the caller, or with SHADOW_INLINE are traced here and their terms
 // added to L at once, in the same order.  Returns whether the path goes on.
 //
-// KEY selects a specialised instantiation: -1 the full shader; otherwise a lean one for waves
-// whose scene has SceneGPU::leanShading and that neither guide nor record, with every feature
-// those waves cannot reach compiled out (so the code fits in registers); KEY >= 0 also fixes the
-// shading key (0 a miss, 1 + material type a surface hit), -2 leaves it to the hit.
+// FEAT: the features the instantiation carries, at least those its waves' scene and settings need
+// (SceneGPU::features, waveFeatures); the others are compiled out, so that the code fits in registers.
+// KEY >= 0 also fixes the shading key (0 a miss, 1 + material type a surface hit), -1 leaves it to the hit.
 // What shadeSlot does with the shadow ray of a NEE sample: appends it to the any-hit queue, traces it
 // at once, or hands it to the caller (one per vertex: waves with one shadow sample).
 enum ShadowMode { SHADOW_QUEUE, SHADOW_INLINE, SHADOW_HAND };
@@ -986,14 +985,14 @@ struct ShadowRec {
     float4 o, d, c, t;
 };
 
-template <ShadowMode SHADOW, bool COUNT, bool OUT, int KEY = -1>
+template <ShadowMode SHADOW, bool COUNT, bool OUT, int FEAT = FEAT_ALL, int KEY = -1>
 __device__ __forceinline__ bool shadeSlot(const SceneGPU& S, const Paths& P, const WaveSeg& A, int slot, int path,
                                           uint32_t& shNodes, uint32_t& shTris, uint32_t& shRays,
                                           ShadowRec* hand = nullptr, bool* handed = nullptr) {
-    constexpr bool LEAN = KEY != -1;
+    constexpr bool MEDIA = (FEAT & FEAT_MEDIA) != 0, GUIDE = (FEAT & FEAT_GUIDE) != 0, REST = (FEAT & FEAT_REST) != 0;
     constexpr int MT = KEY >= 1 ? KEY - 1 : -1; // the material type a surface key fixes
     const TablesGPU* T = S.tables;
-    const bool volumetric = !LEAN && (S.hasVolumes | S.hasSubsurface) != 0;
+    const bool volumetric = MEDIA && (S.hasVolumes | S.hasSubsurface) != 0;
     bool cont = false;
     float4 ro = P.rayO[slot];
     float4 rd = P.rayD[slot];
@@ -1012,7 +1011,7 @@ __device__ __forceinline__ bool shadeSlot(const SceneGPU& S, const Paths& P, con
     uint32_t volCtr = __float_as_uint(md.z);
     float lambda = th.w; // 0 = RGB path; > 0 = single-wavelength path after a dispersive hit
     uint32_t flags = __float_as_uint(ln.w);
-    if (!LEAN && (flags & PF_GUIDE_SNAP)) {
+    if (GUIDE && (flags & PF_GUIDE_SNAP)) {
         // radiance so far, the previous vertex's NEE included: the training record's baseline
         if (P.sdMode & SD_RECORD) {
             const uint32_t n = P.sdCount[slot];
@@ -1042,7 +1041,7 @@ __device__ __forceinline__ bool shadeSlot(const SceneGPU& S, const Paths& P, con
     const bool hit = KEY == 0 ? false : (KEY > 0 ? true : !isMiss(prim));
     const float time = pathTime(S, P, slot);
     // ray cone (path_tracer.cpp:428-454, 777-783, 853-857): only scenes with mipmapped textures
-    const bool cones = !LEAN && S.hasMips && P.cone;
+    const bool cones = REST && S.hasMips && P.cone;
     float2 cone = cones ? P.cone[slot] : make_float2(0.0f, 0.0f);
     Isect is;
     bool done = false;
@@ -1050,7 +1049,7 @@ __device__ __forceinline__ bool shadeSlot(const SceneGPU& S, const Paths& P, con
     bool exitVertex = false; // ... the exit vertex of a subsurface walk
     int shadowRec = -1;      // this vertex's record in the shadow queue
     V3 wo = -dir;
-    if (!LEAN && (flags & PF_WALK)) {
+    if (MEDIA && (flags & PF_WALK)) {
         // one step of the random walk (path_tracer.cpp:263-303)
         const V3 sigT = mk(lp.x, lp.y, lp.z), alb = mk(ln.x, ln.y, ln.z);
         const V3 sigS = alb * sigT;
@@ -1103,7 +1102,7 @@ __device__ __forceinline__ bool shadeSlot(const SceneGPU& S, const Paths& P, con
             // Camera-invisible light quads (for camera rays) and cutouts are passed through;
             // the vertex does not count (path_tracer.cpp:426-439).
             if (skips < 64 && ((cameraRay && (S.shapes[is.shape].flags & SF_CAMERA_INVISIBLE)) ||
-                               (!LEAN && passesCutout(S, S.materials[is.material], is, sb)))) {
+                               (REST && passesCutout(S, S.materials[is.material], is, sb)))) {
                 const V3 no = offsetRayOrigin(is.point, is.pError, is.ng, dir);
                 ro = make_float4(no.x, no.y, no.z, ro.w);
                 if (cones) cone.x = cone.x + cone.y * smax(0.0f, is.t);
@@ -1202,7 +1201,7 @@ __device__ __forceinline__ bool shadeSlot(const SceneGPU& S, const Paths& P, con
                     }
                 }
                 done = true;
-            } else if (!LEAN && cameraRay && is.shape == S.catcherShape) {
+            } else if (REST && cameraRay && is.shape == S.catcherShape) {
                 // the shadow catcher ends the camera path with the shadowed background
                 float ratio = 1.0f;
                 const V3 bg = shadowCatcher(S, is, dir, shadowSamples, sb, ratio, time);
@@ -1228,7 +1227,7 @@ __device__ __forceinline__ bool shadeSlot(const SceneGPU& S, const Paths& P, con
                         li = (sh.flags & SF_AREA_TRIANGLE) ? sh.emitter : sh.emitter + (is.tri - static_cast<int>(sh.firstTri));
                     // Light linking: the previous receiver must be linked to this light
                     // (path_tracer.cpp:571-572; camera rays always see it)
-                    const bool linked = depth == 0 || li < 0 || LEAN || !S.hasLightLinks ||
+                    const bool linked = depth == 0 || li < 0 || !REST || !S.hasLightLinks ||
                                         linkAllows(S.links[li].mode, S.links[li].mask,
                                                    static_cast<int>((flags >> kPrevNodeShift) & 0xFFu));
                     float weight = 1.0f;
@@ -1268,18 +1267,18 @@ __device__ __forceinline__ bool shadeSlot(const SceneGPU& S, const Paths& P, con
     if (vertex) {
         const MatGPU& mat = S.materials[is.material];
         // dispersion: the first wavelength-dependent surface fixes one λ for the path
-        if (!LEAN && lambda == 0.0f && (mat.flags & MF_DISPERSIVE)) {
+        if (MEDIA && lambda == 0.0f && (mat.flags & MF_DISPERSIVE)) {
             V3 w;
             lambda = sampleWavelength(T, get1D(sb), w);
             thr *= w;
         }
         // rounded edges on the first three vertices (not a walk's exit vertex), then contact AO at
         // the camera hit (path_tracer.cpp:612-621)
-        if (!LEAN && depth <= 2 && mat.roundEdge > 0.0f && !exitVertex) {
+        if (REST && depth <= 2 && mat.roundEdge > 0.0f && !exitVertex) {
             const V3 n = roundedEdgeNormal(S, is, mat.roundEdge, sb, time);
             if (dot(n, wo) > 0.02f) is.normal = n;
         }
-        if (!LEAN && A.aoStrength > 0.0f && depth == 0) thr *= approxAo(S, is, sb, A.aoStrength, shadowSamples, time);
+        if (REST && A.aoStrength > 0.0f && depth == 0) thr *= approxAo(S, is, sb, A.aoStrength, shadowSamples, time);
         ShadePoint sp;
         sp.uv = is.uv;
         sp.textures = S.textures;
@@ -1301,11 +1300,11 @@ __device__ __forceinline__ bool shadeSlot(const SceneGPU& S, const Paths& P, con
         const DisneyVertex* dv = &disney;
         if (MT == kDisneyType || (MT < 0 && mat.type == kDisneyType)) disneyVertex(T, mat, wo, sp, disney);
         // this bounce's proposal, when the inference kernel left one for the slot
-        const bool useGuide = !LEAN && P.guiding == 2 && guidable(mat) && P.guideMark[slot] != 0u;
+        const bool useGuide = GUIDE && P.guiding == 2 && guidable(mat) && P.guideMark[slot] != 0u;
         if (useGuide) P.guideMark[slot] = 0u;
         // or the SD-tree's sampling quadtree of the vertex's spatial leaf (path_tracer.cpp:627-629)
         int sdRoot = -1;
-        if (!LEAN && (P.sdMode & SD_SAMPLE) && !useGuide && guidable(mat)) {
+        if (GUIDE && (P.sdMode & SD_SAMPLE) && !useGuide && guidable(mat)) {
             const int leaf = sdLeafWithData(P.sd, is.point);
             if (leaf >= 0) sdRoot = P.sd.leaves[leaf].sampRoot;
         }
@@ -1326,7 +1325,7 @@ __device__ __forceinline__ bool shadeSlot(const SceneGPU& S, const Paths& P, con
                     continue;
                 }
                 const bool fromEnv = lightIndex >= explicitLights;
-                if (!LEAN && !fromEnv && S.hasLightLinks &&
+                if (REST && !fromEnv && S.hasLightLinks &&
                     !linkAllows(S.links[lightIndex].mode, S.links[lightIndex].mask, S.shapes[is.shape].linkNode)) {
                     (void)get2D(T, sb);
                     continue;
@@ -1420,7 +1419,7 @@ __device__ __forceinline__ bool shadeSlot(const SceneGPU& S, const Paths& P, con
         }
         if (!sampled) {
             done = true;
-        } else if (!LEAN && bs.subsurface) {
+        } else if (MEDIA && bs.subsurface) {
             // random-walk entry (path_tracer.cpp:745-761): the walk's coefficients ride
             // in the columns it does not need (lastP, lastN, pickP.x)
             V3 sigT, alb;
@@ -1476,7 +1475,7 @@ __device__ __forceinline__ bool shadeSlot(const SceneGPU& S, const Paths& P, con
             const float cosTheta = fabsf(dot(wi, is.normal));
             const V3 thrBefore = thr;
             thr *= bs.f * (cosTheta / bs.pdf);
-            if (!LEAN && P.guiding && !bs.delta && slot % P.guideStride == 0 && guidable(mat) && isFinite3(thr) &&
+            if (GUIDE && P.guiding && !bs.delta && slot % P.guideStride == 0 && guidable(mat) && isFinite3(thr) &&
                 guideRecord(P, slot, is.point, is.normal, wo, wi, thrBefore))
                 flags |= PF_GUIDE_SNAP;
             if (!isFinite3(thr)) {
@@ -1490,7 +1489,7 @@ __device__ __forceinline__ bool shadeSlot(const SceneGPU& S, const Paths& P, con
                 flags = cameraRay ? (flags | PF_CAMERA_RAY) : (flags & ~PF_CAMERA_RAY);
                 // crossing a volume boundary: enter the object's medium from outside,
                 // leave it from inside
-                if (!LEAN && (mat.flags & MF_VOLUME_BOUNDARY)) {
+                if (MEDIA && (mat.flags & MF_VOLUME_BOUNDARY)) {
                     const float a = dot(wo, is.ng), b = dot(wi, is.ng);
                     if (a * b < 0.0f) {
                         if (a > 0.0f) media.enter(is.material);
@@ -1517,7 +1516,7 @@ __device__ __forceinline__ bool shadeSlot(const SceneGPU& S, const Paths& P, con
                 // SD-tree training vertex (path_tracer.cpp:823-827, recordable ones only): its
                 // incident radiance is what L gains from here on over the throughput after the
                 // bounce and the roulette
-                if (!LEAN && cont && (P.sdMode & SD_RECORD) && !bs.delta && !(mat.flags & MF_VOLUME_BOUNDARY)) {
+                if (GUIDE && cont && (P.sdMode & SD_RECORD) && !bs.delta && !(mat.flags & MF_VOLUME_BOUNDARY)) {
                     const uint32_t n = P.sdCount[slot];
                     if (n < static_cast<uint32_t>(kSdRecords)) {
                         float4* rec = P.sdRec + (static_cast<size_t>(slot) * kSdRecords + n) * 4;
@@ -1557,7 +1556,7 @@ __device__ __forceinline__ bool shadeSlot(const SceneGPU& S, const Paths& P, con
 // OUT: the wave records AOVs or render passes (their code is compiled out of the plain kernel).
 // INLINE: NEE shadow rays are traced here, each sample's term added in the sample loop's order
 // (waves with shadowQuality > 1, whose several records per vertex the shadow queue does not hold).
-template <bool OUT, bool INLINE = false>
+template <int FEAT, bool OUT, bool INLINE = false>
 __global__ void __launch_bounds__(128, 6) kShade(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P, const __grid_constant__ Wave W, int32_t* nextQueue) {
     uint32_t seg[kShadeKeys];
     int n = 0;
@@ -1583,7 +1582,7 @@ __global__ void __launch_bounds__(128, 6) kShade(const __grid_constant__ SceneGP
             slot = P.sortQ[static_cast<size_t>(k) * P.capacity + j];
             const int path = pathOfSlot(P, slot);
             const WaveSeg& A = W.segs[segOfSlot(W, path)];
-            cont = shadeSlot<INLINE ? SHADOW_INLINE : SHADOW_QUEUE, false, OUT>(S, P, A, slot, path, unused0, unused1, unused2);
+            cont = shadeSlot<INLINE ? SHADOW_INLINE : SHADOW_QUEUE, false, OUT, FEAT>(S, P, A, slot, path, unused0, unused1, unused2);
             sweepable = (A.flags & SEG_SWEEP) != 0;
         }
         // a continuous wave sweeps its interactive paths that have lived sweepAge bounces into a
@@ -1614,7 +1613,7 @@ __device__ __forceinline__ void shadeBin(const SceneGPU& S, const Paths& P, cons
             slot = bin[i];
             const int path = pathOfSlot(P, slot);
             const WaveSeg& A = W.segs[segOfSlot(W, path)];
-            cont = shadeSlot<SHADOW_QUEUE, false, OUT, KEY>(S, P, A, slot, path, unused0, unused1, unused2);
+            cont = shadeSlot<SHADOW_QUEUE, false, OUT, 0, KEY>(S, P, A, slot, path, unused0, unused1, unused2);
             sweepable = (A.flags & SEG_SWEEP) != 0;
         }
         if (KEY != 0) {
@@ -1728,7 +1727,7 @@ __global__ void __launch_bounds__(kTailLockstepBlock) kTailLockstep(const __grid
         }
         __syncthreads();
         if (slot >= 0) {
-            if (!shadeSlot<SHADOW_INLINE, false, false, -1>(S, P, *A, slot, path, shNodes, shTris, shRays)) {
+            if (!shadeSlot<SHADOW_INLINE, false, false>(S, P, *A, slot, path, shNodes, shTris, shRays)) {
                 slot = -1;
             } else if (++q >= kMaxPathQueries) {
                 // as kTail: a path past the per-path query bound is ended and reported
@@ -1749,7 +1748,7 @@ __global__ void __launch_bounds__(kTailLockstepBlock) kTailLockstep(const __grid
 // one.  The block's warps shade between barriers (one phase's code at a time, as kTailLockstep).
 // Each path's queries and terms are kTail's, so the film is the same bit for bit.
 constexpr int kTailWarpsBlock = 128;
-template <bool LEAN, bool OUT>
+template <int FEAT, bool OUT>
 __global__ void __launch_bounds__(kTailWarpsBlock) kTailWarps(const __grid_constant__ SceneGPU S,
                                                               const __grid_constant__ Paths P,
                                                               const __grid_constant__ Wave W, const int32_t* queue,
@@ -1809,7 +1808,7 @@ __global__ void __launch_bounds__(kTailWarpsBlock) kTailWarps(const __grid_const
                         ray = -1;
                     } else {
                         if (w.prim == -1) P.hit[slots[ray]] = make_float4(w.tMax, 0.0f, 0.0f, __int_as_float(-1));
-                        if (!LEAN && scattering && scatterOn(S, P, W, slots[ray], next)) {
+                        if ((FEAT & FEAT_MEDIA) && scattering && scatterOn(S, P, W, slots[ray], next)) {
                             w.start(S, root, next.o, next.d, next.mask, 1e30f, -1);
                             ++rays;
                         } else {
@@ -1865,7 +1864,7 @@ __global__ void __launch_bounds__(kTailWarpsBlock) kTailWarps(const __grid_const
         }
         if (slot >= 0) {
             bool handed = false;
-            const bool cont = shadeSlot<SHADOW_HAND, false, OUT, LEAN ? -2 : -1>(S, P, *A, slot, path, unused, unused, unused,
+            const bool cont = shadeSlot<SHADOW_HAND, false, OUT, FEAT>(S, P, *A, slot, path, unused, unused, unused,
                                                                                 &recs[tid], &handed);
             shadow = handed;
             ended = !cont;
@@ -2019,17 +2018,16 @@ static __global__ void kFilm(const __grid_constant__ Paths P, const __grid_const
 
 // ---- instantiations ---------------------------------------------------------------------------
 // The kernels below are compiled in translation units of their own (pe_kernels_*.cu), side by side;
-// PE_LEAN_KERNELS(K) and its siblings expand K(kernel) over a unit's instantiations.
+// PE_FULL_KERNELS(K) and its siblings expand K(kernel) over a unit's instantiations.
 #define PE_SHADE_ARGS                                                                              \
     (const __grid_constant__ SceneGPU, const __grid_constant__ Paths, const __grid_constant__ Wave, int32_t*)
-#define PE_LEAN_KERNELS(K)                                                                         \
-    K(kShadeKey<false, 0, 1>) K(kShadeKey<false, 1, 5>) K(kShadeKey<false, 2, 6>)                  \
-    K(kShadeKey<false, 3, 5>) K(kShadeKey<false, 4, 5>)
-#define PE_LEAN_OUT_KERNELS(K)                                                                     \
-    K(kShadeKey<true, 0, 1>) K(kShadeKey<true, 1, 5>) K(kShadeKey<true, 2, 6>)                     \
-    K(kShadeKey<true, 3, 5>) K(kShadeKey<true, 4, 5>)
-#define PE_FULL_KERNELS(K) K(kShade<false, false>) K(kShade<false, true>)
-#define PE_FULL_OUT_KERNELS(K) K(kShade<true, false>) K(kShade<true, true>)
+// one kernel per shading key: K(AOVs or passes, key, blocks per SM)
+#define PE_LEAN_KEYS(K, OUT) K(OUT, 0, 1) K(OUT, 1, 5) K(OUT, 2, 6) K(OUT, 3, 5) K(OUT, 4, 5)
+#define PE_SHADE_KEY(OUT, KEY, MINB) PE_K(kShadeKey<OUT, KEY, MINB>)
+#define PE_FULL_KERNELS(K) K(kShade<FEAT_ALL, false, false>) K(kShade<FEAT_ALL, false, true>)
+#define PE_FULL_OUT_KERNELS(K) K(kShade<FEAT_ALL, true, false>) K(kShade<FEAT_ALL, true, true>)
+#define PE_MEDIA_KERNELS(K) K(kShade<FEAT_MEDIA, false, false>)
+#define PE_GUIDE_KERNELS(K) K(kShade<FEAT_GUIDE, false, false>)
 #define PE_TAIL_ARGS                                                                               \
     (const __grid_constant__ SceneGPU, const __grid_constant__ Paths, const __grid_constant__ Wave, const int32_t*, \
      const uint32_t*, uint32_t*, int, unsigned long long*)
@@ -2038,8 +2036,8 @@ static __global__ void kFilm(const __grid_constant__ Paths P, const __grid_const
 #define PE_TAIL_WARPS_ARGS                                                                         \
     (const __grid_constant__ SceneGPU, const __grid_constant__ Paths, const __grid_constant__ Wave, const int32_t*, \
      const uint32_t*, uint32_t*, int, int, unsigned long long*)
-#define PE_TAIL_WARPS_LEAN_KERNELS(K) K(kTailWarps<true, false>) K(kTailWarps<true, true>)
-#define PE_TAIL_WARPS_FULL_KERNELS(K) K(kTailWarps<false, false>) K(kTailWarps<false, true>)
+#define PE_TAIL_WARPS_LEAN_KERNELS(K) K(kTailWarps<0, false>) K(kTailWarps<0, true>)
+#define PE_TAIL_WARPS_FULL_KERNELS(K) K(kTailWarps<FEAT_ALL, false>) K(kTailWarps<FEAT_ALL, true>)
 #define PE_TRACE_ARGS                                                                              \
     (const __grid_constant__ SceneGPU, const __grid_constant__ Paths, const __grid_constant__ Wave, const int32_t*, int, \
      unsigned long long*)

@@ -1,8 +1,9 @@
-// pe_kernels_lean.cu — the lean shading kernels of plain waves (pe_integrator.cuh), compiled on their own.
+// pe_kernels_lean.cu — the per-key shading kernels of plain surface scenes (pe_integrator.cuh),
+// compiled on their own.
 #include "pe_integrator.cuh"
 
 namespace pe {
-#define PE_INSTANTIATE(...) template __global__ void __VA_ARGS__ PE_SHADE_ARGS;
-PE_LEAN_KERNELS(PE_INSTANTIATE)
-#undef PE_INSTANTIATE
+#define PE_K(...) template __global__ void __VA_ARGS__ PE_SHADE_ARGS;
+PE_LEAN_KEYS(PE_SHADE_KEY, false)
+#undef PE_K
 } // namespace pe

@@ -1,8 +1,9 @@
-// pe_kernels_lean_out.cu — the lean shading kernels that record AOVs and render passes (pe_integrator.cuh), compiled on their own.
+// pe_kernels_lean_out.cu — the per-key shading kernels of plain surface scenes that record AOVs or passes (pe_integrator.cuh),
+// compiled on their own.
 #include "pe_integrator.cuh"
 
 namespace pe {
-#define PE_INSTANTIATE(...) template __global__ void __VA_ARGS__ PE_SHADE_ARGS;
-PE_LEAN_OUT_KERNELS(PE_INSTANTIATE)
-#undef PE_INSTANTIATE
+#define PE_K(...) template __global__ void __VA_ARGS__ PE_SHADE_ARGS;
+PE_LEAN_KEYS(PE_SHADE_KEY, true)
+#undef PE_K
 } // namespace pe

@@ -2,7 +2,7 @@
 #include "pe_integrator.cuh"
 
 namespace pe {
-#define PE_INSTANTIATE(...) template __global__ void __VA_ARGS__ PE_TAIL_WARPS_ARGS;
-PE_TAIL_WARPS_FULL_KERNELS(PE_INSTANTIATE)
-#undef PE_INSTANTIATE
+#define PE_K(...) template __global__ void __VA_ARGS__ PE_TAIL_WARPS_ARGS;
+PE_TAIL_WARPS_FULL_KERNELS(PE_K)
+#undef PE_K
 } // namespace pe

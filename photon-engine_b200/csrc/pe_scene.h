@@ -61,7 +61,7 @@ constexpr int32_t kMaxBlasRecords = (1 << 21) - 1;
 // A MeshInstance (mesh_instance.cpp): world-to-local and local-to-world (row-major rows 0-3), its
 // BLAS's root in the binary and in the 4-wide tree (a node index or a leaf reference) and first
 // leaf record, the global id of the BLAS's first triangle, the shape and the material.
-struct InstGPU {
+struct alignas(16) InstGPU {
     float4 w2l[4];
     float4 l2w[4];
     int32_t rootBinary, rootWide, recBase, firstTri;
@@ -97,7 +97,7 @@ struct LightLinkGPU {
 };
 
 // Resolved material (pe_material + constants derived on the host).
-struct MatGPU {
+struct alignas(16) MatGPU {
     int32_t type;
     int32_t flags;            // MF_*
     float base[3];
@@ -266,10 +266,7 @@ struct SceneGPU {
     const TexGPU* textures;  // image textures (null without any)
     int32_t nTextures;
     int32_t hasMips;         // some texture has mipmaps: paths carry ray cones for its LOD
-    // 1 when no material or scene setting needs the shading features a plain surface scene
-    // leaves unused (volumes, subsurface walks, dispersion, cutouts, rounded edges, ray cones,
-    // light or shadow links, a shadow catcher): its waves may shade with the lean kernels
-    int32_t leanShading;
+    int32_t features;        // ShadeFeatures its materials and settings need
     int32_t materialTypes;   // bit t: some material has type t
     const InstGPU* instances; // MeshInstances (null without)
     int32_t nInstances;

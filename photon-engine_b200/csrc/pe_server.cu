@@ -566,7 +566,7 @@ void laneThread(pe_server* S, int li) {
         const int nSegs = static_cast<int>(R.segs.size());
         for (; R.aoChecked < nSegs; ++R.aoChecked)
             if (R.hSegs[R.aoChecked].aoStrength > 0.0f) R.anyAo = true;
-        L.lean = L.scene.leanShading && !R.anyAo;
+        L.features = L.scene.features | (R.anyAo ? FEAT_REST : 0);
         const int upFirst = R.uploaded;
         R.uploaded = nSegs;
         const bool draining = R.draining;

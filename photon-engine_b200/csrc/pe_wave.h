@@ -134,6 +134,13 @@ enum PassFilms { PFILM_DEPTH = 8, PFILM_POSITION = 9, PFILM_OBJECT = 10, PFILM_M
 
 // Shading keys: 0 = miss, 1 + material type (Lambert, Disney, Dielectric, Mirror), 5 = random-walk step.
 constexpr int kShadeKeys = 6;
+// Shading features beyond a plain surface scene's, as instantiations of the shading code carry them.
+enum ShadeFeatures {
+    FEAT_MEDIA = 1, // media, subsurface walks, dispersion
+    FEAT_GUIDE = 2, // the learned proposal, the SD-tree
+    FEAT_REST = 4,  // cutouts, rounded edges, ray cones, light and shadow links, shadow catchers, ambient occlusion
+    FEAT_ALL = 7
+};
 constexpr uint8_t kKeyOfPrim = 255; // Paths::key: kBin derives the key from the hit's primitive
 // Counters of one bounce: the closest-hit queue's entries, the shadow records, the work cursors of
 // the trace and shading kernels, the rays per shading key and their bins' cursors.
