@@ -1076,6 +1076,7 @@ static void buildLightSampler(const pe_scene* s, HostBuild& B) {
     B.infinite.clear();
     B.lightNodes.clear();
     B.lights = s->lights;
+    for (LightGPU& l : B.lights) deriveLight(l);
     const int nl = static_cast<int>(B.lights.size());
     const int count = nl + (s->env.present ? 1 : 0);
     B.lightCount = count;
@@ -1106,11 +1107,13 @@ static void buildLightSampler(const pe_scene* s, HostBuild& B) {
                 for (size_t i = 0; i < lb.nodes.size(); ++i) {
                     const LBounds& b = lb.nodeBounds[i];
                     LightNodeGPU& n = B.lightNodes[i];
-                    n.bmin[0] = b.bounds.lo.x; n.bmin[1] = b.bounds.lo.y; n.bmin[2] = b.bounds.lo.z;
-                    n.bmax[0] = b.bounds.hi.x; n.bmax[1] = b.bounds.hi.y; n.bmax[2] = b.bounds.hi.z;
+                    const V3 c = (b.bounds.lo + b.bounds.hi) * 0.5f;
+                    n.centre[0] = c.x; n.centre[1] = c.y; n.centre[2] = c.z;
+                    n.r2 = 0.25f * len2(b.bounds.hi - b.bounds.lo);
                     n.w[0] = b.w.x; n.w[1] = b.w.y; n.w[2] = b.w.z;
                     n.phi = b.phi;
                     n.cosThetaO = b.cosThetaO;
+                    n.sinThetaO = safeSqrtf(1.0f - b.cosThetaO * b.cosThetaO);
                     n.cosThetaE = b.cosThetaE;
                     n.twoSided = b.twoSided ? 1 : 0;
                 }

@@ -39,17 +39,40 @@ PE_HD float angleBetween(V3 a, V3 b) {
     return 2.0f * safeAsinf(length(b - a) * 0.5f);
 }
 
+// LightGPU's derived rows.
+PE_HD void deriveLight(LightGPU& l) {
+    const V3 p0 = m3f(l.p0), p1 = m3f(l.p1), p2 = m3f(l.p2);
+    const V3 c = l.type == LT_TRIANGLE ? (p0 + p1 + p2) * (1.0f / 3.0f) : p0 + (p1 + p2) * 0.5f;
+    l.lum = smax(0.0f, luminance(lightRadiance(l)));
+    V3 x = mk(0.0f), y = mk(0.0f), z = mk(0.0f);
+    if (l.type == LT_AREA) {
+        l.lenU = length(p1);
+        l.lenV = length(p2);
+        if (l.rectangle) {
+            x = p1 / l.lenU;
+            y = p2 / l.lenV;
+            z = cross(x, y);
+        }
+    }
+    for (int i = 0; i < 3; ++i) {
+        l.centre[i] = i == 0 ? c.x : i == 1 ? c.y : c.z;
+        l.axisU[i] = i == 0 ? x.x : i == 1 ? x.y : x.z;
+        l.axisV[i] = i == 0 ? y.x : i == 1 ? y.y : y.z;
+        l.axisN[i] = i == 0 ? z.x : i == 1 ? z.y : z.z;
+    }
+}
+
 struct SphRect {
     Frame frame;
     float x0, y0, z0, x1, y1, b0, b1, g2g3, solidAngle;
 };
-PE_HD SphRect setupSphRect(V3 ref, V3 corner, V3 ex, V3 ey) {
+PE_HD SphRect setupSphRect(V3 ref, const LightGPU& l) {
     SphRect r;
     r.x0 = r.y0 = r.z0 = r.x1 = r.y1 = r.b0 = r.b1 = r.g2g3 = r.solidAngle = 0.0f;
-    const float exl = length(ex), eyl = length(ey);
-    const V3 x = ex / exl, y = ey / eyl;
-    V3 z = cross(x, y);
-    const V3 d = corner - ref;
+    const float exl = l.lenU, eyl = l.lenV;
+    const V3 x = m3f(l.axisU), y = m3f(l.axisV);
+    V3 z = m3f(l.axisN);
+    const V3 d = m3f(l.p0) - ref;
     r.z0 = dot(d, z);
     if (r.z0 > 0.0f) {
         z = -z;
@@ -121,7 +144,7 @@ PE_HDN LightSample sampleLight(const LightGPU& l, V3 p, V2 u) {
     // rectangle
     const V3 pos = m3f(l.p0), lu = m3f(l.p1), lv = m3f(l.p2);
     if (l.rectangle) {
-        const SphRect r = setupSphRect(p, pos, lu, lv);
+        const SphRect r = setupSphRect(p, l);
         if (r.solidAngle >= kMinSolidAngle) {
             const V3 toL = sampleSphRect(r, u);
             const float dist = length(toL);
@@ -160,7 +183,7 @@ PE_HDN float lightPdfHit(const LightGPU& l, V3 ref, V3 pHit) {
     }
     const V3 pos = m3f(l.p0), lu = m3f(l.p1), lv = m3f(l.p2);
     const V3 d = pHit - pos;
-    const float scale = smax(length(lu) + length(lv), 1.0f);
+    const float scale = smax(l.lenU + l.lenV, 1.0f);
     if (fabsf(dot(d, nrm)) > 1e-3f * scale) return 0.0f;
     const float uu = dot(lu, lu), vv = dot(lv, lv), uv = dot(lu, lv);
     const float du = dot(d, lu), dv = dot(d, lv);
@@ -171,7 +194,7 @@ PE_HDN float lightPdfHit(const LightGPU& l, V3 ref, V3 pHit) {
     const float eps = 1e-3f;
     if (s < -eps || t < -eps || s > 1.0f + eps || t > 1.0f + eps) return 0.0f;
     if (l.rectangle) {
-        const float omega = setupSphRect(ref, pos, lu, lv).solidAngle;
+        const float omega = setupSphRect(ref, l).solidAngle;
         if (omega >= kMinSolidAngle) return 1.0f / omega;
     }
     const V3 toL = pHit - ref;
@@ -183,12 +206,9 @@ PE_HDN float lightPdfHit(const LightGPU& l, V3 ref, V3 pHit) {
 
 // Light::importance (area_light.cpp:104-113 and :206-215).
 PE_HD float lightImportance(const LightGPU& l, V3 p, V3 n) {
-    V3 c;
-    if (l.type == LT_TRIANGLE) c = (m3f(l.p0) + m3f(l.p1) + m3f(l.p2)) * (1.0f / 3.0f);
-    else c = m3f(l.p0) + (m3f(l.p1) + m3f(l.p2)) * 0.5f;
-    const V3 d = c - p;
+    const V3 d = m3f(l.centre) - p;
     const float dist2 = len2(d);
-    const float lum = smax(0.0f, luminance(lightRadiance(l)));
+    const float lum = l.lum;
     if (!(dist2 > 0.0f)) return lum * kTwoPi;
     const V3 w = d / sqrtf(dist2);
     const float cosL = smax(fabsf(dot(w, m3f(l.normal))), 0.2f);
@@ -393,22 +413,18 @@ PE_HD float sinSubClamped(float sinA, float cosA, float sinB, float cosB) {
 }
 PE_HD float boundsImportance(const LightNodeGPU& b, V3 p, V3 n) {
     if (!(b.phi > 0.0f)) return 0.0f;
-    const V3 bmin = m3f(b.bmin), bmax = m3f(b.bmax);
-    const V3 pc = (bmin + bmax) * 0.5f;
-    const V3 diag = bmax - bmin;
-    const float d2 = smax(len2(p - pc), 0.25f * len2(diag));
+    V3 wi = p - m3f(b.centre);
+    const float r2 = b.r2, dc2 = len2(wi);
+    const float d2 = smax(dc2, r2);
     if (!(d2 > 0.0f)) return b.phi;
-    V3 wi = p - pc;
     const float len = length(wi);
     wi = len > 0.0f ? wi / len : m3f(b.w);
     float cosW = dot(m3f(b.w), wi);
     if (b.twoSided) cosW = fabsf(cosW);
     const float sinW = safeSqrtf(1.0f - cosW * cosW);
-    const float r2 = 0.25f * len2(diag);
-    const float dc2 = len2(p - pc);
     const float cosB = dc2 <= r2 ? -1.0f : safeSqrtf(1.0f - r2 / dc2);
     const float sinB = safeSqrtf(1.0f - cosB * cosB);
-    const float sinO = safeSqrtf(1.0f - b.cosThetaO * b.cosThetaO);
+    const float sinO = b.sinThetaO;
     const float cosX = cosSubClamped(sinW, cosW, sinO, b.cosThetaO);
     const float sinX = sinSubClamped(sinW, cosW, sinO, b.cosThetaO);
     const float cosP = cosSubClamped(sinX, cosX, sinB, cosB);
@@ -474,29 +490,32 @@ PE_HDN void lightPrepare(const SceneGPU& S, V3 p, V3 n, LightCtx& c) {
     c.uniform = false;
 }
 
+// A level of the descent reads both children whole, so that it waits for one load, not for the node,
+// its second child's index and the child in turn.
 PE_HDN int bvhLightSample(const SceneGPU& S, V3 p, V3 n, float u, float& pmf) {
     pmf = 1.0f;
-    int node = 0;
+    int node = 0, light = S.lightNodes[0].light, child1 = S.lightNodes[0].child1;
     for (int guard = 0; guard < 128; ++guard) {
-        const LightNodeGPU& nd = S.lightNodes[node];
-        if (nd.light >= 0) return nd.light;
-        const int c0 = node + 1, c1 = nd.child1;
-        const float i0 = boundsImportance(S.lightNodes[c0], p, n);
-        const float i1 = boundsImportance(S.lightNodes[c1], p, n);
+        if (light >= 0) return light;
+        const LightNodeGPU a = S.lightNodes[node + 1], b = S.lightNodes[child1];
+        const float i0 = boundsImportance(a, p, n);
+        const float i1 = boundsImportance(b, p, n);
         if (!(i0 > 0.0f) && !(i1 > 0.0f)) {
             pmf = 0.0f;
             return -1;
         }
         const float p0 = i0 / (i0 + i1);
-        if (u < p0) {
-            node = c0;
+        const bool first = u < p0;
+        if (first) {
             u = smin(u / p0, 0.99999994f);
             pmf *= p0;
         } else {
-            node = c1;
             u = smin((u - p0) / (1.0f - p0), 0.99999994f);
             pmf *= 1.0f - p0;
         }
+        node = first ? node + 1 : child1;
+        light = first ? a.light : b.light;
+        child1 = first ? a.child1 : b.child1;
     }
     pmf = 0.0f;
     return -1;
@@ -506,25 +525,22 @@ PE_HDN float bvhLightPmf(const SceneGPU& S, V3 p, V3 n, int index) {
     unsigned long long trail = S.trail[index];
     const int depth = S.trailDepth[index];
     float pmf = 1.0f;
-    int node = 0;
+    int node = 0, light = S.lightNodes[0].light, child1 = S.lightNodes[0].child1;
     for (int d = 0; d < depth; ++d) {
-        const LightNodeGPU& nd = S.lightNodes[node];
-        if (nd.light >= 0) break;
-        const int c0 = node + 1, c1 = nd.child1;
-        const float i0 = boundsImportance(S.lightNodes[c0], p, n);
-        const float i1 = boundsImportance(S.lightNodes[c1], p, n);
+        if (light >= 0) break;
+        const LightNodeGPU a = S.lightNodes[node + 1], b = S.lightNodes[child1];
+        const float i0 = boundsImportance(a, p, n);
+        const float i1 = boundsImportance(b, p, n);
         const float sum = i0 + i1;
         if (!(sum > 0.0f)) return 0.0f;
-        if (trail & 1ull) {
-            pmf *= i1 / sum;
-            node = c1;
-        } else {
-            pmf *= i0 / sum;
-            node = c0;
-        }
+        const bool first = !(trail & 1ull);
+        pmf *= (first ? i0 : i1) / sum;
+        node = first ? node + 1 : child1;
+        light = first ? a.light : b.light;
+        child1 = first ? a.child1 : b.child1;
         trail >>= 1;
     }
-    return S.lightNodes[node].light == index ? pmf : 0.0f;
+    return light == index ? pmf : 0.0f;
 }
 
 // Context::sample (light_sampler.cpp:195-228): candidate index (env = nLights) or -1.

@@ -153,11 +153,12 @@ enum MatFlags : int32_t {
 
 enum LightType : int32_t { LT_TRIANGLE = 0, LT_AREA = 1 };
 
-struct LightGPU {
+// The last five rows are derived from the others (deriveLight), once instead of at every sample.
+struct alignas(16) LightGPU {
     int32_t type;
     int32_t rectangle;  // AreaLight: u ⟂ v (spherical-rectangle sampling allowed)
     float area;
-    float pad0;
+    float lum;          // luminance of the radiance, at least 0
     float p0[3];        // triangle p0 | area position
     float radiance_r;
     float p1[3];        // triangle p1 | area u
@@ -165,18 +166,29 @@ struct LightGPU {
     float p2[3];        // triangle p2 | area v
     float radiance_b;
     float normal[3];
+    float lenU;         // area: |u|
+    float centre[3];
+    float lenV;         // area: |v|
+    float axisU[3];     // rectangle: u / |u|
+    float pad0;
+    float axisV[3];     // rectangle: v / |v|
     float pad1;
+    float axisN[3];     // rectangle: axisU x axisV
+    float pad2;
 };
 
-// Light BVH node (LightSampler::Node with LightBounds, light_sampler.h:57-61, light_bounds.h:16-26).
-struct LightNodeGPU {
-    float bmin[3], bmax[3];
+// Light BVH node (LightSampler::Node with LightBounds, light_sampler.h:57-61, light_bounds.h:16-26),
+// with what boundsImportance asks of its bounds: a node is read whole in four 16-byte loads.
+struct alignas(16) LightNodeGPU {
+    float centre[3];
+    float r2;           // squared half diagonal
     float w[3];
-    float phi, cosThetaO, cosThetaE;
+    float phi;
+    float cosThetaO, sinThetaO, cosThetaE;
     int32_t twoSided;
     int32_t child1;
     int32_t light;
-    int32_t pad;
+    int32_t pad[2];
 };
 
 struct TablesGPU {
