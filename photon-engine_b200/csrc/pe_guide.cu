@@ -41,10 +41,14 @@ __device__ __forceinline__ void storeRow8(unsigned char* tile, int row, int k0, 
     *reinterpret_cast<uint4*>(tile + coreOffset(row, k0, kTcRows)) = *reinterpret_cast<const uint4*>(h);
 }
 
-// Queries: 3 float4 per row (position | shading normal | direction to the viewer).  Row r's 40
-// mixture outputs go to out[slot(r) · 10 ...] as 10 float4; mark[slot] = 1 tells the shading
-// kernel that this bounce's proposal is there.
-__global__ void __launch_bounds__(kTcRows) kGuideInferTC(const __grid_constant__ GuideNet g, const float4* q, const int32_t* slots,
+// Queries: 3 float4 per row (position | shading normal | direction to the viewer).  With `mark`, row r's
+// mixture goes to its slot (putMixture), and mark[slot] = 1 tells the shading kernel that this bounce's
+// proposal is there; without, the row's 40 outputs go to 10 float4 of `out`.
+// Bound by the latency of the grid's gathers (128 of 8 bytes a row) and of four dependent layers, so blocks in
+// flight count: four per SM, a feature pair per load and constant levels took the 14 launches of a guided
+// room pass (320x180 x 16 spp, 2.4M rows) from 2.75 to 1.5 ms.
+constexpr int kTcBlocks = 4; // per SM: TMEM's 512 columns, and 193 of the SM's 228 KB of shared memory
+__global__ void __launch_bounds__(kTcRows, kTcBlocks) kGuideInferTC(const __grid_constant__ GuideNet g, const float4* q, const int32_t* slots,
                                                          const uint32_t* count, int nFixed, float4* out, uint32_t* mark,
                                                          uint32_t* err) {
     extern __shared__ __align__(1024) unsigned char sm[];
@@ -59,9 +63,10 @@ __global__ void __launch_bounds__(kTcRows) kGuideInferTC(const __grid_constant__
     const int bSrc[4] = {kOffB1, kOffB2, kOffB3, kOffB4};
     for (int L = 0; L < 4; ++L) {
         const int K = L == 0 ? kNetIn : kNetHidden;
-        for (int i = tid; i < 64 * K; i += kTcRows) {
-            const int row = i / K, k = i - row * K;
-            *reinterpret_cast<__half*>(sm + wOff[L] + coreOffset(row, k, 64)) = g.mlp16[wSrc[L] + i];
+        for (int i = tid; i < 64 * K / 8; i += kTcRows) {
+            const int row = i & 63, k = (i >> 6) * 8;
+            *reinterpret_cast<uint4*>(sm + wOff[L] + coreOffset(row, k, 64)) =
+                *reinterpret_cast<const uint4*>(g.mlp16 + wSrc[L] + row * K + k);
         }
         for (int j = tid; j < 64; j += kTcRows) bias[L * 64 + j] = g.mlp[bSrc[L] + j];
     }
@@ -123,11 +128,17 @@ __global__ void __launch_bounds__(kTcRows) kGuideInferTC(const __grid_constant__
                 tcFenceAfter();
             } else if (valid) {
                 const int dst = slots ? slots[row] : row;
-                for (int j = 0; j < kNetUsedOut; j += 4)
-                    out[static_cast<size_t>(dst) * 10 + j / 4] =
-                        make_float4(v[j] + bias[192 + j], v[j + 1] + bias[193 + j], v[j + 2] + bias[194 + j],
-                                    v[j + 3] + bias[195 + j]);
-                if (mark) mark[dst] = 1u;
+#pragma unroll
+                for (int j = 0; j < kNetUsedOut; ++j) v[j] += bias[192 + j];
+                if (mark) {
+                    Lobes mix;
+                    decodeLobes(v, mix);
+                    putMixture(out + static_cast<size_t>(dst) * kSlotMixture, mix);
+                    mark[dst] = 1u;
+                } else {
+                    for (int j = 0; j < kNetUsedOut; j += 4)
+                        out[static_cast<size_t>(dst) * 10 + j / 4] = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+                }
             }
         }
         __syncthreads();
@@ -424,7 +435,7 @@ int32_t guideInfer(pe_device* d, cudaStream_t s, const float4* q, const int32_t*
                    int maxRows, float4* out, uint32_t* mark) {
     const int sm = d->prop.multiProcessorCount;
     const int tiles = (maxRows + kTcRows - 1) / kTcRows;
-    const int grid = std::max(1, std::min(tiles, 2 * sm));
+    const int grid = std::max(1, std::min(tiles, kTcBlocks * sm));
     kGuideInferTC<<<grid, kTcRows, kSmBytes, s>>>(guideNet(d), q, slots, count, nFixed, out, mark, d->guide.err);
     PE_CUDA(cudaGetLastError());
     return PE_OK;
@@ -481,7 +492,7 @@ int32_t guideBuffers(pe_device* d) {
     const size_t cap = d->capacity;
     int32_t rc = 0;
     if ((rc = devAlloc(G.laneBufs, P.guideQ, cap * 3)) || (rc = devAlloc(G.laneBufs, P.guideSlot, cap)) ||
-        (rc = devAlloc(G.laneBufs, P.guideOut, cap * 10)) || (rc = devAlloc(G.laneBufs, P.guideMark, cap)) ||
+        (rc = devAlloc(G.laneBufs, P.guideOut, cap * kSlotMixture)) || (rc = devAlloc(G.laneBufs, P.guideMark, cap)) ||
         (rc = devAlloc(G.laneBufs, P.guideRec, cap * 6)) ||
         (rc = devAlloc(G.laneBufs, P.trainBuf, static_cast<size_t>(kGuideTrainRows + 1) * 4))) {
         freeList(G.laneBufs);

@@ -97,13 +97,20 @@ PE_HD V3 guideUnit(const GuideNet& g, V3 p) {
 // Network input row for a query (position, shading normal, direction towards the viewer).
 PE_HD void guideInput(const GuideNet& g, V3 p, V3 n, V3 wo, float* x) {
     const V3 u = guideUnit(g, p);
+#pragma unroll // a level's resolution and whether it hashes are constants
     for (int l = 0; l < kGridLevels; ++l) {
         GridCorners c;
         gridCorners(l, u, c);
         float f0 = 0.0f, f1 = 0.0f;
         for (int k = 0; k < 8; ++k) {
+#if defined(__CUDA_ARCH__)
+            const float2 f = __ldg(reinterpret_cast<const float2*>(g.grid) + c.idx[k]); // an entry's two features
+            f0 += c.w[k] * f.x;
+            f1 += c.w[k] * f.y;
+#else
             f0 += c.w[k] * g.grid[2 * c.idx[k] + 0];
             f1 += c.w[k] * g.grid[2 * c.idx[k] + 1];
+#endif
         }
         x[2 * l + 0] = f0;
         x[2 * l + 1] = f1;
@@ -127,8 +134,10 @@ struct Lobes {
 // Network outputs → mixture: direction normalised, κ = exp(clamped log κ), softmax weights.
 PE_HD void decodeLobes(const float* o, Lobes& L) {
     float mx = -1e30f;
+#pragma unroll
     for (int k = 0; k < kLobes; ++k) mx = smax(mx, o[5 * k + 4]);
     float sum = 0.0f;
+#pragma unroll
     for (int k = 0; k < kLobes; ++k) {
         const V3 m = mk(o[5 * k + 0], o[5 * k + 1], o[5 * k + 2]);
         const float len = sqrtf(len2(m)) + 1e-6f;
@@ -137,37 +146,71 @@ PE_HD void decodeLobes(const float* o, Lobes& L) {
         L.weight[k] = expf(o[5 * k + 4] - mx);
         sum += L.weight[k];
     }
+#pragma unroll
     for (int k = 0; k < kLobes; ++k) L.weight[k] /= sum;
 }
 
 // vMF density on the sphere: κ / (2π (1 − e^{−2κ})) · e^{κ (μ·ω − 1)}.
-PE_HD float vmfPdf(V3 mu, float kappa, V3 w) {
-    const float norm = kappa / (2.0f * kPi * -expm1f(-2.0f * kappa));
-    return norm * expf(kappa * (dot(mu, w) - 1.0f));
-}
+PE_HD float vmfNorm(float kappa) { return kappa / (2.0f * kPi * -expm1f(-2.0f * kappa)); }
+PE_HD float vmfPdf(V3 mu, float kappa, float norm, V3 w) { return norm * expf(kappa * (dot(mu, w) - 1.0f)); }
 
-PE_HD float lobesPdf(const Lobes& L, V3 w) {
-    float p = 0.0f;
-    for (int k = 0; k < kLobes; ++k) p += L.weight[k] * vmfPdf(L.mu[k], L.kappa[k], w);
-    return p;
-}
-
-// One direction from the mixture: lobe by uLobe, then the vMF sample of Jakob 2012
-// ("Numerically stable sampling of the von Mises–Fisher distribution on S²").
-PE_HD V3 lobesSample(const Lobes& L, float uLobe, V2 u) {
-    int k = 0;
-    float acc = L.weight[0];
-    while (k < kLobes - 1 && uLobe >= acc) {
-        ++k;
-        acc += L.weight[k];
-    }
-    const float kappa = L.kappa[k];
+// The vMF sample of Jakob 2012 ("Numerically stable sampling of the von Mises–Fisher distribution on S²").
+PE_HD V3 vmfSample(V3 mu, float kappa, V2 u) {
     const float cosT = 1.0f + logf(u.x + (1.0f - u.x) * expf(-2.0f * kappa)) / kappa;
     const float c = sclamp(cosT, -1.0f, 1.0f);
     const float s = sqrtf(smax(0.0f, 1.0f - c * c));
     const float phi = 2.0f * kPi * u.y;
-    const Frame f = frameFromNormal(L.mu[k]);
-    return normalize(toWorld(f, mk(s * cosf(phi), s * sinf(phi), c)));
+    float sp, cp;
+    sinCos(phi, sp, cp);
+    const Frame f = frameFromNormal(mu);
+    return normalize(toWorld(f, mk(s * cp, s * sp, c)));
+}
+
+// A bounce's mixture in a path slot, decoded once by the inference kernel (each of a vertex's two or three
+// densities used to decode the 40 outputs again): 8 × (μ, κ), the weights, the density's norms.
+constexpr int kSlotMixture = 12; // float4
+PE_HD void putMixture(float4* at, const Lobes& L) {
+    float norm[kLobes];
+#pragma unroll
+    for (int k = 0; k < kLobes; ++k) {
+        at[k] = make_float4(L.mu[k].x, L.mu[k].y, L.mu[k].z, L.kappa[k]);
+        norm[k] = vmfNorm(L.kappa[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        at[8 + k] = make_float4(L.weight[4 * k], L.weight[4 * k + 1], L.weight[4 * k + 2], L.weight[4 * k + 3]);
+        at[10 + k] = make_float4(norm[4 * k], norm[4 * k + 1], norm[4 * k + 2], norm[4 * k + 3]);
+    }
+}
+PE_HD float mixturePdf(const float4* at, V3 w) {
+    float p = 0.0f;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const float4 wt = at[8 + h], nm = at[10 + h];
+        const float weight[4] = {wt.x, wt.y, wt.z, wt.w}, norm[4] = {nm.x, nm.y, nm.z, nm.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float4 m = at[4 * h + k];
+            p += weight[k] * vmfPdf(mk(m.x, m.y, m.z), m.w, norm[k], w);
+        }
+    }
+    return p;
+}
+// One direction from the mixture: a lobe by uLobe, then its sample.
+PE_HD V3 mixtureSample(const float4* at, float uLobe, V2 u) {
+    const float4 a = at[8], b = at[9];
+    const float weight[kLobes] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    int k = 0;
+    float acc = 0.0f;
+    bool found = false;
+#pragma unroll
+    for (int i = 0; i < kLobes; ++i) {
+        acc = i == 0 ? weight[0] : acc + weight[i];
+        if (!found) k = i;
+        found = found || !(uLobe >= acc);
+    }
+    const float4 m = at[k];
+    return vmfSample(mk(m.x, m.y, m.z), m.w, u);
 }
 
 // ∂(−log q(ω))/∂(network outputs) for the mixture decoded from o.
@@ -177,7 +220,7 @@ PE_HD float nllGrad(const float* o, V3 w, float* g) {
     float v[kLobes];
     float q = 0.0f;
     for (int k = 0; k < kLobes; ++k) {
-        v[k] = vmfPdf(L.mu[k], L.kappa[k], w);
+        v[k] = vmfPdf(L.mu[k], L.kappa[k], vmfNorm(L.kappa[k]), w);
         q += L.weight[k] * v[k];
     }
     q = smax(q, 1e-20f);

@@ -760,23 +760,11 @@ __device__ __forceinline__ bool guidable(const MatGPU& m) {
     return (m.flags & (MF_DELTA | MF_VOLUME_BOUNDARY | MF_TRANSMITS_SHADOWS)) == 0;
 }
 
-static __device__ __noinline__ void slotLobes(const Paths& P, int slot, Lobes& L) {
-    float o[kNetUsedOut];
-    for (int j = 0; j < kNetUsedOut / 4; ++j) {
-        const float4 v = P.guideOut[static_cast<size_t>(slot) * 10 + j];
-        o[4 * j + 0] = v.x;
-        o[4 * j + 1] = v.y;
-        o[4 * j + 2] = v.z;
-        o[4 * j + 3] = v.w;
-    }
-    decodeLobes(o, L);
+__device__ __forceinline__ const float4* slotMixture(const Paths& P, int slot) {
+    return P.guideOut + static_cast<size_t>(slot) * kSlotMixture;
 }
 
-static __device__ __noinline__ float guidePdf(const Paths& P, int slot, V3 w) {
-    Lobes L;
-    slotLobes(P, slot, L);
-    return lobesPdf(L, w);
-}
+static __device__ __noinline__ float guidePdf(const Paths& P, int slot, V3 w) { return mixturePdf(slotMixture(P, slot), w); }
 
 // Training record of a path's first guidable vertex; its radiance along wi is what the path adds
 // from here on (kGuideCollect).  False when the path has one already.
@@ -797,12 +785,11 @@ static __device__ __noinline__ bool guideRecord(const Paths& P, int slot, V3 p, 
 // proposal draws a lobe from the rest of it and a direction from one get2D.
 static __device__ __noinline__ bool guidedSample(const TablesGPU* T, const MatGPU& mat, V3 wo, const ShadePoint& sp, const Paths& P,
                                           int slot, const DisneyVertex* dv, Sobol& sb, BsdfSample& bs) {
-    Lobes L;
-    slotLobes(P, slot, L);
+    const float4* mix = slotMixture(P, slot);
     const float uBranch = get1D(sb);
     if (uBranch < 0.5f) {
-        const V3 gwi = lobesSample(L, uBranch * 2.0f, get2D(T, sb));
-        const float gPdf = lobesPdf(L, gwi);
+        const V3 gwi = mixtureSample(mix, uBranch * 2.0f, get2D(T, sb));
+        const float gPdf = mixturePdf(mix, gwi);
         if (!(gPdf > 0.0f)) return false;
         float bPdf = 0.0f;
         const V3 f = bsdfEvalPdfT<-1>(T, mat, wo, gwi, sp, dv, bPdf, nullptr);
@@ -822,7 +809,7 @@ static __device__ __noinline__ bool guidedSample(const TablesGPU* T, const MatGP
     if (!bsdfSampleT<-1>(T, mat, wo, sp, dv, uc, u2, bs)) return false;
     if (bs.subsurface) bs.weight = bs.weight * 2.0f;
     else if (bs.delta || bs.passThrough) bs.pdf *= 0.5f;
-    else if (bs.pdf > 0.0f) bs.pdf = 0.5f * bs.pdf + 0.5f * lobesPdf(L, bs.wi);
+    else if (bs.pdf > 0.0f) bs.pdf = 0.5f * bs.pdf + 0.5f * mixturePdf(mix, bs.wi);
     return true;
 }
 

@@ -75,7 +75,7 @@ struct Paths {
     // learned proposal (null / 0 when off)
     float4* guideQ;      // 3 per query row, compacted per bounce: hit point | shading normal | view direction
     int32_t* guideSlot;  // slot of each query row
-    float4* guideOut;    // 10 per slot: the 40 network outputs of this bounce's proposal
+    float4* guideOut;    // kSlotMixture per slot: this bounce's proposal (putMixture)
     uint32_t* guideMark; // 1 = guideOut holds this bounce's proposal for the slot
     float4* guideRec;    // 6 per slot: training record of the first guidable vertex (see kGuideCollect)
     float4* trainBuf;    // 4 per training sample, compacted per wave
