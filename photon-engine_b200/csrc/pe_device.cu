@@ -382,13 +382,13 @@ void launchTail(pe_device* d, int features, bool inlineShadows, bool out, const 
         return;
     }
     const bool lean = features == 0;
-    const int64_t warps = static_cast<int64_t>(d->blocksTailWarps[lean ? 1 : 0][out ? 1 : 0]) * (kTailWarpsBlock / 32);
+    const int block = tailWarpsBlock(lean ? 0 : FEAT_ALL), blockWarps = block / 32;
+    const int64_t warps = static_cast<int64_t>(d->blocksTailWarps[lean ? 1 : 0][out ? 1 : 0]) * blockWarps;
     const int perWarp = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(32, (n + warps - 1) / warps)));
-    const int64_t perBlock = static_cast<int64_t>(perWarp) * (kTailWarpsBlock / 32);
-    const int grid = static_cast<int>(
-        std::max<int64_t>(1, std::min<int64_t>(warps / (kTailWarpsBlock / 32), (n + perBlock - 1) / perBlock)));
+    const int64_t perBlock = static_cast<int64_t>(perWarp) * blockWarps;
+    const int grid = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(warps / blockWarps, (n + perBlock - 1) / perBlock)));
     const auto tail = [&](auto kernel) {
-        kernel<<<grid, kTailWarpsBlock, 0, cs>>>(S, P, W, queue, count, cursor, hits, perWarp, d->dStats);
+        kernel<<<grid, block, 0, cs>>>(S, P, W, queue, count, cursor, hits, perWarp, d->dStats);
     };
     if (lean) out ? tail(kTailWarps<0, true>) : tail(kTailWarps<0, false>);
     else out ? tail(kTailWarps<FEAT_ALL, true>) : tail(kTailWarps<FEAT_ALL, false>);
@@ -1392,10 +1392,10 @@ pe_device* pe_device_create(int32_t ordinal, char* err, size_t errLen) {
         return sm * std::max(1, nb);
     };
     d->blocksTailLockstep = occ(kTailLockstep<0>, kTailLockstepBlock);
-    d->blocksTailWarps[0][0] = occ(kTailWarps<FEAT_ALL, false>, kTailWarpsBlock);
-    d->blocksTailWarps[0][1] = occ(kTailWarps<FEAT_ALL, true>, kTailWarpsBlock);
-    d->blocksTailWarps[1][0] = occ(kTailWarps<0, false>, kTailWarpsBlock);
-    d->blocksTailWarps[1][1] = occ(kTailWarps<0, true>, kTailWarpsBlock);
+    d->blocksTailWarps[0][0] = occ(kTailWarps<FEAT_ALL, false>, tailWarpsBlock(FEAT_ALL));
+    d->blocksTailWarps[0][1] = occ(kTailWarps<FEAT_ALL, true>, tailWarpsBlock(FEAT_ALL));
+    d->blocksTailWarps[1][0] = occ(kTailWarps<0, false>, tailWarpsBlock(0));
+    d->blocksTailWarps[1][1] = occ(kTailWarps<0, true>, tailWarpsBlock(0));
     for (int out = 0; out < 2; ++out)
         eachKeyKernel(out, [&](auto kernel, int key) { d->blocksShadeKey[out][key] = occ(kernel, 128); });
     d->blocksIntersectBinary = occ(kIntersectBinary<false>, 128);
