@@ -590,14 +590,17 @@ int32_t runWave(pe_device* d, int lane, Paths& P, int nSegs, int nSlots, int nPi
         }
         if ((rc = mark(e))) return rc;
         stats.kernel_launches += launchTrace(d, S, P, W, qIn, shadows, cs);
-        if (P.guiding == 2 && (rc = guideQueries(d, cs, P, W, qIn, &P.now[BC_QUEUE]))) return rc;
+        // the tail kernel's vertices are unguided, its first ones too: no proposal once the count says tail
+        if (P.guiding == 2 && !counted && (rc = readCounts())) return rc;
+        const auto toTail = [&]() { return iter > 0 && static_cast<int64_t>(live) <= tailPaths && nextPath == nSlots; };
+        if (P.guiding == 2 && live > 0 && !toTail() && (rc = guideQueries(d, cs, P, W, qIn, &P.now[BC_QUEUE]))) return rc;
         if ((rc = mark(e))) return rc;
         spent(tm.isect);
         if (!counted && (rc = readCounts())) return rc;
         if (live == 0) break;
         stats.closest_rays += live;
         ++stats.intersect_launches;
-        if (iter > 0 && static_cast<int64_t>(live) <= tailPaths && nextPath == nSlots) {
+        if (toTail()) {
             if ((rc = tail(true))) return rc;
             break;
         }

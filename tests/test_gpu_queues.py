@@ -66,3 +66,62 @@ def test_queue_edges(pe, device, kind):
             assert _same(films[0], aovs[0].beauty), (w, h)
     finally:
         device.set_tail_paths(-1)
+
+
+@pytest.mark.parametrize("kind", ["cornell", "knot", "grid", "media", "room_guided"])
+def test_feature_kernels_equal_the_full_kernel(pe, device, kind):
+    """Waves are shaded by kernels that carry their scene's features only; a counting device takes the
+    kernels with all of them, over the same paths: the films are equal bit for bit.  The guided wave is
+    a fresh network's first, whose training step comes after it."""
+    if kind == "room_guided":
+        S = importlib.import_module("photon_engine_b200.scenes")
+        scene, cam, st = S.room_scene(64, 36, 4, 8)
+    else:
+        scene, cam, st = _scene(kind)
+    scene.build_accelerator()
+    device.set_scene(scene)
+    films = []
+    try:
+        device.set_tail_paths(0)
+        for counting in (False, True):
+            if kind == "room_guided":
+                device.set_guiding(0)
+                device.set_guiding(1, 0, 0.0)
+                pe._capi.check(pe._capi.load().pe_device_guide_reset(device.handle, 7, None, None))
+            device.set_counting(counting)
+            films.append(pe.Film(st.width, st.height))
+            device.render(cam, st, pe.RenderTargets(beauty=films[-1]), 0, 4)
+    finally:
+        device.set_counting(False)
+        device.set_tail_paths(-1)
+        device.set_guiding(0)
+    assert _same(*films)
+
+
+def test_tail_vertices_stay_unguided(pe, device):
+    """The tail kernel runs no inference.  A camera that sees a small mirror and nothing else has no
+    guidable first vertex, and the few paths left go to the tail after it: the guided film is the plain one."""
+    S = importlib.import_module("photon_engine_b200.scenes")
+    scene = pe.Scene()
+    grey = pe.Lambertian((0.6, 0.5, 0.4))
+    for p, u, v, mat in (((-0.5, 0, 3), (1, 0, 0), (0, 1, 0), pe.Mirror((0.9, 0.9, 0.9))),
+                         ((-9, -9, -6), (18, 0, 0), (0, 18, 0), grey), ((-9, -2, -9), (18, 0, 0), (0, 0, 9), grey)):
+        pos, idx = S._wall_grid(tuple(map(float, p)), tuple(map(float, u)), tuple(map(float, v)), 4, 4, None)
+        scene.add_shape(pe.TriangleMesh(pos, None, None, idx, mat))
+    scene.add_light(pe.AreaLight((-1.0, 4.0, -3.0), (2.0, 0.0, 0.0), (0.0, 0.0, 2.0), (9.0, 9.0, 8.0)))
+    scene.build_accelerator()
+    device.set_scene(scene)
+    st = pe.RenderSettings(width=64, height=64, max_bounces=6, seed=3)
+    cam = pe.PerspectiveCamera((0.0, 0.5, 0.0), (0.0, 0.5, 3.0), (0.0, 1.0, 0.0), 40.0, 1.0)
+    films = []
+    try:
+        for guided in (False, True):
+            device.set_guiding(1 if guided else 0, 0, 0.0)
+            films.append(pe.Film(64, 64))
+            device.render(cam, st, pe.RenderTargets(beauty=films[-1]), 0, 1)
+            if guided:
+                assert 0 < device.last_stats().tail_paths <= 2048
+    finally:
+        device.set_guiding(0)
+    assert films[0].sum.max() > 0.0
+    assert _same(*films)
