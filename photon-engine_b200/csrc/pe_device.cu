@@ -574,8 +574,8 @@ int32_t runWave(pe_device* d, int lane, Paths& P, int nSegs, int nSlots, int nPi
             counted = true;
             return PE_OK;
         };
-        if (!counted && regen && nextPath < nSlots) {
-            // the slots of ended paths take the wave's next paths
+        if (!counted && regen && (nextPath < nSlots || !P.direct)) {
+            // the slots of ended paths hand over their radiance, but for direct waves, and take the wave's next paths
             if ((rc = readCounts())) return rc;
             const int freed = static_cast<int>(ln.hCounters[2 * kBounceBlock + CNT_FREE]);
             const int fresh = std::min(freed, nSlots - nextPath);

@@ -125,3 +125,23 @@ def test_tail_vertices_stay_unguided(pe, device):
         device.set_guiding(0)
     assert films[0].sum.max() > 0.0
     assert _same(*films)
+
+
+def test_moving_instances_in_a_regenerating_wave(pe, device):
+    """Waves over moving instances trace their shadow rays before a slot is handed on and flush ended
+    paths bounce by bounce, to the last one: 3.3M paths through 1M slots give the film of a wave whose
+    paths all start at once."""
+    scene, cam, st = importlib.import_module("test_instances").moving_cornell(pe, 64, 64, 8, 6)
+    st.motion_blur = True
+    st.width, st.height = 1100, 1000
+    scene.build_accelerator()
+    device.set_scene(scene)
+    films = []
+    try:
+        for slots, tail in ((1 << 23, -1), (1 << 20, -1), (1 << 20, 0)):
+            device.set_tuning(wave_slots=slots, tail_paths=tail)
+            films.append(pe.Film(1100, 1000))
+            device.render(cam, st, pe.RenderTargets(beauty=films[-1]), 0, 3)
+            assert _same(films[0], films[-1]), (slots, tail)
+    finally:
+        device.set_tuning()
