@@ -71,6 +71,8 @@ struct WaveLane {
     bool segsInFlight = false;
     uint32_t* hCounters = nullptr;    // pinned: the lane's counters (kCounters) after its last shading
     cudaEvent_t evCounts = nullptr;   // ... once that copy has landed
+    cudaStream_t side = nullptr;      // shading kernels beside the lane's stream (launchShade)
+    cudaEvent_t evFork = nullptr, evJoin = nullptr;
     float4* aovA = nullptr;           // AOVs per slot (allocated on first use, in aovBufs)
     float4* aovN = nullptr;
     std::vector<DevBuf> aovBufs;
