@@ -43,6 +43,7 @@ sys.path.insert(0, str(ROOT))
 WIDTH, HEIGHT, DEPTH = 1920, 1080, 12
 SPP_PER_STEP = 4  # one step = 4 samples per pixel of the 1080p frame (one wave of 8.3M paths)
 NODE_BYTES, TRI_BYTES, RAY_BYTES, HIT_BYTES, QUEUE_BYTES = 128, 48, 32, 16, 4  # 4-wide BVH node: 128 B
+SHADOW_RECORD_BYTES = 64
 L2_NOTE = ("inputs larger than L2: 140 MB resident scene + 0.6-1.2 GB of path state for the 4-8M paths in flight "
            "(L2 126 MB)")
 
@@ -265,7 +266,7 @@ def run_ours(args):
                        wave_slots=slots)
         tune_log = "fixed by --tuning"
     else:
-        dev.autotune(cam, st, SPP_PER_STEP)  # untimed set-up: picks traversal, register budget, tail
+        dev.autotune(cam, st, SPP_PER_STEP)  # untimed set-up: picks traversal, tail, paths in flight
         tune_log = dev.autotune_log()
     tuning = dev.tuning()
     tail = tuning["tail_paths"]
@@ -332,13 +333,18 @@ def run_ours(args):
         dev.close()
         return 0
 
-    # roofline of the closest-hit kernel: per-ray algorithmic bytes from the counting pass
+    # roofline of the traversal launches (a bounce's closest hits together with the shadow rays of the
+    # bounce before): per-ray algorithmic bytes from the counting pass
     node_bytes = 64 if tuning["closest_traversal"] == 0 else NODE_BYTES  # binary node 64 B, 4-wide 128 B
     bytes_per_ray = (cs.node_visits * node_bytes + cs.tri_tests * TRI_BYTES) / max(1, cs.closest_rays) + \
         RAY_BYTES + HIT_BYTES + QUEUE_BYTES
     peak, peak_kind = measured_peaks()
-    # only the rays the bounce-by-bounce closest-hit launches traced (the tail kernel's are its own)
-    achieved = (rays_isect * bytes_per_ray) / (ms_isect / 1000.0) / 1e9 if ms_isect > 0 else None
+    any_bytes_per_ray = (cs.shadow_node_visits * node_bytes + cs.shadow_tri_tests * TRI_BYTES) / max(1, cs.shadow_rays) + \
+        SHADOW_RECORD_BYTES + QUEUE_BYTES
+    # only the rays of the bounce-by-bounce launches (the tail kernel's are its own; its share of the
+    # shadow rays is taken as its share of the closest-hit rays)
+    any_isect = shadow_rays * rays_isect / max(1, rays)
+    achieved = (rays_isect * bytes_per_ray + any_isect * any_bytes_per_ray) / (ms_isect / 1000.0) / 1e9 if ms_isect > 0 else None
     traffic = None
     tfile = ROOT / "profiles" / "closest_hit_dram_bytes_per_ray.txt"
     if tfile.exists():
@@ -349,8 +355,8 @@ def run_ours(args):
             traffic = None
     roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
             "frac": (achieved / peak) if achieved else None, "traffic": traffic,
-            "kernel": "kIntersect (closest-hit BVH traversal)", "peak_kind": peak_kind,
-            "bytes_per_ray": bytes_per_ray, "avg_launch_ms": ms_isect / max(1, n_isect),
+            "kernel": "kTrace (closest-hit and any-hit BVH traversal)", "peak_kind": peak_kind,
+            "bytes_per_ray": bytes_per_ray, "any_hit_bytes_per_ray": any_bytes_per_ray, "avg_launch_ms": ms_isect / max(1, n_isect),
             "rays_per_launch": rays_isect / max(1, n_isect)}
 
     # the shading kernels (one lean kernel per shading key): algorithmic bytes per shaded path —

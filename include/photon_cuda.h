@@ -491,16 +491,15 @@ int32_t pe_device_autotune(pe_device* d, const pe_camera* cam, const pe_settings
 typedef struct pe_tuning {
     int64_t tail_paths;        /* as pe_device_set_tail_paths */
     int32_t closest_traversal; /* bounce-by-bounce closest hits: 0 the binary tree in the reference's
-                                  order, a ray per lane; 1-9 (default 6) the 4-wide tree, four lanes
-                                  per ray (one kernel: the numbers are kept for callers that stored
-                                  one of the variants it replaced) */
-    int32_t shade_budget;      /* lean shading kernels: 0-2 (default 1), all at most 128 registers a
-                                  thread for surfaces (four 128-thread blocks per SM) */
-    int32_t any_traversal;     /* plain any-hit shadows: 0-2 (default 2), all the four-lane walk */
+                                  order; 1-9 (default 6) the 4-wide tree (one kernel: the numbers are
+                                  kept for callers that stored one of the variants it replaced) */
+    int32_t shade_budget;      /* lean shading kernels: 0-2 (default 1), all the same kernels (five or
+                                  six 128-thread blocks per SM for surfaces) */
+    int32_t any_traversal;     /* plain any-hit shadows: 0-2 (default 2), all the same walk */
     int64_t wave_slots;        /* paths in flight in a regenerating wave (unguided renders without
                                   AOV or pass targets): 2^20 … 2^23, default 2^23; 0 on input keeps
                                   the current value.  Each of the device's two lanes holds path
-                                  state for that many paths (536 B a slot, 256 B of it the radiance
+                                  state for that many paths (537 B a slot, 256 B of it the radiance
                                   of the paths the slots cycle through: 9 GB for both lanes at
                                   2^23), allocated at the next render and never shrunk */
 } pe_tuning;

@@ -218,9 +218,9 @@ static __global__ void kInitFree(const __grid_constant__ Paths P, int n) {
 
 // ---- closest hit over a queue -----------------------------------------------------------------
 // Closest hit for every queued ray; kBin then bins the rays by shading key (miss or the hit
-// material's type) so that the shading kernels run warps of one material kind.  Traversals of pe_tuning::closest_traversal: 0 the binary tree in the reference's order, one lane
-// per ray; 1-9 the 4-wide tree, four lanes per ray (one kernel: the numbers once told variants apart
-// that the four-lane walk replaced).
+// material's type) so that the shading kernels run warps of one material kind.  Traversals of
+// pe_tuning::closest_traversal: 0 the binary tree in the reference's order, one lane per ray; 1-9 the
+// 4-wide tree in the converged walk of pe_walk.cuh (one kernel for all these numbers).
 enum TraceMode { TRACE_BINARY = 0, TRACE_MODES = 10 };
 
 // The shading key of a closest hit by its primitive.
@@ -1627,8 +1627,8 @@ __global__ void __launch_bounds__(128, MINB) kShadeKey(const __grid_constant__ S
 }
 
 // ---- tail: the last paths of a wave, each run to its end by one thread -------------------------
-// Once a wave's live queue fits in one resident grid, per-bounce launches cost more than they
-// save: each thread takes a path from the queue, alternates closest-hit queries with shadeSlot
+// Once few paths of a wave are left (defaultTailPaths), per-bounce launches cost more than they
+// save.  Here each thread takes a path from the queue, alternates closest-hit queries with shadeSlot
 // (shadow rays inline) until the path ends, then takes the next (`traced`: the queue's paths have
 // their first hits).  The arithmetic and the order of
 // L's terms are the wavefront's, so the film is the same bit for bit.  This one-warp-per-block
@@ -1868,7 +1868,7 @@ __global__ void __launch_bounds__(tailWarpsBlock(FEAT)) kTailWarps(const __grid_
         if (key >= 0 && (peers & below) == 0) keyCount[tid >> 5][key] = static_cast<uint8_t>(__popc(peers));
         __syncthreads();
         if (key >= 0) {
-            int rank = __popc(peers & below), total = 0, spare = kWarps, first = 0, firstWarp = 0, mine = 0;
+            int rank = __popc(peers & below), spare = kWarps, first = 0, firstWarp = 0, mine = 0;
             int most = 0, mostKey = 0;
 #pragma unroll
             for (int k = 0; k < kShadeKeys; ++k) {
@@ -1884,10 +1884,7 @@ __global__ void __launch_bounds__(tailWarpsBlock(FEAT)) kTailWarps(const __grid_
                     first += c;
                     firstWarp += warps;
                 }
-                if (k == key) {
-                    total = c;
-                    mine = warps;
-                }
+                if (k == key) mine = warps;
                 if (c > most) {
                     most = c;
                     mostKey = k;

@@ -579,7 +579,7 @@ __device__ __forceinline__ void cmpx(float& ta, int& ra, int& ka, float& tb, int
 }
 
 // The 4-wide walk by one lane from reference `cur`: rays cast inside the shading code (contact
-// occlusion, rounded edges, transmitted shadows).  The queues' rays take the four-lane walk below.
+// occlusion, rounded edges, transmitted shadows).  The queues' rays take walkTurn (pe_walk.cuh).
 template <bool COUNT, int LEVEL>
 __device__ void walkClosestWide(const SceneGPU& S, int cur, V3 o, V3 d, V3 inv, uint32_t mask, float tMin, float& tMax,
                                 Hit& best, uint32_t& nodeVisits, uint32_t& triTests, float time) {

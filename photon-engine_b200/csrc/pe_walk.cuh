@@ -105,7 +105,8 @@ struct RayWalk {
 // What a warp's rays ask for: the closest hit, any hit, or (RayWalk::any) some the one and some the other.
 enum WalkKind { WALK_CLOSEST, WALK_ANY, WALK_MIXED };
 
-// One turn of the walk for every lane of the warp that has a reference.  T: uint2 (reference, entry distance), or for any hit uint32_t (reference).
+// One turn of the walk for every lane of the warp that has a reference.  T: uint2 (reference, entry
+// distance), or for any hit uint32_t (reference).
 // world(o, d, mask) gives the lane's ray back when it leaves an instance, time() its shutter time;
 // found(t, u, v, prim, meta) takes a closest hit nearer than (or as near as) those before it.
 // INSTANCES: the scene has mesh instances.

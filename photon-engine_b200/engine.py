@@ -1100,8 +1100,8 @@ class CudaDevice:
         capi.check(_lib().pe_device_set_counting(self._h, 1 if on else 0))
 
     def set_tail_paths(self, paths: int):
-        """Live paths at or below which a wave finishes in the per-thread tail kernel
-        (-1 = one resident grid, 0 = never); the film does not depend on it."""
+        """Live paths at or below which a wave finishes in the tail kernel (-1 = the default, 448 per SM for
+        plain surface scenes and 224 for others, 0 = never); the film does not depend on it."""
         capi.check(_lib().pe_device_set_tail_paths(self._h, int(paths)))
 
     @property
