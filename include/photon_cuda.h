@@ -460,7 +460,7 @@ int32_t pe_device_film_clear(pe_device* d);
  * scene with mipmapped image maps (whose level of detail needs a per-path ray cone) are rejected
  * with PE_ERR_INVALID, as is adaptive sampling; render those with pe_device_render.
  *
- * The path state lives in one file-scope device array of 8.5 MB (room for 32768 paths), which
+ * The path state lives in one file-scope device array of 8.6 MB (room for 32768 paths), which
  * every GPU that loads this library holds until the process exits; its address on a device is
  * taken once, when the device is created.  A tile of more than 32768 pixels (w*h) is rejected
  * with PE_ERR_LIMIT.  Every call uses the same array and finds the previous call's contents in

@@ -50,18 +50,10 @@ int32_t allocLane(WaveLane& ln, size_t slots) {
     freeList(ln.bufs);
     int32_t st = 0;
     Paths& P = ln.paths;
-    float4** cols[] = {&P.rayO, &P.rayD, &P.thr, &P.L, &P.lastN, &P.lastP, &P.pickP, &P.pickN, &P.hit, &P.med};
-    for (float4** c : cols)
-        if ((st = devAlloc(ln.bufs, *c, slots))) return st;
-    if ((st = devAlloc(ln.bufs, P.queueA, slots))) return st;
-    if ((st = devAlloc(ln.bufs, P.queueB, slots))) return st;
-    if ((st = devAlloc(ln.bufs, P.key, slots))) return st;
-    if ((st = devAlloc(ln.bufs, P.sortQ, slots * kShadeKeys))) return st;
-    // shadow records: one per slot (shadow quality 1)
-    if ((st = devAlloc(ln.bufs, P.shadowQ, slots))) return st;
-    float4** scols[] = {&P.shO, &P.shD, &P.shC, &P.shT};
-    for (float4** c : scols)
-        if ((st = devAlloc(ln.bufs, *c, slots))) return st;
+    eachWaveColumn(P, [&](auto*& column, size_t entries) {
+        if (!st) st = devAlloc(ln.bufs, column, slots * entries);
+    });
+    if (st) return st;
     uint32_t* counters = nullptr;
     if ((st = devAlloc(ln.bufs, counters, kCounters))) return st;
     setCounters(P, counters);
@@ -230,31 +222,12 @@ int32_t featuresOf(const SceneGPU& G, const std::vector<MatGPU>& mats) {
     return f;
 }
 
-// Scratch of pe_device_render_tile_noalloc: path-state columns, queues, shadow records and
-// counters for kNoAllocSlots paths, carved out of one file-scope device array (8.5 MB).  Every
-// GPU that loads this library holds the array until the process exits.
+// Scratch of pe_device_render_tile_noalloc: the wave's columns and counters for kNoAllocSlots paths,
+// carved out of one file-scope device array (8.6 MB).  Every GPU that loads this library holds the
+// array until the process exits.
 constexpr size_t kNoAllocSlots = size_t(1) << 15;
-constexpr size_t kNoAllocColumn = kNoAllocSlots * sizeof(float4);   // 512 KiB, 256-aligned
-constexpr size_t kNoAllocIndex = kNoAllocSlots * sizeof(int32_t);    // 128 KiB, 256-aligned
-constexpr size_t kNoAllocCounters = 512;                             // bytes
-static_assert(kCounters * sizeof(uint32_t) <= kNoAllocCounters, "the scratch holds every counter");
-constexpr size_t kNoAllocBytes = 14 * kNoAllocColumn + (3 + kShadeKeys) * kNoAllocIndex + kNoAllocCounters;
-static __device__ __align__(256) unsigned char g_noAllocScratch[kNoAllocBytes];
-
-// Path-state view of the scratch whose device address is `base`.
-Paths noAllocPaths(unsigned char* base) {
-    Paths P{};
-    size_t off = 0;
-    auto col = [&](float4*& c) { c = reinterpret_cast<float4*>(base + off); off += kNoAllocColumn; };
-    auto idx = [&](int32_t*& c, size_t n) { c = reinterpret_cast<int32_t*>(base + off); off += n * kNoAllocIndex; };
-    col(P.rayO); col(P.rayD); col(P.thr); col(P.L); col(P.lastN); col(P.lastP); col(P.pickP); col(P.pickN); col(P.hit);
-    col(P.med);
-    col(P.shO); col(P.shD); col(P.shC); col(P.shT);
-    idx(P.queueA, 1); idx(P.queueB, 1); idx(P.shadowQ, 1); idx(P.sortQ, kShadeKeys);
-    setCounters(P, reinterpret_cast<uint32_t*>(base + off));
-    P.capacity = static_cast<uint32_t>(kNoAllocSlots);
-    return P;
-}
+static_assert(kNoAllocSlots % kCarveAlign == 0, "columns of the scratch start aligned");
+static __device__ __align__(256) unsigned char g_noAllocScratch[waveBytes(kNoAllocSlots)];
 
 // f(kernel, key) over the per-key shading kernels.
 template <typename F>
@@ -2098,9 +2071,7 @@ int32_t pe_device_render_tile_noalloc(pe_device* d, const pe_camera* cam, const 
     if (!rc) rc = checkFilmPointer(d, "sum_lum_sq", sumLumSq, px * sizeof(float));
     if (rc) return rc;
     if (count <= 0) return PE_OK;
-    Paths P = noAllocPaths(d->noAllocBase);
-    // The array keeps the previous call's contents; the queue and shadow counters must start at 0.
-    PE_CUDA(cudaMemsetAsync(P.blocks, 0, kNoAllocCounters, d->stream));
+    Paths P = carveWave(d->noAllocBase, kNoAllocSlots);
     return renderWaves(d, cam, st, first, count, nullptr, sumRgb, sampleCount, sumLumSq, &P, kNoAllocSlots, false,
                        Tile{x0, y0, w, h});
 }

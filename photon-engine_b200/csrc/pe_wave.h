@@ -6,7 +6,9 @@
 #include "pe_math.h"
 #include "pe_sdtree.h"
 
+#include <cstddef>
 #include <cstdint>
+#include <type_traits>
 #include <vector_types.h>
 
 namespace pe {
@@ -213,6 +215,37 @@ inline void setCounters(Paths& P, uint32_t* p) {
 inline void setBlock(Paths& P, int b) {
     P.now = P.blocks + b * kBounceBlock;
     P.next = P.blocks + (1 - b) * kBounceBlock;
+}
+
+// The columns that every wave reads or writes, each as f(column, entries per slot).  The lanes and the
+// fixed scratch of pe_device_render_tile_noalloc both take theirs from this list, so that neither can
+// miss one that a kernel takes for granted.
+template <typename F>
+constexpr void eachWaveColumn(Paths& P, F f) {
+    f(P.rayO, 1); f(P.rayD, 1); f(P.thr, 1); f(P.L, 1); f(P.lastN, 1); f(P.lastP, 1); f(P.pickP, 1); f(P.pickN, 1);
+    f(P.hit, 1); f(P.med, 1);
+    f(P.shO, 1); f(P.shD, 1); f(P.shC, 1); f(P.shT, 1); // shadow records: one per slot (shadow quality 1)
+    f(P.queueA, 1); f(P.queueB, 1); f(P.shadowQ, 1); f(P.sortQ, kShadeKeys);
+    f(P.key, 1);
+}
+// Bytes of path state carved by carveWave: the columns of `slots` slots, then every counter.
+constexpr size_t kCarveAlign = 256;
+constexpr size_t waveBytes(size_t slots) {
+    Paths P{};
+    size_t bytes = 0;
+    eachWaveColumn(P, [&](auto*& column, size_t entries) { bytes += entries * slots * sizeof(*column); });
+    return bytes + (kCounters * sizeof(uint32_t) + kCarveAlign - 1) / kCarveAlign * kCarveAlign;
+}
+// Path state of `slots` (a multiple of kCarveAlign) slots in the waveBytes(slots) bytes at `base`.
+inline Paths carveWave(unsigned char* base, size_t slots) {
+    Paths P{};
+    eachWaveColumn(P, [&](auto*& column, size_t entries) {
+        column = reinterpret_cast<std::decay_t<decltype(column)>>(base);
+        base += entries * slots * sizeof(*column);
+    });
+    setCounters(P, reinterpret_cast<uint32_t*>(base));
+    P.capacity = static_cast<uint32_t>(slots);
+    return P;
 }
 
 #ifdef __CUDACC__
