@@ -2091,12 +2091,10 @@ int32_t pe_device_last_stats(pe_device* d, pe_render_stats* out) {
     return PE_OK;
 }
 
-// Times a few tail thresholds on probe renders of the caller's view into a scratch film and keeps
-// the fastest; the film never depends on the threshold, so tuning is free to pick any of them.
 // Coordinate descent over the tuning knobs on probe renders of the caller's frame (samples from
-// 2^24 on, into a scratch film): the closest-hit traversal variant, then the shading kernels'
-// register budget, then the tail threshold; each candidate is timed twice and its faster render
-// counts, after one warm-up render.  The films are the same for every choice.
+// 2^24 on, into a scratch film): paths in flight per wave, then the closest-hit traversal, then the
+// tail threshold; each candidate is timed twice and its faster render counts, after one warm-up
+// render.  The caller's films are untouched.
 int32_t pe_device_autotune(pe_device* d, const pe_camera* cam, const pe_settings* st, int32_t probeSpp,
                            int64_t* chosen) {
     if (!d) {
@@ -2165,7 +2163,9 @@ int32_t pe_device_autotune(pe_device* d, const pe_camera* cam, const pe_settings
              if (!rc) rc = ensureCapacity(d, kWaveSlots);
          },
          {static_cast<int64_t>(kWaveSlots), static_cast<int64_t>(kDefaultWaveSlots), static_cast<int64_t>(kMaxWaveSlots)});
-    tune("closest_traversal", [&](int64_t v) { d->closestMode = static_cast<int>(v); }, {d->closestMode, TRACE_BINARY});
+    // both kernels, whichever is in force: the 4-wide one under the number it was asked for by
+    const int wide = d->closestMode == TRACE_BINARY ? TRACE_DEFAULT : d->closestMode;
+    tune("closest_traversal", [&](int64_t v) { d->closestMode = static_cast<int>(v); }, {wide, TRACE_BINARY});
     const int64_t grid = defaultTailPaths(d, true);
     tune("tail_paths", [&](int64_t v) { d->tailPaths = v; }, {grid / 4, grid / 2, grid, 2 * grid});
     d->guideKind = savedKind;

@@ -221,7 +221,7 @@ static __global__ void kInitFree(const __grid_constant__ Paths P, int n) {
 // material's type) so that the shading kernels run warps of one material kind.  Traversals of
 // pe_tuning::closest_traversal: 0 the binary tree in the reference's order, one lane per ray; 1-9 the
 // 4-wide tree in the converged walk of pe_walk.cuh (one kernel for all these numbers).
-enum TraceMode { TRACE_BINARY = 0, TRACE_MODES = 10 };
+enum TraceMode { TRACE_BINARY = 0, TRACE_DEFAULT = 6, TRACE_MODES = 10 };
 
 // The shading key of a closest hit by its primitive.
 __device__ __forceinline__ int shadeKeyOfPrim(const SceneGPU& S, uint32_t rayMask, int prim) {
