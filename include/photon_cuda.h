@@ -479,6 +479,7 @@ int32_t pe_device_set_counting(pe_device* d, int32_t enabled);
  * remain live; those finish in one launch that runs each path to its end.  The film is the same
  * either way.  -1 (default) = 448 paths per SM in scenes of plain surfaces, 224 in others, 0 = never. */
 int32_t pe_device_set_tail_paths(pe_device* d, int64_t paths);
+/* The threshold set, or with -1 the default for plain renders of the device's scene. */
 int64_t pe_device_tail_paths(pe_device* d);
 /* Autotuner (no reference counterpart): renders probe_spp samples of the view with each of a few
  * tail thresholds (1/4, 1/2, 1 and 2 times the default) into a scratch film, twice, and keeps the

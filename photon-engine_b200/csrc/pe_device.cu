@@ -418,14 +418,20 @@ void launchShadow(pe_device* d, const SceneGPU& S, const Paths& P, cudaStream_t 
     else kShadow<false><<<d->blocksShadow, 128, 0, cs>>>(S, P, st);
 }
 
+// The shading features a wave of scene S needs (kernels that count rays or trace shadow rays inline carry all).
+int waveFeatures(const pe_device* d, const SceneGPU& S, bool guided, bool ao, bool inlineShadows) {
+    if (d->counting || inlineShadows) return FEAT_ALL;
+    return S.features | (guided ? FEAT_GUIDE : 0) | (ao ? FEAT_REST : 0);
+}
+
 // Live paths at or below which a wave's rest goes to the tail kernel unless the caller says otherwise.
 // Below the line a bounce of the whole wave costs more than its rays: it lasts as long as its longest
 // ray and path (about 0.35 ms on the torus knot, however few rays).  448 paths per SM measured best
 // or within 2 % from 64x64 to 1920x1080 films of lean-shading scenes (256x256 x 1 spp, ms, at half
 // this line / at it: Cornell 0.51 / 0.33, knot 2.19 / 2.09, room 2.33 / 1.99, grid 2.81 / 2.48); half of it
 // for the others, whose tail kernel carries all shading code (media 1280x720 x 4 spp: 19.7 / 21.2).
-int64_t defaultTailPaths(const pe_device* d, bool lean) {
-    return static_cast<int64_t>(d->prop.multiProcessorCount) * (lean ? 448 : 224);
+int64_t defaultTailPaths(const pe_device* d, int features) {
+    return static_cast<int64_t>(d->prop.multiProcessorCount) * (features == 0 ? 448 : 224);
 }
 
 // One wave on a lane over the nSegs segments in its segment table (nSlots paths, nPix film
@@ -503,11 +509,9 @@ int32_t runWave(pe_device* d, int lane, Paths& P, int nSegs, int nSlots, int nPi
         noAo = noAo && !(ln.hSegs[k].aoStrength > 0.0f);
         inlineShadows = inlineShadows || ln.hSegs[k].shadowSamples > 1;
     }
-    // the shading features this wave needs (kernels that count rays or trace shadow rays inline carry all)
-    const int features = d->counting || inlineShadows ? FEAT_ALL
-                                                      : S.features | (P.guiding || P.sdMode ? FEAT_GUIDE : 0) | (noAo ? 0 : FEAT_REST);
+    const int features = waveFeatures(d, S, P.guiding || P.sdMode, !noAo, inlineShadows);
     const bool out = P.aovA || P.pass;
-    int64_t tailPaths = d->tailPaths < 0 ? defaultTailPaths(d, features == 0) : d->tailPaths;
+    int64_t tailPaths = d->tailPaths < 0 ? defaultTailPaths(d, features) : d->tailPaths;
     // the tail kernel runs no inference: keep guided bounces in the wavefront until few paths remain
     if (P.guiding == 2) tailPaths = std::min<int64_t>(tailPaths, kGuideTailPaths);
     auto mark = [&](cudaEvent_t& e) -> int32_t {
@@ -2166,7 +2170,7 @@ int32_t pe_device_autotune(pe_device* d, const pe_camera* cam, const pe_settings
     // both kernels, whichever is in force: the 4-wide one under the number it was asked for by
     const int wide = d->closestMode == TRACE_BINARY ? TRACE_DEFAULT : d->closestMode;
     tune("closest_traversal", [&](int64_t v) { d->closestMode = static_cast<int>(v); }, {wide, TRACE_BINARY});
-    const int64_t grid = defaultTailPaths(d, true);
+    const int64_t grid = defaultTailPaths(d, waveFeatures(d, d->scene, false, st->ao_strength > 0.0f, st->shadow_quality > 1));
     tune("tail_paths", [&](int64_t v) { d->tailPaths = v; }, {grid / 4, grid / 2, grid, 2 * grid});
     d->guideKind = savedKind;
     d->guide.mode = savedMode;
@@ -2244,7 +2248,7 @@ int32_t pe_device_set_tail_paths(pe_device* d, int64_t paths) {
 
 int64_t pe_device_tail_paths(pe_device* d) {
     if (!d) return -1;
-    return d->tailPaths < 0 ? defaultTailPaths(d, true) : d->tailPaths;
+    return d->tailPaths < 0 ? defaultTailPaths(d, d->scene.features) : d->tailPaths;
 }
 
 int32_t pe_device_set_counting(pe_device* d, int32_t enabled) {

@@ -281,6 +281,7 @@ inline void freeList(std::vector<DevBuf>& list) {
 }
 
 int32_t ensureCapacity(pe_device* d, size_t slots);
+int64_t defaultTailPaths(const pe_device* d, int features);
 int32_t checkSettings(const pe_camera* cam, const pe_settings* st);
 WaveSeg makeSeg(const pe_camera* cam, const pe_settings* st);
 const float* filterTable(pe_device* d, int type, float width, uint64_t wave, cudaStream_t stream);

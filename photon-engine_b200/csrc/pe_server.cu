@@ -504,8 +504,7 @@ void laneThread(pe_server* S, int li) {
     cudaSetDevice(d->ordinal);
     auto& R = S->lanes[li];
     const cudaStream_t cs = R.stream;
-    // the express lane hands its last paths to the tail kernel earlier: latency over efficiency
-    const int64_t tailPaths = pe_device_tail_paths(d) * (express(li) ? 4 : 1);
+    const int64_t tailSetting = d->tailPaths;
     std::unique_lock<std::mutex> lk(S->mu);
     for (;;) {
         if (S->stop) break;
@@ -567,6 +566,15 @@ void laneThread(pe_server* S, int li) {
         for (; R.aoChecked < nSegs; ++R.aoChecked)
             if (R.hSegs[R.aoChecked].aoStrength > 0.0f) R.anyAo = true;
         L.features = L.scene.features | (R.anyAo ? FEAT_REST : 0);
+        // the threshold of a lone render of the scene (six 320x180 x 8-spp media previews at once: 23.7 ms at that
+        // of plain scenes, 20.7 at the scene's own); the express lane hands its last paths to the tail
+        // kernel earlier: latency over efficiency
+        const int64_t tailPaths =
+            (tailSetting < 0 ? defaultTailPaths(d, L.features) : tailSetting) * (express(li) ? 4 : 1);
+        // an express wave holds only interactive paths: sweeping millions of them into the tail
+        // kernel would be slower than their wavefront bounces, so it sweeps only the stragglers
+        // of a wave that has shrunk to what it would hand over
+        L.sweepLive = express(li) ? tailPaths : 0;
         const int upFirst = R.uploaded;
         R.uploaded = nSegs;
         const bool draining = R.draining;
@@ -722,10 +730,6 @@ pe_server* pe_server_create(pe_device* d, uint64_t budget, char* err, size_t err
         LaneLoop& L = R.loop;
         const size_t cap = ok ? R.loop.ln->paths.capacity : 0;
         L.sweepAge = express(li) ? kExpressSweepAge : kSweepAge;
-        // an express wave holds only interactive paths: sweeping millions of them into the tail
-        // kernel (one thread per path) would be slower than their wavefront bounces, so it sweeps
-        // only the stragglers of a wave that has shrunk to a few tail grids
-        L.sweepLive = express(li) ? 4 * pe_device_tail_paths(d) : 0;
         ok = ok && cudaStreamCreateWithPriority(&L.side, cudaStreamNonBlocking, express(li) ? hiPrio : loPrio) == cudaSuccess &&
              cudaMalloc(&L.born, cap * sizeof(int32_t)) == cudaSuccess &&
              cudaMalloc(&L.sweepCnt, LaneLoop::kSweepBufs * sizeof(uint32_t)) == cudaSuccess &&
