@@ -623,7 +623,7 @@ int32_t runWave(pe_device* d, int lane, Paths& P, int nSegs, int nSlots, int nPi
     PE_CUDA(cudaEventRecord(d->evFilm, cs));
     d->filmLane = lane;
     ++stats.kernel_launches;
-    if (P.guiding && (rc = guideLearn(d, cs, P, nSlots))) return rc;
+    if (P.guiding && (rc = guideLearn(d, cs, P, W))) return rc;
     if ((P.sdMode & SD_RECORD) && (rc = sdRecord(d, cs, P, nSlots))) return rc;
     PE_CUDA(cudaEventRecord(ln.evDone, cs));
     ln.pending = true;

@@ -296,7 +296,7 @@ int32_t uploadScene(pe_device* d, const pe_scene* s, SceneGPU& out, std::vector<
 // Learned proposal in the wave loop (pe_guide.cu): the bounce's queries and their tensor-core
 // inference, and after the film kernel the wave's training samples and one Adam step.
 int32_t guideQueries(pe_device* d, cudaStream_t s, Paths& P, const Wave& W, const int32_t* queue, const uint32_t* count);
-int32_t guideLearn(pe_device* d, cudaStream_t s, Paths& P, int nSlots);
+int32_t guideLearn(pe_device* d, cudaStream_t s, Paths& P, const Wave& W);
 // A continuous wave on one lane (the request server): paths are injected into the slots that
 // ended paths free, bounce after bounce, until the server drains the lane with the tail kernel.
 struct LaneLoop {

@@ -326,9 +326,10 @@ __global__ void kGuideQuery(const __grid_constant__ SceneGPU S, const __grid_con
 // (point, normal, view direction, sampled direction ω, throughput before the bounce) and the
 // radiance the path had gathered before anything arrived along ω; what the path added since,
 // over that throughput, is f·cos·L(ω)/pdf for this one sample — the weight c of −c·log q(ω).
-__global__ void kGuideCollect(const __grid_constant__ Paths P, int nSlots) {
-    for (int s = (blockIdx.x * blockDim.x + threadIdx.x) * P.guideStride; s < nSlots;
-         s += gridDim.x * blockDim.x * P.guideStride) {
+__global__ void kGuideCollect(const __grid_constant__ Paths P, const __grid_constant__ Wave W) {
+    for (int order = (blockIdx.x * blockDim.x + threadIdx.x) * P.guideStride; order < W.nSlots;
+         order += gridDim.x * blockDim.x * P.guideStride) {
+        const int s = pathOfTrainOrder(W.segs[segOfSlot(W, order)], order); // guided waves hold path s in slot s
         float4* rec = P.guideRec + static_cast<size_t>(s) * 6;
         const float4 r4 = rec[4];
         if (r4.w == 0.0f) continue;
@@ -471,10 +472,10 @@ int32_t guideQueries(pe_device* d, cudaStream_t s, Paths& P, const Wave& W, cons
                       P.guideMark);
 }
 
-int32_t guideLearn(pe_device* d, cudaStream_t s, Paths& P, int nSlots) {
+int32_t guideLearn(pe_device* d, cudaStream_t s, Paths& P, const Wave& W) {
     GuideState& G = d->guide;
-    const int maxRows = (nSlots + P.guideStride - 1) / P.guideStride;
-    kGuideCollect<<<std::max(1, (maxRows + 255) / 256), 256, 0, s>>>(P, nSlots);
+    const int maxRows = (W.nSlots + P.guideStride - 1) / P.guideStride;
+    kGuideCollect<<<std::max(1, (maxRows + 255) / 256), 256, 0, s>>>(P, W);
     PE_CUDA(cudaGetLastError());
     const int32_t rc = guideTrain(d, s, P.trainBuf, &P.counters[CNT_TRAIN], 0, maxRows, G.lr);
     if (rc) return rc;

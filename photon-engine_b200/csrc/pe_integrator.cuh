@@ -127,7 +127,7 @@ __device__ __forceinline__ void generatePath(const SceneGPU& S, const Paths& P, 
     if (S.hasVolumes | S.hasSubsurface) P.med[slot] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (P.guiding) {
         P.guideMark[slot] = 0u;
-        if (slot % P.guideStride == 0) P.guideRec[static_cast<size_t>(slot) * 6 + 4] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (trainOrder(A, path) % P.guideStride == 0) P.guideRec[static_cast<size_t>(slot) * 6 + 4] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
     if (S.hasMips && P.cone) P.cone[slot] = make_float2(A.coneWidth, A.coneSpread);
     if (P.pass) {
@@ -1462,7 +1462,8 @@ __device__ __forceinline__ bool shadeSlot(const SceneGPU& S, const Paths& P, con
             const float cosTheta = fabsf(dot(wi, is.normal));
             const V3 thrBefore = thr;
             thr *= bs.f * (cosTheta / bs.pdf);
-            if (GUIDE && P.guiding && !bs.delta && slot % P.guideStride == 0 && guidable(mat) && isFinite3(thr) &&
+            if (GUIDE && P.guiding && !bs.delta && guidable(mat) && isFinite3(thr) &&
+                trainOrder(A, path) % P.guideStride == 0 &&
                 guideRecord(P, slot, is.point, is.normal, wo, wi, thrBefore))
                 flags |= PF_GUIDE_SNAP;
             if (!isFinite3(thr)) {

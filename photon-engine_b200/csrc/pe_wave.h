@@ -82,7 +82,7 @@ struct Paths {
     float4* guideRec;    // 6 per slot: training record of the first guidable vertex (see kGuideCollect)
     float4* trainBuf;    // 4 per training sample, compacted per wave
     int32_t guiding;     // 0 off, 1 record training samples, 2 record and sample with the proposal
-    int32_t guideStride; // one slot in guideStride records a training sample (about 64K per wave)
+    int32_t guideStride; // one path in guideStride records a training sample (trainOrder; about 64K per wave)
     // SD-tree guiding (null / 0 when off)
     SdField sd;          // sampling trees (read), building trees (splats)
     int32_t sdMode;      // bit 0: record training vertices, bit 1: sample with the SD-tree
@@ -248,17 +248,16 @@ inline Paths carveWave(unsigned char* base, size_t slots) {
     return P;
 }
 
-#ifdef __CUDACC__
 // Sample (of the segment's nSamples) of a wave path.
-__device__ __forceinline__ int sampleOfPath(const WaveSeg& A, int path) {
+PE_HD int sampleOfPath(const WaveSeg& A, int path) {
     const int local = path - A.slotFirst;
     return local - (local / A.nSamples) * A.nSamples;
 }
-__device__ __forceinline__ int pathOfSample(const WaveSeg& A, int p, int s) { return A.slotFirst + p * A.nSamples + s; }
+PE_HD int pathOfSample(const WaveSeg& A, int p, int s) { return A.slotFirst + p * A.nSamples + s; }
 // Film position of the segment's tile-linear pixel tp.  The rectangle is numbered in bands of four
 // rows, down each band's columns, so that the 32 paths of a warp look at a compact patch of the film
 // (their camera rays meet the same nodes and their first hits the same surfaces).
-__device__ __forceinline__ void tilePixel(const WaveSeg& A, int tp, int& x, int& y) {
+PE_HD void tilePixel(const WaveSeg& A, int tp, int& x, int& y) {
     if (A.pixList) {
         const int fp = A.pixList[tp];
         x = fp % A.width;
@@ -272,6 +271,33 @@ __device__ __forceinline__ void tilePixel(const WaveSeg& A, int tp, int& x, int&
     x = A.tileX + col;
     y = A.tileY + 4 * band + (in - col * rows);
 }
+// The learned proposal trains on the paths whose place in this order of the wave's paths is a multiple of
+// guideStride: sample by sample, and within a sample the pixels row by row (a wave of part of a rectangle or
+// of a pixel list: in the order of its pixels).  In the paths' own order a stride of the samples per
+// pixel would train on the first sample of each pixel alone, and smaller ones on one row in four.
+PE_HD bool wholeRectangle(const WaveSeg& A) { return !A.pixList && A.nPix == A.tileW * A.tileH; }
+PE_HD int trainOrder(const WaveSeg& A, int path) {
+    const int p = (path - A.slotFirst) / A.nSamples, s = path - A.slotFirst - p * A.nSamples;
+    int r = p;
+    if (wholeRectangle(A)) {
+        int x, y;
+        tilePixel(A, p, x, y);
+        r = (y - A.tileY) * A.tileW + x - A.tileX;
+    }
+    return A.slotFirst + s * A.nPix + r;
+}
+// The path at place `order`.
+PE_HD int pathOfTrainOrder(const WaveSeg& A, int order) {
+    const int s = (order - A.slotFirst) / A.nPix, r = order - A.slotFirst - s * A.nPix;
+    int p = r;
+    if (wholeRectangle(A)) {
+        const int y = r / A.tileW, x = r - y * A.tileW, band = y >> 2;
+        const int rows = A.tileH - 4 * band < 4 ? A.tileH - 4 * band : 4;
+        p = band * 4 * A.tileW + x * rows + (y - 4 * band);
+    }
+    return pathOfSample(A, p, s);
+}
+#ifdef __CUDACC__
 // Wave path index held by a slot.
 __device__ __forceinline__ int pathOfSlot(const Paths& P, int slot) { return P.pathOf ? P.pathOf[slot] : slot; }
 // Segment owning a wave path / a wave pixel (binary search; one segment for a lone request).
