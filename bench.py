@@ -12,10 +12,10 @@ msamplesPerSecond definition).
 ``e2e``     the same K steps through the public RenderDevice::render call with host films:
             camera + settings in, the frame's film (sum, count, sum of squares) read back and
             merged on the host every step.
-``roofline`` closest-hit traversal kernel: algorithmic bytes (4-wide BVH nodes visited × 128 B +
-            triangles tested × 48 B + ray record 32 B + hit record 16 B + queue index 4 B per
-            ray, counted on the device over one untimed step) ÷ its CUDA-event time, against
-            the measured HBM copy bandwidth.
+``roofline`` the traversal launches: bytes the walks ask for (BVH nodes visited × 128 B, binary ones
+            64 B, + triangles tested × 48 B + ray, hit and shadow records + queue indices, counted on
+            the device over one untimed step) ÷ their CUDA-event time, beside the measured HBM copy
+            bandwidth.  L1 and L2 serve most of them; `traffic` is what DRAM moves.
 ``cpu_baseline`` the reference engine's own CPU path (built with its shipping flags) on the same
             scene and camera, all host threads, a bounded number of full-frame samples.
 
@@ -43,6 +43,7 @@ sys.path.insert(0, str(ROOT))
 WIDTH, HEIGHT, DEPTH = 1920, 1080, 12
 SPP_PER_STEP = 4  # one step = 4 samples per pixel of the 1080p frame (one wave of 8.3M paths)
 NODE_BYTES, TRI_BYTES, RAY_BYTES, HIT_BYTES, QUEUE_BYTES = 128, 48, 32, 16, 4  # 4-wide BVH node: 128 B
+BINARY_NODE_BYTES = 64
 SHADOW_RECORD_BYTES = 64
 L2_NOTE = ("inputs larger than L2: 140 MB resident scene + 0.6-1.2 GB of path state for the 4-8M paths in flight "
            "(L2 126 MB)")
@@ -244,6 +245,24 @@ def pe_load():
     return pe_pkg.load()
 
 
+def traversal_roofline(closest_traversal, counted, closest_rays, shadow_rays, ms):
+    """The traversal launches (a bounce's closest hits together with the shadow rays of the bounce before)
+    against the memory: the bytes their walks ask for per ray, from a counting pass.  The binary closest-hit
+    tree (closest_traversal 0) has 64-byte nodes; the shadow rays walk the 4-wide tree in either case."""
+    binary = closest_traversal == 0
+    per_ray = (counted.node_visits * (BINARY_NODE_BYTES if binary else NODE_BYTES) + counted.tri_tests * TRI_BYTES) / \
+        max(1, counted.closest_rays) + RAY_BYTES + HIT_BYTES + QUEUE_BYTES
+    any_per_ray = (counted.shadow_node_visits * NODE_BYTES + counted.shadow_tri_tests * TRI_BYTES) / \
+        max(1, counted.shadow_rays) + SHADOW_RECORD_BYTES + QUEUE_BYTES
+    achieved = (closest_rays * per_ray + shadow_rays * any_per_ray) / (ms / 1000.0) / 1e9 if ms > 0 else None
+    return {"bound": "load latency and issue of divergent warps; the bytes are those the walks ask for, which L1 and L2 "
+                     "serve: DRAM moves `traffic` a launch",
+            "achieved": achieved, "unit": "GB/s",
+            "kernel": "kIntersectBinary (closest hits) and kShadowAny (any hits)" if binary
+            else "kTrace (closest-hit and any-hit BVH traversal)",
+            "bytes_per_ray": per_ray, "any_hit_bytes_per_ray": any_per_ray}
+
+
 def run_ours(args):
     world, rank, local = dist_setup()
     pg = None
@@ -273,11 +292,14 @@ def run_ours(args):
     # disjoint sample indices per replica; step k renders samples base + SPP_PER_STEP·(1 + warmup + k) …
     base = replica_sample_base(rank, args.warmup, args.steps)
 
-    # algorithmic bytes per closest-hit ray, counted on the device over one untimed 1-spp pass
+    # algorithmic bytes per closest-hit ray, counted on the device over one untimed 1-spp pass, bounce by bounce to
+    # its end (the tail kernel walks the 4-wide tree whatever the tuning)
+    dev.set_tail_paths(0)
     dev.set_counting(True)
     dev.render_resident(cam, st, base, 1)
     cs = dev.last_stats()
     dev.set_counting(False)
+    dev.set_tail_paths(tail)
     dev.film_clear()
     for w in range(args.warmup):
         dev.render_resident(cam, st, step_samples(base, 0, w), SPP_PER_STEP)
@@ -333,18 +355,7 @@ def run_ours(args):
         dev.close()
         return 0
 
-    # roofline of the traversal launches (a bounce's closest hits together with the shadow rays of the
-    # bounce before): per-ray algorithmic bytes from the counting pass
-    node_bytes = 64 if tuning["closest_traversal"] == 0 else NODE_BYTES  # binary node 64 B, 4-wide 128 B
-    bytes_per_ray = (cs.node_visits * node_bytes + cs.tri_tests * TRI_BYTES) / max(1, cs.closest_rays) + \
-        RAY_BYTES + HIT_BYTES + QUEUE_BYTES
     peak, peak_kind = measured_peaks()
-    any_bytes_per_ray = (cs.shadow_node_visits * node_bytes + cs.shadow_tri_tests * TRI_BYTES) / max(1, cs.shadow_rays) + \
-        SHADOW_RECORD_BYTES + QUEUE_BYTES
-    # only the rays of the bounce-by-bounce launches (the tail kernel's are its own; its share of the
-    # shadow rays is taken as its share of the closest-hit rays)
-    any_isect = shadow_rays * rays_isect / max(1, rays)
-    achieved = (rays_isect * bytes_per_ray + any_isect * any_bytes_per_ray) / (ms_isect / 1000.0) / 1e9 if ms_isect > 0 else None
     traffic = None
     tfile = ROOT / "profiles" / "closest_hit_dram_bytes_per_ray.txt"
     if tfile.exists():
@@ -353,11 +364,12 @@ def run_ours(args):
             traffic = per_ray * rays_isect / max(1, n_isect)
         except (ValueError, IndexError):
             traffic = None
-    roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-            "frac": (achieved / peak) if achieved else None, "traffic": traffic,
-            "kernel": "kTrace (closest-hit and any-hit BVH traversal)", "peak_kind": peak_kind,
-            "bytes_per_ray": bytes_per_ray, "any_hit_bytes_per_ray": any_bytes_per_ray, "avg_launch_ms": ms_isect / max(1, n_isect),
-            "rays_per_launch": rays_isect / max(1, n_isect)}
+    # only the rays of the bounce-by-bounce launches (the tail kernel's are its own; its share of the
+    # shadow rays is taken as its share of the closest-hit rays)
+    roof = traversal_roofline(tuning["closest_traversal"], cs, rays_isect, shadow_rays * rays_isect / max(1, rays), ms_isect)
+    achieved = roof["achieved"]
+    roof.update({"peak": peak, "frac": (achieved / peak) if achieved else None, "traffic": traffic, "peak_kind": peak_kind,
+                 "avg_launch_ms": ms_isect / max(1, n_isect), "rays_per_launch": rays_isect / max(1, n_isect)})
 
     # the shading kernels (one lean kernel per shading key): algorithmic bytes per shaded path —
     # nine 16-byte state columns and the binned slot index in; eight columns out; the hit record's
