@@ -2,7 +2,7 @@
 // wavefront render loop (RenderDevice::render, src/engine/render_device.h:84-85) and the
 // diagnostics the parity tests call.  Built for sm_100a only.
 #include "pe_device_impl.h"
-#include "pe_integrator.cuh"
+#include "pe_wave_kernels.cuh"
 
 #include <cuda_runtime.h>
 
@@ -366,7 +366,7 @@ void launchTail(pe_device* d, int features, bool inlineShadows, bool out, const 
     if (inlineShadows || !plainShadows(S)) {
         const int grid = static_cast<int>(std::max<int64_t>(
             1, std::min<int64_t>(d->blocksTailLockstep, (n + kTailLockstepBlock - 1) / kTailLockstepBlock)));
-        kTailLockstep<0><<<grid, kTailLockstepBlock, 0, cs>>>(S, P, W, queue, count, cursor, hits, d->dStats);
+        kTailLockstep<false><<<grid, kTailLockstepBlock, 0, cs>>>(S, P, W, queue, count, cursor, hits, d->dStats);
         return;
     }
     const bool lean = features == 0;
@@ -1389,7 +1389,7 @@ pe_device* pe_device_create(int32_t ordinal, char* err, size_t errLen) {
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, threads, 0);
         return sm * std::max(1, nb);
     };
-    d->blocksTailLockstep = occ(kTailLockstep<0>, kTailLockstepBlock);
+    d->blocksTailLockstep = occ(kTailLockstep<false>, kTailLockstepBlock);
     d->blocksTailWarps[0][0] = occ(kTailWarps<FEAT_ALL, false>, tailWarpsBlock(FEAT_ALL));
     d->blocksTailWarps[0][1] = occ(kTailWarps<FEAT_ALL, true>, tailWarpsBlock(FEAT_ALL));
     d->blocksTailWarps[1][0] = occ(kTailWarps<0, false>, tailWarpsBlock(0));

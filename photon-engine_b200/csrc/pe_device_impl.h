@@ -213,7 +213,7 @@ struct pe_device {
     std::vector<cudaEvent_t> evPool;
     bool counting = false;
     pe_render_stats stats{};
-    int blocksIntersect = 0, blocksShade = 0, blocksShadow = 0, blocksGen = 0, blocksTail = 0;
+    int blocksIntersect = 0, blocksShade = 0, blocksShadow = 0, blocksTail = 0;
     int blocksShadeKey[2][pe::kShadeKeys] = {}; // per-key shading kernels: [recording AOVs or passes][key]
     int blocksShadowAny = 0;
     int blocksTailLockstep = 0;     // 128-thread blocks
@@ -221,10 +221,10 @@ struct pe_device {
     int blocksIntersectBinary = 0;
     size_t waveSlots = pe_dev::kDefaultWaveSlots; // pe_tuning::wave_slots: paths in flight per regenerating wave
     size_t laneSlots = 0;                 // slots of path state allocated per lane (>= capacity, waveSlots)
-    int anyMode = 2;               // pe_tuning::any_traversal (every value the one any-hit kernel)
-    // tuning (pe_tuning): closest-hit traversal variant, register budget of the lean shading kernels
-    int closestMode = 6;  // pe_tuning::closest_traversal (TraceMode: 0 the binary tree, else the 4-wide one)
-    int shadeBudget = 1;  // pe_tuning::shade_budget (every value the 128-register kernels)
+    // tuning (pe_tuning)
+    int closestMode = 6;  // closest_traversal (TraceMode: 0 the binary tree, else the 4-wide one)
+    int anyMode = 2;      // any_traversal: kept for pe_device_get_tuning, read by no launch
+    int shadeBudget = 1;  // shade_budget: kept for pe_device_get_tuning, read by no launch
     std::string tuneLog;  // the last autotune's probe times
     int64_t tailPaths = -1; // -1: defaultTailPaths; 0: no tail kernel
     unsigned char* noAllocBase = nullptr; // device address of g_noAllocScratch on this device

@@ -255,9 +255,6 @@ template <bool COUNT, int LEVEL>
 __device__ void walkClosestWide(const SceneGPU& S, int cur, V3 o, V3 d, V3 inv, uint32_t mask, float tMin, float& tMax,
                                 Hit& best, uint32_t& nodeVisits, uint32_t& triTests, float time);
 template <bool COUNT, int LEVEL>
-__device__ bool walkAny(const SceneGPU& S, int cur, V3 o, V3 d, V3 inv, uint32_t mask, float tMin, float tMax,
-                        uint32_t& nodeVisits, uint32_t& triTests, float time);
-template <bool COUNT, int LEVEL>
 __device__ bool walkAnyWide(const SceneGPU& S, int cur, V3 o, V3 d, V3 inv, uint32_t mask, float tMin, float tMax,
                             uint32_t& nodeVisits, uint32_t& triTests, float time);
 
@@ -326,7 +323,7 @@ __device__ __noinline__ void instanceClosest(const SceneGPU& S, int inst, uint32
     best.meta = meta;
 }
 
-template <bool COUNT, bool WIDE>
+template <bool COUNT>
 __device__ __noinline__ bool instanceAny(const SceneGPU& S, int inst, V3 o, V3 d, float tMin, float tMax,
                                          uint32_t& nodeVisits, uint32_t& triTests, float time) {
     const InstGPU& I = S.instances[inst];
@@ -336,8 +333,7 @@ __device__ __noinline__ bool instanceAny(const SceneGPU& S, int inst, V3 o, V3 d
     instancePose(S, I, time, buf, l2w, w2l, uvScale);
     const V3 lo = xfPointD(w2l, o), ld = xfVectorD(w2l, d);
     const V3 linv = mk(1.0f / ld.x, 1.0f / ld.y, 1.0f / ld.z);
-    return WIDE ? walkAnyWide<COUNT, 1>(S, I.rootWide, lo, ld, linv, 0x1Fu, tMin, tMax, nodeVisits, triTests, 0.0f)
-                : walkAny<COUNT, 1>(S, I.rootBinary, lo, ld, linv, 0x1Fu, tMin, tMax, nodeVisits, triTests, 0.0f);
+    return walkAnyWide<COUNT, 1>(S, I.rootWide, lo, ld, linv, 0x1Fu, tMin, tMax, nodeVisits, triTests, 0.0f);
 }
 
 // The primitives of one leaf, in order: triangles (lean Möller–Trumbore), spheres and, at the top
@@ -372,7 +368,7 @@ __device__ __forceinline__ void testLeafClosest(const SceneGPU& S, int first, in
     }
 }
 
-template <bool COUNT, int LEVEL, bool WIDE>
+template <bool COUNT, int LEVEL>
 __device__ __forceinline__ bool testLeafAny(const SceneGPU& S, int first, int count, V3 o, V3 d, uint32_t mask,
                                             float tMin, float tMax, uint32_t& nodeVisits, uint32_t& triTests,
                                             float time) {
@@ -383,7 +379,7 @@ __device__ __forceinline__ bool testLeafAny(const SceneGPU& S, int first, int co
         const uint32_t meta = __float_as_uint(b.w);
         if ((meta & mask) == 0u) continue;
         if (LEVEL == 0 && (meta & PRIM_INSTANCE)) {
-            if (instanceAny<COUNT, WIDE>(S, __float_as_int(a.x), o, d, tMin, tMax, nodeVisits, triTests, time)) return true;
+            if (instanceAny<COUNT>(S, __float_as_int(a.x), o, d, tMin, tMax, nodeVisits, triTests, time)) return true;
             continue;
         }
         if (COUNT) ++triTests;
@@ -482,57 +478,6 @@ __device__ Hit traceClosest(const SceneGPU& S, V3 o, V3 d, uint32_t mask, float 
         return best;
     walkClosest<COUNT, 0>(S, rootRef(S), o, d, inv, mask, tMin, tMax, best, nodeVisits, triTests, time);
     return best;
-}
-
-// BVH::intersectAny (bvh.cpp:404-446) from reference `cur`.
-template <bool COUNT, int LEVEL>
-__device__ bool walkAny(const SceneGPU& S, int cur, V3 o, V3 d, V3 inv, uint32_t mask, float tMin, float tMax,
-                        uint32_t& nodeVisits, uint32_t& triTests, float time) {
-    int stackRef[kMaxStack];
-    int sp = 0;
-    for (;;) {
-        while (cur >= 0) {
-            if (COUNT) ++nodeVisits;
-            const float4 n0 = __ldg(&S.nodes[4 * cur + 0]);
-            const float4 n1 = __ldg(&S.nodes[4 * cur + 1]);
-            const float4 n2 = __ldg(&S.nodes[4 * cur + 2]);
-            const float4 n3 = __ldg(&S.nodes[4 * cur + 3]);
-            float t0, t1;
-            const bool h0 = slab(n0.x, n0.y, n0.z, n0.w, n2.x, n2.y, o, inv, tMin, tMax, t0);
-            const bool h1 = slab(n1.x, n1.y, n1.z, n1.w, n2.z, n2.w, o, inv, tMin, tMax, t1);
-            const int c0 = __float_as_int(n3.x), c1 = __float_as_int(n3.y);
-            if (h0 && h1) {
-                const bool farFirst = t1 < t0;
-                stackRef[sp++] = farFirst ? c0 : c1;
-                cur = farFirst ? c1 : c0;
-            } else if (h0) {
-                cur = c0;
-            } else if (h1) {
-                cur = c1;
-            } else {
-                if (sp == 0) return false;
-                cur = stackRef[--sp];
-            }
-        }
-        int first, count;
-        leafRange(cur, first, count);
-        if (testLeafAny<COUNT, LEVEL, false>(S, first, count, o, d, mask, tMin, tMax, nodeVisits, triTests, time)) return true;
-        if (sp == 0) return false;
-        cur = stackRef[--sp];
-    }
-}
-
-// BVH::intersectAny (bvh.cpp:404-446): true when any primitive in [tMin, tMax] passes the mask.
-// The answer does not depend on visiting order; near child first for early exit.
-template <bool COUNT>
-__device__ bool traceAny(const SceneGPU& S, V3 o, V3 d, uint32_t mask, float tMin, float tMax, uint32_t& nodeVisits,
-                         uint32_t& triTests, float time = 0.0f) {
-    const V3 inv = mk(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
-    float tn;
-    if (S.nTris == 0) return false;
-    if (!slab(S.rootMin[0], S.rootMax[0], S.rootMin[1], S.rootMax[1], S.rootMin[2], S.rootMax[2], o, inv, tMin, tMax, tn))
-        return false;
-    return walkAny<COUNT, 0>(S, rootRef(S), o, d, inv, mask, tMin, tMax, nodeVisits, triTests, time);
 }
 
 // ---- 4-wide traversal ----------------------------------------------------------------------
@@ -686,7 +631,7 @@ __device__ bool walkAnyWide(const SceneGPU& S, int cur, V3 o, V3 d, V3 inv, uint
         }
         int first, count;
         leafRange(cur, first, count);
-        if (testLeafAny<COUNT, LEVEL, true>(S, first, count, o, d, mask, tMin, tMax, nodeVisits, triTests, time)) return true;
+        if (testLeafAny<COUNT, LEVEL>(S, first, count, o, d, mask, tMin, tMax, nodeVisits, triTests, time)) return true;
         if (sp == 0) return false;
         cur = stackRef[--sp];
     }
