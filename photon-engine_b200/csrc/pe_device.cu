@@ -243,9 +243,10 @@ void eachKeyKernel(bool out, F f) {
 // keys — a kernel per key measured slower for them (media 1280x720 x 4 spp 6.1 -> 6.5 ms of shading,
 // guided room 320x180 x 16 spp 3.45 -> 4.17: their bounces have fewer paths, and each launch its own last warps) —
 // with only the features of scenes with media or walks (6.1 -> 5.7 ms), of guided plain scenes (3.45 -> 3.25 ms),
-// or with all.  Key kernels share nothing but counters: with `beside`, the commonest kind's runs on the lane's
-// stream and the others on its side stream, so that one's last warps (40 us a launch) overlap the other's
-// (room 1920x1080 x 2 spp 23.0 -> 22.3 ms, knot 333x217 x 5 spp 5.16 -> 5.08 ms).
+// or with all.  Key kernels share nothing but counters: with `beside`, Disney's (Lambert's in a scene without
+// Disney materials) runs on the lane's stream and the others on its side stream, so that one's last warps
+// (40 us a launch) overlap the other's (room 1920x1080 x 2 spp 23.0 -> 22.3 ms, knot 333x217 x 5 spp 5.16 ->
+// 5.08 ms).
 int launchShade(pe_device* d, int features, bool inlineShadows, bool out, const SceneGPU& S, const Paths& P,
                 const Wave& W, int32_t* qOut, cudaStream_t cs, const WaveLane* beside) {
     if (features == 0) {
@@ -524,7 +525,7 @@ int32_t runWave(pe_device* d, int lane, Paths& P, int nSegs, int nSlots, int nPi
     auto spent = [&](std::vector<std::pair<size_t, size_t>>& v) {
         if (tm.timing) v.push_back({tm.evUsed - 2, tm.evUsed - 1});
     };
-    // the rest of the wave: one thread per path until it ends
+    // the rest of the wave, each path to its end in one launch
     auto tail = [&](bool traced) -> int32_t {
         const int grid = static_cast<int>(
             std::min<int64_t>(d->blocksTail, (static_cast<int64_t>(live) + kTailBlock - 1) / kTailBlock));

@@ -370,10 +370,9 @@ inline float4 f4(float x, float y, float z, float w) {
 // children left after repeatedly replacing its largest-area interior child by that child's two
 // children (at most four; leaves are never opened), in the binary tree's left-to-right order, so
 // every box and leaf is one of the binary tree's.  Layout per node, 8 float4 (128 bytes, one L2
-// line), child by child, so that lane k of the four that walk a ray reads child k with two
-// 16-byte loads: (lo.x, lo.y, lo.z, hi.x) of children 0-3, then (hi.y, hi.z, reference, 1) of
-// children 0-3; reference: interior, wide node index; leaf, ~(first << 8 | count-1); all zero
-// for an absent child.  Nodes are written depth-first, a node before its children.
+// line), child by child, so that a child's box and reference are two 16-byte loads:
+// (lo.x, lo.y, lo.z, hi.x) of children 0-3, then (hi.y, hi.z, reference, 1) of children 0-3;
+// reference: interior, wide node index; leaf, ~(first << 8 | count-1); all zero for an absent child.  Nodes are written depth-first, a node before its children.
 static void putWideBox(float4* w, int k, V3 lo, V3 hi) {
     w[k].x = lo.x;
     w[k].y = lo.y;

@@ -1,10 +1,12 @@
 // pe_integrator.cuh — the wavefront form of PathTracer::Li (src/integrators/path_tracer.cpp:321-890).
 //
 // One path slot per (pixel, sample) of a wave.  A slot's state lives in HBM as SoA float4
-// columns; each bounce runs three persistent kernels over compacted queues:
-//   closest-hit  (queue of live rays)            → hit records
-//   shade        (same queue) → next-ray queue + shadow queue (warp-aggregated appends)
-//   any-hit      (shadow queue)                  → adds visible NEE terms to the slot's L
+// columns; each bounce runs persistent kernels over compacted queues:
+//   trace   (queue of live rays, shadow records of the bounce before) → hit records; visible NEE terms
+//           added to the slots' L
+//   bin     (the queue) → a bin per shading key
+//   shade   (the bins) → next-ray queue + shadow records (warp-aggregated appends)
+// and the last paths of a wave run to their ends in a tail kernel.
 // The state machine below is Li's loop body split at its two scene queries.  Radiance terms are
 // added to L in the reference's order (emission of vertex k, NEE of vertex k, emission of
 // vertex k+1, ...), and each slot draws Sobol dimensions in the reference's order.

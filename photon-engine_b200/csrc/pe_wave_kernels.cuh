@@ -128,8 +128,9 @@ static __global__ void kInitFree(const __grid_constant__ Paths P, int n) {
 // state reads scatter (8.3 against 7.1 ms of shading per 8.3M-path knot wave); here a bin keeps the
 // queue's order but for the interleaving of blocks.  Bound by the latency of its loads and of the bins'
 // counters: the walk leaves a ray's key in a byte (instances' hits excepted), and a block takes each
-// bin's share for 1024 entries at once: 30 -> 11 us per million rays (traversal and binning of the
-// 256x256 x 64-spp Cornell wave 2.48 -> 2.21 ms, of the 1920x1080 x 4-spp knot wave 6.86 -> 6.53 ms).
+// bin's share for 1024 entries at once (traversal and binning of the 256x256 x 64-spp Cornell wave 2.48 ->
+// 2.21 ms, of the 1920x1080 x 4-spp knot wave 6.86 -> 6.53 ms).  5 us per million rays over that wave's
+// launches, 14 to 17 in launches of 0.4-0.5 M rays.
 constexpr int kBinBlock = 256, kBinEach = 4;
 static __global__ void __launch_bounds__(kBinBlock) kBin(const __grid_constant__ SceneGPU S, const __grid_constant__ Paths P, const int32_t* queue) {
     constexpr int kWarps = kBinBlock / 32;

@@ -1109,7 +1109,8 @@ class CudaDevice:
         return int(_lib().pe_device_tail_paths(self._h))
 
     def autotune(self, camera: PerspectiveCamera, settings: RenderSettings, probe_spp: int = 4) -> int:
-        """Picks the tail threshold that renders this view fastest (films are unaffected)."""
+        """Picks the paths in flight, the closest-hit traversal and the tail threshold that render this view fastest
+        (films are unaffected); returns the threshold."""
         chosen = C.c_int64(0)
         capi.check(_lib().pe_device_autotune(self._h, C.byref(camera.describe_gpu()), C.byref(settings.to_c()),
                                              int(probe_spp), C.byref(chosen)))
